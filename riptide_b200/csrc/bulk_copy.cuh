@@ -25,6 +25,11 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
                  : "memory");
 }
 
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
 // Order earlier generic-proxy accesses of this thread before later async-proxy accesses.
 __device__ __forceinline__ void fence_proxy_async_smem()
 {
@@ -39,6 +44,31 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
             "r"(smem_u32(dst)),
         "l"(src), "r"(bytes), "r"(smem_u32(bar))
         : "memory");
+}
+
+// Copy `bytes` (a multiple of 16; both addresses 16-byte aligned) from shared to global memory
+// as one bulk group of this thread.
+__device__ __forceinline__ void bulk_s2g(void* dst, const void* src, size_t bytes)
+{
+    constexpr size_t kChunk = 32768;
+    for (size_t o = 0; o < bytes; o += kChunk) {
+        const uint32_t n = (uint32_t)(bytes - o < kChunk ? bytes - o : kChunk);
+        asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(
+                         reinterpret_cast<unsigned char*>(dst) + o),
+                     "r"(smem_u32(reinterpret_cast<const unsigned char*>(src) + o)), "r"(n)
+                     : "memory");
+    }
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+
+// Wait until this thread's bulk stores have read their shared memory / have completed.
+__device__ __forceinline__ void bulk_s2g_wait_read()
+{
+    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+}
+__device__ __forceinline__ void bulk_s2g_wait_all()
+{
+    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
 // Bounded wait for the completion of phase `parity` of the barrier. Returns false when the
@@ -59,12 +89,18 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, long l
     return false;
 }
 
+// Offset (0..3 floats) at which stage_rows_async places the value at global address `src`.
+__device__ __forceinline__ int staged_delta(const float* src)
+{
+    return (int)((reinterpret_cast<uintptr_t>(src) & 15) / sizeof(float));
+}
+
 // Stage `nfloats` floats starting at global address `src` into shared memory at `dst`
-// (16-byte aligned), as whole 16-byte units: the data lands at dst + returned offset
-// (0..3 floats). Reads up to 12 bytes before `src` and after its end: the source allocation
-// must be padded accordingly. Called by one thread; returns the offset in floats.
-__device__ __forceinline__ int stage_rows_async(float* dst, const float* src, size_t nfloats,
-                                                uint64_t* bar)
+// (16-byte aligned), as whole 16-byte units: the data lands at dst + staged_delta(src).
+// Reads up to 12 bytes before `src` and after its end: the source allocation must be padded
+// accordingly. Called by one thread.
+__device__ __forceinline__ void stage_rows_async(float* dst, const float* src, size_t nfloats,
+                                                 uint64_t* bar)
 {
     const uintptr_t a = reinterpret_cast<uintptr_t>(src);
     const uintptr_t a0 = a & ~uintptr_t(15);
@@ -78,7 +114,6 @@ __device__ __forceinline__ int stage_rows_async(float* dst, const float* src, si
         bulk_g2s(reinterpret_cast<unsigned char*>(dst) + off,
                  reinterpret_cast<const unsigned char*>(a0) + off, n, bar);
     }
-    return (int)((a - a0) / sizeof(float));
 }
 
 }  // namespace rt

@@ -49,10 +49,6 @@ struct WorkItem {
 constexpr size_t kEngineTreeBytes = (sizeof(JobTree) + 255) & ~size_t(255);
 constexpr size_t kEngineSnrBytes = (sizeof(SnrParams) + 255) & ~size_t(255);
 constexpr size_t kEngineDynBytes = kFfaSmemBytes - 2 * (kEngineTreeBytes + kEngineSnrBytes);
-RT_HD int engine_cap_rows(int b)
-{
-    return ffa_cap_rows_for(kEngineDynBytes, 0, b);
-}
 
 constexpr int kSlots = 256;          // scratch slots for multi-stage transforms
 constexpr size_t kLagItems = 640;    // work items emitted between two stages of a transform
@@ -79,6 +75,7 @@ struct EngineArgs {
     unsigned long long* phase_cycles;  // optional [kPhases] SM-cycle totals (thread 0 of each CTA)
     long long spin_limit;    // polls before a wait gives up with RT_ETIMEOUT
     int dep_bias;            // added to later-stage dependency targets (fault injection; 0)
+    FfaLayout layout;        // operations and level buffers in dynamic shared memory
 };
 
 // Phases of one work item, for the optional in-kernel profile.
@@ -94,17 +91,20 @@ __device__ __forceinline__ int ld_acquire(const int* p)
     return v;
 }
 
-template <int TPR>
-__device__ void final_stage_outputs(const JobTree& T, const XformRec& X, const EngineArgs& A,
-                                    const SnrParams& S, float* buf0, float* buf1, int fstride,
-                                    int cap_rows)
+// Boxcar S/N and the period rows of a final-stage job's root rows (`root`); `work` is the
+// other level buffer.
+template <int TPR, bool kUnrolled>
+__device__ __forceinline__ void final_stage_outputs(const JobTree& T, const XformRec& X, const EngineArgs& A,
+                                    const SnrParams& S, const float* root, float* work,
+                                    int fstride)
 {
     const Node r = T.nodes[0];
     const int b = X.b;
     const int cs = prefix_stride(b, S.wmax, TPR);
-    const int groups = (int)(((size_t)cap_rows * fstride) / cs);
-    snr_rows<TPR, 34>(buf0, fstride, r.hi - r.lo, b, S, X.stdnoise,
-                      A.snrs + ((size_t)X.out_row + r.lo) * S.nw, S.nw, buf1, cs, groups);
+    const int groups = A.layout.buf_floats / cs;
+    snr_rows_impl<TPR, 34, kUnrolled>(root, fstride, r.hi - r.lo, b, S, X.stdnoise,
+                                      A.snrs + ((size_t)X.out_row + r.lo) * S.nw, S.nw, work, cs,
+                                      groups);
     double* per_out = A.periods + X.out_row;
     uint32_t* fb_out = A.foldbins + X.out_row;
     for (int s = r.lo + threadIdx.x; s < r.hi; s += kThreads) {
@@ -115,16 +115,19 @@ __device__ void final_stage_outputs(const JobTree& T, const XformRec& X, const E
 
 // The persistent kernel has kThreads compute threads and one scheduling warp. The scheduler
 // claims the next ticket, loads its descriptors into one of two shared slots and waits for
-// its dependencies while the compute threads work on the other slot; slot hand-over uses
-// named barriers (full: scheduler -> compute, empty: compute -> scheduler), one pair per slot.
+// its dependencies while the compute threads work on the other slot. A slot is handed over by
+// an mbarrier that every compute warp waits for by itself (a warp that is done with an item
+// goes on to build the next one's operations), and handed back by a named barrier.
 constexpr int kEngineThreads = kThreads + 32;
-constexpr int kBarFull = 2;   // + slot
-constexpr int kBarEmpty = 4;  // + slot
+constexpr int kBarEmpty = 2;  // + slot
+constexpr int kBarRead = 4;   // the previous item's root rows have left their level buffer
 
 struct ItemSlot {
     long long ticket;   // >= nitems: no more work
     int ok;             // 0: a wait failed, stop
     int done_ok;        // set by the compute threads: 0 if the item failed
+    int root;           // set by the compute threads: level buffer (0, 1) of the root rows to
+                        // store as a stage output, -1: nothing to store
     int stage, last, cap_rows, jobs_of_stage;
     JobSpec J;
     XformRec X;
@@ -218,8 +221,58 @@ __device__ void sched_decode(const EngineArgs& A, long long t, SchedItem& it)
 // have smaller tickets), so whichever scheduler holds it hands it over; every wait is bounded.
 constexpr int kParked = 4;
 
+// The level buffer that an item's source rows are staged in: the one that does not hold the
+// root rows which the previous item leaves to be stored.
+__device__ __forceinline__ int staging_buffer(int prev_root) { return prev_root < 0 ? 1 : 1 - prev_root; }
+
+__device__ __forceinline__ float* level_buffer(unsigned char* smem, const EngineArgs& A, int i)
+{
+    return reinterpret_cast<float*>(smem + (size_t)A.layout.ops_units * 16) +
+           (size_t)i * A.layout.buf_floats;
+}
+
+__device__ __forceinline__ float* stage_output(const EngineArgs& A, const XformRec& X, int stage)
+{
+    return A.scratch + ((size_t)(X.seq % kSlots) * 2 + (stage & 1)) * A.slot_floats;
+}
+
+// Whether an item's source rows come by bulk copies (issued by the scheduling warp).
+__device__ __forceinline__ bool staged_async(const ItemSlot& L, const JobTree& T)
+{
+    if (L.J.hi <= L.J.lo || T.error) return false;
+    return L.stage == 0 ? !L.X.src_norm : T.pstaged != 0;
+}
+
+// Issues the bulk copies of an item's source rows into level buffer `buf` (one warp): for
+// stage-0 jobs (whole subtrees) one contiguous block of the downsampled arena, in whole 16-byte
+// units (the arena is padded); for later stages the blocks of the previous stage's output that
+// the cone needs.
+__device__ __forceinline__ void stage_item(const EngineArgs& A, const ItemSlot& L, const JobTree& T,
+                                           float* buf, uint64_t* bar)
+{
+    if (!staged_async(L, T)) return;
+    const int b = L.X.b;
+    if (L.stage > 0)
+        stage_source_rows_async(T, stage_output(A, L.X, L.stage - 1), ffa_stride(b), buf, bar);
+    else if ((threadIdx.x & 31) == 0)
+        stage_rows_async(buf, A.ds + L.X.src_off + (size_t)L.J.root_row0 * b,
+                         (size_t)L.J.root_rows * b, bar);
+}
+
+// Issues the bulk store of a stage's root rows [lo, hi), one block in the level buffer and in
+// the stage output (same stride, a multiple of 16 bytes). One thread; the writers of the rows
+// have made them visible to the async proxy.
+__device__ __forceinline__ void store_root_rows(const EngineArgs& A, const ItemSlot& L,
+                                                const float* buf)
+{
+    const int fstride = ffa_stride(L.X.b);
+    bulk_s2g(stage_output(A, L.X, L.stage) + (size_t)(L.J.root_row0 + L.J.lo) * fstride, buf,
+             (size_t)(L.J.hi - L.J.lo) * fstride * sizeof(float));
+}
+
 __device__ void scheduler_warp(const EngineArgs& A, ItemSlot* slots, JobTree* trees,
-                               SnrParams* snr, unsigned* finished)
+                               SnrParams* snr, unsigned* finished, unsigned char* smem,
+                               uint64_t* bar, uint64_t* full)
 {
     const int lane = threadIdx.x & 31;
     SchedItem parked[kParked];
@@ -227,10 +280,14 @@ __device__ void scheduler_warp(const EngineArgs& A, ItemSlot* slots, JobTree* tr
     bool exhausted = false;
     // items handed over whose completion is not signalled yet (lane 0): signalled as soon as
     // every compute warp has released them, also while this warp waits for a dependency (an
-    // item it waits for may be the one running here)
+    // item it waits for may be the one running here); a stage output is stored first
     bool pending[2] = {false, false};
-    auto try_signal = [&](int s) {
+    auto finish = [&](int s) {
         if (pending[s] && warps_done_acquire(finished + s) >= (unsigned)kWarps) {
+            if (slots[s].root >= 0) {
+                store_root_rows(A, slots[s], level_buffer(smem, A, slots[s].root));
+                bulk_s2g_wait_all();
+            }
             signal_item_done(A, slots[s]);
             pending[s] = false;
         }
@@ -238,15 +295,33 @@ __device__ void scheduler_warp(const EngineArgs& A, ItemSlot* slots, JobTree* tr
     int k = 0;
     for (;; ++k) {
         const int s = k & 1;
-        if (k >= 2) named_sync(kBarEmpty + s, kEngineThreads);  // compute is done with item k-2
+        if (k >= 2) {
+            named_sync(kBarEmpty + s, kEngineThreads);  // compute is done with item k-2
+            // ... and starts item k-1: its source rows, then the stage output of item k-2
+            stage_item(A, slots[s ^ 1], trees[s ^ 1],
+                       level_buffer(smem, A, staging_buffer(slots[s].root)), bar);
+            if (slots[s].root >= 0) {
+                if (lane == 0 && pending[s]) {
+                    store_root_rows(A, slots[s], level_buffer(smem, A, slots[s].root));
+                    bulk_s2g_wait_read();
+                }
+                __syncwarp();
+                named_arrive(kBarRead, kEngineThreads);
+                if (lane == 0 && pending[s]) {
+                    bulk_s2g_wait_all();
+                    signal_item_done(A, slots[s]);
+                    pending[s] = false;
+                }
+            }
+        }
         if (lane == 0) {
-            try_signal(s);  // item k-2
+            finish(s);  // item k-2
             ItemSlot& L = slots[s];
             const long long w0 = clock64();
             bool chosen = false;
             unsigned ns = 32;
             for (long long spin = 0; !chosen; ++spin) {
-                try_signal(s ^ 1);  // item k-1, running
+                finish(s ^ 1);  // item k-1, running
                 for (int i = 0; i < nparked && !chosen; ++i) {
                     if (sched_ready(parked[i])) {
                         L = parked[i].slot;
@@ -295,6 +370,7 @@ __device__ void scheduler_warp(const EngineArgs& A, ItemSlot* slots, JobTree* tr
             }
             if (A.phase_cycles) atomicAdd(A.phase_cycles + 7, (unsigned long long)(clock64() - w0));
             L.done_ok = 1;
+            L.root = -1;
             finished[s] = 0;
             __threadfence_block();
         }
@@ -303,153 +379,158 @@ __device__ void scheduler_warp(const EngineArgs& A, ItemSlot* slots, JobTree* tr
         // the job tree and boxcar coefficients of the item, prepared while the compute threads
         // run the previous item
         if (!stop && slots[s].J.hi > slots[s].J.lo) {
-            build_job_tree_warp(trees[s], slots[s].J, slots[s].cap_rows, slots[s].stage > 0);
+            build_job_tree_warp(trees[s], slots[s].J, slots[s].X.b, slots[s].cap_rows,
+                                A.layout.ops_units, slots[s].stage == 0);
             if (slots[s].last) snr_params_fill_warp(snr[s], A.widths, A.nw, A.nfast, slots[s].X.b);
+            if (k == 0) stage_item(A, slots[0], trees[0], level_buffer(smem, A, staging_buffer(-1)), bar);
         }
-        named_arrive(kBarFull + s, kEngineThreads);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(full + s);
         if (stop) break;
         if (lane == 0) pending[s] = true;
     }
     // the compute threads still hand back the slot of item k-1
     if (k >= 1) {
         named_sync(kBarEmpty + ((k - 1) & 1), kEngineThreads);
-        if (lane == 0) try_signal((k - 1) & 1);
+        if (lane == 0) finish((k - 1) & 1);
     }
 }
 
-// BC: the bins class of the plan's transforms (which unrolled level loops the instance holds);
-// TPRS: the S/N threads per profile its transforms use (bit 0: 8, bit 1: 16). The host picks
-// the instance (search_kernel_for).
-template <int BC, int TPRS>
+// KINDS: the kinds of S/N code (snr_kind) the instance holds. The host picks the instance
+// (search_kernel_for).
+template <int KINDS>
 __global__ void __launch_bounds__(kEngineThreads, 1) k_search_persistent(EngineArgs A)
 {
-    extern __shared__ __align__(16) unsigned char smem[];
-    unsigned char* layout = smem;
+    extern __shared__ __align__(128) unsigned char smem[];
     __shared__ ItemSlot slots[2];
     __shared__ JobTree trees[2];
     __shared__ SnrParams snr[2];
     __shared__ unsigned finished[2];
-    __shared__ __align__(8) uint64_t s_bar;  // completion of the bulk copy of a job's rows
+    __shared__ __align__(8) uint64_t s_bar;     // completion of the bulk copy of a job's rows
+    __shared__ __align__(8) uint64_t s_full[2];  // slot handed to the compute threads
 
-    if (threadIdx.x == 0) mbar_init(&s_bar, 1);
+    if (threadIdx.x == 0) {
+        mbar_init(&s_bar, 1);
+        mbar_init(s_full, 1);
+        mbar_init(s_full + 1, 1);
+    }
     __syncthreads();
     if (threadIdx.x >= kThreads) {
-        scheduler_warp(A, slots, trees, snr, finished);
+        scheduler_warp(A, slots, trees, snr, finished, smem, &s_bar, s_full);
         return;
     }
+    uint4* ops = reinterpret_cast<uint4*>(smem);
     uint32_t bar_phase = 0;
     const bool prof = A.phase_cycles != nullptr;
-    unsigned long long ph[kPhases] = {0, 0, 0, 0, 0, 0, 0, 0};
-    unsigned long long cnt[4] = {0, 0, 0, 0};  // counters 12..15
     long long tprev = prof ? clock64() : 0;
     auto mark = [&](int phase) {
         if (prof && threadIdx.x == 0) {
             const long long t = clock64();
-            ph[phase] += (unsigned long long)(t - tprev);
+            atomicAdd(A.phase_cycles + phase, (unsigned long long)(t - tprev));
             tprev = t;
         }
     };
+    int prev_root = -1;  // level buffer of the previous item's root rows while they are stored
     for (int k = 0;; ++k) {
         const int sl = k & 1;
-        named_sync(kBarFull + sl, kEngineThreads);
+        // the scheduling warp's own waits are bounded and it always hands a slot over: this
+        // limit is far beyond them
+        if (!mbar_wait(s_full + sl, (k >> 1) & 1, 1ll << 40)) break;
         mark(kPhWait);
         const ItemSlot& L = slots[sl];
         const JobTree& T = trees[sl];
         const SnrParams& S = snr[sl];
         if (L.ticket >= A.nitems || !L.ok) break;
-        const XformRec X = L.X;
-        const JobSpec J = L.J;
-        const int stage = L.stage;
-        const bool last = L.last != 0;
+        const XformRec& X = L.X;
+        const JobSpec& J = L.J;
         const int b = X.b;
         const int fstride = ffa_stride(b);
-        const int cap_rows = L.cap_rows;
-        const FfaSmem Lay = ffa_smem(layout, cap_rows, b);
-        float* slot = (X.seq >= 0) ? A.scratch + (size_t)(X.seq % kSlots) * 2 * A.slot_floats
-                                   : nullptr;
-        mark(6);
-        mark(kPhFetch);
+        const int buf = staging_buffer(prev_root);
+        int root = -1;
         bool failed = false;
         if (J.hi > J.lo) {
-            const float* src =
-                (stage == 0) ? (X.src_norm ? A.norm : A.ds) + X.src_off
-                             : slot + (size_t)((stage - 1) & 1) * A.slot_floats;
+            // The source rows are staged by the scheduling warp in the background of the
+            // operations' build, except those of the normalised series (it may be the caller's
+            // buffer, which bulk copies of whole 16-byte units could leave).
+            float* sbuf = level_buffer(smem, A, buf);
             LevelIO io;
-            io.src = src;
-            io.src_stride = (stage == 0) ? b : fstride;  // stage outputs: level stride
-            io.bar = &s_bar;
             io.phase = &bar_phase;
-            // Level G's source rows are copied (bulk copies) into the level buffer that level G
-            // does not write, in the background of the row-operation build: for stage-0 jobs
-            // (whole subtrees) one contiguous block of the downsampled arena (padded); for
-            // later stages the blocks of the previous stage's output that the cone needs.
-            float* sbuf = (J.G & 1) ? Lay.buf0 : Lay.buf1;
-            const bool staged0 = stage == 0 && !X.src_norm && J.root_rows <= cap_rows &&
-                                 (size_t)J.root_rows * b + 8 <= (size_t)cap_rows * fstride;
-            const bool staged = staged0 || (stage > 0 && T.pstaged && !T.error);
-            if (staged0) {
-                __shared__ int s_delta;
-                if (threadIdx.x == 0)
-                    s_delta = stage_rows_async(sbuf, src + (size_t)J.root_row0 * b,
-                                               (size_t)J.root_rows * b, &s_bar);
-                cta_sync();
-                io.staged = sbuf + s_delta - (ptrdiff_t)J.root_row0 * b;
-            } else if (staged) {
-                if (threadIdx.x < 32) stage_source_rows_async(T, src, fstride, sbuf, &s_bar);
-                io.staged = sbuf;
+            if (L.stage == 0) {
+                const float* from =
+                    (X.src_norm ? A.norm : A.ds) + X.src_off + (size_t)J.root_row0 * b;
+                int delta = 0;
+                if (X.src_norm) {
+                    cta_sync();  // every warp is done with the previous item's buffers
+                    const int nraw = J.root_rows * b;
+#pragma unroll 4
+                    for (int i = threadIdx.x; i < nraw; i += kThreads) sbuf[i] = __ldg(from + i);
+                } else {
+                    delta = staged_delta(from);
+                }
+                io.staged = sbuf + delta - (ptrdiff_t)J.root_row0 * b;
+            } else {
+                io.src = stage_output(A, X, L.stage - 1);
+                io.src_stride = fstride;  // stage outputs: level rows with halo
                 io.staged_rows = true;
+                if (T.pstaged) io.staged = sbuf;
             }
+            if (staged_async(L, T)) io.bar = &s_bar;
             failed = T.error != 0;
+            mark(kPhTree);
+            if (!failed) build_ops(T, b, ops);
+            // the other level buffer is free once the previous item's root rows have left it
+            if (prev_root >= 0) named_sync(kBarRead, kEngineThreads);
+            else cta_sync();
+            mark(kPhFetch);
             if (failed) {
                 if (threadIdx.x == 0) atomicExch(A.error, RT_EINTERNAL);
-                if (staged) {  // still let the copy land before the buffer is reused
-                    mbar_wait(&s_bar, bar_phase);
-                    bar_phase ^= 1u;
-                }
             } else {
-                mark(kPhTree);
                 if (prof && threadIdx.x == 0) {
-                    for (int d = 0; d <= T.depth; ++d)
-                        cnt[0] += (unsigned long long)T.level_rows[d] * b;
-                    cnt[1] += T.depth + 1;
-                    cnt[2] += J.hi - J.lo;
-                    cnt[3] += stage > 0;
+                    unsigned long long rows = T.fused ? 2 * T.level_rows[T.depth] : 0;
+                    for (int d = 0; d <= T.depth; ++d) rows += T.level_rows[d];
+                    atomicAdd(A.phase_cycles + 12, rows * b);
+                    atomicAdd(A.phase_cycles + 13, (unsigned long long)(J.G + 1));
+                    atomicAdd(A.phase_cycles + 14, (unsigned long long)(J.hi - J.lo));
+                    atomicAdd(A.phase_cycles + 15, (unsigned long long)(L.stage > 0));
                 }
-                // stage outputs other than the last are written by the root level itself
-                if (!last) {
-                    io.root_dst =
-                        root_rows_dst(T, fstride, slot + (size_t)(stage & 1) * A.slot_floats);
-                    io.root_stride = fstride;
-                }
-                if (!run_job_levels<BC>(T, b, Lay.buf0, Lay.buf1, fstride, Lay.ops, io)) {
-                    if (threadIdx.x == 0) atomicExch(A.error, RT_ETIMEOUT);
-                }
+                bool ok = true;
+                float* other = level_buffer(smem, A, buf ^ 1);
+                float* rows = run_job_levels(T, b, sbuf, other, fstride, ops, io, &ok);
+                if (!ok && threadIdx.x == 0) atomicExch(A.error, RT_ETIMEOUT);
                 mark(kPhLevels);
-                if (last) {
-                    if constexpr (TPRS == 1)
-                        final_stage_outputs<8>(T, X, A, S, Lay.buf0, Lay.buf1, fstride, cap_rows);
-                    else if constexpr (TPRS == 2)
-                        final_stage_outputs<16>(T, X, A, S, Lay.buf0, Lay.buf1, fstride, cap_rows);
-                    else if ((X.tune >> 16) == 8)
-                        final_stage_outputs<8>(T, X, A, S, Lay.buf0, Lay.buf1, fstride, cap_rows);
-                    else
-                        final_stage_outputs<16>(T, X, A, S, Lay.buf0, Lay.buf1, fstride, cap_rows);
+                if (L.last) {
+                    float* work = rows == sbuf ? other : sbuf;
+                    const int kind = KINDS == kSnr8 || KINDS == kSnr16
+                                         ? KINDS : snr_kind(b, X.tune >> 16);
+                    if ((KINDS & kSnr8) && kind == kSnr8)
+                        final_stage_outputs<8, true>(T, X, A, S, rows, work, fstride);
+                    else if ((KINDS & kSnr16) && kind == kSnr16)
+                        final_stage_outputs<16, true>(T, X, A, S, rows, work, fstride);
+                    else if (KINDS & kSnr16Loop)
+                        final_stage_outputs<16, false>(T, X, A, S, rows, work, fstride);
                     mark(kPhSnr);
+                } else {
+                    // the scheduling warp stores the root rows (bulk copy): make this thread's
+                    // writes visible to the async proxy
+                    root = rows == sbuf ? buf : buf ^ 1;
+                    fence_proxy_async_smem();
                 }
             }
+        } else if (prev_root >= 0) {
+            named_sync(kBarRead, kEngineThreads);
         }
+        prev_root = root;
         // hand the item back: the scheduling warp signals its completion to the other CTAs
         // once every compute warp has released it
-        if (threadIdx.x == 0 && failed) slots[sl].done_ok = 0;
+        if (threadIdx.x == 0) {
+            slots[sl].root = root;
+            if (failed) slots[sl].done_ok = 0;
+        }
         __syncwarp();
         if ((threadIdx.x & 31) == 0) warp_done_release(finished + sl);
         mark(kPhStore);
         named_arrive(kBarEmpty + sl, kEngineThreads);
     }
-    if (prof && threadIdx.x == 0)
-        for (int i = 0; i < kPhases; ++i) atomicAdd(A.phase_cycles + i, ph[i]);
-    if (prof && threadIdx.x == 0)
-        for (int i = 0; i < 4; ++i) atomicAdd(A.phase_cycles + 12 + i, cnt[i]);
 }
 
 // ------------------------------------------------------------------------------------
@@ -1029,8 +1110,7 @@ struct SearchPlan {
     std::vector<rt_tile_rule> rules;    // per (rows, bins) tile choices, first match wins
     std::vector<int> widths;
     int nfast = 0;
-    int bins_used[2] = {1 << 30, 0};  // smallest and largest b of the transforms
-    int tpr_mask = 0;                 // S/N threads per profile used: bit 0 = 8, bit 1 = 16
+    int snr_kinds = 0;                // kinds of S/N code the transforms need (snr_kind)
     std::vector<size_t> lengths, offsets;
     size_t total_len = 0, max_len = 0;
     // cycles (cpp/periodogram.hpp:135-158)
@@ -1052,6 +1132,7 @@ struct SearchPlan {
     std::vector<WorkItem> items;
     int nseq = 0;
     size_t slot_floats = 0;
+    FfaLayout layout{};                  // shared-memory layout of the persistent kernel
     // device buffers
     bool dev_ready = false;
     int* d_widths = nullptr;
@@ -1175,6 +1256,7 @@ static int plan_build(SearchPlan& P)
         }
     };
 
+    P.layout = ffa_layout(kEngineDynBytes, (int)c.bins_min, P.max_len / c.bins_min);
     size_t ds_total = 0;
     for (int t = 0; t < T; ++t) {
         const size_t N = P.lengths[t];
@@ -1198,7 +1280,7 @@ static int plan_build(SearchPlan& P)
                     return set_error(RT_EINVAL, "transform of %zu rows is too large", rows);
                 // rows per job: the shared-memory capacity, scaled by the tuning (its own
                 // fraction for transforms of more than 8 jobs' worth of rows)
-                const int cap_full = engine_cap_rows((int)b);
+                const int cap_full = ffa_cap_rows(P.layout, (int)b);
                 double frac = P.tuning.rows_fraction > 0 ? std::min(1.0, P.tuning.rows_fraction) : 1.0;
                 if (rows > 8 * (size_t)cap_full && P.tuning.rows_fraction_deep > 0)
                     frac = std::min(1.0, P.tuning.rows_fraction_deep);
@@ -1221,8 +1303,9 @@ static int plan_build(SearchPlan& P)
                     StagePlan sp;
                     // a rule's level count that needs more stages than a plan holds falls back
                     // to the default depth
-                    if (capr < 4 || (!plan_stages((int)rows, (int)re, capr, &sp, max_depth) &&
-                                     !plan_stages((int)rows, (int)re, capr, &sp)))
+                    if (capr < 4 ||
+                        (!plan_stages((int)rows, (int)b, (int)re, capr, &sp, max_depth) &&
+                         !plan_stages((int)rows, (int)b, (int)re, capr, &sp)))
                         return set_error(RT_EINVAL, "no device plan for a %zu x %zu transform", rows, b);
                     pi = (int)P.plans.size();
                     P.plans.push_back(sp);
@@ -1255,9 +1338,7 @@ static int plan_build(SearchPlan& P)
                     if (X.seq >= kSlots) finish_seq(X.seq - kSlots);
                 }
                 P.xforms.push_back(X);
-                P.bins_used[0] = std::min(P.bins_used[0], (int)b);
-                P.bins_used[1] = std::max(P.bins_used[1], (int)b);
-                P.tpr_mask |= (tpr == 8) ? 1 : 2;
+                P.snr_kinds |= snr_kind((int)b, tpr);
                 P.xform_tc.push_back(make_int2(t, ci));
                 rows_total += re;
                 emit_stage(xi, 0);
@@ -1390,17 +1471,13 @@ static int plan_alloc_device(SearchPlan& P)
     return RT_OK;
 }
 
-// The instance of k_search_persistent for a plan whose transforms have bins in
-// [bmin, bmax] and use the S/N thread counts of tpr_mask (bit 0: 8, bit 1: 16). Plans of bins
-// 449-544 with 16 S/N threads (the bins 480-520 searches) get the instance without the
-// 256-bin loops and the 8-thread S/N: 2.0% faster on the large sweep. An instance for bins
-// 225-288 measured 3.6-3.8% slower than the full one on the 240-260 searches (with both S/N
-// thread counts or with 8 only), so those keep the full instance.
-static void (*search_kernel_for(int bmin, int bmax, int tpr_mask))(EngineArgs)
+// The instance of k_search_persistent for a plan whose transforms need the kinds of S/N code in
+// `kinds`: the usual searches need one kind only.
+static void (*search_kernel_for(int kinds))(EngineArgs)
 {
-    if (bins_class(bmin, bmax) == kBins512 && tpr_mask == 2)
-        return k_search_persistent<kBins512, 2>;
-    return k_search_persistent<kBinsAny, 3>;
+    if (kinds == kSnr8) return k_search_persistent<kSnr8>;
+    if (kinds == kSnr16) return k_search_persistent<kSnr16>;
+    return k_search_persistent<kSnr8 | kSnr16 | kSnr16Loop>;
 }
 
 static int engine_grid(void (*kernel)(EngineArgs))
@@ -1516,7 +1593,8 @@ static int plan_run(SearchPlan& P, const float* data, float* normalised_out, dou
     A.phase_cycles = P.d_phase;
     A.spin_limit = P.spin_limit;
     A.dep_bias = P.dep_bias;
-    void (*kernel)(EngineArgs) = search_kernel_for(P.bins_used[0], P.bins_used[1], P.tpr_mask);
+    A.layout = P.layout;
+    void (*kernel)(EngineArgs) = search_kernel_for(P.snr_kinds);
     RT_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)kEngineDynBytes));
     if (A.nitems > 0) {

@@ -13,8 +13,30 @@
 //   * going down the tree, a contiguous output range of a node needs a contiguous range of
 //     rows of each child, so every level is a list of (node, row range) stored back to back
 //     in a shared-memory buffer; two buffers alternate between levels;
-//   * the root rows are then either written to global memory (to feed a job higher in the
-//     tree, or as the ffa2 result) or turned into boxcar S/N (snr_core.cuh).
+//   * the root rows are left in one of the two buffers, from where the caller writes them to
+//     global memory (to feed a job higher in the tree, or as the ffa2 result) or turns them
+//     into boxcar S/N (snr_core.cuh).
+//
+// What bounds the levels is shared memory: an output value of a level is two reads, an add and
+// a write, and one warp-wide access of 32 words is one of the SM's cycles. Three choices
+// follow:
+//   * a lane owns kLaneCols = 9 consecutive columns (an odd stride, so the 32 lanes of an
+//     access fall in 32 banks, and one warp covers the 240-279 bins of the usual searches,
+//     two the 480-520). Rows s and s + 1 of a node mostly read the same head and tail rows,
+//     the tail shifted by one more column for the second: computed together they take
+//     9 + 10 reads for 18 values instead of 36;
+//   * every row is stored with its first kHalo columns repeated after its last one, computed
+//     as columns b .. b + 8 of the row, so that the 10 consecutive columns a lane reads from a
+//     rolled row never wrap: one address per lane and row, then immediate offsets;
+//   * the bottom three levels of a subtree of whole rows (nodes of 4 to 8 input rows) are
+//     computed in registers from the input rows, one node per warp (ffa_nodes_fused): 92 reads
+//     and 72 writes of a lane for 3 x 72 values. Above them, two levels are computed per pass
+//     over shared memory where the row numbers follow the usual pattern (level_quads).
+//
+// Against one level per pass with lanes 32 columns apart (a wrap test per value, unrolled for
+// each count of column chunks), the search kernel over 16 trials of ~2^22 samples, bins
+// 240-260, went from 12.1 to 9.4 ms (411 to 290 M warp instructions a trial), and 3 trials of
+// 2^21 samples at bins 960-1040, which had taken a loop without unrolling, from 13.0 to 6.5 ms.
 // Additions are float32 and performed in exactly the reference's order, so the result is
 // bit-identical to cpp/transforms.hpp.
 #pragma once
@@ -23,10 +45,17 @@
 
 namespace rt {
 
-constexpr int kMaxJobDepth = 7;      // levels computed inside one job (<= 128 nodes at the bottom)
-constexpr int kMaxJobNodes = 256;    // total nodes of all levels of one job
+constexpr int kMaxJobDepth = 7;      // levels below the root computed inside one job
+constexpr int kMaxTreeDepth = 5;     // deepest level of a job with a node list
+constexpr int kMaxJobNodes = (2 << kMaxTreeDepth) - 1;  // nodes of all listed levels of one job
 constexpr int kThreads = 480;        // compute threads per CTA of every FFA kernel (1 CTA per SM)
 constexpr int kWarps = kThreads / 32;
+
+constexpr int kLaneCols = 9;         // consecutive columns of a lane
+constexpr int kHalo = kLaneCols + 2; // columns repeated past the end of a row
+// Below this many bins a column window of a lane can wrap twice: such transforms take the
+// plain level loop (level_rows_direct) throughout.
+constexpr int kWideMinBins = 17;
 
 // Barrier of the compute threads only (named barrier 1). The persistent search kernel adds a
 // scheduling warp that does not take part; in the other kernels every thread computes.
@@ -41,25 +70,35 @@ struct Node {
     int lo;     // first needed output row (node-local)
     int hi;     // one past the last needed output row
     int off;    // row of `lo` inside this level's shared buffer
+    int goff;   // first row group of the node at its level
+    int qoff;   // first row quad of the node at its level
+    float kh;   // head slope of the node (merge_coef)
+};
+
+// One pass over a job's shared-memory levels: level d from level d + 1 by row groups, or
+// (`two`) from level d + 2 by row quads. Its operations start at 16-byte unit `unit`.
+struct Step {
+    int d, two, unit, count;
 };
 
 struct JobTree {
-    Node nodes[kMaxJobNodes];
-    int level_start[kMaxJobDepth + 2];  // index of the first node of each level
-    int level_rows[kMaxJobDepth + 2];   // rows stored for each level
-    int op_start[kMaxJobDepth + 2];     // first row operation of each level
-    int depth;                          // G: nodes at this level read the global source
+    Node nodes[kMaxJobNodes];           // node i of level d at (1 << d) - 1 + i
+    int level_rows[kMaxTreeDepth + 1];  // rows stored for each level
+    Step steps[kMaxTreeDepth + 1];      // levels first_op .. 0, deepest first
+    int nsteps;
+    int depth;                          // deepest level with a node list
+    int first_op;                       // levels first_op .. 0 are computed by `steps`
+    int fused;                          // level `depth` is computed from the raw input rows
+    int regular;                        // the root has at most kRegularRows rows
     int error;                          // nonzero if the job does not fit
-    // Source rows of level G staged in shared memory (jobs of later stages, whose source is
-    // the previous stage's output with 16-byte aligned rows; G <= kMaxStagedDepth): node i
-    // of level G reads its head child's source rows src_rng[i].x + [0, src_rng[i].y) from
-    // staged rows src_off[i] + ..., and its tail child's rows src_rng[i].z + [0, .w) right
-    // after them. pstaged = 0: level G reads global rows.
+    // Source rows of level `depth` staged in shared memory (jobs of later stages, whose source
+    // is the previous stage's output): node i reads its head child's source rows
+    // src_rng[i].x + [0, src_rng[i].y) from staged rows src_off[i] + ..., and its tail child's
+    // rows src_rng[i].z + [0, .w) right after them. pstaged = 0: the level reads global rows.
     int pstaged;
-    int src_off[33];
-    int4 src_rng[32];
+    int src_off[(1 << kMaxTreeDepth) + 1];
+    int4 src_rng[1 << kMaxTreeDepth];
 };
-constexpr int kMaxStagedDepth = 5;
 
 // Description of one job, produced by the planners (host).
 struct JobSpec {
@@ -77,189 +116,83 @@ RT_HD int full_depth(int rows)
     return d;
 }
 
-// Builds the per-level node lists of a job (all threads of the CTA, 3 barriers).
-// Node q of the flat array is node i = q - (2^d - 1) of level d; its row range follows from
-// the root range by applying the head/tail row maps along the bits of i.
-__device__ inline void build_job_tree(JobTree& T, const JobSpec& J, int cap_rows)
-{
-    const int tid = threadIdx.x;
-    const int G = J.G;
-    const bool bad = (G > kMaxJobDepth || (2 << G) - 1 > kMaxJobNodes);
-    if (tid == 0) {
-        T.depth = G;
-        T.error = bad ? 1 : 0;
-        T.pstaged = 0;
-    }
-    if (bad) {
-        cta_sync();
-        return;
-    }
-    const int nnodes = (2 << G) - 1;
-    for (int q = tid; q < nnodes; q += kThreads) {
-        const int d = 31 - __clz(q + 1);
-        const int i = q + 1 - (1 << d);
-        int row0 = J.root_row0, rows = J.root_rows, lo = J.lo, hi = J.hi;
-        for (int k = d - 1; k >= 0; --k) {
-            const int mh = rows >> 1;
-            const MergeCoef c = merge_coef(rows);
-            if ((i >> k) & 1) {
-                const int nlo = merge_row(c.kt, lo), nhi = merge_row(c.kt, hi - 1) + 1;
-                row0 += mh;
-                rows -= mh;
-                lo = nlo;
-                hi = nhi;
-            } else {
-                const int nlo = merge_row(c.kh, lo), nhi = merge_row(c.kh, hi - 1) + 1;
-                rows = mh;
-                lo = nlo;
-                hi = nhi;
-            }
-        }
-        Node nd;
-        nd.row0 = row0;
-        nd.rows = rows;
-        nd.lo = lo;
-        nd.hi = hi;
-        nd.off = 0;
-        T.nodes[q] = nd;
-    }
-    if (tid <= G) T.level_start[tid] = (1 << tid) - 1;
-    cta_sync();
-    // one warp per level: exclusive prefix of the row counts -> buffer offsets
-    const int warp = tid >> 5, lane = tid & 31;
-    if (warp <= G) {
-        const int d = warp, n = 1 << d, base = (1 << d) - 1;
-        int carry = 0;
-        for (int b0 = 0; b0 < n; b0 += 32) {
-            const int i = b0 + lane;
-            const int v = (i < n) ? (T.nodes[base + i].hi - T.nodes[base + i].lo) : 0;
-            int incl = v;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += y;
-            }
-            if (i < n) T.nodes[base + i].off = carry + incl - v;
-            carry += __shfl_sync(0xffffffffu, incl, 31);
-        }
-        if (lane == 0) {
-            T.level_rows[d] = carry;
-            if (carry > cap_rows) T.error = 2;
-        }
-    }
-    cta_sync();
-    if (tid == 0) {
-        int acc = 0;
-        for (int d = 0; d <= G; ++d) {
-            T.op_start[d] = acc;
-            acc += T.level_rows[d];
-        }
-        T.op_start[G + 1] = acc;
-    }
-    cta_sync();
-}
+// Whether the bottom three levels (G, G - 1, G - 2) of a full-depth job are computed together:
+// the nodes of level G - 2 then have 4 to 8 rows.
+RT_HD bool job_fused(int G, int b) { return G >= 2 && b >= kWideMinBins; }
 
-// The same job tree built by one warp (no CTA barrier), level by level: node i of level d is
-// the head (i even) or tail (i odd) child of node i >> 1 of level d - 1, which gives the
-// node list of build_job_tree.
-// With stage_source, also lays out the level-G source rows for staging (src_off, pstaged):
-// set when every level-G node has two children and the rows fit the level buffer.
-__device__ inline void build_job_tree_warp(JobTree& T, const JobSpec& J, int cap_rows,
-                                           bool stage_source = false)
+// Largest full depth of a stage-0 job whose node lists fit a JobTree.
+RT_HD int max_full_depth(int b) { return b >= kWideMinBins ? kMaxJobDepth : kMaxTreeDepth; }
+
+// Rows of a node are computed in groups of two consecutive rows, aligned so that the two rows
+// share their tail row (t(s) = t(s + 1), and mostly their head row): for a node of n rows the
+// group of row s is (s + n % 2) / 2. For every n up to kRegularRows that number is t(s) itself,
+// and h(s) is t(s) (n even), t(s) - 1 (n odd, s odd), or one of the two (n odd, s even: t(s) up
+// to a middle row, t(s) - 1 beyond it): checked exhaustively by the CPU tests. Beyond that the
+// float32 slope may round a row to its neighbour, and only the row groups (which read each
+// row's own numbers) are used.
+constexpr int kRegularRows = 65536;
+RT_HD int group_of(int n, int s) { return (s + (n & 1)) >> 1; }
+
+// Builds the node lists of a job (one warp, no CTA barrier), level by level: node i of level d
+// is the head (i even) or tail (i odd) child of node i >> 1 of level d - 1, its row range
+// follows from the parent's by the head/tail row maps. `raw`: a stage-0 job (whole subtree over
+// raw input rows); otherwise the level-G source rows are laid out for staging (src_off,
+// pstaged): set when every level-G node has two children and the rows fit a level buffer.
+__device__ inline void build_job_tree_warp(JobTree& T, const JobSpec& J, int b, int cap_rows,
+                                           int ops_units, bool raw)
 {
     const int lane = threadIdx.x & 31;
-    const int G = J.G;
-    const bool bad = (G > kMaxJobDepth || (2 << G) - 1 > kMaxJobNodes);
+    const bool fused = raw && job_fused(J.G, b);
+    const int depth = fused ? J.G - 2 : J.G;
+    const bool bad = depth > kMaxTreeDepth;
     if (lane == 0) {
-        T.depth = G;
+        T.depth = depth;
+        T.fused = fused ? 1 : 0;
         T.error = bad ? 1 : 0;
         T.pstaged = 0;
+        T.first_op = depth - 1;
     }
     if (bad) {
         __syncwarp();
         return;
     }
-    if (lane == 0) {
-        Node nd;
-        nd.row0 = J.root_row0;
-        nd.rows = J.root_rows;
-        nd.lo = J.lo;
-        nd.hi = J.hi;
-        nd.off = 0;
-        T.nodes[0] = nd;
-    }
-    __syncwarp();
-    for (int d = 1; d <= G; ++d) {
-        const int base = (1 << d) - 1, pbase = (1 << (d - 1)) - 1;
-        for (int i = lane; i < (1 << d); i += 32) {
-            const Node p = T.nodes[pbase + (i >> 1)];
-            const int mh = p.rows >> 1;
-            const MergeCoef c = merge_coef(p.rows);
-            Node nd;
-            if (i & 1) {
-                nd.row0 = p.row0 + mh;
-                nd.rows = p.rows - mh;
-                nd.lo = merge_row(c.kt, p.lo);
-                nd.hi = merge_row(c.kt, p.hi - 1) + 1;
-            } else {
-                nd.row0 = p.row0;
-                nd.rows = mh;
-                nd.lo = merge_row(c.kh, p.lo);
-                nd.hi = merge_row(c.kh, p.hi - 1) + 1;
-            }
-            nd.off = 0;
-            T.nodes[base + i] = nd;
-        }
-        __syncwarp();
-    }
-    // per level: exclusive prefix of the row counts -> buffer offsets; then op_start
-    int acc = 0;
-    for (int d = 0; d <= G; ++d) {
+    Node nd;  // node `lane` of the current level
+    nd.row0 = J.root_row0;
+    nd.rows = J.root_rows;
+    nd.lo = J.lo;
+    nd.hi = J.hi;
+    nd.qoff = 0;
+    float kt = 0.f;  // tail slope of the node
+    int groups = 0, quads = 0;  // lane d: of level d
+    for (int d = 0; d <= depth; ++d) {
         const int n = 1 << d, base = n - 1;
-        int carry = 0;
-        for (int b0 = 0; b0 < n; b0 += 32) {
-            const int i = b0 + lane;
-            const int v = (i < n) ? (T.nodes[base + i].hi - T.nodes[base + i].lo) : 0;
-            int incl = v;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += y;
-            }
-            if (i < n) T.nodes[base + i].off = carry + incl - v;
-            carry += __shfl_sync(0xffffffffu, incl, 31);
+        if (d > 0) {
+            Node p;
+            const int from = lane >> 1;
+            p.row0 = __shfl_sync(0xffffffffu, nd.row0, from);
+            p.rows = __shfl_sync(0xffffffffu, nd.rows, from);
+            p.lo = __shfl_sync(0xffffffffu, nd.lo, from);
+            p.hi = __shfl_sync(0xffffffffu, nd.hi, from);
+            const float pkh = __shfl_sync(0xffffffffu, nd.kh, from);
+            const float pkt = __shfl_sync(0xffffffffu, kt, from);
+            const int mh = p.rows >> 1;
+            const float k = (lane & 1) ? pkt : pkh;
+            nd.row0 = p.row0 + ((lane & 1) ? mh : 0);
+            nd.rows = (lane & 1) ? p.rows - mh : mh;
+            nd.lo = merge_row(k, p.lo);
+            nd.hi = merge_row(k, p.hi - 1) + 1;
         }
-        if (lane == 0) {
-            T.level_start[d] = base;
-            T.level_rows[d] = carry;
-            T.op_start[d] = acc;
-            if (carry > cap_rows) T.error = 2;
-        }
-        acc += carry;
-    }
-    if (lane == 0) T.op_start[G + 1] = acc;
-    if (stage_source && G <= kMaxStagedDepth) {
-        // rows each level-G node needs from its two children, as consecutive staged blocks
-        // (one lane per node: at most 32 nodes)
-        const int n = 1 << G, base = n - 1;
-        const int i = lane;
+        const MergeCoef mc = merge_coef(nd.rows);
+        nd.kh = mc.kh;
+        kt = mc.kt;
+        // rows stored and row groups of the node, scanned together (both below 2^15); the
+        // fused level stores whole nodes
         int v = 0;
-        bool two = true;
-        if (i < n) {
-            const Node nd = T.nodes[base + i];
-            int4 rg = make_int4(nd.row0, 0, nd.row0 + (nd.rows >> 1), 0);
-            if (nd.rows < 2) {
-                two = false;
-            } else if (nd.hi > nd.lo) {
-                const MergeCoef c = merge_coef(nd.rows);
-                const int hlo = merge_row(c.kh, nd.lo), tlo = merge_row(c.kt, nd.lo);
-                rg.x += hlo;
-                rg.y = merge_row(c.kh, nd.hi - 1) + 1 - hlo;
-                rg.z += tlo;
-                rg.w = merge_row(c.kt, nd.hi - 1) + 1 - tlo;
-            }
-            v = rg.y + rg.w;
-            T.src_rng[i] = rg;
+        if (lane < n) {
+            const int rows = (fused && d == depth) ? nd.rows : nd.hi - nd.lo;
+            const int grp = nd.hi > nd.lo
+                                ? group_of(nd.rows, nd.hi - 1) - group_of(nd.rows, nd.lo) + 1 : 0;
+            v = rows | (grp << 16);
         }
         int incl = v;
 #pragma unroll
@@ -267,361 +200,623 @@ __device__ inline void build_job_tree_warp(JobTree& T, const JobSpec& J, int cap
             const int y = __shfl_up_sync(0xffffffffu, incl, o);
             if (lane >= o) incl += y;
         }
-        if (i < n) T.src_off[i] = incl - v;
+        nd.off = (incl - v) & 0xffff;
+        nd.goff = (incl - v) >> 16;
+        if (lane < n) T.nodes[base + lane] = nd;
+        const int total = __shfl_sync(0xffffffffu, incl, 31);
+        if (lane == 0) {
+            T.level_rows[d] = total & 0xffff;
+            if ((total & 0xffff) > cap_rows) T.error = 2;
+        }
+        if (lane == d) groups = total >> 16;
+        if (d > 0) {
+            // the quads of a node of level d - 1 are the row groups of its tail child
+            const int odd = (lane & 1) ? v >> 16 : 0;
+            int qincl = odd;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, qincl, o);
+                if (lane >= o) qincl += y;
+            }
+            if (lane < n && (lane & 1)) T.nodes[base - (n >> 1) + (lane >> 1)].qoff = qincl - odd;
+            const int qtotal = __shfl_sync(0xffffffffu, qincl, 31);
+            if (lane == d - 1) quads = qtotal;
+        }
+    }
+    if (!raw) {
+        // rows each level-G node needs from its two children, as consecutive staged blocks
+        const int n = 1 << depth;
+        int v = 0;
+        bool two = true;
+        if (lane < n) {
+            int4 rg = make_int4(nd.row0, 0, nd.row0 + (nd.rows >> 1), 0);
+            if (nd.rows < 2) {
+                two = false;
+            } else if (nd.hi > nd.lo) {
+                const int hlo = merge_row(nd.kh, nd.lo), tlo = merge_row(kt, nd.lo);
+                rg.x += hlo;
+                rg.y = merge_row(nd.kh, nd.hi - 1) + 1 - hlo;
+                rg.z += tlo;
+                rg.w = merge_row(kt, nd.hi - 1) + 1 - tlo;
+            }
+            v = rg.y + rg.w;
+            T.src_rng[lane] = rg;
+        }
+        int incl = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        if (lane < n) T.src_off[lane] = incl - v;
         const int total = __shfl_sync(0xffffffffu, incl, 31);
         two = __all_sync(0xffffffffu, two);
         if (lane == 0) {
             T.src_off[n] = total;
-            T.pstaged = (two && total <= cap_rows) ? 1 : 0;
+            const bool staged = two && total <= cap_rows;
+            T.pstaged = staged ? 1 : 0;
+            if (staged) T.first_op = depth;
         }
+    }
+    __syncwarp();
+    // the passes over levels first_op .. 0: two levels at a time from the deepest up, a single
+    // one last when their number is odd
+    if (b < kWideMinBins && lane == 0) T.first_op = -1;
+    __syncwarp();
+    const bool regular = J.root_rows <= kRegularRows;
+    int ns = 0, unit = 0;
+    for (int d = T.first_op; d >= 0;) {
+        const bool two = d >= 1 && regular;
+        if (two) --d;
+        const int count = __shfl_sync(0xffffffffu, two ? quads : groups, d);
+        if (lane == 0) T.steps[ns] = Step{d, two ? 1 : 0, unit, count};
+        unit += two ? 2 * count : count;
+        ++ns;
+        --d;
+    }
+    if (lane == 0) {
+        T.nsteps = ns;
+        T.regular = regular ? 1 : 0;
+        if (unit > ops_units) T.error = 3;
     }
     __syncwarp();
 }
 
-// Index of the node holding buffer row r at a level (nodes sorted by `off`).
-__device__ __forceinline__ int find_node(const Node* nodes, int n, int r)
-{
-    int lo = 0, hi = n - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (nodes[mid].off <= r) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
-}
+// Chunks of kLaneCols columns of a row with its halo, and the stride of level rows in shared
+// memory and in stage outputs (whole chunks, 16-byte aligned rows).
+RT_HD int ffa_chunks(int b) { return (b + kHalo + kLaneCols - 1) / kLaneCols; }
+RT_HD int ffa_stride(int b) { return (ffa_chunks(b) * kLaneCols + 3) & ~3; }
 
-// Level rows in shared memory: b values, 16-byte aligned rows. For the bins ranges of the
-// usual searches (bins_min 240 or 480) the level loops are unrolled for exactly ceil(b / 64)
-// two-column chunks per lane (4, 5, 8, 9) and the global level for ceil(b / 32) columns
-// (8, 9, 15, 16, 17).
-RT_HD bool halo_mode(int b) { return (b >= 225 && b <= 288) || (b >= 449 && b <= 544); }
-RT_HD int ffa_stride(int b) { return (b + 3) & ~3; }
-
-// One output row of a level: out = row h + roll(row t, -shift) of the level below.
-// For the level read from global memory, h and t are global row indices; t < 0 marks a
-// single-row node (out = row h).
-struct RowOp {
-    int h, t, shift;
+// One group of a level: output rows `out` and, with kOpTwo, `out` + 1 of the level buffer;
+// row i is head row h_i + roll(tail row t_i, -shift_i) of the level below.
+struct GroupOp {
+    unsigned h;      // h_0 | h_1 << 16
+    unsigned t;      // t_0 | t_1 << 16
+    unsigned shift;  // shift_0 | shift_1 << 13 | flags
+    int out;
+};
+enum : unsigned {
+    kOpTwo = 1u << 26,       // two rows
+    kOpSameHead = 1u << 27,  // h_1 = h_0
+    kOpSameTail = 1u << 28,  // t_1 = t_0 and shift_1 = shift_0 + 1
 };
 
-// Row operation of buffer row r of level d.
-__device__ __forceinline__ RowOp make_row_op(const JobTree& T, int d, int r, int b)
+// One quad of a level: up to four consecutive output rows k = 0 .. 3 (row `out` + k of the
+// level buffer for the k of the mask) that read tail rows T_0 (k < 2) and T_1 of the level
+// below, shifted by sC, sC + 1, sC + 1, sC + 2, and head rows H_0 (k = 0; k = 1 without
+// kQuadH1), H_1 (k = 2; k = 1 with kQuadH1; k = 3 without kQuadH2) and H_2 (k = 3 with
+// kQuadH2). Those rows are not stored: each is formed from the level below it,
+//     H_0 = A_a0 + roll(B_b0, -sB),  H_1 = A_a1 + roll(B_b0, -(sB + 1)),
+//     H_2 = A_a2 + roll(B_b2, -sB2),
+//     T_0 = C_c0 + roll(D_d0, -(sD - sC)),  T_1 = C_c1 + roll(D_d0, -(sD - sC + 1)).
+struct QuadOp {
+    unsigned a01, b0a2, b2c0, c1d0;  // 16-bit row numbers of level d + 2, low half first
+    unsigned sB;                     // sB | sB2 << 13
+    unsigned sCD;                    // sC | sD << 13
+    unsigned flags;                  // mask of valid rows | flags
+    int out;
+};
+enum : unsigned {
+    kQuadSameA = 16u,  // a1 = a0
+    kQuadSameC = 32u,  // c1 = c0
+    kQuadH1 = 64u,
+    kQuadH2 = 128u,
+};
+static_assert(sizeof(GroupOp) == 16 && sizeof(QuadOp) == 32, "operations are read as 16-byte units");
+
+// Where row r of child `tail` (0 head, 1 tail) of node i of level d is found: its row in the
+// level below's buffer, in the staged rows (deepest level, pstaged), or of the transform.
+__device__ __forceinline__ int child_row(const JobTree& T, int d, int i, const Node& nd, int tail,
+                                         int r)
 {
-    const Node* lvl = T.nodes + T.level_start[d];
-    const int i = find_node(lvl, 1 << d, r);
-    const Node nd = lvl[i];
-    const int s = nd.lo + (r - nd.off);
-    RowOp op;
-    if (nd.rows == 1) {
-        op.h = nd.row0;
-        op.t = -1;
-        op.shift = 0;
-    } else {
-        const MergeCoef c = merge_coef(nd.rows);
-        const int h = merge_row(c.kh, s), t = merge_row(c.kt, s);
-        op.shift = (s - t) % b;
-        if (d == T.depth && T.pstaged) {
-            const int4 rg = T.src_rng[i];
-            op.h = T.src_off[i] + (nd.row0 + h - rg.x);
-            op.t = T.src_off[i] + rg.y + (nd.row0 + (nd.rows >> 1) + t - rg.z);
-        } else if (d == T.depth) {
-            op.h = nd.row0 + h;
-            op.t = nd.row0 + (nd.rows >> 1) + t;
-        } else {
-            const Node* child = T.nodes + T.level_start[d + 1];
-            const Node hn = child[2 * i], tn = child[2 * i + 1];
-            op.h = hn.off + h - hn.lo;
-            op.t = tn.off + t - tn.lo;
-        }
+    if (d < T.depth) {
+        const Node& c = T.nodes[(2 << d) - 1 + 2 * i + tail];
+        return c.off + r - c.lo;
+    }
+    const int row = nd.row0 + (tail ? (nd.rows >> 1) : 0) + r;
+    if (!T.pstaged) return row;
+    const int4 rg = T.src_rng[i];
+    return T.src_off[i] + (tail ? rg.y + row - rg.z : row - rg.x);
+}
+
+// Source row numbers and shift of output row s of node i of level d.
+__device__ __forceinline__ void source_rows(const JobTree& T, int d, int i, const Node& nd, int s,
+                                            int* h, int* t, int* shift)
+{
+    const int hs = merge_row(nd.kh, s);
+    const int ts = T.regular ? group_of(nd.rows, s) : merge_row(merge_coef(nd.rows).kt, s);
+    *shift = s - ts;
+    *h = child_row(T, d, i, nd, 0, hs);
+    *t = child_row(T, d, i, nd, 1, ts);
+}
+
+// x mod b by one multiply-high, `inv` = ceil(2^32 / b): exact while x b < 2^32 (the shifts of a
+// transform of at most kRegularRows rows); x >= -1.
+__device__ __forceinline__ int mod_bins(int x, int b, unsigned inv)
+{
+    if (x < 0) x += b;
+    return x - (int)__umulhi((unsigned)x, inv) * b;
+}
+
+// Row group r of level d.
+__device__ inline GroupOp make_group(const JobTree& T, int d, int r, int b, unsigned inv)
+{
+    const Node* lvl = T.nodes + (1 << d) - 1;
+    int lo = 0, hi = (1 << d) - 1;  // node holding group r (nodes sorted by goff)
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (lvl[mid].goff <= r) lo = mid;
+        else hi = mid - 1;
+    }
+    const Node nd = lvl[lo];
+    const int q = group_of(nd.rows, nd.lo) + (r - nd.goff);
+    const int s0 = max(nd.lo, 2 * q - (nd.rows & 1));
+    const int s1 = min(nd.hi - 1, 2 * q - (nd.rows & 1) + 1);
+    GroupOp op;
+    int h0, t0, sh0;
+    source_rows(T, d, lo, nd, s0, &h0, &t0, &sh0);
+    sh0 = T.regular ? mod_bins(sh0, b, inv) : sh0 % b;
+    op.out = nd.off + s0 - nd.lo;
+    op.h = h0;
+    op.t = t0;
+    op.shift = sh0;
+    if (s1 > s0) {
+        int h1, t1, sh1;
+        source_rows(T, d, lo, nd, s1, &h1, &t1, &sh1);
+        sh1 = T.regular ? mod_bins(sh1, b, inv) : sh1 % b;
+        op.h |= h1 << 16;
+        op.t |= t1 << 16;
+        op.shift |= (sh1 << 13) | kOpTwo | (h1 == h0 ? kOpSameHead : 0) |
+                    (t1 == t0 && sh1 == (sh0 + 1 == b ? 0 : sh0 + 1) ? kOpSameTail : 0);
     }
     return op;
 }
 
-// Row operations of every level of the job (one thread per output row, all levels at once).
-// Call after build_job_tree; the caller synchronises before using `ops`.
-__device__ inline void build_all_ops(const JobTree& T, int b, RowOp* ops)
+// Row quad r of level d (over level d + 1, whose rows are not stored).
+__device__ inline QuadOp make_quad(const JobTree& T, int d, int r, int b, unsigned inv)
 {
-    const int total = T.op_start[T.depth + 1];
-    for (int g = threadIdx.x; g < total; g += kThreads) {
-        int d = 0;
-        while (T.op_start[d + 1] <= g) ++d;
-        ops[g] = make_row_op(T, d, g - T.op_start[d], b);
+    const Node* lvl = T.nodes + (1 << d) - 1;
+    int i = 0, hi = (1 << d) - 1;  // node holding quad r (nodes sorted by qoff)
+    while (i < hi) {
+        const int mid = (i + hi + 1) >> 1;
+        if (lvl[mid].qoff <= r) i = mid;
+        else hi = mid - 1;
+    }
+    const Node N = lvl[i];
+    const Node Hn = T.nodes[(2 << d) - 1 + 2 * i], Tn = T.nodes[(2 << d) + 2 * i];
+    const int p = N.rows & 1, pT = Tn.rows & 1;
+    const int gid = group_of(Tn.rows, Tn.lo) + (r - N.qoff);  // tail row of T_0 and T_1
+    const int t0 = 2 * gid - pT, s0 = 2 * t0 - p;             // T_0 and output row k = 0
+    const int k0 = max(0, N.lo - s0), k1 = min(4, N.hi - s0);  // rows [k0, k1) are wanted
+    const int hb = t0 - p;                                     // H_0
+    const bool v0 = k0 == 0, v1 = k0 <= 1 && k1 > 1, v2 = k0 <= 2 && k1 > 2, v3 = k1 > 3;
+    const bool h1 = v1 && merge_row(N.kh, s0 + 1) != hb;      // k = 1 reads H_1
+    const bool h2 = v3 && merge_row(N.kh, s0 + 3) == hb + 2;  // k = 3 reads H_2
+    const bool need0 = v0 || (v1 && !h1), need1 = h1 || v2 || (v3 && !h2);
+    // a row that nothing reads stands in for another, so that every row number is valid
+    const int r0 = need0 ? hb : need1 ? hb + 1 : hb + 2;
+    const int r1 = need1 ? hb + 1 : r0;
+    const int r2 = h2 ? hb + 2 : r0;
+    const int u0 = (v0 || v1) ? t0 : t0 + 1, u1 = (v2 || v3) ? t0 + 1 : t0;
+    const int e = d + 1;
+    const int a0 = child_row(T, e, 2 * i, Hn, 0, merge_row(Hn.kh, r0));
+    const int a1 = child_row(T, e, 2 * i, Hn, 0, merge_row(Hn.kh, r1));
+    const int a2 = child_row(T, e, 2 * i, Hn, 0, merge_row(Hn.kh, r2));
+    const int gB = group_of(Hn.rows, r0), gB2 = group_of(Hn.rows, r2);
+    const int b0 = child_row(T, e, 2 * i, Hn, 1, gB), b2 = child_row(T, e, 2 * i, Hn, 1, gB2);
+    const int c0 = child_row(T, e, 2 * i + 1, Tn, 0, merge_row(Tn.kh, u0));
+    const int c1 = child_row(T, e, 2 * i + 1, Tn, 0, merge_row(Tn.kh, u1));
+    const int d0 = child_row(T, e, 2 * i + 1, Tn, 1, gid);
+    QuadOp op;
+    op.a01 = a0 | (a1 << 16);
+    op.b0a2 = b0 | (a2 << 16);
+    op.b2c0 = b2 | (c0 << 16);
+    op.c1d0 = c1 | (d0 << 16);
+    op.sB = mod_bins(hb - gB, b, inv) | (mod_bins(r2 - gB2, b, inv) << 13);
+    op.sCD = mod_bins(s0 - t0, b, inv) | (mod_bins(s0 - gid, b, inv) << 13);
+    op.flags = (v0 ? 1u : 0) | (v1 ? 2u : 0) | (v2 ? 4u : 0) | (v3 ? 8u : 0) |
+               (a1 == a0 ? kQuadSameA : 0) | (c1 == c0 ? kQuadSameC : 0) | (h1 ? kQuadH1 : 0) |
+               (h2 ? kQuadH2 : 0);
+    op.out = N.off + s0 - N.lo;  // negative when row 0 is not wanted
+    return op;
+}
+
+// Operations of all steps of the job, one thread per operation, dealt from the last thread down
+// (the boxcar S/N of the search's previous job keeps the first warps longest). Call after
+// build_job_tree_warp; the caller synchronises before using `ops`.
+__device__ inline void build_ops(const JobTree& T, int b, uint4* ops)
+{
+    const unsigned inv = 0xffffffffu / (unsigned)b + 1u;
+    const int nsteps = T.nsteps;
+    for (int g = kThreads - 1 - (int)threadIdx.x;; g += kThreads) {
+        int r = g, k = 0;
+        while (k < nsteps && r >= T.steps[k].count) r -= T.steps[k++].count;
+        if (k >= nsteps) break;
+        const Step st = T.steps[k];
+        if (st.two)
+            *reinterpret_cast<QuadOp*>(ops + st.unit + 2 * r) = make_quad(T, st.d, r, b, inv);
+        else
+            *reinterpret_cast<GroupOp*>(ops + st.unit + r) = make_group(T, st.d, r, b, inv);
     }
 }
 
-// Computes the rows of one level, one warp per row, NIT = ceil(b / 32) columns per lane.
-// kGlobal: operands are rows of the global source (packed, stride b).
-template <int NIT, bool kGlobal>
-__device__ __forceinline__ void level_rows_unrolled(const RowOp* ops, int nrows,
-                                                    const float* __restrict__ src, int sstride,
-                                                    float* __restrict__ dst, int stride, int b)
+// a + b of two values at once: two round-to-nearest float32 additions
+__device__ __forceinline__ void add2(float a0, float a1, float b0, float b1, float& s0, float& s1)
+{
+    asm("{\n .reg .b64 a, b, d;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n"
+        " add.rn.f32x2 d, a, b;\n mov.b64 {%0, %1}, d;\n}"
+        : "=f"(s0), "=f"(s1)
+        : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
+}
+
+// First column of a lane's window in a rolled row: (c0 + shift) mod b, for c0 < b + kHalo and
+// shift < b (b >= kWideMinBins, so two subtractions are enough).
+__device__ __forceinline__ int rolled_col(int c0, int shift, int b)
+{
+    const unsigned i = (unsigned)(c0 + shift);
+    const unsigned j = min(i, i - (unsigned)b);
+    return (int)min(j, j - (unsigned)b);
+}
+
+// Computes one level by row groups, from rows of stride `stride` with halo to rows of the same
+// layout. A warp takes one group (two rows) at a time, or 32 / W groups when a row has at most
+// W = 16 or 8 chunks; rows of more than 32 chunks are several warp tasks.
+__device__ __forceinline__ void level_groups(const uint4* ops, int ngroups,
+                                             const float* __restrict__ src,
+                                             float* __restrict__ dst, int stride, int b)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int r = warp; r < nrows; r += kWarps) {
-        const RowOp op = ops[r];
-        float* out = dst + (size_t)r * stride;
-        const float* H = src + (size_t)op.h * sstride;
-        float v[NIT];
-        if (op.t < 0) {
-#pragma unroll
-            for (int j = 0; j < NIT; ++j) {
-                const int c = lane + 32 * j;
-                if (j < NIT - 1 || c < b) v[j] = kGlobal ? __ldcg(H + c) : H[c];
-            }
+    const int nq = ffa_chunks(b);
+    const int lw = nq <= 8 ? 3 : nq <= 16 ? 4 : 5;  // log2 of the lanes of a group
+    const int nblk = (nq + 31) >> 5;
+    const unsigned inv = (65536u + nblk - 1) / nblk;  // task / nblk: exact, task * nblk < 65536
+    const int ntask = (ngroups * nblk + (32 >> lw) - 1) >> (5 - lw);
+    const int sub = lane >> lw, ql = lane & ((1 << lw) - 1);
+    for (int task = warp; task < ntask; task += kWarps) {
+        int g = task, q = ql;
+        if (nblk > 1) {
+            g = (int)(((unsigned)task * inv) >> 16);
+            q += 32 * (task - g * nblk);
         } else {
-            // column c reads the rolled row at c + shift, or c + shift - b past the wrap
-            // (c + shift < 2 b): the test 32 j >= b - shift - lane picks the base pointer
-            const float* T0 = src + (size_t)op.t * sstride + op.shift + lane;
-            const float* T1 = T0 - b;
-            const int thr = b - op.shift - lane;
-#pragma unroll
-            for (int j = 0; j < NIT; j += 2) {
-                const int c = lane + 32 * j;
-                const float* p = (32 * j >= thr) ? T1 : T0;
-                if (j + 1 < NIT - 1) {
-                    // two columns, both inside the row: one packed f32x2 addition
-                    const float* q = (32 * j + 32 >= thr) ? T1 : T0;
-                    asm("{\n .reg .b64 a, b, d;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n"
-                        " add.rn.f32x2 d, a, b;\n mov.b64 {%0, %1}, d;\n}"
-                        : "=f"(v[j]), "=f"(v[j + 1])
-                        : "f"(kGlobal ? __ldcg(H + c) : H[c]), "f"(kGlobal ? __ldcg(H + c + 32) : H[c + 32]),
-                          "f"(kGlobal ? __ldcg(p + 32 * j) : p[32 * j]),
-                          "f"(kGlobal ? __ldcg(q + 32 * j + 32) : q[32 * j + 32]));
-                } else {
-                    if (j < NIT - 1 || c < b)
-                        v[j] = __fadd_rn(kGlobal ? __ldcg(H + c) : H[c],
-                                         kGlobal ? __ldcg(p + 32 * j) : p[32 * j]);
-                    if (j + 1 < NIT) {
-                        const float* q = (32 * j + 32 >= thr) ? T1 : T0;
-                        if (c + 32 < b)
-                            v[j + 1] = __fadd_rn(kGlobal ? __ldcg(H + c + 32) : H[c + 32],
-                                                 kGlobal ? __ldcg(q + 32 * j + 32) : q[32 * j + 32]);
-                    }
-                }
-            }
+            g = (task << (5 - lw)) + sub;
         }
+        if (q >= nq || g >= ngroups) continue;
+        const uint4 v = ops[g];  // a GroupOp
+        const int c0 = kLaneCols * q;
+        const float* ph = src + (int)(v.x & 0xffff) * stride + c0;
+        float* po = dst + (int)v.w * stride + c0;
+        float H[kLaneCols], Tl[kLaneCols + 1];
 #pragma unroll
-        for (int j = 0; j < NIT; ++j) {
-            const int c = lane + 32 * j;
-            if (j < NIT - 1 || c < b) out[c] = v[j];
+        for (int k = 0; k < kLaneCols; ++k) H[k] = ph[k];
+        const float* pt = src + (int)(v.y & 0xffff) * stride + rolled_col(c0, v.z & 0x1fff, b);
+#pragma unroll
+        for (int k = 0; k <= kLaneCols; ++k) Tl[k] = pt[k];
+#pragma unroll
+        for (int k = 0; k + 1 < kLaneCols; k += 2) {
+            float s0, s1;
+            add2(H[k], H[k + 1], Tl[k], Tl[k + 1], s0, s1);
+            po[k] = s0;
+            po[k + 1] = s1;
+        }
+        po[kLaneCols - 1] = __fadd_rn(H[kLaneCols - 1], Tl[kLaneCols - 1]);
+        if (!(v.z & kOpTwo)) continue;
+        if (!(v.z & kOpSameHead)) {
+            const float* ph1 = src + (int)(v.x >> 16) * stride + c0;
+#pragma unroll
+            for (int k = 0; k < kLaneCols; ++k) H[k] = ph1[k];
+        }
+        if (!(v.z & kOpSameTail)) {
+            const float* pt1 =
+                src + (int)(v.y >> 16) * stride + rolled_col(c0, (v.z >> 13) & 0x1fff, b);
+#pragma unroll
+            for (int k = 0; k < kLaneCols; ++k) Tl[k + 1] = pt1[k];
+        }
+        po += stride;
+#pragma unroll
+        for (int k = 0; k < kLaneCols; ++k) po[k] = __fadd_rn(H[k], Tl[k + 1]);
+    }
+}
+
+// Computes level d from level d + 2 by row quads, both of stride `stride` with halo: 42 reads
+// and 36 writes of a lane for the 4 x 9 values of level d and the as many of level d + 1 that
+// stay in registers (two passes of level_groups: 76 and 72).
+__device__ __forceinline__ void level_quads(const uint4* ops, int nquads,
+                                            const float* __restrict__ src,
+                                            float* __restrict__ dst, int stride, int b)
+{
+    constexpr int K = kLaneCols;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nq = ffa_chunks(b);
+    const int lw = nq <= 8 ? 3 : nq <= 16 ? 4 : 5;  // log2 of the lanes of a quad
+    const int nblk = (nq + 31) >> 5;
+    const unsigned inv = (65536u + nblk - 1) / nblk;  // task / nblk: exact, task * nblk < 65536
+    const int ntask = (nquads * nblk + (32 >> lw) - 1) >> (5 - lw);
+    const int sub = lane >> lw, ql = lane & ((1 << lw) - 1);
+    for (int task = warp; task < ntask; task += kWarps) {
+        int g = task, q = ql;
+        if (nblk > 1) {
+            g = (int)(((unsigned)task * inv) >> 16);
+            q += 32 * (task - g * nblk);
+        } else {
+            g = (task << (5 - lw)) + sub;
+        }
+        if (q >= nq || g >= nquads) continue;
+        const uint4 v = ops[2 * g], w = ops[2 * g + 1];  // a QuadOp
+        const int c0 = K * q;
+        float T0[K + 1], T1[K + 1];
+        {
+            const float* pc = src + (int)(v.z >> 16) * stride + rolled_col(c0, w.y & 0x1fff, b);
+            const float* pd =
+                src + (int)(v.w >> 16) * stride + rolled_col(c0, (w.y >> 13) & 0x1fff, b);
+            float C[K + 2], D[K + 3];
+#pragma unroll
+            for (int k = 0; k < K + 2; ++k) C[k] = pc[k];
+#pragma unroll
+            for (int k = 0; k < K + 3; ++k) D[k] = pd[k];
+#pragma unroll
+            for (int k = 0; k < K + 1; ++k) T0[k] = __fadd_rn(C[k], D[k]);
+            if (!(w.z & kQuadSameC)) {
+                pc += ((int)(v.w & 0xffff) - (int)(v.z >> 16)) * stride;
+#pragma unroll
+                for (int k = 0; k < K + 1; ++k) C[k + 1] = pc[k + 1];
+            }
+#pragma unroll
+            for (int k = 0; k < K + 1; ++k) T1[k] = __fadd_rn(C[k + 1], D[k + 2]);
+        }
+        float H0[K], H1[K];
+        {
+            const float* pa = src + (int)(v.x & 0xffff) * stride + c0;
+            const float* pb = src + (int)(v.y & 0xffff) * stride + rolled_col(c0, w.x & 0x1fff, b);
+            float A[K], B[K + 1];
+#pragma unroll
+            for (int k = 0; k < K; ++k) A[k] = pa[k];
+#pragma unroll
+            for (int k = 0; k < K + 1; ++k) B[k] = pb[k];
+#pragma unroll
+            for (int k = 0; k < K; ++k) H0[k] = __fadd_rn(A[k], B[k]);
+            if (!(w.z & kQuadSameA)) {
+                pa += ((int)(v.x >> 16) - (int)(v.x & 0xffff)) * stride;
+#pragma unroll
+                for (int k = 0; k < K; ++k) A[k] = pa[k];
+            }
+#pragma unroll
+            for (int k = 0; k < K; ++k) H1[k] = __fadd_rn(A[k], B[k + 1]);
+        }
+        float* po = dst + (int)w.w * stride + c0;
+        if (w.z & 1u) {
+#pragma unroll
+            for (int k = 0; k < K; ++k) po[k] = __fadd_rn(H0[k], T0[k]);
+        }
+        po += stride;
+        if (w.z & 2u) {
+            if (w.z & kQuadH1) {
+#pragma unroll
+                for (int k = 0; k < K; ++k) H0[k] = H1[k];
+            }
+#pragma unroll
+            for (int k = 0; k < K; ++k) po[k] = __fadd_rn(H0[k], T0[k + 1]);
+        }
+        po += stride;
+        if (w.z & 4u) {
+#pragma unroll
+            for (int k = 0; k < K; ++k) po[k] = __fadd_rn(H1[k], T1[k]);
+        }
+        po += stride;
+        if (w.z & 8u) {
+            if (w.z & kQuadH2) {
+                const float* pa = src + (int)(v.y >> 16) * stride + c0;
+                const float* pb =
+                    src + (int)(v.z & 0xffff) * stride + rolled_col(c0, (w.x >> 13) & 0x1fff, b);
+#pragma unroll
+                for (int k = 0; k < K; ++k) H1[k] = __fadd_rn(pa[k], pb[k]);
+            }
+#pragma unroll
+            for (int k = 0; k < K; ++k) po[k] = __fadd_rn(H1[k], T1[k + 1]);
         }
     }
 }
 
-// Shared-memory level for the usual bins ranges: in each 64-column chunk a lane computes
-// columns c = 64 j + lane and c + 32, so every load and store of the warp touches 32
-// consecutive words (mod b). Column c reads the rolled row at c + shift before the wrap and
-// at c + shift - b after it (c + shift < 2 b: one wrap at most); with c = 64 j + lane (+ 32)
-// the wrap test is 64 j (+ 32) >= b - shift - lane, an immediate compared with one register
-// per row, and picks one of two base pointers: one compare and one select per element, and
-// no dependency chain from chunk to chunk.
-template <int NIT2>
-__device__ __forceinline__ void level_rows_pairs(const RowOp* ops, int nrows,
-                                                 const float* __restrict__ src, int sstride,
-                                                 float* __restrict__ dst, int stride, int b)
+// One level row by row with a modulo per column: any bins, any source (raw rows or rows with
+// halo, shared or global memory, `sstride` apart). For what the other two loops do not take:
+// fewer than kWideMinBins bins, whole subtrees of at most 4 rows, and stages whose source rows
+// do not fit a level buffer.
+__device__ __forceinline__ void level_rows_direct(const JobTree& T, int d, const float* src,
+                                               size_t sstride, float* dst, int stride, int b)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int r = warp; r < nrows; r += kWarps) {
-        const RowOp op = ops[r];
-        float* out = dst + (size_t)r * stride + lane;
-        const float* H = src + (size_t)op.h * sstride + lane;
-        const float* T0 = src + (size_t)op.t * sstride + op.shift + lane;
-        const float* T1 = T0 - b;
-        const int thr = b - op.shift - lane;
-#pragma unroll
-        for (int j = 0; j < NIT2; ++j) {
-            const int c = 64 * j + lane;
-            const float* p0 = (64 * j >= thr) ? T1 : T0;
-            const float* p1 = (64 * j + 32 >= thr) ? T1 : T0;
-            if (j < NIT2 - 1) {
-                // both columns' adds in one packed f32x2 addition
-                float s0, s1;
-                asm("{\n .reg .b64 a, b, d;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n"
-                    " add.rn.f32x2 d, a, b;\n mov.b64 {%0, %1}, d;\n}"
-                    : "=f"(s0), "=f"(s1)
-                    : "f"(H[64 * j]), "f"(H[64 * j + 32]), "f"(p0[64 * j]), "f"(p1[64 * j + 32]));
-                out[64 * j] = s0;
-                out[64 * j + 32] = s1;
-            } else {
-                if (c < b) out[64 * j] = __fadd_rn(H[64 * j], p0[64 * j]);
-                // the last chunk's second half (columns from 64 (NIT2 - 1) + 32) is empty for
-                // every b of the 5- and 9-chunk ranges (b <= 288 and b <= 544)
-                constexpr bool kHalf2 = NIT2 != 5 && NIT2 != 9;
-                if (kHalf2 && c + 32 < b) out[64 * j + 32] = __fadd_rn(H[64 * j + 32], p1[64 * j + 32]);
-            }
+    const Node* lvl = T.nodes + (1 << d) - 1;
+    for (int r = warp; r < T.level_rows[d]; r += kWarps) {
+        int lo = 0, hi = (1 << d) - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (lvl[mid].off <= r) lo = mid;
+            else hi = mid - 1;
         }
-    }
-}
-
-// Any b: per-element wrap, no unrolling.
-template <bool kGlobal>
-__device__ __forceinline__ void level_rows_generic(const RowOp* ops, int nrows,
-                                                   const float* __restrict__ src, int sstride,
-                                                   float* __restrict__ dst, int stride, int b)
-{
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int r = warp; r < nrows; r += kWarps) {
-        const RowOp op = ops[r];
+        const Node nd = lvl[lo];
         float* out = dst + (size_t)r * stride;
-        const float* H = src + (size_t)op.h * sstride;
-        const float* Tr = src + (size_t)(op.t < 0 ? 0 : op.t) * sstride;
-        for (int c = lane; c < b; c += 32) {
-            float v;
-            if (op.t < 0) {
-                v = kGlobal ? __ldcg(H + c) : H[c];
-            } else {
-                int idx = c + op.shift;
-                idx -= (idx >= b) ? b : 0;
-                v = kGlobal ? __fadd_rn(__ldcg(H + c), __ldcg(Tr + idx)) : __fadd_rn(H[c], Tr[idx]);
-            }
-            out[c] = v;
+        if (nd.rows == 1) {
+            const int h = d < T.depth ? T.nodes[(2 << d) - 1 + 2 * lo].off : nd.row0;
+            for (int c = lane; c < b + kHalo; c += 32) out[c] = src[(size_t)h * sstride + c % b];
+            continue;
+        }
+        int h, t, shift;
+        source_rows(T, d, lo, nd, nd.lo + (r - nd.off), &h, &t, &shift);
+        const float *H = src + (size_t)h * sstride, *Tl = src + (size_t)t * sstride;
+        for (int c = lane; c < b + kHalo; c += 32)
+            out[c] = __fadd_rn(H[c % b], Tl[(c + shift) % b]);
+    }
+}
+
+// Head and tail rows of output row s of a node of n <= 8 rows, as merge_row gives them: the
+// rounded quotients s (n_child - 1) / (n - 1).
+__host__ __device__ constexpr int small_row(int n, int child, int s)
+{
+    return n < 2 ? 0 : (2 * s * (child - 1) + (n - 1)) / (2 * (n - 1));
+}
+
+// The transform of N input rows on LEN consecutive columns, entirely in registers (the row and
+// column numbers are compile-time constants; values nothing uses are never computed). off[j]:
+// offset of column c0 + j (mod b) in a row.
+template <int N, int LEN>
+struct SmallNode {
+    static __device__ __forceinline__ void run(const float* x, int b, const int* off,
+                                               float (&o)[N][LEN])
+    {
+        constexpr int NH = N / 2, NT = N - NH;
+        float H[NH][LEN], Tl[NT][LEN + NH];  // the largest shift s - t(s) is N - NT = NH
+        SmallNode<NH, LEN>::run(x, b, off, H);
+        SmallNode<NT, LEN + NH>::run(x + NH * b, b, off, Tl);
+#pragma unroll
+        for (int s = 0; s < N; ++s) {
+#pragma unroll
+            for (int j = 0; j < LEN; ++j)
+                o[s][j] = __fadd_rn(H[small_row(N, NH, s)][j],
+                                    Tl[small_row(N, NT, s)][j + s - small_row(N, NT, s)]);
         }
     }
-}
-
-// Bins classes of a kernel instance: which unrolled level loops it contains. A kernel that
-// only ever sees b in [225, 288] (kBins256) or in [449, 544] (kBins512) leaves out the loops of
-// the other range (smaller code); kBinsAny has all of them. Any b still runs correctly in any
-// class (the generic loop), only slower.
-enum BinsClass { kBinsAny = 0, kBins256 = 1, kBins512 = 2 };
-
-RT_HD int bins_class(int bmin, int bmax)
-{
-    if (bmin >= 225 && bmax <= 288) return kBins256;
-    if (bmin >= 449 && bmax <= 544) return kBins512;
-    return kBinsAny;
-}
-
-template <bool kGlobal, int BC = kBinsAny>
-__device__ __forceinline__ void level_rows(const RowOp* ops, int nrows, const float* src,
-                                           int sstride, float* dst, int stride, int b)
-{
-    constexpr bool k256 = BC != kBins512, k512 = BC != kBins256;
-    // each case runs its unrolled loop and returns when the class holds it, else falls
-    // through to the generic loop below
-#define RT_PAIRS_CASE(N, K)                                                   \
-    case N:                                                                   \
-        if constexpr (K) {                                                    \
-            level_rows_pairs<N>(ops, nrows, src, sstride, dst, stride, b);    \
-            return;                                                           \
-        }                                                                     \
-        break;
-    if (!kGlobal && halo_mode(b)) {
-        switch ((b + 63) >> 6) {
-            RT_PAIRS_CASE(4, k256)
-            RT_PAIRS_CASE(5, k256)
-            RT_PAIRS_CASE(8, k512)
-            default:  // 9
-                if constexpr (k512) {
-                    level_rows_pairs<9>(ops, nrows, src, sstride, dst, stride, b);
-                    return;
-                }
-                break;
-        }
+};
+template <int LEN>
+struct SmallNode<1, LEN> {
+    static __device__ __forceinline__ void run(const float* x, int, const int* off,
+                                               float (&o)[1][LEN])
+    {
+#pragma unroll
+        for (int j = 0; j < LEN; ++j) o[0][j] = x[off[j]];
     }
-#undef RT_PAIRS_CASE
-#define RT_NIT_CASE(N, K)                                                              \
-    case N:                                                                            \
-        if constexpr (K) {                                                             \
-            level_rows_unrolled<N, kGlobal>(ops, nrows, src, sstride, dst, stride, b); \
-            return;                                                                    \
-        }                                                                              \
-        break;
-    switch ((b + 31) >> 5) {
-        // bins 225-288 and 449-544 cover the usual searches (bins_min 240 / 480)
-        RT_NIT_CASE(8, k256)
-        RT_NIT_CASE(9, k256)
-        RT_NIT_CASE(15, k512)
-        RT_NIT_CASE(16, k512)
-        RT_NIT_CASE(17, k512)
-        default: break;
-    }
-#undef RT_NIT_CASE
-    level_rows_generic<kGlobal>(ops, nrows, src, sstride, dst, stride, b);
-}
-
-// Level computed from source rows staged in shared memory (packed, stride b): same loop as
-// the global level, plain loads.
-template <int BC = kBinsAny>
-__device__ __forceinline__ void level_rows_staged(const RowOp* ops, int nrows, const float* src,
-                                                  float* dst, int stride, int b)
-{
-    constexpr bool k256 = BC != kBins512, k512 = BC != kBins256;
-#define RT_NIT_CASE(N, K)                                                         \
-    case N:                                                                       \
-        if constexpr (K) {                                                        \
-            level_rows_unrolled<N, false>(ops, nrows, src, b, dst, stride, b);    \
-            return;                                                               \
-        }                                                                         \
-        break;
-    switch ((b + 31) >> 5) {
-        RT_NIT_CASE(8, k256)
-        RT_NIT_CASE(9, k256)
-        RT_NIT_CASE(15, k512)
-        RT_NIT_CASE(16, k512)
-        RT_NIT_CASE(17, k512)
-        default: break;
-    }
-#undef RT_NIT_CASE
-    level_rows_generic<false>(ops, nrows, src, b, dst, stride, b);
-}
-
-// Where a job's levels read and write outside the two level buffers.
-struct LevelIO {
-    const float* src = nullptr;     // global source: row j at src + j * src_stride
-    int src_stride = 0;
-    const float* staged = nullptr;  // optional source rows being copied into shared memory
-    bool staged_rows = false;       // staged: true = rows of the layout in JobTree::src_off
-                                    // (stride = the level stride); false = global row j at
-                                    // staged + j * b
-    uint64_t* bar = nullptr;        // the copy completes on phase *phase of bar
-    uint32_t* phase = nullptr;
-    float* root_dst = nullptr;      // optional: root rows go to root_dst + i * root_stride
-    int root_stride = 0;
 };
 
-// Runs all levels of the job. On return, the root rows [lo, hi) are in buf0 (stride
-// `stride`, row i of the buffer = root output row lo + i), or in global memory if
-// io.root_dst is given. `ops` has room for the largest level. Returns false if the wait for
-// staged rows ran out.
-template <int BC = kBinsAny>
-__device__ inline bool run_job_levels(const JobTree& T, int b, float* buf0, float* buf1,
-                                      int stride, RowOp* ops, const LevelIO& io)
+constexpr int kFusedWindow = kLaneCols + 7;  // columns a lane reads from the last of 8 rows
+
+template <int N>
+__device__ __forceinline__ void fused_node(const float* x, int b, const int* off, float* out,
+                                           int stride)
 {
-    build_all_ops(T, b, ops);
-    cta_sync();
-    bool ok = true;
-    if (io.staged) {
-        ok = mbar_wait(io.bar, *io.phase);
-        *io.phase ^= 1u;
+    float o[N][kLaneCols];
+    SmallNode<N, kLaneCols>::run(x, b, off, o);
+#pragma unroll
+    for (int s = 0; s < N; ++s) {
+#pragma unroll
+        for (int k = 0; k < kLaneCols; ++k) out[s * stride + k] = o[s][k];
     }
-    for (int d = T.depth; d >= 0; --d) {
-        // the root level goes straight to global memory when the caller wants it there
-        const bool out_global = d == 0 && io.root_dst != nullptr;
-        float* dst = out_global ? io.root_dst : ((d & 1) ? buf1 : buf0);
-        const int dstride = out_global ? io.root_stride : stride;
-        const RowOp* lops = ops + T.op_start[d];
-        // one call site per level loop kind (the loops are large once unrolled)
-        const bool first = d == T.depth;
-        if (first && !io.staged) {
-            level_rows<true, BC>(lops, T.level_rows[d], io.src, io.src_stride, dst, dstride, b);
-        } else if (first && !io.staged_rows) {
-            level_rows_staged<BC>(lops, T.level_rows[d], io.staged, dst, dstride, b);
-        } else {
-            // shared-memory source: level d + 1, or the staged rows of level G's children
-            const float* from = first ? io.staged : ((d & 1) ? buf0 : buf1);
-            level_rows<false, BC>(lops, T.level_rows[d], from, stride, dst, dstride, b);
-        }
-        cta_sync();
-    }
-    return ok;
 }
 
-// Global address of the root rows of a job in a stage output (row stride `rstride`).
-__device__ __forceinline__ float* root_rows_dst(const JobTree& T, int rstride, float* dst)
+// Level T.depth of a fused job: a warp computes all rows of one node from its 4 to 8 raw input
+// rows (row j of the transform at raw + j * b, no halo: a lane's window wraps at a column that
+// is the same for every row, so one offset per window column serves all rows).
+__device__ __forceinline__ void ffa_nodes_fused(const JobTree& T, const float* raw, float* dst,
+                                                int stride, int b)
 {
-    const Node r = T.nodes[0];
-    return dst + (size_t)(r.row0 + r.lo) * rstride;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nq = ffa_chunks(b);
+    const int lw = nq <= 8 ? 3 : nq <= 16 ? 4 : 5;
+    const int nblk = (nq + 31) >> 5;
+    const unsigned inv = (65536u + nblk - 1) / nblk;
+    const int nnodes = 1 << T.depth;
+    const int ntask = (nnodes * nblk + (32 >> lw) - 1) >> (5 - lw);
+    const int sub = lane >> lw, ql = lane & ((1 << lw) - 1);
+    const Node* lvl = T.nodes + nnodes - 1;
+    for (int task = warp; task < ntask; task += kWarps) {
+        int i = task, q = ql;
+        if (nblk > 1) {
+            i = (int)(((unsigned)task * inv) >> 16);
+            q += 32 * (task - i * nblk);
+        } else {
+            i = (task << (5 - lw)) + sub;
+        }
+        if (q >= nq || i >= nnodes) continue;
+        const int c0 = kLaneCols * q;
+        const int w0 = c0 < b ? c0 : c0 - b;
+        int off[kFusedWindow];
+#pragma unroll
+        for (int j = 0; j < kFusedWindow; ++j) off[j] = w0 + j - (w0 + j >= b ? b : 0);
+        const float* x = raw + (size_t)lvl[i].row0 * b;
+        float* out = dst + (size_t)lvl[i].off * stride + c0;
+        switch (lvl[i].rows) {
+            case 4: fused_node<4>(x, b, off, out, stride); break;
+            case 5: fused_node<5>(x, b, off, out, stride); break;
+            case 6: fused_node<6>(x, b, off, out, stride); break;
+            case 7: fused_node<7>(x, b, off, out, stride); break;
+            default: fused_node<8>(x, b, off, out, stride); break;
+        }
+    }
+}
+
+// Where a job's levels read.
+struct LevelIO {
+    const float* src = nullptr;     // global source: row j at src + j * src_stride (used when
+    size_t src_stride = 0;          // nothing is staged)
+    const float* staged = nullptr;  // source rows in shared memory
+    bool staged_rows = false;       // staged: true = rows of the layout in JobTree::src_off
+                                    // (stride = the level stride, with halo); false = raw row
+                                    // j at staged + j * b
+    uint64_t* bar = nullptr;        // staged by a bulk copy that completes on phase *phase of
+    uint32_t* phase = nullptr;      // bar (null: already in place)
+};
+
+// Runs all levels of the job; the operations are built (build_ops) and the CTA synchronised.
+// `src` is the level buffer that holds the staged source rows, `dst` the other one. Returns
+// the one that holds the root rows [lo, hi) (stride `stride`, row i of the buffer = root output
+// row lo + i). *ok is cleared if the wait for staged rows ran out.
+__device__ inline float* run_job_levels(const JobTree& T, int b, float* src, float* dst,
+                                        int stride, const uint4* ops, const LevelIO& io, bool* ok)
+{
+    if (io.bar) {
+        *ok = mbar_wait(io.bar, *io.phase);
+        *io.phase ^= 1u;
+    }
+    for (int d = T.depth; d > T.first_op; --d) {
+        const bool first = d == T.depth;
+        if (T.fused) {
+            ffa_nodes_fused(T, io.staged, dst, stride, b);
+        } else {
+            const float* from = src;
+            size_t fstride = stride;
+            if (first && !io.staged) {
+                from = io.src;
+                fstride = io.src_stride;
+            } else if (first && !io.staged_rows) {
+                from = io.staged;
+                fstride = b;
+            }
+            level_rows_direct(T, d, from, fstride, dst, stride, b);
+        }
+        cta_sync();
+        float* x = src;
+        src = dst;
+        dst = x;
+    }
+    for (int k = 0; k < T.nsteps; ++k) {
+        const Step st = T.steps[k];
+        if (st.two)
+            level_quads(ops + st.unit, st.count, src, dst, stride, b);
+        else
+            level_groups(ops + st.unit, st.count, src, dst, stride, b);
+        cta_sync();
+        float* x = src;
+        src = dst;
+        dst = x;
+    }
+    return src;
 }
 
 // Issued by one warp: bulk copies of the level-G source rows of a job laid out by
@@ -658,32 +853,36 @@ __device__ inline void stage_source_rows_async(const JobTree& T, const float* sr
     }
 }
 
-// Shared-memory layout of a CTA running FFA jobs: [fixed part][ops][buf0][buf1].
-// Rows per level buffer for `smem_bytes` with `fixed_bytes` already used.
-constexpr int kOpsPerCapRow = kMaxJobDepth + 1;  // row operations of all levels of a job
-
-RT_HD int ffa_cap_rows_for(size_t smem_bytes, size_t fixed_bytes, int b)
+// Shared-memory layout of a CTA running FFA jobs: [fixed part][operations][buffer][buffer].
+// Operations (in 16-byte units) of a job whose levels hold at most cap_rows rows. A node with L
+// rows wanted has at most L / 2 + 1 groups, and at most L / 2 + 1 rows wanted of its tail child
+// (t(s) = group_of) and so L / 4 + 3 / 2 quads. Levels 5 .. 0 by three passes of quads (two
+// units each) or by two and a single level: at most 3 cap_rows / 2 + 80 units; by single levels
+// (more than kRegularRows rows): 6 (cap_rows / 2) + 63.
+RT_HD int ffa_ops_units(int cap_rows, bool regular)
 {
-    const size_t per_row =
-        2 * (size_t)ffa_stride(b) * sizeof(float) + kOpsPerCapRow * sizeof(RowOp);
-    return (int)((smem_bytes - fixed_bytes - 64) / per_row);
+    return regular ? 3 * cap_rows / 2 + 80
+                   : (kMaxTreeDepth + 1) * ((cap_rows + 1) / 2) + (2 << kMaxTreeDepth);
 }
 
-struct FfaSmem {
-    RowOp* ops;
-    float* buf0;
-    float* buf1;
+struct FfaLayout {
+    int ops_units;     // room for operations, in 16-byte units
+    int buf_floats;    // floats per level buffer (a multiple of 16)
 };
 
-__device__ __forceinline__ FfaSmem ffa_smem(unsigned char* base, int cap_rows, int b)
+// Layout of `bytes` of shared memory for transforms of at least bmin bins and at most max_rows
+// rows: fixed by the smallest b, which has the most rows per level.
+RT_HD FfaLayout ffa_layout(size_t bytes, int bmin, size_t max_rows)
 {
-    FfaSmem L;
-    L.ops = reinterpret_cast<RowOp*>(base);
-    size_t off = ((size_t)cap_rows * kOpsPerCapRow * sizeof(RowOp) + 63) & ~size_t(63);
-    L.buf0 = reinterpret_cast<float*>(base + off);
-    L.buf1 = L.buf0 + (size_t)cap_rows * ffa_stride(b);
+    FfaLayout L;
+    const int most = (int)(bytes / (2 * sizeof(float) * ffa_stride(bmin)));
+    L.ops_units = (ffa_ops_units(most, max_rows <= (size_t)kRegularRows) + 3) & ~3;
+    L.buf_floats = (int)((bytes - (size_t)L.ops_units * 16) / (2 * sizeof(float))) & ~15;
     return L;
 }
+
+// Rows per level buffer.
+RT_HD int ffa_cap_rows(const FfaLayout& L, int b) { return L.buf_floats / ffa_stride(b); }
 
 // ------------------------------------------------------------------------------------
 // Host-side planning of the stages of one transform.
@@ -692,7 +891,7 @@ __device__ __forceinline__ FfaSmem ffa_smem(unsigned char* base, int cap_rows, i
 // computes the needed rows of nodes at depth D[k] from the outputs of depth D[k-1]; the
 // last stage has D = 0 (the root) and produces rows [0, rows_out).
 // ------------------------------------------------------------------------------------
-constexpr int kMaxStages = 4;
+constexpr int kMaxStages = 6;
 
 struct StagePlan {
     int nstages;
@@ -708,7 +907,8 @@ struct StagePlan {
 // rows, since kh, kt <= 1/2).
 // max_depth: the largest depth G of a job (G + 1 levels computed in shared memory); smaller
 // values cut deep transforms into more stages, whose outputs pass through L2.
-bool plan_stages(int m, int rows_out, int cap_rows, StagePlan* P, int max_depth = kMaxJobDepth);
+bool plan_stages(int m, int b, int rows_out, int cap_rows, StagePlan* P,
+                 int max_depth = kMaxJobDepth);
 // Job k of stage s of a transform (host or device).
 RT_HD void node_at(int m, int d, int i, int* row0, int* rows)
 {

@@ -149,35 +149,83 @@ int circular_prefix_sum(const float* x, size_t size, size_t nsum, float* out, cu
 // ------------------------------------------------------------------------------------
 constexpr size_t kStageTreeBytes = (sizeof(JobTree) + 255) & ~size_t(255);
 
-int ffa_cap_rows(int b) { return ffa_cap_rows_for(kFfaSmemBytes, kStageTreeBytes, b); }
+static FfaLayout stage_layout(int m, int b)
+{
+    return ffa_layout(kFfaSmemBytes - kStageTreeBytes, b, (size_t)m);
+}
+
+// Copies the source rows of a later-stage job (rows of b floats in global memory, laid out by
+// build_job_tree_warp) into `sbuf`, each with its halo.
+__device__ void stage_rows_halo(const JobTree& T, const float* __restrict__ src, int b, float* sbuf,
+                                int stride)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n = 1 << T.depth;
+    for (int r = warp; r < T.src_off[n]; r += kWarps) {
+        int lo = 0, hi = n - 1;  // node whose block holds staged row r
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (T.src_off[mid] <= r) lo = mid;
+            else hi = mid - 1;
+        }
+        const int4 rg = T.src_rng[lo];
+        const int k = r - T.src_off[lo];
+        const float* from = src + (size_t)(k < rg.y ? rg.x + k : rg.z + k - rg.y) * b;
+        float* to = sbuf + (size_t)r * stride;
+#pragma unroll 4
+        for (int c = lane; c < b + kHalo; c += 32) to[c] = __ldg(from + (c < b ? c : c % b));
+    }
+}
 
 __global__ void __launch_bounds__(kThreads, 1)
     k_ffa_stage(const float* __restrict__ src, float* __restrict__ dst, int m, int b,
-                int rows_out, StagePlan P, int stage, int cap_rows, int* err)
+                int rows_out, StagePlan P, int stage, FfaLayout L, int* err)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     JobTree& T = *reinterpret_cast<JobTree*>(smem);
-    const FfaSmem L = ffa_smem(smem + kStageTreeBytes, cap_rows, b);
+    uint4* ops = reinterpret_cast<uint4*>(smem + kStageTreeBytes);
+    float* buf0 = reinterpret_cast<float*>(ops + L.ops_units);
+    float* buf1 = buf0 + L.buf_floats;
     const int stride = ffa_stride(b);
     const JobSpec J = stage_job(m, rows_out, P, stage, blockIdx.x);
     if (J.hi <= J.lo) return;
-    build_job_tree(T, J, cap_rows);
+    LevelIO io;
+    io.src = src;
+    io.src_stride = b;
+    if (stage == 0) {
+        // raw input rows, as one block (it fits: no more rows than a level holds)
+        const float* from = src + (size_t)J.root_row0 * b;
+        const int n = J.root_rows * b;
+#pragma unroll 4
+        for (int i = threadIdx.x; i < n; i += kThreads) buf1[i] = __ldg(from + i);
+        io.staged = buf1 - (ptrdiff_t)J.root_row0 * b;
+    }
+    if (threadIdx.x < 32) build_job_tree_warp(T, J, b, ffa_cap_rows(L, b), L.ops_units, stage == 0);
+    cta_sync();
     if (T.error) {
         if (threadIdx.x == 0) atomicExch(err, RT_EINTERNAL);
         return;
     }
-    LevelIO io;
-    io.src = src;
-    io.src_stride = b;
-    io.root_dst = root_rows_dst(T, b, dst);
-    io.root_stride = b;
-    run_job_levels(T, b, L.buf0, L.buf1, stride, L.ops, io);
+    if (stage > 0 && T.pstaged) {
+        stage_rows_halo(T, src, b, buf1, stride);
+        io.staged = buf1;
+        io.staged_rows = true;
+    }
+    build_ops(T, b, ops);
+    cta_sync();
+    bool ok = true;
+    const float* root = run_job_levels(T, b, buf1, buf0, stride, ops, io, &ok);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int r = warp; r < J.hi - J.lo; r += kWarps) {
+        float* to = dst + (size_t)(J.root_row0 + J.lo + r) * b;
+        for (int c = lane; c < b; c += 32) to[c] = root[(size_t)r * stride + c];
+    }
 }
 
-bool plan_stages(int m, int rows_out, int cap_rows, StagePlan* P, int max_depth)
+bool plan_stages(int m, int b, int rows_out, int cap_rows, StagePlan* P, int max_depth)
 {
     memset(P, 0, sizeof(*P));
-    max_depth = std::max(0, std::min(max_depth, kMaxJobDepth));
+    max_depth = std::max(0, std::min(max_depth, max_full_depth(b)));
     if (m <= cap_rows && full_depth(m) <= max_depth) {
         P->nstages = 1;
         P->D[0] = 0;
@@ -200,7 +248,7 @@ bool plan_stages(int m, int rows_out, int cap_rows, StagePlan* P, int max_depth)
     while (D > 0) {
         if (ns >= kMaxStages) return false;
         // largest step e such that R = cap - 3 * 2^(e-1) stays >= cap / 2 (at least 1 level)
-        int e = std::min(D, max_depth + 1);
+        int e = std::min({D, max_depth + 1, kMaxTreeDepth + 1});
         int R = 0;
         for (; e >= 1; --e) {
             R = cap_rows - 3 * (1 << (e - 1));
@@ -224,9 +272,10 @@ bool plan_stages(int m, int rows_out, int cap_rows, StagePlan* P, int max_depth)
 int ffa_transform(const float* in, int m, int b, int rows_out, float* out, float* scratch,
                   int* d_err, cudaStream_t st)
 {
-    const int cap = ffa_cap_rows(b);
+    const FfaLayout L = stage_layout(m, b);
+    const int cap = ffa_cap_rows(L, b);
     StagePlan P;
-    if (cap < 4 || !plan_stages(m, rows_out, cap, &P))
+    if (cap < 4 || !plan_stages(m, b, rows_out, cap, &P))
         return set_error(RT_EINVAL, "FFA transform of %d x %d does not fit the device plan", m, b);
     if (P.nstages > 1 && scratch == nullptr)
         return set_error(RT_EINTERNAL, "FFA transform of %d x %d needs scratch memory", m, b);
@@ -236,7 +285,7 @@ int ffa_transform(const float* in, int m, int b, int rows_out, float* out, float
     for (int s = 0; s < P.nstages; ++s) {
         float* dst = (s == P.nstages - 1) ? out : scratch + (size_t)(s & 1) * m * b;
         k_ffa_stage<<<P.jobs[s], kThreads, kFfaSmemBytes, st>>>(src, dst, m, b, rows_out, P, s,
-                                                               cap, d_err);
+                                                               L, d_err);
         RT_TRY_CUDA(cudaGetLastError());
         src = dst;
     }
@@ -247,7 +296,7 @@ size_t ffa_scratch_floats(int m, int b)
 {
     // multi-stage plans (too many rows, or too deep for one job) need two scratch copies
     StagePlan P;
-    if (!plan_stages(m, m, ffa_cap_rows(b), &P) || P.nstages == 1) return 0;
+    if (!plan_stages(m, b, m, ffa_cap_rows(stage_layout(m, b), b), &P) || P.nstages == 1) return 0;
     return 2 * (size_t)m * b;
 }
 

@@ -8,7 +8,6 @@ namespace rt {
 // Dynamic shared memory of the FFA / S/N kernels (one CTA per SM).
 constexpr size_t kFfaSmemBytes = 226 * 1024;
 
-int ffa_cap_rows(int b);
 size_t ffa_scratch_floats(int m, int b);
 int detect_fast_widths(const int* w, int nw);
 const char* last_error();

@@ -156,7 +156,7 @@ __device__ __forceinline__ void window_max(const float* cr, int start, float (&m
 // Phases per thread of a TPR-thread profile for which the prefix passes are unrolled (the
 // thread's values held in registers): bins up to 264 with 8 threads, up to 544 with 16.
 template <int TPR>
-constexpr int snr_unrolled_phases() { return TPR == 8 ? 33 : 35; }
+__host__ __device__ constexpr int snr_unrolled_phases() { return TPR == 8 ? 33 : 35; }
 
 template <int TPR, int SB, bool kUnrolled>
 __device__ void snr_rows_impl(const float* X, int xs, int nrows, int b, const SnrParams& S,
@@ -316,5 +316,15 @@ RT_HD int prefix_stride(int b, int wmax, int tpr)
 }
 
 RT_HD int snr_tpr(int b) { return b <= 264 ? 8 : 16; }
+
+// Kinds of S/N code a kernel instance may hold, one bit each: 8 threads a profile, 16 threads
+// with the prefix passes unrolled, 16 threads with loops.
+enum : int { kSnr8 = 1, kSnr16 = 2, kSnr16Loop = 4 };
+
+RT_HD int snr_kind(int b, int tpr)
+{
+    if (tpr == 8) return kSnr8;  // at most 264 bins: always unrolled
+    return ((b + 15) / 16 | 1) <= snr_unrolled_phases<16>() ? kSnr16 : kSnr16Loop;
+}
 
 }  // namespace rt
