@@ -58,8 +58,6 @@ struct EngineArgs {
     const float* ds;         // downsampled series arena
     const float* norm;       // normalised series arena (cycles with f == 1)
     float* snrs;
-    double* periods;
-    uint32_t* foldbins;
     const XformRec* xforms;
     const WorkItem* items;
     long long nitems;
@@ -91,8 +89,7 @@ __device__ __forceinline__ int ld_acquire(const int* p)
     return v;
 }
 
-// Boxcar S/N and the period rows of a final-stage job's root rows (`root`); `work` is the
-// other level buffer.
+// Boxcar S/N of a final-stage job's root rows (`root`); `work` is the other level buffer.
 template <int TPR, bool kUnrolled>
 __device__ __forceinline__ void final_stage_outputs(const JobTree& T, const XformRec& X, const EngineArgs& A,
                                     const SnrParams& S, const float* root, float* work,
@@ -102,14 +99,27 @@ __device__ __forceinline__ void final_stage_outputs(const JobTree& T, const Xfor
     const int b = X.b;
     const int cs = prefix_stride(b, S.wmax, TPR);
     const int groups = A.layout.buf_floats / cs;
-    snr_rows_impl<TPR, 34, kUnrolled>(root, fstride, r.hi - r.lo, b, S, X.stdnoise,
-                                      A.snrs + ((size_t)X.out_row + r.lo) * S.nw, S.nw, work, cs,
-                                      groups);
-    double* per_out = A.periods + X.out_row;
-    uint32_t* fb_out = A.foldbins + X.out_row;
-    for (int s = r.lo + threadIdx.x; s < r.hi; s += kThreads) {
-        per_out[s] = trial_period(X.tau, b, s, X.m);
-        fb_out[s] = (uint32_t)b;
+    snr_rows_impl<TPR, 34, kUnrolled, false>(root, fstride, r.hi - r.lo, b, S, X.stdnoise,
+                                             A.snrs + ((size_t)X.out_row + r.lo) * S.nw, S.nw,
+                                             work, cs, groups);
+}
+
+// Trial periods and fold bins of every transform (periodogram.hpp:190-194), a warp per
+// transform. In the persistent kernel they were a tail of float64 divisions that two of the
+// fifteen compute warps ran while the others waited: 0.3 of 9.5 ms for 16 trials of 2^22
+// samples, against 15 us here.
+__global__ void __launch_bounds__(256) k_search_periods(const XformRec* __restrict__ xforms, int n,
+                                                        double* __restrict__ periods,
+                                                        uint32_t* __restrict__ foldbins)
+{
+    const int lane = threadIdx.x & 31;
+    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n;
+         i += (gridDim.x * blockDim.x) >> 5) {
+        const XformRec X = xforms[i];
+        for (int s = lane; s < X.rows_eval; s += 32) {
+            periods[X.out_row + s] = trial_period(X.tau, X.b, s, X.m);
+            foldbins[X.out_row + s] = (uint32_t)X.b;
+        }
     }
 }
 
@@ -122,6 +132,8 @@ constexpr int kEngineThreads = kThreads + 32;
 constexpr int kBarEmpty = 2;  // + slot
 constexpr int kBarRead = 4;   // the previous item's root rows have left their level buffer
 
+// A claimed work item. The scheduling warp keeps a pool of them: two handed to the compute
+// threads, the others waiting for a dependency or decoded ahead.
 struct ItemSlot {
     long long ticket;   // >= nitems: no more work
     int ok;             // 0: a wait failed, stop
@@ -129,9 +141,13 @@ struct ItemSlot {
     int root;           // set by the compute threads: level buffer (0, 1) of the root rows to
                         // store as a stage output, -1: nothing to store
     int stage, last, cap_rows, jobs_of_stage;
+    int target;         // the item may start once *dep reaches this value
+    const int* dep;     // (null: at once)
     JobSpec J;
     XformRec X;
 };
+constexpr int kParked = 4;            // items waiting for a dependency
+constexpr int kPool = 2 + kParked + 1;  // at most 16: parked entries are numbered in 4 bits
 
 __device__ __forceinline__ void named_sync(int id, int n)
 {
@@ -159,38 +175,34 @@ __device__ __forceinline__ unsigned warps_done_acquire(const unsigned* counter)
 
 // Completion of an item for the other CTAs: its stage counter and, after the last job of the
 // last stage, the release of the transform's scratch slot. Called by one thread after every
-// compute warp of the CTA has released the item (CTA scope); the fence makes their global
-// writes visible at GPU scope before the counters.
+// compute warp of the CTA has released the item (CTA scope) and its stage output is stored;
+// the fence makes their global writes visible at GPU scope before the counters.
 __device__ __forceinline__ void signal_item_done(const EngineArgs& A, const ItemSlot& P)
 {
     if (P.X.seq < 0 || !P.done_ok) return;
-    __threadfence();
     int* d = A.done + (size_t)P.X.seq * kMaxStages + P.stage;
+    if (!P.last) {
+        asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(d) : "memory");
+        return;
+    }
+    __threadfence();
     const int prev = atomicAdd(d, 1);
-    if (P.last && prev + 1 == P.jobs_of_stage) {
+    if (prev + 1 == P.jobs_of_stage) {
         __threadfence();
         atomicAdd(A.slot_release + (P.X.seq % kSlots), 1);
     }
 }
 
-// Scheduler-side view of a claimed item: its slot contents and its dependency.
-struct SchedItem {
-    ItemSlot slot;
-    const int* dep;     // counter to wait for (null: no dependency)
-    int target;         // ... until it reaches this value
-};
-
-__device__ __forceinline__ bool sched_ready(const SchedItem& it)
+__device__ __forceinline__ bool sched_ready(const ItemSlot& L)
 {
-    return it.dep == nullptr || ld_acquire(it.dep) >= it.target;
+    return L.dep == nullptr || ld_acquire(L.dep) >= L.target;
 }
 
-__device__ void sched_decode(const EngineArgs& A, long long t, SchedItem& it)
+__device__ __forceinline__ void sched_decode(const EngineArgs& A, long long t, ItemSlot& L)
 {
-    ItemSlot& L = it.slot;
     const WorkItem W = A.items[t];
     const XformRec X = A.xforms[W.xform];
-    const StagePlan P = A.plans[X.plan];
+    const StagePlan& P = A.plans[X.plan];
     const int stage = W.stage_job >> 24, job = W.stage_job & 0xffffff;
     const JobSpec J = stage_job(X.m, X.rows_eval, P, stage, job);
     L.ticket = t;
@@ -201,25 +213,21 @@ __device__ void sched_decode(const EngineArgs& A, long long t, SchedItem& it)
     L.last = stage == P.nstages - 1;
     L.jobs_of_stage = P.jobs[stage];
     L.cap_rows = X.tune & 0xffff;
-    it.dep = nullptr;
-    it.target = 0;
+    const int* dep = nullptr;
+    int target = 0;
     if (J.hi > J.lo && X.seq >= 0) {
         const int seq = X.seq;
         if (stage == 0) {
-            it.dep = A.slot_release + (seq % kSlots);
-            it.target = seq / kSlots;
+            dep = A.slot_release + (seq % kSlots);
+            target = seq / kSlots;
         } else {
-            it.dep = A.done + (size_t)seq * kMaxStages + stage - 1;
-            it.target = P.jobs[stage - 1] + A.dep_bias;
+            dep = A.done + (size_t)seq * kMaxStages + stage - 1;
+            target = P.jobs[stage - 1] + A.dep_bias;
         }
     }
+    L.dep = dep;
+    L.target = target;
 }
-
-// Hands the compute threads one ready item per slot. Items whose dependency is not met yet
-// are parked (up to kParked) while later tickets are tried, so a waiting stage does not stall
-// the CTA. Progress: the smallest unfinished ticket has all its dependencies finished (they
-// have smaller tickets), so whichever scheduler holds it hands it over; every wait is bounded.
-constexpr int kParked = 4;
 
 // The level buffer that an item's source rows are staged in: the one that does not hold the
 // root rows which the previous item leaves to be stored.
@@ -270,129 +278,175 @@ __device__ __forceinline__ void store_root_rows(const EngineArgs& A, const ItemS
              (size_t)(L.J.hi - L.J.lo) * fstride * sizeof(float));
 }
 
-__device__ void scheduler_warp(const EngineArgs& A, ItemSlot* slots, JobTree* trees,
-                               SnrParams* snr, unsigned* finished, unsigned char* smem,
-                               uint64_t* bar, uint64_t* full)
+// What the compute threads see of the scheduling warp.
+struct Handover {
+    ItemSlot pool[kPool + 1];    // the last entry: no more work
+    int item[2];              // pool entry of each slot's item
+    unsigned finished[2];     // compute warps done with the slot's item
+    unsigned long long full[2];  // mbarriers: the slot's item is ready
+    unsigned long long staged;   // mbarrier: the item's source rows have landed
+};
+
+// Hands the compute threads one ready item per slot. Items whose dependency is not met yet
+// are parked (up to kParked) while later tickets are tried, so a waiting stage does not stall
+// the CTA. Progress: the smallest unfinished ticket has all its dependencies finished (they
+// have smaller tickets), so whichever scheduler holds it hands it over; every wait is bounded.
+//
+// The compute threads need an item every ten thousand cycles or so, and a claim with the loads
+// behind it takes three to four thousand: the next ticket is claimed and decoded after an item
+// is handed over, while the compute threads run the one before (not near the end of the list,
+// where a ticket held ahead could have gone to an idle CTA).
+__device__ void scheduler_warp(const EngineArgs& A, Handover& H, JobTree* trees, SnrParams* snr,
+                               unsigned char* smem)
 {
     const int lane = threadIdx.x & 31;
-    SchedItem parked[kParked];
-    int nparked = 0;
+    uint64_t* bar = reinterpret_cast<uint64_t*>(&H.staged);
+    // lane 0: free pool entries; parked entries in order of their tickets, 4 bits each
+    unsigned free_mask = (1u << kPool) - 1, parked = 0;
+    int nparked = 0, ahead = -1;
     bool exhausted = false;
-    // items handed over whose completion is not signalled yet (lane 0): signalled as soon as
-    // every compute warp has released them, also while this warp waits for a dependency (an
-    // item it waits for may be the one running here); a stage output is stored first
-    bool pending[2] = {false, false};
-    auto finish = [&](int s) {
-        if (pending[s] && warps_done_acquire(finished + s) >= (unsigned)kWarps) {
-            if (slots[s].root >= 0) {
-                store_root_rows(A, slots[s], level_buffer(smem, A, slots[s].root));
-                bulk_s2g_wait_all();
-            }
-            signal_item_done(A, slots[s]);
-            pending[s] = false;
+    // items handed over whose completion is not signalled yet (lane 0), and whether their
+    // stage output is on its way: signalled as soon as every compute warp has released them,
+    // also while this warp waits for a dependency (an item it waits for may be the one here)
+    bool pending[2] = {false, false}, stored[2] = {false, false};
+    // signals an item that every compute warp has released
+    auto settle = [&](int i, bool is_stored) {
+        ItemSlot& L = H.pool[i];
+        if (L.root >= 0) {
+            if (!is_stored) store_root_rows(A, L, level_buffer(smem, A, L.root));
+            bulk_s2g_wait_all();
         }
+        signal_item_done(A, L);
+    };
+    auto claim = [&]() {  // a pool entry with the next item, -1: no more
+        const long long t = (long long)atomicAdd(A.ticket, 1ull);
+        if (t >= A.nitems) {
+            exhausted = true;
+            return -1;
+        }
+        const int i = __ffs(free_mask) - 1;
+        free_mask &= ~(1u << i);
+        sched_decode(A, t, H.pool[i]);
+        if (A.phase_cycles) atomicAdd(A.phase_cycles + 10, 1ull);
+        return i;
     };
     int k = 0;
     for (;; ++k) {
         const int s = k & 1;
         if (k >= 2) {
             named_sync(kBarEmpty + s, kEngineThreads);  // compute is done with item k-2
-            // ... and starts item k-1: its source rows, then the stage output of item k-2
-            stage_item(A, slots[s ^ 1], trees[s ^ 1],
-                       level_buffer(smem, A, staging_buffer(slots[s].root)), bar);
-            if (slots[s].root >= 0) {
-                if (lane == 0 && pending[s]) {
-                    store_root_rows(A, slots[s], level_buffer(smem, A, slots[s].root));
-                    bulk_s2g_wait_read();
-                }
+            // ... and starts item k-1: the stage output of item k-2 and the source rows of k-1
+            const ItemSlot& P = H.pool[H.item[s]];
+            if (lane == 0 && P.root >= 0 && !stored[s])
+                store_root_rows(A, P, level_buffer(smem, A, P.root));
+            stage_item(A, H.pool[H.item[s ^ 1]], trees[s ^ 1],
+                       level_buffer(smem, A, staging_buffer(P.root)), bar);
+            if (P.root >= 0) {
+                if (lane == 0 && !stored[s]) bulk_s2g_wait_read();
+                if (lane == 0) stored[s] = true;
                 __syncwarp();
                 named_arrive(kBarRead, kEngineThreads);
-                if (lane == 0 && pending[s]) {
-                    bulk_s2g_wait_all();
-                    signal_item_done(A, slots[s]);
-                    pending[s] = false;
-                }
             }
         }
+        int owed = -1;  // pool entry of item k-2 while it is not signalled
         if (lane == 0) {
-            finish(s);  // item k-2
-            ItemSlot& L = slots[s];
             const long long w0 = clock64();
-            bool chosen = false;
+            if (k >= 2 && pending[s]) owed = H.item[s];
+            else if (k >= 2) free_mask |= 1u << H.item[s];
+            int chosen = -1;
+            bool stop = false;
             unsigned ns = 32;
-            for (long long spin = 0; !chosen; ++spin) {
-                finish(s ^ 1);  // item k-1, running
-                for (int i = 0; i < nparked && !chosen; ++i) {
-                    if (sched_ready(parked[i])) {
-                        L = parked[i].slot;
-                        for (int q = i; q + 1 < nparked; ++q) parked[q] = parked[q + 1];
+            for (long long spin = 0; chosen < 0 && !stop; ++spin) {
+                for (int i = 0; i < nparked; ++i) {
+                    const int c = (parked >> (4 * i)) & 15;
+                    if (sched_ready(H.pool[c])) {
+                        chosen = c;
+                        const unsigned low = parked & ((1u << (4 * i)) - 1);
+                        parked = low | ((parked >> (4 * i + 4)) << (4 * i));
                         --nparked;
-                        chosen = true;
+                        break;
                     }
                 }
-                if (chosen) break;
-                if (ld_acquire(A.error) != RT_OK) exhausted = true;
-                if (!exhausted && nparked < kParked) {
-                    const long long t = (long long)atomicAdd(A.ticket, 1ull);
-                    if (t >= A.nitems) {
-                        exhausted = true;
-                    } else {
-                        SchedItem it;
-                        sched_decode(A, t, it);
-                        if (A.phase_cycles) atomicAdd(A.phase_cycles + 10, 1ull);
-                        if (sched_ready(it)) {
-                            L = it.slot;
-                            chosen = true;
-                        } else {
-                            if (A.phase_cycles)
-                                atomicAdd(A.phase_cycles + (it.slot.stage == 0 ? 8 : 9), 1ull);
-                            parked[nparked++] = it;
-                        }
+                if (chosen >= 0) break;
+                if (ahead < 0 && !exhausted && nparked < kParked) ahead = claim();
+                if (ahead >= 0) {
+                    if (sched_ready(H.pool[ahead])) {
+                        chosen = ahead;
+                        ahead = -1;
+                        break;
                     }
-                    continue;
+                    if (nparked < kParked) {
+                        if (A.phase_cycles)
+                            atomicAdd(A.phase_cycles + (H.pool[ahead].stage == 0 ? 8 : 9), 1ull);
+                        parked |= (unsigned)ahead << (4 * nparked++);
+                        ahead = -1;
+                        continue;
+                    }
                 }
-                if (exhausted && (nparked == 0 || ld_acquire(A.error) != RT_OK)) {
-                    L.ticket = A.nitems;  // no more work
-                    L.ok = 1;
-                    chosen = true;
-                    break;
+                if (owed >= 0) {
+                    settle(owed, stored[s]);
+                    free_mask |= 1u << owed;
+                    owed = -1;
                 }
-                if (spin > A.spin_limit) {
+                if (pending[s ^ 1] && warps_done_acquire(H.finished + (s ^ 1)) >= (unsigned)kWarps) {
+                    settle(H.item[s ^ 1], stored[s ^ 1]);  // item k-1
+                    stored[s ^ 1] = true;
+                    pending[s ^ 1] = false;
+                }
+                if (ld_acquire(A.error) != RT_OK) {
+                    stop = true;
+                } else if (exhausted && nparked == 0 && ahead < 0) {
+                    stop = true;
+                } else if (spin > A.spin_limit) {
                     atomicExch(A.error, RT_ETIMEOUT);
-                    L.ticket = A.nitems;
-                    L.ok = 0;
-                    chosen = true;
-                    break;
+                    stop = true;
+                } else if (exhausted || nparked == kParked) {
+                    if (A.phase_cycles) atomicAdd(A.phase_cycles + 11, 1ull);
+                    __nanosleep(ns);
+                    if (ns < 1024) ns <<= 1;
                 }
-                if (A.phase_cycles) atomicAdd(A.phase_cycles + 11, 1ull);
-                __nanosleep(ns);
-                if (ns < 1024) ns <<= 1;
             }
             if (A.phase_cycles) atomicAdd(A.phase_cycles + 7, (unsigned long long)(clock64() - w0));
-            L.done_ok = 1;
-            L.root = -1;
-            finished[s] = 0;
-            __threadfence_block();
+            if (stop) chosen = kPool;
+            H.pool[chosen].done_ok = 1;
+            H.pool[chosen].root = -1;
+            H.item[s] = chosen;
+            H.finished[s] = 0;
         }
         __syncwarp();
-        const bool stop = slots[s].ticket >= A.nitems || !slots[s].ok;
+        const ItemSlot& L = H.pool[H.item[s]];
+        const bool stop = !L.ok;
+        // the previous stage's output was written before the counter that lane 0 acquired; it
+        // is read by bulk copies
+        asm volatile("fence.proxy.async.global;" ::: "memory");
         // the job tree and boxcar coefficients of the item, prepared while the compute threads
         // run the previous item
-        if (!stop && slots[s].J.hi > slots[s].J.lo) {
-            build_job_tree_warp(trees[s], slots[s].J, slots[s].X.b, slots[s].cap_rows,
-                                A.layout.ops_units, slots[s].stage == 0);
-            if (slots[s].last) snr_params_fill_warp(snr[s], A.widths, A.nw, A.nfast, slots[s].X.b);
-            if (k == 0) stage_item(A, slots[0], trees[0], level_buffer(smem, A, staging_buffer(-1)), bar);
+        if (!stop && L.J.hi > L.J.lo) {
+            build_job_tree_warp(trees[s], L.J, L.X.b, L.cap_rows, A.layout.ops_units, L.stage == 0);
+            const bool fill = L.last && snr[s].b != L.X.b;
+            __syncwarp();
+            if (fill) snr_params_fill_warp(snr[s], A.widths, A.nw, A.nfast, L.X.b);
+            if (k == 0) stage_item(A, L, trees[0], level_buffer(smem, A, staging_buffer(-1)), bar);
         }
         __syncwarp();
-        if (lane == 0) mbar_arrive(full + s);
+        if (lane == 0) {
+            mbar_arrive(reinterpret_cast<uint64_t*>(H.full + s));
+            if (owed >= 0) {
+                settle(owed, stored[s]);
+                free_mask |= 1u << owed;
+            }
+            pending[s] = true;
+            stored[s] = false;
+            if (!stop && ahead < 0 && !exhausted && L.ticket + 8 * (long long)gridDim.x < A.nitems)
+                ahead = claim();
+        }
         if (stop) break;
-        if (lane == 0) pending[s] = true;
     }
     // the compute threads still hand back the slot of item k-1
     if (k >= 1) {
-        named_sync(kBarEmpty + ((k - 1) & 1), kEngineThreads);
-        if (lane == 0) finish((k - 1) & 1);
+        const int s = (k - 1) & 1;
+        named_sync(kBarEmpty + s, kEngineThreads);
+        if (lane == 0 && pending[s]) settle(H.item[s], stored[s]);
     }
 }
 
@@ -402,21 +456,23 @@ template <int KINDS>
 __global__ void __launch_bounds__(kEngineThreads, 1) k_search_persistent(EngineArgs A)
 {
     extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ ItemSlot slots[2];
+    __shared__ Handover H;
     __shared__ JobTree trees[2];
     __shared__ SnrParams snr[2];
-    __shared__ unsigned finished[2];
-    __shared__ __align__(8) uint64_t s_bar;     // completion of the bulk copy of a job's rows
-    __shared__ __align__(8) uint64_t s_full[2];  // slot handed to the compute threads
 
+    uint64_t* full = reinterpret_cast<uint64_t*>(H.full);
+    uint64_t* staged = reinterpret_cast<uint64_t*>(&H.staged);
     if (threadIdx.x == 0) {
-        mbar_init(&s_bar, 1);
-        mbar_init(s_full, 1);
-        mbar_init(s_full + 1, 1);
+        mbar_init(staged, 1);
+        mbar_init(full, 1);
+        mbar_init(full + 1, 1);
+        snr[0].b = snr[1].b = 0;
+        H.pool[kPool].ok = 0;
+        H.pool[kPool].ticket = A.nitems;
     }
     __syncthreads();
     if (threadIdx.x >= kThreads) {
-        scheduler_warp(A, slots, trees, snr, finished, smem, &s_bar, s_full);
+        scheduler_warp(A, H, trees, snr, smem);
         return;
     }
     uint4* ops = reinterpret_cast<uint4*>(smem);
@@ -435,12 +491,12 @@ __global__ void __launch_bounds__(kEngineThreads, 1) k_search_persistent(EngineA
         const int sl = k & 1;
         // the scheduling warp's own waits are bounded and it always hands a slot over: this
         // limit is far beyond them
-        if (!mbar_wait(s_full + sl, (k >> 1) & 1, 1ll << 40)) break;
+        if (!mbar_wait(full + sl, (k >> 1) & 1, 1ll << 40)) break;
         mark(kPhWait);
-        const ItemSlot& L = slots[sl];
+        ItemSlot& L = H.pool[H.item[sl]];
         const JobTree& T = trees[sl];
         const SnrParams& S = snr[sl];
-        if (L.ticket >= A.nitems || !L.ok) break;
+        if (!L.ok) break;
         const XformRec& X = L.X;
         const JobSpec& J = L.J;
         const int b = X.b;
@@ -474,7 +530,7 @@ __global__ void __launch_bounds__(kEngineThreads, 1) k_search_persistent(EngineA
                 io.staged_rows = true;
                 if (T.pstaged) io.staged = sbuf;
             }
-            if (staged_async(L, T)) io.bar = &s_bar;
+            if (staged_async(L, T)) io.bar = staged;
             failed = T.error != 0;
             mark(kPhTree);
             if (!failed) build_ops(T, b, ops);
@@ -500,14 +556,18 @@ __global__ void __launch_bounds__(kEngineThreads, 1) k_search_persistent(EngineA
                 mark(kPhLevels);
                 if (L.last) {
                     float* work = rows == sbuf ? other : sbuf;
-                    const int kind = KINDS == kSnr8 || KINDS == kSnr16
-                                         ? KINDS : snr_kind(b, X.tune >> 16);
-                    if ((KINDS & kSnr8) && kind == kSnr8)
+                    constexpr bool one = (KINDS & (KINDS - 1)) == 0;
+                    const int kind = one ? KINDS : snr_kind(b, X.tune >> 16);
+                    if ((KINDS & kSnr4) && kind == kSnr4)
+                        final_stage_outputs<4, true>(T, X, A, S, rows, work, fstride);
+                    else if ((KINDS & kSnr8) && kind == kSnr8)
                         final_stage_outputs<8, true>(T, X, A, S, rows, work, fstride);
                     else if ((KINDS & kSnr16) && kind == kSnr16)
                         final_stage_outputs<16, true>(T, X, A, S, rows, work, fstride);
-                    else if (KINDS & kSnr16Loop)
-                        final_stage_outputs<16, false>(T, X, A, S, rows, work, fstride);
+                    else if ((KINDS & kSnr32) && kind == kSnr32)
+                        final_stage_outputs<32, true>(T, X, A, S, rows, work, fstride);
+                    else if (KINDS & kSnr32Loop)
+                        final_stage_outputs<32, false>(T, X, A, S, rows, work, fstride);
                     mark(kPhSnr);
                 } else {
                     // the scheduling warp stores the root rows (bulk copy): make this thread's
@@ -523,11 +583,11 @@ __global__ void __launch_bounds__(kEngineThreads, 1) k_search_persistent(EngineA
         // hand the item back: the scheduling warp signals its completion to the other CTAs
         // once every compute warp has released it
         if (threadIdx.x == 0) {
-            slots[sl].root = root;
-            if (failed) slots[sl].done_ok = 0;
+            L.root = root;
+            if (failed) L.done_ok = 0;
         }
         __syncwarp();
-        if ((threadIdx.x & 31) == 0) warp_done_release(finished + sl);
+        if ((threadIdx.x & 31) == 0) warp_done_release(H.finished + sl);
         mark(kPhStore);
         named_arrive(kBarEmpty + sl, kEngineThreads);
     }
@@ -1256,7 +1316,9 @@ static int plan_build(SearchPlan& P)
         }
     };
 
-    P.layout = ffa_layout(kEngineDynBytes, (int)c.bins_min, P.max_len / c.bins_min);
+    // (the first cycle has the smallest factor, and so the most rows)
+    const size_t most_rows = C > 0 ? downsampled_size(P.max_len, P.f[0]) / c.bins_min : 0;
+    P.layout = ffa_layout(kEngineDynBytes, (int)c.bins_min, most_rows);
     size_t ds_total = 0;
     for (int t = 0; t < T; ++t) {
         const size_t N = P.lengths[t];
@@ -1294,8 +1356,9 @@ static int plan_build(SearchPlan& P)
                     break;
                 }
                 const int capr = std::max(4, (int)((double)cap_full * frac));
-                // S/N threads per profile: 8 where the register window allows it, unless tuned
-                const int tpr = (tune_tpr == 16) ? 16 : snr_tpr((int)b);
+                // S/N threads per profile: the default for these bins, or 16 where that is tuned
+                // and 16 segments hold a profile
+                const int tpr = (tune_tpr == 16 && b <= 16 * kSnrPhases) ? 16 : snr_tpr((int)b);
                 const auto key = std::make_pair((int)rows, (long long)re * 8192 + (long long)b);
                 int pi;
                 auto itp = plan_index.find(key);
@@ -1304,8 +1367,8 @@ static int plan_build(SearchPlan& P)
                     // a rule's level count that needs more stages than a plan holds falls back
                     // to the default depth
                     if (capr < 4 ||
-                        (!plan_stages((int)rows, (int)b, (int)re, capr, &sp, max_depth) &&
-                         !plan_stages((int)rows, (int)b, (int)re, capr, &sp)))
+                        (!plan_stages((int)rows, (int)b, (int)re, capr, kThreads / tpr, &sp, max_depth) &&
+                         !plan_stages((int)rows, (int)b, (int)re, capr, kThreads / tpr, &sp)))
                         return set_error(RT_EINVAL, "no device plan for a %zu x %zu transform", rows, b);
                     pi = (int)P.plans.size();
                     P.plans.push_back(sp);
@@ -1477,7 +1540,8 @@ static void (*search_kernel_for(int kinds))(EngineArgs)
 {
     if (kinds == kSnr8) return k_search_persistent<kSnr8>;
     if (kinds == kSnr16) return k_search_persistent<kSnr16>;
-    return k_search_persistent<kSnr8 | kSnr16 | kSnr16Loop>;
+    if (kinds == kSnr32) return k_search_persistent<kSnr32>;
+    return k_search_persistent<kSnr4 | kSnr8 | kSnr16 | kSnr32 | kSnr32Loop>;
 }
 
 static int engine_grid(void (*kernel)(EngineArgs))
@@ -1575,8 +1639,6 @@ static int plan_run(SearchPlan& P, const float* data, float* normalised_out, dou
     A.ds = P.d_ds;
     A.norm = zsrc;
     A.snrs = snrs;
-    A.periods = periods;
-    A.foldbins = foldbins;
     A.xforms = P.d_xforms;
     A.items = P.d_items;
     A.nitems = (long long)P.items.size();
@@ -1598,6 +1660,11 @@ static int plan_run(SearchPlan& P, const float* data, float* normalised_out, dou
     RT_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)kEngineDynBytes));
     if (A.nitems > 0) {
+        const int nx = (int)P.xforms.size();
+        k_search_periods<<<std::min((nx + 7) / 8, 148 * 8), 256, 0, st>>>(P.d_xforms, nx, periods,
+                                                                         foldbins);
+        RT_TRY_CUDA(cudaGetLastError());
+        launches += 1;
         kernel<<<engine_grid(kernel), kEngineThreads, kEngineDynBytes, st>>>(A);
         RT_TRY_CUDA(cudaGetLastError());
         launches += 1;

@@ -72,6 +72,9 @@ struct Node {
     int off;    // row of `lo` inside this level's shared buffer
     int goff;   // first row group of the node at its level
     int qoff;   // first row quad of the node at its level
+    int hbias, tbias;  // row r of the head / tail child is row hbias + r / tbias + r of the
+                       // level below's buffer, of the staged rows, or of the transform
+    int thr;    // last even row s with h(s) = s / 2 (odd rows: see head_row)
     float kh;   // head slope of the node (merge_coef)
 };
 
@@ -83,7 +86,9 @@ struct Step {
 
 struct JobTree {
     Node nodes[kMaxJobNodes];           // node i of level d at (1 << d) - 1 + i
-    int level_rows[kMaxTreeDepth + 1];  // rows stored for each level
+    int level_rows[kMaxTreeDepth + 1];    // rows stored for each level
+    int level_groups[kMaxTreeDepth + 1];  // row groups of each level
+    int level_tails[kMaxTreeDepth + 1];   // row groups of its tail children: quads a level up
     Step steps[kMaxTreeDepth + 1];      // levels first_op .. 0, deepest first
     int nsteps;
     int depth;                          // deepest level with a node list
@@ -127,156 +132,172 @@ RT_HD int max_full_depth(int b) { return b >= kWideMinBins ? kMaxJobDepth : kMax
 // share their tail row (t(s) = t(s + 1), and mostly their head row): for a node of n rows the
 // group of row s is (s + n % 2) / 2. For every n up to kRegularRows that number is t(s) itself,
 // and h(s) is t(s) (n even), t(s) - 1 (n odd, s odd), or one of the two (n odd, s even: t(s) up
-// to a middle row, t(s) - 1 beyond it): checked exhaustively by the CPU tests. Beyond that the
-// float32 slope may round a row to its neighbour, and only the row groups (which read each
-// row's own numbers) are used.
-constexpr int kRegularRows = 65536;
+// to the middle row n / 2 or the even row before it, t(s) - 1 beyond it): the CPU tests check
+// every n and s. From n = 8195 on the float32 slope moves that middle row, and only the row
+// groups (which read each row's own numbers) are used.
+constexpr int kRegularRows = 8192;
 RT_HD int group_of(int n, int s) { return (s + (n & 1)) >> 1; }
 
-// Builds the node lists of a job (one warp, no CTA barrier), level by level: node i of level d
-// is the head (i even) or tail (i odd) child of node i >> 1 of level d - 1, its row range
-// follows from the parent's by the head/tail row maps. `raw`: a stage-0 job (whole subtree over
-// raw input rows); otherwise the level-G source rows are laid out for staging (src_off,
-// pstaged): set when every level-G node has two children and the rows fit a level buffer.
+// h(s) of a node of at most kRegularRows rows, thr as in Node.
+__device__ __forceinline__ int head_row(const Node& nd, int s)
+{
+    return (s >> 1) - (int)((s > nd.thr) & ((s & 1) ^ 1));
+}
+
+// Node q of a job's node list in heap order (1: the root, 2 q and 2 q + 1: the head and tail
+// children of q): its row range follows from the root's by the head/tail row maps along the
+// path to it. Every lane of a warp walks to a node of its own.
+__device__ __forceinline__ Node walk_to_node(const JobSpec& J, int q, int maxdepth)
+{
+    Node nd;
+    nd.row0 = J.root_row0;
+    nd.rows = J.root_rows;
+    nd.lo = J.lo;
+    nd.hi = J.hi;
+    const int d = 31 - __clz(q);
+    for (int k = 0; k < maxdepth; ++k) {
+        if (k >= d) break;
+        const int tail = (q >> (d - 1 - k)) & 1;
+        const int mh = nd.rows >> 1;
+        const int n = tail ? nd.rows - mh : mh;
+        const float slope = __fdiv_rn((float)n - 1.0f, (float)nd.rows - 1.0f);  // merge_coef
+        nd.row0 += tail ? mh : 0;
+        nd.rows = n;
+        nd.lo = merge_row(slope, nd.lo);
+        nd.hi = merge_row(slope, nd.hi - 1) + 1;
+    }
+    nd.kh = merge_coef(nd.rows).kh;
+    const int half = (nd.rows >> 1) & ~1;
+    nd.thr = !(nd.rows & 1) ? 0x7fffffff : merge_row(nd.kh, half) == half >> 1 ? half : half - 2;
+    nd.hbias = nd.row0;
+    nd.tbias = nd.row0 + (nd.rows >> 1);
+    nd.off = nd.goff = nd.qoff = 0;
+    return nd;
+}
+
+// Builds the node lists of a job (one warp, no CTA barrier): every lane walks to its nodes (31
+// of levels 0 to 4, 32 of level 5), then the rows, groups and quads before each node in its
+// level come from one scan over all levels. Level by level, with a scan each, it took the
+// scheduling warp 6,600 cycles a job and kept the compute warps waiting.
+// `raw`: a stage-0 job (whole subtree over raw input rows); otherwise the level-G source rows
+// are laid out for staging (src_off, pstaged): set when every level-G node has two children and
+// the rows fit a level buffer.
 __device__ inline void build_job_tree_warp(JobTree& T, const JobSpec& J, int b, int cap_rows,
                                            int ops_units, bool raw)
 {
     const int lane = threadIdx.x & 31;
     const bool fused = raw && job_fused(J.G, b);
     const int depth = fused ? J.G - 2 : J.G;
-    const bool bad = depth > kMaxTreeDepth;
-    if (lane == 0) {
-        T.depth = depth;
-        T.fused = fused ? 1 : 0;
-        T.error = bad ? 1 : 0;
-        T.pstaged = 0;
-        T.first_op = depth - 1;
-    }
-    if (bad) {
+    if (depth > kMaxTreeDepth) {
+        if (lane == 0) T.error = 1;
         __syncwarp();
         return;
     }
-    Node nd;  // node `lane` of the current level
-    nd.row0 = J.root_row0;
-    nd.rows = J.root_rows;
-    nd.lo = J.lo;
-    nd.hi = J.hi;
-    nd.qoff = 0;
-    float kt = 0.f;  // tail slope of the node
-    int groups = 0, quads = 0;  // lane d: of level d
-    for (int d = 0; d <= depth; ++d) {
-        const int n = 1 << d, base = n - 1;
-        if (d > 0) {
-            Node p;
-            const int from = lane >> 1;
-            p.row0 = __shfl_sync(0xffffffffu, nd.row0, from);
-            p.rows = __shfl_sync(0xffffffffu, nd.rows, from);
-            p.lo = __shfl_sync(0xffffffffu, nd.lo, from);
-            p.hi = __shfl_sync(0xffffffffu, nd.hi, from);
-            const float pkh = __shfl_sync(0xffffffffu, nd.kh, from);
-            const float pkt = __shfl_sync(0xffffffffu, kt, from);
-            const int mh = p.rows >> 1;
-            const float k = (lane & 1) ? pkt : pkh;
-            nd.row0 = p.row0 + ((lane & 1) ? mh : 0);
-            nd.rows = (lane & 1) ? p.rows - mh : mh;
-            nd.lo = merge_row(k, p.lo);
-            nd.hi = merge_row(k, p.hi - 1) + 1;
-        }
-        const MergeCoef mc = merge_coef(nd.rows);
-        nd.kh = mc.kh;
-        kt = mc.kt;
-        // rows stored and row groups of the node, scanned together (both below 2^15); the
-        // fused level stores whole nodes
-        int v = 0;
-        if (lane < n) {
+    const bool regular = J.root_rows <= kRegularRows;
+    if (lane == 0) {
+        T.depth = depth;
+        T.fused = fused ? 1 : 0;
+        T.regular = regular ? 1 : 0;
+        T.error = 0;
+        T.pstaged = 0;
+    }
+    __syncwarp();
+    int first_op = b < kWideMinBins ? -1 : depth - 1;
+    for (int half = 0; half < (depth == kMaxTreeDepth ? 2 : 1); ++half) {
+        const int q = half ? 32 + lane : lane + 1;
+        const int d = 31 - __clz(q), i = q - (1 << d);  // level, node of the level
+        const bool live = d <= depth && d < (half ? 6 : 5);
+        Node nd = walk_to_node(J, live ? q : 1, depth);
+        // rows stored, row groups, and row groups of tail children (the quads of the level
+        // above) of the node, scanned together: 11, 10 and 10 bits. The fused level stores
+        // whole nodes.
+        unsigned v = 0;
+        if (live) {
             const int rows = (fused && d == depth) ? nd.rows : nd.hi - nd.lo;
-            const int grp = nd.hi > nd.lo
-                                ? group_of(nd.rows, nd.hi - 1) - group_of(nd.rows, nd.lo) + 1 : 0;
-            v = rows | (grp << 16);
+            const int grp = group_of(nd.rows, nd.hi - 1) - group_of(nd.rows, nd.lo) + 1;
+            v = rows | (grp << 11) | ((i & 1) ? (unsigned)grp << 21 : 0u);
         }
-        int incl = v;
+        unsigned incl = v;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += y;
+            const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (i >= o) incl += y;
         }
-        nd.off = (incl - v) & 0xffff;
-        nd.goff = (incl - v) >> 16;
-        if (lane < n) T.nodes[base + lane] = nd;
-        const int total = __shfl_sync(0xffffffffu, incl, 31);
-        if (lane == 0) {
-            T.level_rows[d] = total & 0xffff;
-            if ((total & 0xffff) > cap_rows) T.error = 2;
+        const unsigned excl = incl - v;
+        if (live) {
+            nd.off = excl & 0x7ff;
+            nd.goff = (excl >> 11) & 0x3ff;
+            T.nodes[q - 1] = nd;
+            if (i == (1 << d) - 1) {  // last node of the level
+                T.level_rows[d] = incl & 0x7ff;
+                T.level_groups[d] = (incl >> 11) & 0x3ff;
+                T.level_tails[d] = incl >> 21;
+                if ((int)(incl & 0x7ff) > cap_rows) T.error = 2;
+            }
         }
-        if (lane == d) groups = total >> 16;
-        if (d > 0) {
-            // the quads of a node of level d - 1 are the row groups of its tail child
-            const int odd = (lane & 1) ? v >> 16 : 0;
-            int qincl = odd;
+        __syncwarp();
+        if (live && d > 0) {
+            Node& parent = T.nodes[(q >> 1) - 1];
+            if (i & 1) {
+                parent.qoff = excl >> 21;
+                parent.tbias = nd.off - nd.lo;
+            } else {
+                parent.hbias = nd.off - nd.lo;
+            }
+        }
+        if (!raw && half == (depth == kMaxTreeDepth ? 1 : 0)) {
+            // rows each level-G node needs from its two children, as consecutive staged blocks
+            const bool mine = live && d == depth;
+            int v2 = 0;
+            bool two = true;
+            int4 rg = make_int4(0, 0, 0, 0);
+            if (mine) {
+                rg = make_int4(nd.row0, 0, nd.row0 + (nd.rows >> 1), 0);
+                two = nd.rows >= 2;
+                if (two) {
+                    const float kt = regular ? 0.f : merge_coef(nd.rows).kt;
+                    const int hlo = merge_row(nd.kh, nd.lo), hhi = merge_row(nd.kh, nd.hi - 1);
+                    const int tlo = regular ? group_of(nd.rows, nd.lo) : merge_row(kt, nd.lo);
+                    const int thi = regular ? group_of(nd.rows, nd.hi - 1) : merge_row(kt, nd.hi - 1);
+                    rg = make_int4(rg.x + hlo, hhi + 1 - hlo, rg.z + tlo, thi + 1 - tlo);
+                }
+                v2 = rg.y + rg.w;
+                T.src_rng[i] = rg;
+            }
+            int incl2 = v2;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, qincl, o);
-                if (lane >= o) qincl += y;
+                const int y = __shfl_up_sync(0xffffffffu, incl2, o);
+                if (i >= o) incl2 += y;
             }
-            if (lane < n && (lane & 1)) T.nodes[base - (n >> 1) + (lane >> 1)].qoff = qincl - odd;
-            const int qtotal = __shfl_sync(0xffffffffu, qincl, 31);
-            if (lane == d - 1) quads = qtotal;
-        }
-    }
-    if (!raw) {
-        // rows each level-G node needs from its two children, as consecutive staged blocks
-        const int n = 1 << depth;
-        int v = 0;
-        bool two = true;
-        if (lane < n) {
-            int4 rg = make_int4(nd.row0, 0, nd.row0 + (nd.rows >> 1), 0);
-            if (nd.rows < 2) {
-                two = false;
-            } else if (nd.hi > nd.lo) {
-                const int hlo = merge_row(nd.kh, nd.lo), tlo = merge_row(kt, nd.lo);
-                rg.x += hlo;
-                rg.y = merge_row(nd.kh, nd.hi - 1) + 1 - hlo;
-                rg.z += tlo;
-                rg.w = merge_row(kt, nd.hi - 1) + 1 - tlo;
+            if (mine) T.src_off[i] = incl2 - v2;
+            const int total = __shfl_sync(0xffffffffu, incl2, half ? 31 : (2 << depth) - 2);
+            const bool staged = __all_sync(0xffffffffu, two) && total <= cap_rows;
+            if (lane == 0) {
+                T.src_off[1 << depth] = total;
+                T.pstaged = staged ? 1 : 0;
             }
-            v = rg.y + rg.w;
-            T.src_rng[lane] = rg;
+            if (staged && mine) {
+                T.nodes[q - 1].hbias += incl2 - v2 - rg.x;
+                T.nodes[q - 1].tbias += incl2 - v2 + rg.y - rg.z;
+            }
+            if (staged && b >= kWideMinBins) first_op = depth;
         }
-        int incl = v;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += y;
-        }
-        if (lane < n) T.src_off[lane] = incl - v;
-        const int total = __shfl_sync(0xffffffffu, incl, 31);
-        two = __all_sync(0xffffffffu, two);
-        if (lane == 0) {
-            T.src_off[n] = total;
-            const bool staged = two && total <= cap_rows;
-            T.pstaged = staged ? 1 : 0;
-            if (staged) T.first_op = depth;
-        }
+        __syncwarp();
     }
-    __syncwarp();
     // the passes over levels first_op .. 0: two levels at a time from the deepest up, a single
     // one last when their number is odd
-    if (b < kWideMinBins && lane == 0) T.first_op = -1;
-    __syncwarp();
-    const bool regular = J.root_rows <= kRegularRows;
-    int ns = 0, unit = 0;
-    for (int d = T.first_op; d >= 0;) {
-        const bool two = d >= 1 && regular;
-        if (two) --d;
-        const int count = __shfl_sync(0xffffffffu, two ? quads : groups, d);
-        if (lane == 0) T.steps[ns] = Step{d, two ? 1 : 0, unit, count};
-        unit += two ? 2 * count : count;
-        ++ns;
-        --d;
-    }
     if (lane == 0) {
+        int ns = 0, unit = 0;
+        for (int d = first_op; d >= 0; --d) {
+            const bool two = d >= 1 && regular;
+            const int count = two ? T.level_tails[d] : T.level_groups[d];
+            if (two) --d;
+            T.steps[ns++] = Step{d, two ? 1 : 0, unit, count};
+            unit += two ? 2 * count : count;
+        }
+        T.first_op = first_op;
         T.nsteps = ns;
-        T.regular = regular ? 1 : 0;
         if (unit > ops_units) T.error = 3;
     }
     __syncwarp();
@@ -324,30 +345,15 @@ enum : unsigned {
 };
 static_assert(sizeof(GroupOp) == 16 && sizeof(QuadOp) == 32, "operations are read as 16-byte units");
 
-// Where row r of child `tail` (0 head, 1 tail) of node i of level d is found: its row in the
-// level below's buffer, in the staged rows (deepest level, pstaged), or of the transform.
-__device__ __forceinline__ int child_row(const JobTree& T, int d, int i, const Node& nd, int tail,
-                                         int r)
+// Source row numbers and shift of output row s of a node.
+__device__ __forceinline__ void source_rows(const JobTree& T, const Node& nd, int s, int* h, int* t,
+                                            int* shift)
 {
-    if (d < T.depth) {
-        const Node& c = T.nodes[(2 << d) - 1 + 2 * i + tail];
-        return c.off + r - c.lo;
-    }
-    const int row = nd.row0 + (tail ? (nd.rows >> 1) : 0) + r;
-    if (!T.pstaged) return row;
-    const int4 rg = T.src_rng[i];
-    return T.src_off[i] + (tail ? rg.y + row - rg.z : row - rg.x);
-}
-
-// Source row numbers and shift of output row s of node i of level d.
-__device__ __forceinline__ void source_rows(const JobTree& T, int d, int i, const Node& nd, int s,
-                                            int* h, int* t, int* shift)
-{
-    const int hs = merge_row(nd.kh, s);
+    const int hs = T.regular ? head_row(nd, s) : merge_row(nd.kh, s);
     const int ts = T.regular ? group_of(nd.rows, s) : merge_row(merge_coef(nd.rows).kt, s);
     *shift = s - ts;
-    *h = child_row(T, d, i, nd, 0, hs);
-    *t = child_row(T, d, i, nd, 1, ts);
+    *h = nd.hbias + hs;
+    *t = nd.tbias + ts;
 }
 
 // x mod b by one multiply-high, `inv` = ceil(2^32 / b): exact while x b < 2^32 (the shifts of a
@@ -374,7 +380,7 @@ __device__ inline GroupOp make_group(const JobTree& T, int d, int r, int b, unsi
     const int s1 = min(nd.hi - 1, 2 * q - (nd.rows & 1) + 1);
     GroupOp op;
     int h0, t0, sh0;
-    source_rows(T, d, lo, nd, s0, &h0, &t0, &sh0);
+    source_rows(T, nd, s0, &h0, &t0, &sh0);
     sh0 = T.regular ? mod_bins(sh0, b, inv) : sh0 % b;
     op.out = nd.off + s0 - nd.lo;
     op.h = h0;
@@ -382,7 +388,7 @@ __device__ inline GroupOp make_group(const JobTree& T, int d, int r, int b, unsi
     op.shift = sh0;
     if (s1 > s0) {
         int h1, t1, sh1;
-        source_rows(T, d, lo, nd, s1, &h1, &t1, &sh1);
+        source_rows(T, nd, s1, &h1, &t1, &sh1);
         sh1 = T.regular ? mod_bins(sh1, b, inv) : sh1 % b;
         op.h |= h1 << 16;
         op.t |= t1 << 16;
@@ -393,7 +399,7 @@ __device__ inline GroupOp make_group(const JobTree& T, int d, int r, int b, unsi
 }
 
 // Row quad r of level d (over level d + 1, whose rows are not stored).
-__device__ inline QuadOp make_quad(const JobTree& T, int d, int r, int b, unsigned inv)
+__device__ __forceinline__ QuadOp make_quad(const JobTree& T, int d, int r, int b, unsigned inv)
 {
     const Node* lvl = T.nodes + (1 << d) - 1;
     int i = 0, hi = (1 << d) - 1;  // node holding quad r (nodes sorted by qoff)
@@ -402,36 +408,32 @@ __device__ inline QuadOp make_quad(const JobTree& T, int d, int r, int b, unsign
         if (lvl[mid].qoff <= r) i = mid;
         else hi = mid - 1;
     }
-    const Node N = lvl[i];
-    const Node Hn = T.nodes[(2 << d) - 1 + 2 * i], Tn = T.nodes[(2 << d) + 2 * i];
+    const Node& N = lvl[i];
+    const Node& Hn = T.nodes[(2 << d) - 1 + 2 * i];
+    const Node& Tn = T.nodes[(2 << d) + 2 * i];
     const int p = N.rows & 1, pT = Tn.rows & 1;
-    const int gid = group_of(Tn.rows, Tn.lo) + (r - N.qoff);  // tail row of T_0 and T_1
-    const int t0 = 2 * gid - pT, s0 = 2 * t0 - p;             // T_0 and output row k = 0
+    const int gid = group_of(Tn.rows, Tn.lo) + (r - N.qoff);   // tail row of T_0 and T_1
+    const int t0 = 2 * gid - pT, s0 = 2 * t0 - p;              // T_0 and output row k = 0
     const int k0 = max(0, N.lo - s0), k1 = min(4, N.hi - s0);  // rows [k0, k1) are wanted
     const int hb = t0 - p;                                     // H_0
     const bool v0 = k0 == 0, v1 = k0 <= 1 && k1 > 1, v2 = k0 <= 2 && k1 > 2, v3 = k1 > 3;
-    const bool h1 = v1 && merge_row(N.kh, s0 + 1) != hb;      // k = 1 reads H_1
-    const bool h2 = v3 && merge_row(N.kh, s0 + 3) == hb + 2;  // k = 3 reads H_2
+    const bool h1 = v1 && p && 2 * t0 <= N.thr;      // k = 1 reads H_1: h(s0 + 1) = hb + 1
+    const bool h2 = v3 && p && 2 * t0 + 2 <= N.thr;  // k = 3 reads H_2: h(s0 + 3) = hb + 2
     const bool need0 = v0 || (v1 && !h1), need1 = h1 || v2 || (v3 && !h2);
     // a row that nothing reads stands in for another, so that every row number is valid
     const int r0 = need0 ? hb : need1 ? hb + 1 : hb + 2;
     const int r1 = need1 ? hb + 1 : r0;
     const int r2 = h2 ? hb + 2 : r0;
     const int u0 = (v0 || v1) ? t0 : t0 + 1, u1 = (v2 || v3) ? t0 + 1 : t0;
-    const int e = d + 1;
-    const int a0 = child_row(T, e, 2 * i, Hn, 0, merge_row(Hn.kh, r0));
-    const int a1 = child_row(T, e, 2 * i, Hn, 0, merge_row(Hn.kh, r1));
-    const int a2 = child_row(T, e, 2 * i, Hn, 0, merge_row(Hn.kh, r2));
     const int gB = group_of(Hn.rows, r0), gB2 = group_of(Hn.rows, r2);
-    const int b0 = child_row(T, e, 2 * i, Hn, 1, gB), b2 = child_row(T, e, 2 * i, Hn, 1, gB2);
-    const int c0 = child_row(T, e, 2 * i + 1, Tn, 0, merge_row(Tn.kh, u0));
-    const int c1 = child_row(T, e, 2 * i + 1, Tn, 0, merge_row(Tn.kh, u1));
-    const int d0 = child_row(T, e, 2 * i + 1, Tn, 1, gid);
+    const int a0 = Hn.hbias + head_row(Hn, r0), a1 = Hn.hbias + head_row(Hn, r1);
+    const int a2 = Hn.hbias + head_row(Hn, r2);
+    const int c0 = Tn.hbias + head_row(Tn, u0), c1 = Tn.hbias + head_row(Tn, u1);
     QuadOp op;
     op.a01 = a0 | (a1 << 16);
-    op.b0a2 = b0 | (a2 << 16);
-    op.b2c0 = b2 | (c0 << 16);
-    op.c1d0 = c1 | (d0 << 16);
+    op.b0a2 = (Hn.tbias + gB) | (a2 << 16);
+    op.b2c0 = (Hn.tbias + gB2) | (c0 << 16);
+    op.c1d0 = c1 | ((Tn.tbias + gid) << 16);
     op.sB = mod_bins(hb - gB, b, inv) | (mod_bins(r2 - gB2, b, inv) << 13);
     op.sCD = mod_bins(s0 - t0, b, inv) | (mod_bins(s0 - gid, b, inv) << 13);
     op.flags = (v0 ? 1u : 0) | (v1 ? 2u : 0) | (v2 ? 4u : 0) | (v3 ? 8u : 0) |
@@ -444,7 +446,7 @@ __device__ inline QuadOp make_quad(const JobTree& T, int d, int r, int b, unsign
 // Operations of all steps of the job, one thread per operation, dealt from the last thread down
 // (the boxcar S/N of the search's previous job keeps the first warps longest). Call after
 // build_job_tree_warp; the caller synchronises before using `ops`.
-__device__ inline void build_ops(const JobTree& T, int b, uint4* ops)
+__device__ __forceinline__ void build_ops(const JobTree& T, int b, uint4* ops)
 {
     const unsigned inv = 0xffffffffu / (unsigned)b + 1u;
     const int nsteps = T.nsteps;
@@ -655,12 +657,12 @@ __device__ __forceinline__ void level_rows_direct(const JobTree& T, int d, const
         const Node nd = lvl[lo];
         float* out = dst + (size_t)r * stride;
         if (nd.rows == 1) {
-            const int h = d < T.depth ? T.nodes[(2 << d) - 1 + 2 * lo].off : nd.row0;
+            const int h = nd.hbias;
             for (int c = lane; c < b + kHalo; c += 32) out[c] = src[(size_t)h * sstride + c % b];
             continue;
         }
         int h, t, shift;
-        source_rows(T, d, lo, nd, nd.lo + (r - nd.off), &h, &t, &shift);
+        source_rows(T, nd, nd.lo + (r - nd.off), &h, &t, &shift);
         const float *H = src + (size_t)h * sstride, *Tl = src + (size_t)t * sstride;
         for (int c = lane; c < b + kHalo; c += 32)
             out[c] = __fadd_rn(H[c % b], Tl[(c + shift) % b]);
@@ -821,15 +823,14 @@ __device__ inline float* run_job_levels(const JobTree& T, int b, float* src, flo
 
 // Issued by one warp: bulk copies of the level-G source rows of a job laid out by
 // build_job_tree_warp (pstaged), from a global source of 16-byte aligned rows of `stride`
-// floats into `sbuf` (same stride), completing on `bar` (one arrival with the byte count).
+// floats into `sbuf` (same stride), completing on `bar` (one arrival with the byte count). The
+// caller has ordered the source's writes before the copies (fence.proxy.async.global).
 __device__ inline void stage_source_rows_async(const JobTree& T, const float* src, int stride,
                                                float* sbuf, uint64_t* bar)
 {
     const int lane = threadIdx.x & 31;
     const int n = 1 << T.depth;
     const size_t row_bytes = (size_t)stride * sizeof(float);
-    // the source was written by other CTAs (generic proxy) before they signalled it
-    asm volatile("fence.proxy.async.global;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     if (lane == 0) mbar_arrive_expect_tx(bar, (uint32_t)(T.src_off[n] * row_bytes));
     __syncwarp();
@@ -865,6 +866,8 @@ RT_HD int ffa_ops_units(int cap_rows, bool regular)
                    : (kMaxTreeDepth + 1) * ((cap_rows + 1) / 2) + (2 << kMaxTreeDepth);
 }
 
+constexpr int kPadFloats = 256;
+
 struct FfaLayout {
     int ops_units;     // room for operations, in 16-byte units
     int buf_floats;    // floats per level buffer (a multiple of 16)
@@ -877,7 +880,9 @@ RT_HD FfaLayout ffa_layout(size_t bytes, int bmin, size_t max_rows)
     FfaLayout L;
     const int most = (int)(bytes / (2 * sizeof(float) * ffa_stride(bmin)));
     L.ops_units = (ffa_ops_units(most, max_rows <= (size_t)kRegularRows) + 3) & ~3;
-    L.buf_floats = (int)((bytes - (size_t)L.ops_units * 16) / (2 * sizeof(float))) & ~15;
+    // (kPadFloats behind the second buffer: the boxcar S/N reads past the end of its rows)
+    L.buf_floats = (int)((bytes - (size_t)L.ops_units * 16 - kPadFloats * sizeof(float)) /
+                         (2 * sizeof(float))) & ~15;
     return L;
 }
 
@@ -907,7 +912,8 @@ struct StagePlan {
 // rows, since kh, kt <= 1/2).
 // max_depth: the largest depth G of a job (G + 1 levels computed in shared memory); smaller
 // values cut deep transforms into more stages, whose outputs pass through L2.
-bool plan_stages(int m, int b, int rows_out, int cap_rows, StagePlan* P,
+// snr_rows: most rows of a last-stage job (0: no limit but cap_rows).
+bool plan_stages(int m, int b, int rows_out, int cap_rows, int snr_rows, StagePlan* P,
                  int max_depth = kMaxJobDepth);
 // Job k of stage s of a transform (host or device).
 RT_HD void node_at(int m, int d, int i, int* row0, int* rows)

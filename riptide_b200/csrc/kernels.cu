@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
 }
 
-bool plan_stages(int m, int b, int rows_out, int cap_rows, StagePlan* P, int max_depth)
+bool plan_stages(int m, int b, int rows_out, int cap_rows, int snr_rows, StagePlan* P, int max_depth)
 {
     memset(P, 0, sizeof(*P));
     max_depth = std::max(0, std::min(max_depth, max_full_depth(b)));
@@ -255,12 +255,17 @@ bool plan_stages(int m, int b, int rows_out, int cap_rows, StagePlan* P, int max
             if (R >= cap_rows / 2 || e == 1) break;
         }
         if (R < 1) return false;
+        // (the staged source rows of 1 to 3 levels can be two more than the bound of the levels)
+        if (e <= 3 && R > 4) R -= 2;
         const int Dn = D - e;
         const int node_rows = (m + (1 << Dn) - 1) >> Dn;
         const int need = (Dn == 0) ? rows_out : node_rows;
+        // the last stage's jobs hold no more rows than the boxcar S/N takes at a time
+        if (Dn == 0 && snr_rows > 0) R = std::min(R, snr_rows);
+        const int per_node = std::max(1, (need + R - 1) / R);
         P->D[ns] = Dn;
-        P->R[ns] = R;
-        P->jobs_per_node[ns] = std::max(1, (need + R - 1) / R);
+        P->R[ns] = std::max(1, (need + per_node - 1) / per_node);
+        P->jobs_per_node[ns] = per_node;
         P->jobs[ns] = P->jobs_per_node[ns] << Dn;
         ++ns;
         D = Dn;
@@ -275,7 +280,7 @@ int ffa_transform(const float* in, int m, int b, int rows_out, float* out, float
     const FfaLayout L = stage_layout(m, b);
     const int cap = ffa_cap_rows(L, b);
     StagePlan P;
-    if (cap < 4 || !plan_stages(m, b, rows_out, cap, &P))
+    if (cap < 4 || !plan_stages(m, b, rows_out, cap, 0, &P))
         return set_error(RT_EINVAL, "FFA transform of %d x %d does not fit the device plan", m, b);
     if (P.nstages > 1 && scratch == nullptr)
         return set_error(RT_EINTERNAL, "FFA transform of %d x %d needs scratch memory", m, b);
@@ -296,7 +301,7 @@ size_t ffa_scratch_floats(int m, int b)
 {
     // multi-stage plans (too many rows, or too deep for one job) need two scratch copies
     StagePlan P;
-    if (!plan_stages(m, b, m, ffa_cap_rows(stage_layout(m, b), b), &P) || P.nstages == 1) return 0;
+    if (!plan_stages(m, b, m, ffa_cap_rows(stage_layout(m, b), b), 0, &P) || P.nstages == 1) return 0;
     return 2 * (size_t)m * b;
 }
 
@@ -346,18 +351,17 @@ int snr2(const float* x, size_t rows, size_t cols, const int* d_widths, const in
     if (tile < 1) return set_error(RT_EINVAL, "profiles of %zu bins are too long", cols);
     const int grid = (int)std::min<size_t>((rows + tile - 1) / tile, 148 * 4);
     if (nw > kMaxWidths) return set_error(RT_EINVAL, "at most %d trial widths are supported", kMaxWidths);
-    const int tpr = snr_tpr((int)cols);
-    if (tpr == 8) {
-        RT_TRY_CUDA(cudaFuncSetAttribute(k_snr2<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)kFfaSmemBytes));
-        k_snr2<8><<<grid, kThreads, kFfaSmemBytes, st>>>(x, (int)rows, (int)cols, d_widths, nw,
-                                                         nfast, stdnoise, out, tile);
-    } else {
-        RT_TRY_CUDA(cudaFuncSetAttribute(k_snr2<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)kFfaSmemBytes));
-        k_snr2<16><<<grid, kThreads, kFfaSmemBytes, st>>>(x, (int)rows, (int)cols, d_widths, nw,
-                                                          nfast, stdnoise, out, tile);
+    void (*kernel)(const float*, int, int, const int*, int, int, float, float*, int);
+    switch (snr_tpr((int)cols)) {
+        case 4: kernel = k_snr2<4>; break;
+        case 8: kernel = k_snr2<8>; break;
+        case 16: kernel = k_snr2<16>; break;
+        default: kernel = k_snr2<32>; break;
     }
+    RT_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)kFfaSmemBytes));
+    kernel<<<grid, kThreads, kFfaSmemBytes, st>>>(x, (int)rows, (int)cols, d_widths, nw, nfast,
+                                                  stdnoise, out, tile);
     return check_cuda(cudaGetLastError(), "snr2");
 }
 

@@ -7,13 +7,18 @@
 //     S/N = ((h + beta) * dmax - beta * C[b-1]) / stdnoise
 // (snr.hpp:49-52; the reference build fuses the first product and the subtraction, which is
 // reproduced with __fmaf_rn). Everything below follows that arithmetic exactly; the only
-// change of order is the prefix sum: the TPR threads of a profile sum their segments (in
-// double), scan the segment totals and accumulate their running prefixes (in double-float
-// pairs), which is identical to the reference's sequential double sum whenever the sums are
-// exact (float inputs whose magnitudes within one profile span less than about 2^24).
+// change of order is the prefix sum: the TPR threads of a profile sum their segments, scan the
+// segment totals and accumulate their running prefixes, all in double, which is identical to
+// the reference's sequential double sum whenever the sums are exact (float inputs whose
+// magnitudes within one profile span less than about 2^29).
 //
 // Work split: TPR threads share one profile; each builds its segment of C, then holds a
-// window C[i .. i+SB+WMAX) in registers so that every width reads registers only.
+// window C[i .. i+SB+WMAX) in registers so that every width reads registers only. What bounds
+// it is the number of instructions (about 21 per phase, of which 12.5 are the differences and
+// maxima of the ten widths). A round of 60 profiles of 250 bins takes a CTA 6,800 cycles, of
+// which 2,500 are the window and 1,000 the double-precision prefixes; the prefix in double-float
+// pairs (eight float additions a value against one double addition and two conversions) and a
+// guard on every load and store made it 8,000.
 #pragma once
 #include "common.cuh"
 #include "ffa_core.cuh"
@@ -39,6 +44,7 @@ struct SnrParams {
     int nw;                  // number of trial widths
     int nfast;               // leading widths handled by the register window (0 or 10)
     int wmax;                // largest width
+    int b;                   // profile length the coefficients are for
     int w[kMaxWidths];
     float hb[kMaxWidths];    // h + beta (per width, for the current b)
     float beta[kMaxWidths];  // beta
@@ -61,6 +67,7 @@ __device__ inline void snr_params_fill(SnrParams& S, const int* widths, int nw, 
         int wm = 0;
         for (int k = 0; k < nw; ++k) wm = widths[k] > wm ? widths[k] : wm;
         S.wmax = wm;
+        S.b = b;
     }
     for (int k = threadIdx.x; k < nw; k += kThreads) {
         S.w[k] = widths[k];
@@ -80,34 +87,13 @@ __device__ inline void snr_params_fill_warp(SnrParams& S, const int* widths, int
         int wm = 0;
         for (int k = 0; k < nw; ++k) wm = widths[k] > wm ? widths[k] : wm;
         S.wmax = wm;
+        S.b = b;
     }
     for (int k = lane; k < nw; k += 32) {
         S.w[k] = widths[k];
         boxcar_coefs(b, widths[k], &S.hb[k], &S.beta[k]);
     }
     __syncwarp();
-}
-
-// Double-float accumulation (Knuth's TwoSum): (hi, lo) holds a sum exactly while it needs no
-// more than about 48 significant bits -- the float32 counterpart of the reference's double
-// accumulator (kernels.hpp:75-83), which is exact up to 53 bits. round(hi + lo) is then the
-// correctly rounded prefix, i.e. the reference's float(acc). Pure FP32 adds: no conversions.
-__device__ __forceinline__ void df_add(float& hi, float& lo, float x)
-{
-    const float s = __fadd_rn(hi, x);
-    const float bp = __fsub_rn(s, hi);
-    const float e = __fadd_rn(__fsub_rn(hi, __fsub_rn(s, bp)), __fsub_rn(x, bp));
-    hi = s;
-    lo = __fadd_rn(lo, e);
-}
-
-__device__ __forceinline__ void df_add2(float& hi, float& lo, float bhi, float blo)
-{
-    const float s = __fadd_rn(hi, bhi);
-    const float bp = __fsub_rn(s, hi);
-    const float e = __fadd_rn(__fsub_rn(hi, __fsub_rn(s, bp)), __fsub_rn(bhi, bp));
-    hi = s;
-    lo = __fadd_rn(__fadd_rn(lo, blo), e);
 }
 
 __device__ __forceinline__ float fmax3(float a, float b, float c)
@@ -148,108 +134,133 @@ __device__ __forceinline__ void window_max(const float* cr, int start, float (&m
     }
 }
 
+// Folds the N per-width maxima of TPR lanes by halves: at each step a lane keeps the maxima of
+// one half of its widths (the middle one of an odd number goes to both sides) and sends the
+// other half to its partner, until each lane holds the TPR-wide maxima of widths *k and up.
+// 2 N + ... instead of N log2(TPR) shuffles. Returns how many a lane holds at the end.
+template <int N, int OFF>
+__device__ __forceinline__ void fold_maxima(float (&mx)[FastWidths10::NW], unsigned mask, int t, int* k)
+{
+    if constexpr (OFF > 0) {
+        constexpr int KEEP = (N + 1) / 2, SKIP = N - KEEP;
+        const bool up = t & OFF;
+#pragma unroll
+        for (int i = 0; i < KEEP; ++i) {
+            const float send = up ? mx[i] : mx[i + SKIP];
+            const float keep = up ? mx[i + SKIP] : mx[i];
+            mx[i] = fmaxf(keep, __shfl_xor_sync(mask, send, OFF));
+        }
+        if (up) *k += SKIP;
+        fold_maxima<KEEP, OFF / 2>(mx, mask, t, k);
+    }
+}
+// Widths a lane holds after fold_maxima over TPR lanes.
+constexpr int folded_widths(int n, int tpr) { return tpr > 1 ? folded_widths((n + 1) / 2, tpr / 2) : n; }
+
+// Phases of a thread whose prefix passes are unrolled, the values held in registers: up to 264
+// bins with 8 threads, 528 with 16. (An odd number: the threads of a profile hit distinct banks.)
+constexpr int kSnrPhases = 33;
+RT_HD int snr_phases(int b, int tpr)
+{
+    return b <= tpr * kSnrPhases ? kSnrPhases : ((b + tpr - 1) / tpr) | 1;
+}
+
 // Boxcar S/N of `nrows` folded profiles (rows of X, stride xs) straight from the FFA output:
 // TPR threads per profile build its circular prefix sum (double accumulation, group scan) in
 // the scratch rows C (stride cs), then take the width maxima from a register window. Only
 // warp-level synchronisation: a profile's TPR threads are lanes of one warp. Writes
 // out[r * out_stride + k]. `groups` profiles are processed at a time (C holds `groups` rows).
-// Phases per thread of a TPR-thread profile for which the prefix passes are unrolled (the
-// thread's values held in registers): bins up to 264 with 8 threads, up to 544 with 16.
-template <int TPR>
-__host__ __device__ constexpr int snr_unrolled_phases() { return TPR == 8 ? 33 : 35; }
-
-template <int TPR, int SB, bool kUnrolled>
-__device__ void snr_rows_impl(const float* X, int xs, int nrows, int b, const SnrParams& S,
-                              float stdnoise, float* __restrict__ out, size_t out_stride,
-                              float* C, int cs, int groups)
+// kUnrolled: kSnrPhases phases per thread. kGuard: X must not be read past a row's end; without
+// it all TPR * kSnrPhases values from the row's start are read: anything may be past bin b - 1,
+// it only reaches prefix values past b - 1, which the wrap-around part replaces as far as they
+// are read.
+template <int TPR, int SB, bool kUnrolled, bool kGuard>
+__device__ __forceinline__ void snr_rows_impl(const float* X, int xs, int nrows, int b,
+                                              const SnrParams& S, float stdnoise,
+                                              float* __restrict__ out, size_t out_stride, float* C,
+                                              int cs, int groups)
 {
-    constexpr int PMAX = kUnrolled ? snr_unrolled_phases<TPR>() : 1;
+    constexpr int PMAX = kUnrolled ? kSnrPhases : 1, PH = (kSnrPhases + 1) / 2;
+    constexpr int NW = FastWidths10::NW;
     const int tid = threadIdx.x;
     const int g = tid / TPR, t = tid - g * TPR;
     const int ngroups = min(groups, kThreads / TPR);
-    const int P = ((b + TPR - 1) / TPR) | 1;  // odd: threads of a profile hit distinct banks
-    const int i0 = min(b, t * P), i1 = min(b, i0 + P);
+    const int P = kUnrolled ? kSnrPhases : snr_phases(b, TPR);
+    const int i0 = kGuard ? min(b, t * P) : t * P, i1 = min(b, t * P + P);
     const unsigned gmask = (TPR == 32) ? 0xffffffffu : (((1u << TPR) - 1u) << ((tid & 31) & ~(TPR - 1)));
     if (g >= ngroups) return;  // whole groups leave together
     float* cr = C + (size_t)g * cs;
     for (int r = g; r < nrows; r += ngroups) {
-        const float* xr = X + (size_t)r * xs;
-        // prefix sums (kernels.hpp:73-101): exact sums, float stores. The thread's segment
-        // total is summed in double (cheaper here than double-float pairs) and split into a
-        // double-float pair for the scan; the running prefix is accumulated in double-float.
-        // With at most PMAX phases per thread, the thread's values are loaded once into
-        // registers.
-        constexpr bool unrolled = kUnrolled;
+        const float* xr = X + (size_t)r * xs + i0;
+        // prefix sums (kernels.hpp:73-101): the thread's segment total (two halves, so that the
+        // additions form two chains), a scan of the totals, the running prefix of each half
         float v[PMAX];
-        double seg = 0.0;
-        if (unrolled) {
+        double s0 = 0.0, s1 = 0.0;
+        if (kUnrolled) {
 #pragma unroll
-            for (int j = 0; j < PMAX; ++j) v[j] = (j < i1 - i0) ? xr[i0 + j] : 0.0f;
+            for (int j = 0; j < PMAX; ++j) v[j] = (!kGuard || j < i1 - i0) ? xr[j] : 0.0f;
 #pragma unroll
-            for (int j = 0; j < PMAX; ++j) seg = __dadd_rn(seg, (double)v[j]);
+            for (int j = 0; j < PH; ++j) {
+                s0 = __dadd_rn(s0, (double)v[j]);
+                if (j + PH < PMAX) s1 = __dadd_rn(s1, (double)v[j + PH]);
+            }
         } else {
-            for (int i = i0; i < i1; ++i) seg = __dadd_rn(seg, (double)xr[i]);
+            const int n = max(0, i1 - i0);
+#pragma unroll 8
+            for (int j = 0; j < n; ++j) s0 = __dadd_rn(s0, (double)xr[j]);
         }
-        const float lh = __double2float_rn(seg);
-        const float ll = __double2float_rn(__dsub_rn(seg, (double)lh));
-        float ih = lh, il = ll;  // inclusive scan over the TPR segments
+        double incl = __dadd_rn(s0, s1);
 #pragma unroll
         for (int o = 1; o < TPR; o <<= 1) {
-            const float yh = __shfl_up_sync(gmask, ih, o, TPR);
-            const float yl = __shfl_up_sync(gmask, il, o, TPR);
-            if (t >= o) {
-                // (earlier segments) + (this range), in order of increasing phase
-                float nh = yh, nl = yl;
-                df_add2(nh, nl, ih, il);
-                ih = nh;
-                il = nl;
-            }
+            const double y = __shfl_up_sync(gmask, incl, o, TPR);
+            if (t >= o) incl = __dadd_rn(y, incl);
         }
-        float rh = __shfl_up_sync(gmask, ih, 1, TPR), rl = __shfl_up_sync(gmask, il, 1, TPR);
-        if (t == 0) rh = rl = 0.f;
-        if (unrolled) {
+        double run = __shfl_up_sync(gmask, incl, 1, TPR);
+        if (t == 0) run = 0.0;
+        float* c0 = cr + i0;
+        if (kUnrolled) {
+            double run1 = __dadd_rn(run, s0);
 #pragma unroll
-            for (int j = 0; j < PMAX; ++j) {
-                df_add(rh, rl, v[j]);  // adding the zero padding changes nothing stored
-                if (j < i1 - i0) cr[i0 + j] = __fadd_rn(rh, rl);
+            for (int j = 0; j < PH; ++j) {
+                run = __dadd_rn(run, (double)v[j]);
+                if (!kGuard || j < i1 - i0) c0[j] = __double2float_rn(run);
+                if (j + PH < PMAX) {
+                    run1 = __dadd_rn(run1, (double)v[j + PH]);
+                    if (!kGuard || j + PH < i1 - i0) c0[j + PH] = __double2float_rn(run1);
+                }
             }
         } else {
-            for (int i = i0; i < i1; ++i) {
-                df_add(rh, rl, xr[i]);
-                cr[i] = __fadd_rn(rh, rl);
+            const int n = max(0, i1 - i0);
+#pragma unroll 8
+            for (int j = 0; j < n; ++j) {
+                run = __dadd_rn(run, (double)xr[j]);
+                c0[j] = __double2float_rn(run);
             }
         }
-        const float th = __shfl_sync(gmask, ih, TPR - 1, TPR), tl = __shfl_sync(gmask, il, TPR - 1, TPR);
-        const float sumx = __fadd_rn(th, tl);
-        __syncwarp(gmask);
-        for (int j = t; j < S.wmax; j += TPR) cr[b + j] = __fadd_rn(cr[j], sumx);
         __syncwarp(gmask);
         const float sum = cr[b - 1];
-        float mx[FastWidths10::NW];
+        // the wrap-around part (it also replaces what unguarded tails left past bin b - 1)
+        for (int j = t; j < S.wmax; j += TPR) cr[b + j] = __fadd_rn(cr[j], sum);
+        __syncwarp(gmask);
+        float* orow = out + (size_t)r * out_stride;
+        if (S.nfast == NW) {
+            float mx[NW];
 #pragma unroll
-        for (int k = 0; k < FastWidths10::NW; ++k) mx[k] = -INFINITY;
-        if (S.nfast == FastWidths10::NW) {
-            if (b >= SB && P <= SB) {
+            for (int k = 0; k < NW; ++k) mx[k] = -INFINITY;
+            // (b > 42 >= SB: the fast widths end at 42)
+            if (kUnrolled) {
                 window_max<FastWidths10, SB>(cr, min(i0, b - SB), mx);
             } else {
-                for (int i = i0; i < i1; ++i)
-#pragma unroll
-                    for (int k = 0; k < FastWidths10::NW; ++k)
-                        mx[k] = fmaxf(mx[k], __fsub_rn(cr[i + FastWidths10::w(k)], cr[i]));
+#pragma unroll 1
+                for (int i = i0; i < i1; i += SB) window_max<FastWidths10, SB>(cr, min(i, b - SB), mx);
             }
-        }
+            int k0 = 0;
+            fold_maxima<NW, TPR / 2>(mx, gmask, t, &k0);
 #pragma unroll
-        for (int k = 0; k < FastWidths10::NW; ++k) {
-#pragma unroll
-            for (int o = TPR / 2; o > 0; o >>= 1)
-                mx[k] = fmaxf(mx[k], __shfl_xor_sync(gmask, mx[k], o, TPR));
-        }
-        float* orow = out + (size_t)r * out_stride;
-        for (int k = t; k < S.nfast; k += TPR) {
-            float dm = mx[0];
-#pragma unroll
-            for (int q = 1; q < FastWidths10::NW; ++q) dm = (k == q) ? mx[q] : dm;
-            orow[k] = __fdiv_rn(__fmaf_rn(S.hb[k], dm, -__fmul_rn(S.beta[k], sum)), stdnoise);
+            for (int q = 0; q < folded_widths(NW, TPR); ++q) {
+                const int k = k0 + q;
+                orow[k] = __fdiv_rn(__fmaf_rn(S.hb[k], mx[q], -__fmul_rn(S.beta[k], sum)), stdnoise);
+            }
         }
         // remaining widths (63 and 94 for bins_min 480), two at a time straight from shared
         // memory: each phase's C[i] is loaded once for both widths, eight phases per step
@@ -258,6 +269,7 @@ __device__ void snr_rows_impl(const float* X, int xs, int nrows, int b, const Sn
             const int w1 = S.w[k], w2 = two ? S.w[k + 1] : w1;
             float m1 = -INFINITY, m2 = -INFINITY;
             int i = i0;
+#pragma unroll 1
             for (; i + 8 <= i1; i += 8) {
                 float a[8], p[8], q[8];
 #pragma unroll
@@ -272,6 +284,7 @@ __device__ void snr_rows_impl(const float* X, int xs, int nrows, int b, const Sn
                     m2 = fmax3(m2, __fsub_rn(q[j], a[j]), __fsub_rn(q[j + 1], a[j + 1]));
                 }
             }
+#pragma unroll 1
             for (; i < i1; ++i) {
                 const float a = cr[i];
                 m1 = fmaxf(m1, __fsub_rn(cr[i + w1], a));
@@ -293,38 +306,45 @@ __device__ void snr_rows_impl(const float* X, int xs, int nrows, int b, const Sn
     }
 }
 
+// Profiles in global memory.
 template <int TPR, int SB>
 __device__ __forceinline__ void snr_rows(const float* X, int xs, int nrows, int b,
                                          const SnrParams& S, float stdnoise,
                                          float* __restrict__ out, size_t out_stride, float* C,
                                          int cs, int groups)
 {
-    if ((((b + TPR - 1) / TPR) | 1) <= snr_unrolled_phases<TPR>())
-        snr_rows_impl<TPR, SB, true>(X, xs, nrows, b, S, stdnoise, out, out_stride, C, cs, groups);
+    if (b <= TPR * kSnrPhases)
+        snr_rows_impl<TPR, SB, true, true>(X, xs, nrows, b, S, stdnoise, out, out_stride, C, cs, groups);
     else
-        snr_rows_impl<TPR, SB, false>(X, xs, nrows, b, S, stdnoise, out, out_stride, C, cs, groups);
+        snr_rows_impl<TPR, SB, false, true>(X, xs, nrows, b, S, stdnoise, out, out_stride, C, cs, groups);
 }
 
-// Row stride for prefix-sum rows: >= b + wmax and = TPR (mod 32), so that with an odd
-// per-thread phase count the TPR threads of a profile and the 32/TPR profiles of a warp read
-// distinct banks.
+// Row stride for prefix-sum rows: >= b + wmax and the whole segments of the TPR threads, and
+// = TPR (mod 32), so that with an odd per-thread phase count the TPR threads of a profile and
+// the 32/TPR profiles of a warp read distinct banks.
 RT_HD int prefix_stride(int b, int wmax, int tpr)
 {
-    int s = b + wmax;
+    const int seg = tpr * snr_phases(b, tpr);
+    int s = b + wmax > seg ? b + wmax : seg;
     s = (s + 31) & ~31;
     return s + tpr;
 }
 
-RT_HD int snr_tpr(int b) { return b <= 264 ? 8 : 16; }
+// Threads per profile: the fewest whose kSnrPhases phases each hold it, at least 4 (a window of
+// 33 phases costs 75 reads, one of half the phases 58: fewer threads with long segments read
+// and scan less), 32 beyond 1056 bins.
+RT_HD int snr_tpr(int b)
+{
+    return b <= 4 * kSnrPhases ? 4 : b <= 8 * kSnrPhases ? 8 : b <= 16 * kSnrPhases ? 16 : 32;
+}
 
-// Kinds of S/N code a kernel instance may hold, one bit each: 8 threads a profile, 16 threads
-// with the prefix passes unrolled, 16 threads with loops.
-enum : int { kSnr8 = 1, kSnr16 = 2, kSnr16Loop = 4 };
+// Kinds of S/N code a kernel instance may hold, one bit each: 4, 8, 16 or 32 threads a profile
+// with the prefix passes unrolled, 32 threads with loops.
+enum : int { kSnr4 = 1, kSnr8 = 2, kSnr16 = 4, kSnr32 = 8, kSnr32Loop = 16 };
 
 RT_HD int snr_kind(int b, int tpr)
 {
-    if (tpr == 8) return kSnr8;  // at most 264 bins: always unrolled
-    return ((b + 15) / 16 | 1) <= snr_unrolled_phases<16>() ? kSnr16 : kSnr16Loop;
+    return tpr < 32 ? tpr >> 2 : b <= 32 * kSnrPhases ? kSnr32 : kSnr32Loop;
 }
 
 }  // namespace rt

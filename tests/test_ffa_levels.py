@@ -20,21 +20,16 @@ def _rows(n):
             (kt * s + 0.5).astype(np.float32).astype(np.int64))
 
 
-@pytest.mark.parametrize("ns", [range(2, 3000), range(3000, 65537, 977),
-                                list(range(65520, 65537))])
-def test_row_pattern(ns):
-    for n in ns:
+def test_row_pattern():
+    # every node size for which the kernels use it (kRegularRows)
+    for n in range(2, 8193):
         h, t = _rows(n)
         s = np.arange(n)
         p = n & 1
         assert np.array_equal(t, (s + p) >> 1), n
-        if p == 0:
-            assert np.array_equal(h, t), n
-        else:
-            low = h == t  # even rows up to a middle one
-            assert np.array_equal(h[s % 2 == 1], t[s % 2 == 1] - 1), n
-            e = low[::2]
-            assert np.array_equal(h[::2], t[::2] - ~e) and not np.any(np.diff(e.astype(int)) > 0), n
+        half = (n >> 1) & ~1
+        thr = (half if h[half] == half // 2 else half - 2) if p else n
+        assert np.array_equal(h, (s >> 1) - ((s > thr) & (s % 2 == 0))), n
 
 
 EDGE_BINS = [2, 9, 16, 17, 18, 61, 62, 133, 134, 277, 278, 288, 289, 565, 566, 4096]
