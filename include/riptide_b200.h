@@ -35,6 +35,9 @@ extern "C" {
 const char* rt_last_error(void);
 /* Library version, 100 * major + minor. */
 int rt_version(void);
+/* Gives back the device memory (at most 512 MiB) that the library keeps for the scratch of
+ * later calls on the current device. */
+int rt_release_scratch(void);
 
 /* ---------------------------------------------------------------------------------
  * Drop-ins for the riptide.libcpp functions (device buffers).

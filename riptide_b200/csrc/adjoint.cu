@@ -305,7 +305,7 @@ extern "C" int rt_snr2_backward(const float* d_in, size_t rows, size_t cols,
     int wpb = (int)std::min<size_t>(8, (160 * 1024) / per_warp);
     if (wpb < 1) return set_error(RT_EINVAL, "profiles of %zu bins are too long", cols);
     int* d_w = nullptr;
-    RT_TRY_CUDA(cudaMallocAsync((void**)&d_w, std::max<size_t>(num_widths, 1) * sizeof(int), st));
+    RT_TRY_CUDA(scratch_malloc((void**)&d_w, std::max<size_t>(num_widths, 1) * sizeof(int), st));
     int s = check_cuda(cudaMemcpyAsync(d_w, w.data(), num_widths * sizeof(int),
                                        cudaMemcpyHostToDevice, st), "snr2_backward");
     const size_t smem = (size_t)wpb * per_warp;
@@ -340,8 +340,8 @@ extern "C" int rt_ffa2_transpose(const float* d_gout, size_t rows, size_t cols, 
                                           cudaMemcpyDeviceToDevice, st), "ffa2_transpose");
     TRow* d_tab = nullptr;
     float* tmp = nullptr;
-    RT_TRY_CUDA(cudaMallocAsync((void**)&d_tab, tabs.size() * sizeof(TRow), st));
-    int s = check_cuda(cudaMallocAsync((void**)&tmp, rows * cols * sizeof(float), st), "ffa2_transpose");
+    RT_TRY_CUDA(scratch_malloc((void**)&d_tab, tabs.size() * sizeof(TRow), st));
+    int s = check_cuda(scratch_malloc((void**)&tmp, rows * cols * sizeof(float), st), "ffa2_transpose");
     if (s == RT_OK)
         s = check_cuda(cudaMemcpyAsync(d_tab, tabs.data(), tabs.size() * sizeof(TRow),
                                        cudaMemcpyHostToDevice, st), "ffa2_transpose");
@@ -381,7 +381,7 @@ extern "C" int rt_normalise_adjoint(const float* d_g, const float* d_z, size_t s
     if (!(std_ > 0.0)) return set_error(RT_EINVAL, "std must be > 0");
     const int blocks = (int)std::min<size_t>((size + kNormBwdThreads - 1) / kNormBwdThreads, 512);
     double* part = nullptr;
-    RT_TRY_CUDA(cudaMallocAsync((void**)&part, (size_t)blocks * 2 * sizeof(double), st));
+    RT_TRY_CUDA(scratch_malloc((void**)&part, (size_t)blocks * 2 * sizeof(double), st));
     k_norm_adj_sums<<<blocks, kNormBwdThreads, 0, st>>>(d_g, d_z, size, part);
     int s = check_cuda(cudaGetLastError(), "normalise_adjoint");
     if (s == RT_OK) {

@@ -17,6 +17,12 @@ using namespace rt;
 extern "C" const char* rt_last_error(void) { return rt::last_error(); }
 extern "C" int rt_version(void) { return 100; }
 
+extern "C" int rt_release_scratch(void)
+{
+    rt::release_scratch();
+    return RT_OK;
+}
+
 extern "C" int rt_rollback(const float* d_x, size_t size, size_t shift, float* d_out,
                            void* stream)
 {
@@ -38,42 +44,23 @@ extern "C" int rt_circular_prefix_sum(const float* d_x, size_t size, size_t nsum
 // ------------------------------------------------------------------------------------
 // ffa2
 // ------------------------------------------------------------------------------------
-static int ffa2_impl(const float* d_in, size_t rows, size_t cols, float* d_out, cudaStream_t st,
-                     bool sync)
+extern "C" int rt_ffa2(const float* d_in, size_t rows, size_t cols, float* d_out, void* stream)
 {
+    cudaStream_t st = (cudaStream_t)stream;
     if (rows == 0 || cols == 0) return RT_OK;
     if (rows >= (1u << 24) || cols > 4096)
         return set_error(RT_EINVAL, "ffa2 input of %zu x %zu is larger than supported", rows, cols);
     const int m = (int)rows, b = (int)cols;
     float* scratch = nullptr;
-    int* d_err = nullptr;
     const size_t sf = ffa_scratch_floats(m, b);
-    RT_TRY_CUDA(cudaMallocAsync((void**)&d_err, sizeof(int), st));
-    RT_TRY_CUDA(cudaMemsetAsync(d_err, 0, sizeof(int), st));
     if (sf) {
-        cudaError_t e = cudaMallocAsync((void**)&scratch, sf * sizeof(float), st);
-        if (e != cudaSuccess) {
-            cudaFreeAsync(d_err, st);
-            return check_cuda(e, "ffa2 scratch");
-        }
+        const cudaError_t e = scratch_malloc((void**)&scratch, sf * sizeof(float), st);
+        if (e != cudaSuccess) return check_cuda(e, "ffa2 scratch");
     }
-    int s = ffa_transform(d_in, m, b, m, d_out, scratch, d_err, st);
-    int herr = 0;
-    if (s == RT_OK) {
-        cudaMemcpyAsync(&herr, d_err, sizeof(int), cudaMemcpyDeviceToHost, st);
-    }
+    // (the plan is checked on the host before any launch: nothing to read back)
+    const int s = ffa_transform(d_in, m, b, m, d_out, scratch, nullptr, st);
     if (scratch) cudaFreeAsync(scratch, st);
-    cudaFreeAsync(d_err, st);
-    if (s != RT_OK) return s;
-    (void)sync;
-    RT_TRY_CUDA(cudaStreamSynchronize(st));
-    if (herr) return set_error(RT_EINTERNAL, "ffa2 device plan check failed (%d)", herr);
-    return RT_OK;
-}
-
-extern "C" int rt_ffa2(const float* d_in, size_t rows, size_t cols, float* d_out, void* stream)
-{
-    return ffa2_impl(d_in, rows, cols, d_out, (cudaStream_t)stream, true);
+    return s;
 }
 
 extern "C" int rt_benchmark_ffa2(size_t rows, size_t cols, size_t loops, double* h_seconds)
@@ -140,14 +127,7 @@ extern "C" int rt_snr2(const float* d_in, size_t rows, size_t cols, const uint64
     RT_TRY(check_widths(h_widths, num_widths, cols, w));
     if (rows == 0 || num_widths == 0) return RT_OK;
     if (cols > 4096) return set_error(RT_EINVAL, "profiles longer than 4096 bins are not supported");
-    int* d_w = nullptr;
-    RT_TRY_CUDA(cudaMallocAsync((void**)&d_w, w.size() * sizeof(int), st));
-    cudaMemcpyAsync(d_w, w.data(), w.size() * sizeof(int), cudaMemcpyHostToDevice, st);
-    int s = rt::snr2(d_in, rows, cols, d_w, w.data(), (int)w.size(), stdnoise, d_out, st);
-    cudaFreeAsync(d_w, st);
-    if (s != RT_OK) return s;
-    RT_TRY_CUDA(cudaStreamSynchronize(st));  // h_widths staging must outlive the copy
-    return RT_OK;
+    return rt::snr2(d_in, rows, cols, w.data(), (int)w.size(), stdnoise, d_out, st);
 }
 
 // ------------------------------------------------------------------------------------
@@ -157,37 +137,17 @@ extern "C" size_t rt_downsampled_size(size_t size, double f) { return downsample
 
 static int downsample_one(const float* d_in, size_t size, double f, float* d_out, cudaStream_t st)
 {
-    // device-side descriptor arrays for one series, one factor
-    struct Hdr {
-        size_t in_off, len, out_off;
-        double f;
-        int use_seg;
-    };
-    Hdr h{0, size, 0, f, ds_use_segments(f) ? 1 : 0};
-    unsigned char* d = nullptr;
-    RT_TRY_CUDA(cudaMallocAsync((void**)&d, sizeof(Hdr), st));
-    RT_TRY_CUDA(cudaMemcpyAsync(d, &h, sizeof(Hdr), cudaMemcpyHostToDevice, st));
-    Hdr* dh = reinterpret_cast<Hdr*>(d);
-    DsJob job;
+    DsJob job{};
     job.in = d_in;
-    job.in_off = &dh->in_off;
-    job.lengths = &dh->len;
-    job.mean = nullptr;
-    job.norm = nullptr;
-    job.norm_out = nullptr;
-    job.f = &dh->f;
-    job.use_seg = &dh->use_seg;
+    job.one_len = size;
+    job.one_f = f;
     job.out = d_out;
-    job.out_off = &dh->out_off;
     job.ncycles = 1;
-    const int use_seg = h.use_seg, skip = 0;
+    const int use_seg = ds_use_segments(f) ? 1 : 0, skip = 0;
     job.use_seg_host = &use_seg;
     job.f_host = &f;
     job.skip_host = &skip;
-    int s = launch_downsample(job, 1, size, st);
-    cudaFreeAsync(d, st);
-    if (s == RT_OK) s = check_cuda(cudaStreamSynchronize(st), "downsample");
-    return s;
+    return launch_downsample(job, 1, size, st);
 }
 
 extern "C" int rt_downsample(const float* d_in, size_t size, double f, float* d_out,
@@ -208,15 +168,8 @@ extern "C" int rt_running_median(const float* d_in, size_t size, size_t width, f
     // running_median.hpp:103-107
     if (!(width % 2)) return set_error(RT_EINVAL, "width must be an odd number");
     if (!(width < size)) return set_error(RT_EINVAL, "width must be < size");
-    cudaStream_t st = (cudaStream_t)stream;
-    size_t* d = nullptr;
-    const size_t hv[2] = {size, 0};
-    RT_TRY_CUDA(cudaMallocAsync((void**)&d, sizeof(hv), st));
-    RT_TRY_CUDA(cudaMemcpyAsync(d, hv, sizeof(hv), cudaMemcpyHostToDevice, st));
-    int s = launch_running_median(d_in, d, d + 1, 1, size, (int)width, d_out, st);
-    cudaFreeAsync(d, st);
-    if (s == RT_OK) s = check_cuda(cudaStreamSynchronize(st), "running_median");
-    return s;
+    return launch_running_median(d_in, nullptr, nullptr, 1, size, (int)width, d_out,
+                                 (cudaStream_t)stream);
 }
 
 // ------------------------------------------------------------------------------------
@@ -330,16 +283,14 @@ extern "C" int rt_periodogram_plain(const float* d_data, size_t size, double tsa
     const size_t nds = (size_t)ceil(log(period_max / period_min) / log(ds_geo));
     const size_t bufsize = downsampled_size(size, ds_ini);
     float *input = nullptr, *ffaout = nullptr, *scratch = nullptr;
-    int *d_w = nullptr, *d_err = nullptr;
+    int* d_err = nullptr;
     size_t scratch_floats = 0;
     for (size_t b = bins_min; b <= bins_max && b <= bufsize; ++b)
         scratch_floats = std::max(scratch_floats, ffa_scratch_floats((int)(bufsize / b), (int)b));
-    RT_TRY_CUDA(cudaMallocAsync((void**)&input, std::max<size_t>(bufsize, 1) * sizeof(float), st));
-    RT_TRY_CUDA(cudaMallocAsync((void**)&ffaout, std::max<size_t>(bufsize, 1) * sizeof(float), st));
-    RT_TRY_CUDA(cudaMallocAsync((void**)&scratch, std::max<size_t>(scratch_floats, 1) * sizeof(float), st));
-    RT_TRY_CUDA(cudaMallocAsync((void**)&d_w, w.size() * sizeof(int), st));
-    RT_TRY_CUDA(cudaMallocAsync((void**)&d_err, sizeof(int), st));
-    RT_TRY_CUDA(cudaMemcpyAsync(d_w, w.data(), w.size() * sizeof(int), cudaMemcpyHostToDevice, st));
+    RT_TRY_CUDA(scratch_malloc((void**)&input, std::max<size_t>(bufsize, 1) * sizeof(float), st));
+    RT_TRY_CUDA(scratch_malloc((void**)&ffaout, std::max<size_t>(bufsize, 1) * sizeof(float), st));
+    RT_TRY_CUDA(scratch_malloc((void**)&scratch, std::max<size_t>(scratch_floats, 1) * sizeof(float), st));
+    RT_TRY_CUDA(scratch_malloc((void**)&d_err, sizeof(int), st));
     RT_TRY_CUDA(cudaMemsetAsync(d_err, 0, sizeof(int), st));
     int s = RT_OK;
     double* periods = d_periods;
@@ -367,7 +318,7 @@ extern "C" int rt_periodogram_plain(const float* d_data, size_t size, double tsa
             if (re == 0) continue;
             s = ffa_transform(in, (int)rows, (int)b, (int)rows, ffaout, scratch, d_err, st);
             if (s != RT_OK) break;
-            s = rt::snr2(ffaout, re, b, d_w, w.data(), (int)w.size(), stdnoise, snr, st);
+            s = rt::snr2(ffaout, re, b, w.data(), (int)w.size(), stdnoise, snr, st);
             if (s != RT_OK) break;
             s = launch_periods(periods, foldbins, re, tau, (int)b, rows, st);
             snr += re * w.size();
@@ -380,7 +331,6 @@ extern "C" int rt_periodogram_plain(const float* d_data, size_t size, double tsa
     cudaFreeAsync(input, st);
     cudaFreeAsync(ffaout, st);
     cudaFreeAsync(scratch, st);
-    cudaFreeAsync(d_w, st);
     cudaFreeAsync(d_err, st);
     if (s != RT_OK) return s;
     RT_TRY_CUDA(cudaStreamSynchronize(st));

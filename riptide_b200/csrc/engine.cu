@@ -597,10 +597,16 @@ __global__ void __launch_bounds__(kEngineThreads, 1) k_search_persistent(EngineA
 // Deredden / normalise (batched)
 // ------------------------------------------------------------------------------------
 struct TrialArrays {
-    const size_t* len;       // [T]
+    const size_t* len;       // [T]; null: one series, its lengths below and its offsets 0
     const size_t* off;       // [T] offsets into the packed series
     const size_t* lo_len;    // [T] scrunched lengths
     const size_t* lo_off;    // [T] offsets into the packed scrunched series
+    size_t one_len, one_lo_len;
+
+    __device__ size_t length(int t) const { return len ? len[t] : one_len; }
+    __device__ size_t offset(int t) const { return len ? off[t] : 0; }
+    __device__ size_t lo_length(int t) const { return len ? lo_len[t] : one_lo_len; }
+    __device__ size_t lo_offset(int t) const { return len ? lo_off[t] : 0; }
 };
 
 // ---- numpy's pairwise summation -----------------------------------------------------
@@ -773,9 +779,9 @@ __global__ void k_scrunch_batched(const float* __restrict__ x, TrialArrays A, in
     }
     __syncthreads();
     const int trial = blockIdx.y;
-    const size_t nl = A.lo_len[trial];
-    const float* xr = x + A.off[trial];
-    float* o = lores + A.lo_off[trial];
+    const size_t nl = A.lo_length(trial);
+    const float* xr = x + A.offset(trial);
+    float* o = lores + A.lo_offset(trial);
     const int lane = threadIdx.x & 31;
     const int grp = lane >> 3, c = lane & 7;
     const size_t w0 = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5;
@@ -837,9 +843,9 @@ __global__ void k_scrunch(const float* __restrict__ x, TrialArrays A, int k, int
     if (threadIdx.x == 0) pw_leaf_table(k, leaves);
     __syncthreads();
     const int trial = blockIdx.y;
-    const size_t nl = A.lo_len[trial];
-    const float* xr = x + A.off[trial];
-    float* o = lores + A.lo_off[trial];
+    const size_t nl = A.lo_length(trial);
+    const float* xr = x + A.offset(trial);
+    float* o = lores + A.lo_offset(trial);
     const int lane = threadIdx.x & 31;
     const int grp = lane >> 3, c = lane & 7;
     const size_t w0 = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5;
@@ -951,9 +957,9 @@ __global__ void k_interp_coef(TrialArrays A, int k, const float* __restrict__ rm
                               double2* __restrict__ coef)
 {
     const int trial = blockIdx.y;
-    const size_t nl = A.lo_len[trial];
-    const float* fp = rmed + A.lo_off[trial];
-    double2* c = coef + A.lo_off[trial];
+    const size_t nl = A.lo_length(trial);
+    const float* fp = rmed + A.lo_offset(trial);
+    double2* c = coef + A.lo_offset(trial);
     for (size_t j = blockIdx.x * (size_t)blockDim.x + threadIdx.x; j < nl;
          j += (size_t)gridDim.x * blockDim.x) {
         const double a = (double)fp[j];
@@ -974,12 +980,12 @@ __global__ void __launch_bounds__(kStatThreads)
             float* __restrict__ y, double* __restrict__ part, int blocks_per_trial)
 {
     const int trial = blockIdx.y;
-    const size_t N = A.len[trial];
-    const float* xr = x + A.off[trial];
-    float* yr = y + A.off[trial];
-    const float* fp = rmed + (k > 1 ? A.lo_off[trial] : A.off[trial]);
-    const double2* cf = coef + (k > 1 ? A.lo_off[trial] : 0);
-    const size_t nl = A.lo_len[trial];
+    const size_t N = A.length(trial);
+    const float* xr = x + A.offset(trial);
+    float* yr = y + A.offset(trial);
+    const float* fp = rmed + (k > 1 ? A.lo_offset(trial) : A.offset(trial));
+    const double2* cf = coef + (k > 1 ? A.lo_offset(trial) : 0);
+    const size_t nl = A.lo_length(trial);
     double s1 = 0.0, s2 = 0.0;
     const float shift = xr[0];
     float shift_y;
@@ -1061,8 +1067,8 @@ __global__ void __launch_bounds__(kStatThreads)
            int blocks_per_trial)
 {
     const int trial = blockIdx.y;
-    const size_t N = A.len[trial];
-    const float* xr = x + A.off[trial];
+    const size_t N = A.length(trial);
+    const float* xr = x + A.offset(trial);
     const float shift = xr[0];
     double s1 = 0.0, s2 = 0.0;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < N;
@@ -1091,8 +1097,7 @@ __global__ void __launch_bounds__(kStatThreads)
 }
 
 // mean and standard deviation per trial (population variance, ddof = 0).
-__global__ void k_stats(const double* __restrict__ part, const size_t* __restrict__ len,
-                        int blocks_per_trial, int ntrials, double* __restrict__ mean,
+__global__ void k_stats(const double* __restrict__ part, TrialArrays A, int blocks_per_trial, int ntrials, double* __restrict__ mean,
                         double* __restrict__ norm)
 {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1104,7 +1109,7 @@ __global__ void k_stats(const double* __restrict__ part, const size_t* __restric
         s2 += p[1];
         shift = p[2];
     }
-    const double N = (double)len[t];
+    const double N = (double)A.length(t);
     const double d = s1 / N;
     const double var = s2 / N - d * d;
     mean[t] = shift + d;
@@ -1117,10 +1122,10 @@ __global__ void k_interp_rmed(TrialArrays A, int k, const float* __restrict__ rm
                               double* __restrict__ out)
 {
     const int trial = blockIdx.y;
-    const size_t N = A.len[trial];
-    const float* fp = rmed + A.lo_off[trial];
-    const size_t nl = A.lo_len[trial];
-    double* o = out + A.off[trial];
+    const size_t N = A.length(trial);
+    const float* fp = rmed + A.lo_offset(trial);
+    const size_t nl = A.lo_length(trial);
+    double* o = out + A.offset(trial);
     const double half = 0.5 * (double)(k - 1);
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < N;
          i += (size_t)gridDim.x * blockDim.x) {
@@ -1151,9 +1156,9 @@ __global__ void k_normalise(const float* __restrict__ x, TrialArrays A, const do
                             const double* norm, float* __restrict__ z)
 {
     const int trial = blockIdx.y;
-    const size_t N = A.len[trial];
-    const float* xr = x + A.off[trial];
-    float* zr = z + A.off[trial];
+    const size_t N = A.length(trial);
+    const float* xr = x + A.offset(trial);
+    float* zr = z + A.offset(trial);
     const double m = mean[trial], s = norm[trial];
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < N;
          i += (size_t)gridDim.x * blockDim.x)
@@ -1470,8 +1475,13 @@ static int dalloc(SearchPlan& P, T** p, size_t n)
     if (P.alloc_fail_at > 0 && P.alloc_calls == P.alloc_fail_at)
         return set_error(RT_ENOMEM, "device allocation %d of the plan failed (injected)",
                          P.alloc_calls);
-    RT_TRY_CUDA(cudaMalloc((void**)p, n * sizeof(T)));
-    return RT_OK;
+    cudaError_t e = cudaMalloc((void**)p, n * sizeof(T));
+    if (e == cudaErrorMemoryAllocation) {  // without the scratch pool's kept memory, then
+        cudaGetLastError();
+        release_scratch();
+        e = cudaMalloc((void**)p, n * sizeof(T));
+    }
+    return check_cuda(e, "device allocation of the plan");
 }
 
 template <class T>
@@ -1560,7 +1570,7 @@ static int plan_run(SearchPlan& P, const float* data, float* normalised_out, dou
     RT_TRY(plan_prepare_device(P));
     const int T = (int)P.lengths.size();
     const int C = (int)P.f.size();
-    TrialArrays TA{P.d_len, P.d_off, P.d_lo_len, P.d_lo_off};
+    TrialArrays TA{P.d_len, P.d_off, P.d_lo_len, P.d_lo_off, 0, 0};
     const float* series = data;  // series before normalisation
     int launches = 0;
     if (P.timing) RT_TRY_CUDA(cudaEventRecord(P.ev[0], st));
@@ -1593,7 +1603,7 @@ static int plan_run(SearchPlan& P, const float* data, float* normalised_out, dou
     }
     const bool affine = !P.cfg.already_normalised;
     if (affine) {
-        k_stats<<<(T + 127) / 128, 128, 0, st>>>(P.d_part, P.d_len, P.stat_blocks, T, P.d_mean,
+        k_stats<<<(T + 127) / 128, 128, 0, st>>>(P.d_part, TA, P.stat_blocks, T, P.d_mean,
                                                  P.d_normv);
         RT_TRY_CUDA(cudaGetLastError());
         launches += 1;
@@ -1895,7 +1905,7 @@ static int plan_backward(SearchPlan& P, const float* d_z, const float* d_gsnr, f
     if (L == 0 || nw == 0) return RT_OK;
     // rows that carry a gradient
     unsigned long long *d_list = nullptr, *d_count = nullptr;
-    RT_TRY_CUDA(cudaMallocAsync((void**)&d_list, (max_rows + 1) * sizeof(unsigned long long), st));
+    RT_TRY_CUDA(scratch_malloc((void**)&d_list, (max_rows + 1) * sizeof(unsigned long long), st));
     d_count = d_list + max_rows;
     RT_TRY_CUDA(cudaMemsetAsync(d_count, 0, sizeof(unsigned long long), st));
     k_live_rows<<<(unsigned)std::min<size_t>((L + 255) / 256, 148 * 16), 256, 0, st>>>(
@@ -1981,7 +1991,7 @@ static int plan_backward(SearchPlan& P, const float* d_z, const float* d_gsnr, f
     const size_t bytes = groups.size() * sizeof(BwdGroup) + jobs.size() * sizeof(BwdJob) +
                          nwave * sizeof(int) + (gds_total + 4) * sizeof(float) +
                          (sig_total + 4) * sizeof(int) + 64;
-    RT_TRY_CUDA(cudaMallocAsync((void**)&blob, bytes, st));
+    RT_TRY_CUDA(scratch_malloc((void**)&blob, bytes, st));
     BwdGroup* d_groups = reinterpret_cast<BwdGroup*>(blob);
     BwdJob* d_jobs = reinterpret_cast<BwdJob*>(d_groups + groups.size());
     int* d_wave = reinterpret_cast<int*>(d_jobs + jobs.size());
@@ -2384,22 +2394,9 @@ extern "C" void rt_search_plan_destroy(rt_search_plan* plan)
 // ------------------------------------------------------------------------------------
 // Single-series deredden / normalise (TimeSeries.deredden / normalise, fast_running_median)
 // ------------------------------------------------------------------------------------
-namespace {
-struct OneSeries {
-    size_t v[4];  // len, off, lo_len, lo_off
-};
-}  // namespace
-
-static int one_series_arrays(size_t N, size_t nl, size_t** d, cudaStream_t st, TrialArrays* A)
+static TrialArrays one_series(size_t N, size_t nl)
 {
-    OneSeries h{{N, 0, nl, 0}};
-    RT_TRY_CUDA(cudaMallocAsync((void**)d, sizeof(h), st));
-    RT_TRY_CUDA(cudaMemcpyAsync(*d, &h, sizeof(h), cudaMemcpyHostToDevice, st));
-    A->len = *d;
-    A->off = *d + 1;
-    A->lo_len = *d + 2;
-    A->lo_off = *d + 3;
-    return RT_OK;
+    return TrialArrays{nullptr, nullptr, nullptr, nullptr, N, nl};
 }
 
 // width_samples / min_points -> (scrunch factor, running-median width, scrunched length)
@@ -2423,16 +2420,14 @@ extern "C" int rt_fast_running_median(const float* d_x, size_t size, size_t widt
     int k, w;
     size_t nl;
     RT_TRY(rmed_geometry(size, width_samples, min_points, &k, &w, &nl));
-    size_t* d = nullptr;
-    TrialArrays A;
-    RT_TRY(one_series_arrays(size, nl, &d, st, &A));
+    const TrialArrays A = one_series(size, nl);
     float *lores = nullptr, *rmed = nullptr;
     int s = RT_OK;
     if (k > 1) {
-        RT_TRY_CUDA(cudaMallocAsync((void**)&lores, nl * sizeof(float), st));
-        RT_TRY_CUDA(cudaMallocAsync((void**)&rmed, nl * sizeof(float), st));
+        RT_TRY_CUDA(scratch_malloc((void**)&lores, nl * sizeof(float), st));
+        RT_TRY_CUDA(scratch_malloc((void**)&rmed, nl * sizeof(float), st));
         s = launch_scrunch(d_x, A, k, 1, nl, lores, st);
-        if (s == RT_OK) s = launch_running_median(lores, A.lo_len, A.lo_off, 1, nl, w, rmed, st);
+        if (s == RT_OK) s = launch_running_median(lores, nullptr, nullptr, 1, nl, w, rmed, st);
         if (s == RT_OK) {
             k_interp_rmed<<<dim3(std::max(1, (int)std::min<size_t>((size + 255) / 256, 4096)), 1), 256, 0, st>>>(
                 A, k, rmed, d_out);
@@ -2440,18 +2435,16 @@ extern "C" int rt_fast_running_median(const float* d_x, size_t size, size_t widt
         }
     } else {
         // no scrunching: the exact running median (float32), widened to float64
-        RT_TRY_CUDA(cudaMallocAsync((void**)&rmed, size * sizeof(float), st));
-        s = launch_running_median(d_x, A.len, A.off, 1, size, w, rmed, st);
+        RT_TRY_CUDA(scratch_malloc((void**)&rmed, size * sizeof(float), st));
+        s = launch_running_median(d_x, nullptr, nullptr, 1, size, w, rmed, st);
         if (s == RT_OK) {
             k_interp_rmed<<<dim3(std::max(1, (int)std::min<size_t>((size + 255) / 256, 4096)), 1), 256, 0, st>>>(
-                TrialArrays{A.len, A.off, A.len, A.off}, 1, rmed, d_out);
+                one_series(size, size), 1, rmed, d_out);
             s = check_cuda(cudaGetLastError(), "fast_running_median");
         }
     }
     if (lores) cudaFreeAsync(lores, st);
     if (rmed) cudaFreeAsync(rmed, st);
-    cudaFreeAsync(d, st);
-    if (s == RT_OK) s = check_cuda(cudaStreamSynchronize(st), "fast_running_median");
     return s;
 }
 
@@ -2464,29 +2457,27 @@ extern "C" int rt_deredden(const float* d_x, size_t size, double tsamp, double w
     int k, w;
     size_t nl;
     RT_TRY(rmed_geometry(size, (size_t)ws, min_points, &k, &w, &nl));
-    size_t* d = nullptr;
-    TrialArrays A;
-    RT_TRY(one_series_arrays(size, nl, &d, st, &A));
+    const TrialArrays A = one_series(size, nl);
     float *lores = nullptr, *rmed = nullptr;
     double2* coef = nullptr;
     double* part = nullptr;
     int s = RT_OK;
     const int blocks = 64;
-    RT_TRY_CUDA(cudaMallocAsync((void**)&part, blocks * 3 * sizeof(double), st));
+    RT_TRY_CUDA(scratch_malloc((void**)&part, blocks * 3 * sizeof(double), st));
     if (k > 1) {
-        RT_TRY_CUDA(cudaMallocAsync((void**)&lores, nl * sizeof(float), st));
-        RT_TRY_CUDA(cudaMallocAsync((void**)&rmed, nl * sizeof(float), st));
-        RT_TRY_CUDA(cudaMallocAsync((void**)&coef, nl * sizeof(double2), st));
+        RT_TRY_CUDA(scratch_malloc((void**)&lores, nl * sizeof(float), st));
+        RT_TRY_CUDA(scratch_malloc((void**)&rmed, nl * sizeof(float), st));
+        RT_TRY_CUDA(scratch_malloc((void**)&coef, nl * sizeof(double2), st));
         s = launch_scrunch(d_x, A, k, 1, nl, lores, st);
-        if (s == RT_OK) s = launch_running_median(lores, A.lo_len, A.lo_off, 1, nl, w, rmed, st);
+        if (s == RT_OK) s = launch_running_median(lores, nullptr, nullptr, 1, nl, w, rmed, st);
         if (s == RT_OK) {
             k_interp_coef<<<dim3((unsigned)std::min<size_t>((nl + 255) / 256, 1024), 1), 256, 0, st>>>(
                 A, k, rmed, coef);
             s = check_cuda(cudaGetLastError(), "deredden");
         }
     } else {
-        RT_TRY_CUDA(cudaMallocAsync((void**)&rmed, size * sizeof(float), st));
-        s = launch_running_median(d_x, A.len, A.off, 1, size, w, rmed, st);
+        RT_TRY_CUDA(scratch_malloc((void**)&rmed, size * sizeof(float), st));
+        s = launch_running_median(d_x, nullptr, nullptr, 1, size, w, rmed, st);
     }
     if (s == RT_OK) {
         k_dered<<<dim3(blocks, 1), kStatThreads, 0, st>>>(d_x, A, k, div_magic(2u * (unsigned)k),
@@ -2497,8 +2488,6 @@ extern "C" int rt_deredden(const float* d_x, size_t size, double tsamp, double w
     if (lores) cudaFreeAsync(lores, st);
     if (rmed) cudaFreeAsync(rmed, st);
     cudaFreeAsync(part, st);
-    cudaFreeAsync(d, st);
-    if (s == RT_OK) s = check_cuda(cudaStreamSynchronize(st), "deredden");
     return s;
 }
 
@@ -2506,21 +2495,17 @@ extern "C" int rt_normalise(const float* d_x, size_t size, float* d_out, void* s
 {
     cudaStream_t st = (cudaStream_t)stream;
     if (size == 0) return RT_OK;
-    size_t* d = nullptr;
-    TrialArrays A;
-    RT_TRY(one_series_arrays(size, 0, &d, st, &A));
+    const TrialArrays A = one_series(size, 0);
     double* part = nullptr;
     const int blocks = 64;
-    RT_TRY_CUDA(cudaMallocAsync((void**)&part, (blocks * 3 + 2) * sizeof(double), st));
+    RT_TRY_CUDA(scratch_malloc((void**)&part, (blocks * 3 + 2) * sizeof(double), st));
     double* mean = part + blocks * 3;
     double* norm = mean + 1;
     k_sums<<<dim3(blocks, 1), kStatThreads, 0, st>>>(d_x, A, part, blocks);
-    k_stats<<<1, 32, 0, st>>>(part, A.len, blocks, 1, mean, norm);
+    k_stats<<<1, 32, 0, st>>>(part, A, blocks, 1, mean, norm);
     k_normalise<<<dim3(std::max(1, (int)std::min<size_t>((size + 255) / 256, 4096)), 1), 256, 0, st>>>(
         d_x, A, mean, norm, d_out);
     int s = check_cuda(cudaGetLastError(), "normalise");
     cudaFreeAsync(part, st);
-    cudaFreeAsync(d, st);
-    if (s == RT_OK) s = check_cuda(cudaStreamSynchronize(st), "normalise");
     return s;
 }

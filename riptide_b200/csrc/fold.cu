@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "kernels.cuh"
 
 namespace rt {
 
@@ -185,7 +186,7 @@ extern "C" int rt_fold_batched(const float* d_in, size_t size, double tsamp,
     }
     if (most == 0) return RT_OK;
     FoldJob* d_jobs = nullptr;
-    RT_TRY_CUDA(cudaMallocAsync((void**)&d_jobs, count * sizeof(FoldJob), stream));
+    RT_TRY_CUDA(scratch_malloc((void**)&d_jobs, count * sizeof(FoldJob), stream));
     cudaError_t e = cudaMemcpyAsync(d_jobs, jobs.data(), count * sizeof(FoldJob),
                                     cudaMemcpyHostToDevice, stream);
     if (e == cudaSuccess) {

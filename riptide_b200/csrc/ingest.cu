@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "kernels.cuh"
 
 namespace rt {
 
@@ -198,7 +199,7 @@ extern "C" int rt_ingest_files(const char* const* paths, const uint64_t* offsets
         if (e != cudaSuccess) fail_cuda(e, "cudaEventCreateWithFlags");
     }
     if (status == RT_OK && any8) {
-        cudaError_t e = cudaMallocAsync((void**)&dstage, 2 * half, stream);
+        cudaError_t e = rt::scratch_malloc((void**)&dstage, 2 * half, stream);
         if (e != cudaSuccess) fail_cuda(e, "cudaMallocAsync");
     }
     uint64_t out_pos = 0;

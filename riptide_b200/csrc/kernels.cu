@@ -6,7 +6,11 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <cuda.h>
+
 #include <algorithm>
+#include <map>
+#include <mutex>
 #include <vector>
 
 #include "common.cuh"
@@ -42,6 +46,52 @@ int check_cuda(cudaError_t e, const char* where)
 }
 
 const char* last_error() { return g_err; }
+
+// ------------------------------------------------------------------------------------
+// Device scratch
+// ------------------------------------------------------------------------------------
+static std::mutex g_pool_mutex;
+static std::map<int, cudaMemPool_t> g_pools;  // by device
+
+cudaError_t scratch_malloc(void** p, size_t bytes, cudaStream_t st)
+{
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    cudaMemPool_t pool = nullptr;
+    {
+        std::lock_guard<std::mutex> lock(g_pool_mutex);
+        auto it = g_pools.find(dev);
+        if (it == g_pools.end()) {
+            cudaMemPoolProps props;
+            memset(&props, 0, sizeof(props));
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = dev;
+            e = cudaMemPoolCreate(&pool, &props);
+            if (e != cudaSuccess) return e;
+            cuuint64_t kept = kScratchKept;
+            e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &kept);
+            if (e != cudaSuccess) {
+                cudaMemPoolDestroy(pool);
+                return e;
+            }
+            g_pools[dev] = pool;
+        } else {
+            pool = it->second;
+        }
+    }
+    return cudaMallocFromPoolAsync(p, bytes, pool, st);
+}
+
+void release_scratch()
+{
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return;
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    auto it = g_pools.find(dev);
+    if (it != g_pools.end()) cudaMemPoolTrimTo(it->second, 0);
+}
 
 // ------------------------------------------------------------------------------------
 // Elementwise helpers (kernels.hpp:19-38, 73-101)
@@ -203,7 +253,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (threadIdx.x < 32) build_job_tree_warp(T, J, b, ffa_cap_rows(L, b), L.ops_units, stage == 0);
     cta_sync();
     if (T.error) {
-        if (threadIdx.x == 0) atomicExch(err, RT_EINTERNAL);
+        if (threadIdx.x == 0 && err) atomicExch(err, RT_EINTERNAL);
         return;
     }
     if (stage > 0 && T.pstaged) {
@@ -282,6 +332,14 @@ int ffa_transform(const float* in, int m, int b, int rows_out, float* out, float
     StagePlan P;
     if (cap < 4 || !plan_stages(m, b, rows_out, cap, 0, &P))
         return set_error(RT_EINVAL, "FFA transform of %d x %d does not fit the device plan", m, b);
+    // what the device checks of every job (level rows and node lists that fit), for all of them:
+    // a level d of a later-stage job of R rows holds at most R + 3 2^d rows
+    for (int s = 0; s < P.nstages; ++s) {
+        const int G = s == 0 ? full_depth((m + (1 << P.D[0]) - 1) >> P.D[0]) : P.D[s - 1] - P.D[s] - 1;
+        const int rows = s == 0 ? (m + (1 << P.D[0]) - 1) >> P.D[0] : P.R[s] + 3 * (1 << G);
+        if (rows > cap || G > (s == 0 ? max_full_depth(b) : kMaxTreeDepth))
+            return set_error(RT_EINTERNAL, "ffa2 plan check failed (%d x %d, stage %d)", m, b, s);
+    }
     if (P.nstages > 1 && scratch == nullptr)
         return set_error(RT_EINTERNAL, "FFA transform of %d x %d needs scratch memory", m, b);
     RT_TRY_CUDA(cudaFuncSetAttribute(k_ffa_stage, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -308,15 +366,19 @@ size_t ffa_scratch_floats(int m, int b)
 // ------------------------------------------------------------------------------------
 // S/N of rows in global memory (snr.hpp:58-65)
 // ------------------------------------------------------------------------------------
+struct WidthList {
+    int w[kMaxWidths];
+};
+
 template <int TPR>
 __global__ void __launch_bounds__(kThreads, 1)
-    k_snr2(const float* __restrict__ x, int rows, int b, const int* __restrict__ widths, int nw,
-           int nfast, float stdnoise, float* __restrict__ out, int tile_rows)
+    k_snr2(const float* __restrict__ x, int rows, int b, WidthList W, int nw, int nfast,
+           float stdnoise, float* __restrict__ out, int tile_rows)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     SnrParams& S = *reinterpret_cast<SnrParams*>(smem);
     float* C = reinterpret_cast<float*>(smem + ((sizeof(SnrParams) + 255) & ~size_t(255)));
-    snr_params_fill(S, widths, nw, nfast, b);
+    snr_params_fill(S, W.w, nw, nfast, b);
     const int cs = prefix_stride(b, S.wmax, TPR);
     const int groups = min(tile_rows, kThreads / TPR);
     for (int r0 = blockIdx.x * tile_rows; r0 < rows; r0 += gridDim.x * tile_rows) {
@@ -340,8 +402,8 @@ int detect_fast_widths(const int* w, int nw)
     return FastWidths10::NW;
 }
 
-int snr2(const float* x, size_t rows, size_t cols, const int* d_widths, const int* h_widths,
-         int nw, float stdnoise, float* out, cudaStream_t st)
+int snr2(const float* x, size_t rows, size_t cols, const int* h_widths, int nw, float stdnoise,
+         float* out, cudaStream_t st)
 {
     if (rows == 0 || nw == 0) return RT_OK;
     int wmax = 0;
@@ -351,7 +413,9 @@ int snr2(const float* x, size_t rows, size_t cols, const int* d_widths, const in
     if (tile < 1) return set_error(RT_EINVAL, "profiles of %zu bins are too long", cols);
     const int grid = (int)std::min<size_t>((rows + tile - 1) / tile, 148 * 4);
     if (nw > kMaxWidths) return set_error(RT_EINVAL, "at most %d trial widths are supported", kMaxWidths);
-    void (*kernel)(const float*, int, int, const int*, int, int, float, float*, int);
+    WidthList W{};
+    std::copy(h_widths, h_widths + nw, W.w);
+    void (*kernel)(const float*, int, int, WidthList, int, int, float, float*, int);
     switch (snr_tpr((int)cols)) {
         case 4: kernel = k_snr2<4>; break;
         case 8: kernel = k_snr2<8>; break;
@@ -360,7 +424,7 @@ int snr2(const float* x, size_t rows, size_t cols, const int* d_widths, const in
     }
     RT_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)kFfaSmemBytes));
-    kernel<<<grid, kThreads, kFfaSmemBytes, st>>>(x, (int)rows, (int)cols, d_widths, nw, nfast,
+    kernel<<<grid, kThreads, kFfaSmemBytes, st>>>(x, (int)rows, (int)cols, W, nw, nfast,
                                                   stdnoise, out, tile);
     return check_cuda(cudaGetLastError(), "snr2");
 }
@@ -435,16 +499,16 @@ __global__ void __launch_bounds__(kDsThreads, 2)
     __shared__ unsigned char s_tab[kDsTab];
 
     const int trial = blockIdx.y;
-    const size_t N = job.lengths[trial];
+    const size_t N = job.length(trial);
     const int seg = job.seg;
     const size_t seg0 = (size_t)blockIdx.x * seg;
     if (seg0 >= N) return;
-    const float* z = job.in + job.in_off[trial] + seg0;
+    const float* z = job.in + job.input(trial) + seg0;
     const int L = (int)std::min<size_t>(kDsStage, N - seg0);
     const double mean = job.mean ? job.mean[trial] : 0.0;
     const double inv = job.norm ? job.norm[trial] : 1.0;
     const bool affine = job.mean != nullptr;
-    float* zout = job.norm_out ? job.norm_out + job.in_off[trial] + seg0 : nullptr;
+    float* zout = job.norm_out ? job.norm_out + job.input(trial) + seg0 : nullptr;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nc = job.ncycles;
 
@@ -452,11 +516,11 @@ __global__ void __launch_bounds__(kDsThreads, 2)
     const size_t seg1 = std::min(N, seg0 + (size_t)seg);
     if (tid < nc) {
         const int c = tid;
-        const double f = job.f[c];
+        const double f = job.factor(c);
         const size_t n = downsampled_size(N, f);
         int cnt = 0;
         size_t k0 = 0;
-        if (job.use_seg[c] && n > 0) {
+        if (job.segments(c) && n > 0) {
             k0 = first_k_at_or_after(seg0, f);
             size_t k1 = (seg1 >= N) ? n : first_k_at_or_after(seg1, f);
             k1 = std::min(k1, n);
@@ -465,7 +529,7 @@ __global__ void __launch_bounds__(kDsThreads, 2)
         s_cnt[c] = cnt;
         s_kb[c] = (long long)k0;
         s_f[c] = f;
-        s_o[c] = job.out + job.out_off[(size_t)trial * nc + c];
+        s_o[c] = job.out + job.output(trial, c);
     }
 
     // Stage the segment + halo. A = z - sh is 16-byte aligned; staged sample i is A[i + sh].
@@ -613,15 +677,15 @@ __global__ void __launch_bounds__(kDsThreads, 2)
 __global__ void k_downsample_wide(DsJob job, int cycle)
 {
     const int trial = blockIdx.y;
-    const size_t N = job.lengths[trial];
-    const double f = job.f[cycle];
+    const size_t N = job.length(trial);
+    const double f = job.factor(cycle);
     const size_t n = downsampled_size(N, f);
-    const float* z = job.in + job.in_off[trial];
+    const float* z = job.in + job.input(trial);
     const double mean = job.mean ? job.mean[trial] : 0.0;
     const double inv = job.norm ? job.norm[trial] : 1.0;
     const double rinv = 1.0 / inv;
     const bool affine = job.mean != nullptr;
-    float* o = job.out + job.out_off[(size_t)trial * job.ncycles + cycle];
+    float* o = job.out + job.output(trial, cycle);
     const int lane = threadIdx.x & 31;
     const size_t wid = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5;
     const size_t nwarp = ((size_t)gridDim.x * blockDim.x) >> 5;
@@ -683,14 +747,15 @@ int launch_downsample(const DsJob& job_in, int ntrials, size_t max_len, cudaStre
 // edge-padded window. Counting selection over a shared-memory tile.
 // ------------------------------------------------------------------------------------
 __global__ void k_running_median(const float* __restrict__ x, const size_t* __restrict__ lengths,
-                                 const size_t* __restrict__ offsets, int width,
+                                 const size_t* __restrict__ offsets, size_t one_len, int width,
                                  float* __restrict__ out, int tile)
 {
     extern __shared__ float sx[];
     const int trial = blockIdx.y;
-    const size_t N = lengths[trial];
-    const float* xr = x + offsets[trial];
-    float* orow = out + offsets[trial];
+    const size_t N = lengths ? lengths[trial] : one_len;
+    const size_t off = lengths ? offsets[trial] : 0;
+    const float* xr = x + off;
+    float* orow = out + off;
     const int half = width / 2;
     const size_t t0 = (size_t)blockIdx.x * tile;
     if (t0 >= N) return;
@@ -732,16 +797,17 @@ constexpr int kRmedSortSpan = 512;  // tile + width - 1 <= span
 
 __global__ void __launch_bounds__(kRmedSortTile)
     k_running_median_sorted(const float* __restrict__ x, const size_t* __restrict__ lengths,
-                            const size_t* __restrict__ offsets, int width,
+                            const size_t* __restrict__ offsets, size_t one_len, int width,
                             float* __restrict__ out)
 {
     __shared__ float sv[kRmedSortSpan];
     __shared__ short sp[kRmedSortSpan];
     const int trial = blockIdx.y;
-    const size_t N = lengths[trial];
+    const size_t N = lengths ? lengths[trial] : one_len;
+    const size_t off = lengths ? offsets[trial] : 0;
     const size_t t0 = (size_t)blockIdx.x * kRmedSortTile;
     if (t0 >= N) return;
-    const float* xr = x + offsets[trial];
+    const float* xr = x + off;
     const int half = width / 2;
     const int span = kRmedSortTile + width - 1;
     for (int i = threadIdx.x; i < kRmedSortSpan; i += blockDim.x) {
@@ -788,7 +854,7 @@ __global__ void __launch_bounds__(kRmedSortTile)
             break;
         }
     }
-    out[offsets[trial] + t0 + t] = med;
+    out[off + t0 + t] = med;
 }
 
 int launch_running_median(const float* x, const size_t* d_lengths, const size_t* d_offsets,
@@ -796,7 +862,7 @@ int launch_running_median(const float* x, const size_t* d_lengths, const size_t*
 {
     if (width >= 1 && kRmedSortTile + width - 1 <= kRmedSortSpan) {
         dim3 grid((unsigned)((max_len + kRmedSortTile - 1) / kRmedSortTile), (unsigned)ntrials);
-        k_running_median_sorted<<<grid, kRmedSortTile, 0, st>>>(x, d_lengths, d_offsets, width, out);
+        k_running_median_sorted<<<grid, kRmedSortTile, 0, st>>>(x, d_lengths, d_offsets, max_len, width, out);
         return check_cuda(cudaGetLastError(), "running_median");
     }
     int tile = 256;
@@ -807,7 +873,7 @@ int launch_running_median(const float* x, const size_t* d_lengths, const size_t*
         RT_TRY_CUDA(cudaFuncSetAttribute(k_running_median,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     dim3 grid((unsigned)((max_len + tile - 1) / tile), (unsigned)ntrials);
-    k_running_median<<<grid, 256, smem, st>>>(x, d_lengths, d_offsets, width, out, tile);
+    k_running_median<<<grid, 256, smem, st>>>(x, d_lengths, d_offsets, max_len, width, out, tile);
     return check_cuda(cudaGetLastError(), "running_median");
 }
 

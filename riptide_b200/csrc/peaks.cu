@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "kernels.cuh"
 
 namespace rt {
 
@@ -245,7 +246,7 @@ extern "C" int rt_peak_segments(const double* d_periods, const float* d_snrs, si
         double* d_ends = nullptr;
         const size_t ro_bytes = (ntrials + 1) * sizeof(uint64_t);
         const size_t ro_room = (ro_bytes + 15) & ~size_t(15);
-        RT_TRY_CUDA(cudaMallocAsync((void**)&d_ro, ro_room + 2 * ntrials * sizeof(double), st));
+        RT_TRY_CUDA(scratch_malloc((void**)&d_ro, ro_room + 2 * ntrials * sizeof(double), st));
         d_ends = reinterpret_cast<double*>(reinterpret_cast<char*>(d_ro) + ro_room);
         cudaError_t e = cudaMemcpyAsync(d_ro, h_row_offsets, ro_bytes, cudaMemcpyHostToDevice, st);
         if (e == cudaSuccess) {
@@ -289,7 +290,7 @@ extern "C" int rt_peak_segments(const double* d_periods, const float* d_snrs, si
     if (!d_snrs) return set_error(RT_EINVAL, "null argument");
     if (seg >= (1ull << 31)) return set_error(RT_EINVAL, "too many segments");
     SegTrial* d_tr = nullptr;
-    RT_TRY_CUDA(cudaMallocAsync((void**)&d_tr, ntrials * sizeof(SegTrial), st));
+    RT_TRY_CUDA(scratch_malloc((void**)&d_tr, ntrials * sizeof(SegTrial), st));
     int s = check_cuda(cudaMemcpyAsync(d_tr, tr.data(), ntrials * sizeof(SegTrial),
                                        cudaMemcpyHostToDevice, st), "peak_segments");
     int n2 = 2;
@@ -337,7 +338,7 @@ extern "C" int rt_peak_select(const double* d_periods, const float* d_snrs, size
     if (num_coef == 0 || num_widths == 0) return set_error(RT_EINVAL, "bad coefficient count");
     const uint64_t rows = h_row_offsets[ntrials];
     unsigned long long* d_aux = nullptr;  // [ntrials] trial row ends, then the counter
-    RT_TRY_CUDA(cudaMallocAsync((void**)&d_aux, (ntrials + 1) * sizeof(unsigned long long), st));
+    RT_TRY_CUDA(scratch_malloc((void**)&d_aux, (ntrials + 1) * sizeof(unsigned long long), st));
     int s = check_cuda(cudaMemcpyAsync(d_aux, h_row_offsets + 1, ntrials * sizeof(uint64_t),
                                        cudaMemcpyHostToDevice, st), "peak_select");
     if (s == RT_OK)

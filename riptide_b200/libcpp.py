@@ -52,6 +52,9 @@ def _as_f32(x, ndim=None):
         elif not t.is_contiguous():
             raise ValueError("Input numpy array must be contiguous in memory")
         dev = True
+        # the kernels read it on the current stream, after the call has returned: its memory
+        # must not be reused before (it may belong to another stream)
+        t.record_stream(torch.cuda.current_stream())
     else:
         a = np.asarray(x)
         if a.dtype != np.float32:
