@@ -693,89 +693,55 @@ __device__ float pw_combine(const float* leaf_sums, int n)
     return ret;
 }
 
-// The additions of the recursion tree of n values as a program: nodes 0 .. L-1 are the leaves
-// (left to right), node L + q = node prog[q].x + node prog[q].y, in the order numpy adds
-// them (children before parents); the root is node 2L - 2 (node 0 when L = 1).
-__device__ void pw_program(int n, int2* prog)
+// The recursion over k values of at most 32 leaves, and its additions as a program: nodes 0 ..
+// L-1 are the leaves (left to right), node L + q = node a[q] + node b[q], in the order numpy
+// adds them (children before parents); the root is node 2L - 2 (node 0 when L = 1).
+constexpr int kScrunchBatchLeaves = 32;
+struct ScrunchTab {
+    int nleaves;
+    unsigned short start[kScrunchBatchLeaves];
+    unsigned char len[kScrunchBatchLeaves];
+    unsigned char a[kScrunchBatchLeaves], b[kScrunchBatchLeaves];
+};
+
+static int scrunch_tab(ScrunchTab& T, int nleaves, int start, int n, int* leaf, int* add)
 {
-    int fn[40], fstate[40], fleft[40];
-    int sp = 1, li = 0, q = 0, ret = 0;
-    fn[0] = n;
-    fstate[0] = 0;
-    int nleaves = 0;
-    // first pass: count leaves (node ids of internal nodes start after them)
-    {
-        int gn[40], gs[40], gp = 1;
-        gn[0] = n;
-        gs[0] = 0;
-        while (gp > 0) {
-            const int t = gp - 1, m = gn[t];
-            if (m <= kPwLeaf) {
-                ++nleaves;
-                --gp;
-                continue;
-            }
-            int m2 = m / 2;
-            m2 -= m2 % 8;
-            if (gs[t] == 0) {
-                gs[t] = 1;
-                gn[gp] = m2;
-                gs[gp++] = 0;
-            } else if (gs[t] == 1) {
-                gs[t] = 2;
-                gn[gp] = m - m2;
-                gs[gp++] = 0;
-            } else {
-                --gp;
-            }
-        }
+    if (n <= kPwLeaf) {
+        T.start[*leaf] = (unsigned short)start;
+        T.len[*leaf] = (unsigned char)n;
+        return (*leaf)++;
     }
-    while (sp > 0) {
-        const int t = sp - 1;
-        const int m = fn[t];
-        if (m <= kPwLeaf) {
-            ret = li++;
-            --sp;
-            continue;
-        }
-        int m2 = m / 2;
-        m2 -= m2 % 8;
-        if (fstate[t] == 0) {
-            fstate[t] = 1;
-            fn[sp] = m2;
-            fstate[sp++] = 0;
-        } else if (fstate[t] == 1) {
-            fleft[t] = ret;
-            fstate[t] = 2;
-            fn[sp] = m - m2;
-            fstate[sp++] = 0;
-        } else {
-            prog[q] = make_int2(fleft[t], ret);
-            ret = nleaves + q;
-            ++q;
-            --sp;
-        }
-    }
+    int n2 = n / 2;
+    n2 -= n2 % 8;
+    const int l = scrunch_tab(T, nleaves, start, n2, leaf, add);
+    const int r = scrunch_tab(T, nleaves, start + n2, n - n2, leaf, add);
+    T.a[*add] = (unsigned char)l;
+    T.b[*add] = (unsigned char)r;
+    return nleaves + (*add)++;
 }
 
 // Scrunch for factors whose recursion has at most 32 leaves (k up to a few thousand): a warp
-// takes 32 scrunched points at a time; its four 8-lane groups compute their leaves (one leaf
-// per group per step, one strided accumulator per lane), then every lane adds up one
-// point's leaves along the program above, so the additions of 32 points run side by side.
-// Dynamic shared memory: leaf table, program, and per warp 32 points x (2L - 1) node values.
-constexpr int kScrunchBatchLeaves = 32;
-
-__global__ void k_scrunch_batched(const float* __restrict__ x, TrialArrays A, int k, int nleaves,
-                                  float* __restrict__ lores)
+// takes `pts` scrunched points at a time; its four 8-lane groups compute their leaves (one leaf
+// per group per step, one strided accumulator per lane), then one lane per point adds up the
+// leaves along the program above. What bounds it is the latency of the loads: a lane issues all
+// of a leaf's (at most 16) before it adds them in order, and points per warp are chosen for
+// warps enough to fill the GPU. (32 points a warp with one load in flight took 117 us for one
+// series of 2^22 samples.)
+// Dynamic shared memory: per warp pts points x (2L - 1) node values.
+__global__ void __launch_bounds__(256)
+    k_scrunch_batched(const float* __restrict__ x, TrialArrays A, int k, ScrunchTab T, int pts,
+                      float* __restrict__ lores)
 {
-    extern __shared__ __align__(16) unsigned char sm_scb[];
-    int2* leaves = reinterpret_cast<int2*>(sm_scb);
-    int2* prog = leaves + nleaves;
+    extern __shared__ float sm_scb[];
+    __shared__ ScrunchTab S;
+    const int nleaves = T.nleaves;
     const int nn = 2 * nleaves - 1, vs = nn | 1;  // odd per-point stride: no bank conflicts
-    float* V = reinterpret_cast<float*>(prog + nleaves) + (threadIdx.x >> 5) * 32 * vs;
-    if (threadIdx.x == 0) {
-        pw_leaf_table(k, leaves);
-        pw_program(k, prog);
+    float* V = sm_scb + (threadIdx.x >> 5) * pts * vs;
+    if (threadIdx.x < kScrunchBatchLeaves) {
+        S.start[threadIdx.x] = T.start[threadIdx.x];
+        S.len[threadIdx.x] = T.len[threadIdx.x];
+        S.a[threadIdx.x] = T.a[threadIdx.x];
+        S.b[threadIdx.x] = T.b[threadIdx.x];
     }
     __syncthreads();
     const int trial = blockIdx.y;
@@ -786,44 +752,41 @@ __global__ void k_scrunch_batched(const float* __restrict__ x, TrialArrays A, in
     const int grp = lane >> 3, c = lane & 7;
     const size_t w0 = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5;
     const size_t nwarp = ((size_t)gridDim.x * blockDim.x) >> 5;
-    for (size_t p0 = w0 * 32; p0 < nl; p0 += nwarp * 32) {
-        const int np = (int)min((size_t)32, nl - p0);
+    for (size_t p0 = w0 * pts; p0 < nl; p0 += nwarp * pts) {
+        const int np = (int)min((size_t)pts, nl - p0);
         const int tasks = np * nleaves;
         for (int u0 = 0; u0 < tasks; u0 += 4) {
             const int u = u0 + grp;
             const bool ok = u < tasks;
             const int pt = ok ? u / nleaves : 0, l = ok ? u - pt * nleaves : 0;
-            const float* a = xr + (p0 + pt) * (size_t)k;
-            float v = 0.0f;
-            int2 lf = make_int2(0, 0);
-            if (ok) {
-                lf = leaves[l];
-                if (lf.y >= 8) {
-                    const int full = lf.y - lf.y % 8;
-                    v = __ldg(a + lf.x + c);
-                    for (int i = 8; i < full; i += 8) v = __fadd_rn(v, __ldg(a + lf.x + i + c));
-                }
-            }
+            const int len = ok ? S.len[l] : 0, full = len & ~7;
+            const float* a = xr + (p0 + pt) * (size_t)k + S.start[l];
+            float r[kPwLeaf / 8];
+#pragma unroll
+            for (int q = 0; q < kPwLeaf / 8; ++q) r[q] = 8 * q < full ? __ldg(a + 8 * q + c) : 0.0f;
+            const float tail = full + c < len ? __ldg(a + full + c) : 0.0f;
+            float v = r[0];
+#pragma unroll
+            for (int q = 1; q < kPwLeaf / 8; ++q)
+                if (8 * q < full) v = __fadd_rn(v, r[q]);
             v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 1));
             v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 2));
             v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 4));
-            if (ok && c == 0) {
-                int i = lf.y - lf.y % 8;
-                if (lf.y < 8) {
-                    v = -0.0f;
-                    i = 0;
+            if (full == 0) v = -0.0f;
+            if (__any_sync(0xffffffffu, full < len)) {
+#pragma unroll
+                for (int q = 0; q < 7; ++q) {
+                    const float y = __shfl_sync(0xffffffffu, tail, q, 8);
+                    if (full + q < len) v = __fadd_rn(v, y);
                 }
-                for (; i < lf.y; ++i) v = __fadd_rn(v, __ldg(a + lf.x + i));
-                V[pt * vs + l] = v;
             }
+            if (ok && c == 0) V[pt * vs + l] = v;
         }
         __syncwarp();
         if (lane < np) {
             float* Vp = V + lane * vs;
-            for (int q = 0; q + 1 < nleaves; ++q) {
-                const int2 ab = prog[q];
-                Vp[nleaves + q] = __fadd_rn(Vp[ab.x], Vp[ab.y]);
-            }
+            for (int q = 0; q + 1 < nleaves; ++q)
+                Vp[nleaves + q] = __fadd_rn(Vp[S.a[q]], Vp[S.b[q]]);
             o[p0 + lane] = __fdiv_rn(Vp[nn - 1], (float)k);
         }
         __syncwarp();
@@ -890,16 +853,21 @@ static int launch_scrunch(const float* x, const TrialArrays& A, int k, int ntria
 {
     const int nleaves = pw_num_leaves(k);
     if (nleaves <= kScrunchBatchLeaves) {
-        // 8 warps, each with 32 points x (2L - 1) node values
-        const size_t smem = 2 * (size_t)nleaves * sizeof(int2) +
-                            8 * 32 * (size_t)((2 * nleaves - 1) | 1) * sizeof(float);
-        const size_t per_trial = std::max<size_t>(8, 4096 / (size_t)std::max(ntrials, 1));
-        dim3 g((unsigned)std::max<size_t>(1, std::min<size_t>((max_lo + 255) / 256, per_trial)),
+        ScrunchTab T;
+        memset(&T, 0, sizeof(T));
+        int leaf = 0, add = 0;
+        T.nleaves = nleaves;
+        scrunch_tab(T, nleaves, 0, k, &leaf, &add);
+        // 8 warps of `pts` points: as many points a warp as leave 32 warps per SM
+        int pts = 32;
+        while (pts > 1 && (size_t)ntrials * max_lo < (size_t)pts * 148 * 32) pts >>= 1;
+        const size_t smem = 8 * (size_t)pts * ((2 * nleaves - 1) | 1) * sizeof(float);
+        dim3 g((unsigned)std::max<size_t>(1, std::min<size_t>((max_lo + 8 * pts - 1) / (8 * pts), 1 << 16)),
                (unsigned)ntrials);
         if (smem > 48 * 1024)
             RT_TRY_CUDA(cudaFuncSetAttribute(k_scrunch_batched,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_scrunch_batched<<<g, 256, smem, st>>>(x, A, k, nleaves, lores);
+        k_scrunch_batched<<<g, 256, smem, st>>>(x, A, k, T, pts, lores);
         return check_cuda(cudaGetLastError(), "scrunch");
     }
     const size_t per_warp = (size_t)nleaves * sizeof(float);
@@ -950,204 +918,223 @@ __device__ __forceinline__ unsigned div_by_magic(unsigned n, const DivMagic& g)
     return (t + ((n - t) >> g.sh1)) >> g.sh2;
 }
 
-// np.interp coefficients of the scrunched running median (running_medians.py:82-85):
-// coef[j] = (fp[j], (fp[j+1] - fp[j]) / k) in float64, so that the interpolated value at
-// x = j*k + (k-1)/2 + dx is fp[j] + slope * dx as numpy evaluates it.
-__global__ void k_interp_coef(TrialArrays A, int k, const float* __restrict__ rmed,
-                              double2* __restrict__ coef)
-{
-    const int trial = blockIdx.y;
-    const size_t nl = A.lo_length(trial);
-    const float* fp = rmed + A.lo_offset(trial);
-    double2* c = coef + A.lo_offset(trial);
-    for (size_t j = blockIdx.x * (size_t)blockDim.x + threadIdx.x; j < nl;
-         j += (size_t)gridDim.x * blockDim.x) {
-        const double a = (double)fp[j];
-        const double s = (j + 1 < nl) ? __ddiv_rn(__dsub_rn((double)fp[j + 1], a), (double)k) : 0.0;
-        c[j] = make_double2(a, s);
+// np.interp of the scrunched running median (running_medians.py:82-85) over kInterpSpan
+// consecutive samples of a series: with v = 2 i - (k - 1) = 2 k j + 2 dx, sample i lies dx past
+// point j, and the value is fp[j] + slope_j * dx in float64 as numpy evaluates it (fp[j] at
+// dx = 0, the end values outside). The CTA puts the points and slopes under its span in shared
+// memory first (one division each); positions are then relative to the span, in 32 bits.
+constexpr int kInterpSpan = 4096;
+constexpr int kInterpCoefs = kInterpSpan / 2 + 2;  // k >= 2
+
+struct InterpSpan {
+    long long vb;       // v of the span's first sample
+    unsigned rel0;      // vb relative to its first point's v (vb >= 0)
+    double first, last;
+    long long vlast;    // v >= vlast is at or right of the last point
+
+    __device__ __forceinline__ void load(const float* fp, size_t nl, int k, size_t i0, int n,
+                                         double2* coef)
+    {
+        vb = 2LL * (long long)i0 - (k - 1);
+        const long long j0 = vb > 0 ? vb / (2LL * k) : 0;
+        rel0 = (unsigned)(vb - 2LL * k * j0);
+        const int nj = n / k + 2;
+        for (int j = threadIdx.x; j < nj; j += blockDim.x) {
+            const size_t jj = (size_t)(j0 + j);
+            double2 c = make_double2(0.0, 0.0);
+            if (jj < nl) {
+                c.x = (double)fp[jj];
+                if (jj + 1 < nl) c.y = __ddiv_rn(__dsub_rn((double)fp[jj + 1], c.x), (double)k);
+            }
+            coef[j] = c;
+        }
+        vlast = 2LL * k * (long long)(nl - 1) - vb;  // relative to vb from here on
+        first = (double)fp[0];
+        last = (double)fp[nl - 1];
     }
+    // sample i of the span
+    __device__ __forceinline__ double value(int i, int k, const DivMagic& g2k,
+                                            const double2* coef) const
+    {
+        const int v = 2 * i;
+        if (v < -vb) return first;
+        if (v >= vlast) return last;
+        const unsigned rel = rel0 + (unsigned)v;  // below 2 kInterpSpan + 2 k
+        const unsigned j = div_by_magic(rel, g2k);
+        const unsigned twodx = rel - j * 2u * (unsigned)k;
+        const double2 c = coef[j];
+        // (an integer below 2^32 as a double by its bits: no conversion)
+        const double dx2 = __dsub_rn(__hiloint2double(0x43300000, (int)twodx), 4503599627370496.0);
+        return twodx == 0 ? c.x : __dadd_rn(__dmul_rn(c.y, 0.5 * dx2), c.x);
+    }
+};
+
+// Sum of a CTA's two per-thread values, in a fixed order (thread 0 has it).
+__device__ __forceinline__ double2 block_sum2(double a, double b)
+{
+    __shared__ double2 w[kStatThreads / 32];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, o);
+        b += __shfl_xor_sync(0xffffffffu, b, o);
+    }
+    if ((threadIdx.x & 31) == 0) w[threadIdx.x >> 5] = make_double2(a, b);
+    __syncthreads();
+    double2 r = w[0];
+    if (threadIdx.x == 0)
+#pragma unroll
+        for (int i = 1; i < kStatThreads / 32; ++i) {
+            r.x += w[i].x;
+            r.y += w[i].y;
+        }
+    return r;
 }
 
-// y = float32(x - running median); per-block shifted sums for the statistics.
-// k > 1: rmed = np.interp(i, j*k + (k-1)/2, rmed_lores) in float64 (running_medians.py:82-85),
-// from the coefficients of k_interp_coef; with v = 2i - (k-1) = 2k*j + 2*dx, the segment j
-// and the offset dx = v mod 2k / 2 come from one invariant division (exact in 32 bits while
-// 2N < 2^32; longer series take 64-bit division);
-// k == 1: rmed is the full-resolution float32 running median (float32 subtraction).
+// CTAs of a series in k_dered, k_sums and k_interp_rmed.
+RT_HD size_t interp_blocks(size_t n) { return (n + kInterpSpan - 1) / kInterpSpan; }
+
+// y = float32(x - running median); per-CTA shifted sums for the statistics.
+// k > 1: the interpolated scrunched running median (InterpSpan); k == 1: rmed is the
+// full-resolution float32 running median (float32 subtraction).
+// Bound by the float64 work between a 4-byte read and a 4-byte write: a CTA takes 4,096
+// consecutive samples, 16 loads a thread in flight. (64 CTAs a series striding over it, with a
+// 64-bit division per sample and the slopes in global memory, took 267 us for 16 series of
+// ~2^22 samples, and left half the GPU idle for one series.)
 __global__ void __launch_bounds__(kStatThreads)
     k_dered(const float* __restrict__ x, TrialArrays A, int k, DivMagic g2k,
-            const float* __restrict__ rmed, const double2* __restrict__ coef,
-            float* __restrict__ y, double* __restrict__ part, int blocks_per_trial)
+            const float* __restrict__ rmed, float* __restrict__ y, double* __restrict__ part)
 {
+    constexpr int Q = kInterpSpan / kStatThreads;
+    __shared__ double2 coef[kInterpCoefs];
     const int trial = blockIdx.y;
-    const size_t N = A.length(trial);
+    const size_t N = A.length(trial), i0 = blockIdx.x * (size_t)kInterpSpan;
+    if (i0 >= N) return;
+    const int n = (int)min((size_t)kInterpSpan, N - i0);
     const float* xr = x + A.offset(trial);
-    float* yr = y + A.offset(trial);
-    const float* fp = rmed + (k > 1 ? A.lo_offset(trial) : A.offset(trial));
-    const double2* cf = coef + (k > 1 ? A.lo_offset(trial) : 0);
-    const size_t nl = A.lo_length(trial);
-    double s1 = 0.0, s2 = 0.0;
-    const float shift = xr[0];
-    float shift_y;
-    {
-        // shift for the sums: y[0]
-        double r0;
-        if (k > 1) r0 = (double)fp[0];  // x = 0 <= xp[0]
-        else r0 = 0.0;
-        shift_y = (k > 1) ? __double2float_rn((double)shift - r0) : __fsub_rn(shift, fp[0]);
+    float* yr = y + A.offset(trial) + i0;
+    float xv[Q];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+        const int i = threadIdx.x + q * kStatThreads;
+        xv[q] = i < n ? xr[i0 + i] : 0.0f;
     }
-    const double shift_yd = (double)shift_y;
-    // v = 2i - (k-1) ranges: v < 0 is left of xp[0]; v >= 2k(nl-1) is at or right of xp[-1]
-    const long long vlast = 2LL * k * (long long)(nl - 1);
-    const bool small = 2 * (unsigned long long)N < (1ull << 32);
-    const double first = (k > 1) ? (double)fp[0] : 0.0;
-    const double last = (k > 1) ? (double)fp[nl - 1] : 0.0;
-    auto body = [&](size_t i, float xv) {
-        float yv;
-        if (k > 1) {
-            const long long v = 2LL * (long long)i - (k - 1);
-            double r;
-            if (v < 0) {
-                r = first;
-            } else if (v >= vlast) {
-                r = last;
-            } else {
-                long long j;
-                if (small) j = (long long)div_by_magic((unsigned)v, g2k);
-                else j = v / (2LL * k);
-                const int twodx = (int)(v - j * 2LL * k);  // 2 (x - xp[j]), 0 <= . < 2k
-                const double2 c = cf[j];
-                // x - xp[j] is exact in double; numpy's interp returns fp[j] at x == xp[j]
-                r = (twodx == 0) ? c.x : __dadd_rn(__dmul_rn(c.y, 0.5 * (double)twodx), c.x);
-            }
-            yv = __double2float_rn(__dsub_rn((double)xv, r));
-        } else {
-            yv = __fsub_rn(xv, fp[i]);
-        }
+    const float* fp = rmed + (k > 1 ? A.lo_offset(trial) : A.offset(trial));
+    // the sums are shifted by y[0] (x = 0 <= xp[0]: its running median is fp[0])
+    const float shift = k > 1 ? __double2float_rn((double)xr[0] - (double)fp[0])
+                              : __fsub_rn(xr[0], fp[0]);
+    const double shift_d = (double)shift;
+    InterpSpan S;
+    if (k > 1) S.load(fp, A.lo_length(trial), k, i0, n, coef);
+    __syncthreads();
+    double s1 = 0.0, s2 = 0.0;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+        const int i = threadIdx.x + q * kStatThreads;
+        if (i >= n) continue;
+        const float yv = k > 1 ? __double2float_rn(__dsub_rn((double)xv[q], S.value(i, k, g2k, coef)))
+                               : __fsub_rn(xv[q], fp[i0 + i]);
         yr[i] = yv;
-        const double d = (double)yv - shift_yd;
+        const double d = (double)yv - shift_d;
         s1 += d;
         s2 += d * d;
-    };
-    // four grid-stride steps per pass with their loads issued first; the sums keep the
-    // order of the plain loop
-    const size_t stride = (size_t)blocks_per_trial * blockDim.x;
-    size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    for (; i + 3 * stride < N; i += 4 * stride) {
-        float xv[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) xv[q] = xr[i + q * stride];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) body(i + q * stride, xv[q]);
     }
-    for (; i < N; i += stride) body(i, xr[i]);
-    // block reduction (fixed order)
-    __shared__ double r1[kStatThreads], r2[kStatThreads];
-    r1[threadIdx.x] = s1;
-    r2[threadIdx.x] = s2;
-    __syncthreads();
-    for (int o = kStatThreads / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) {
-            r1[threadIdx.x] += r1[threadIdx.x + o];
-            r2[threadIdx.x] += r2[threadIdx.x + o];
-        }
-        __syncthreads();
-    }
+    const double2 s = block_sum2(s1, s2);
     if (threadIdx.x == 0) {
-        double* p = part + ((size_t)trial * blocks_per_trial + blockIdx.x) * 3;
-        p[0] = r1[0];
-        p[1] = r2[0];
-        p[2] = (double)shift_y;
+        double* p = part + ((size_t)trial * gridDim.x + blockIdx.x) * 3;
+        p[0] = s.x;
+        p[1] = s.y;
+        p[2] = shift_d;
     }
 }
 
 // Same statistics without deredden (normalise only).
 __global__ void __launch_bounds__(kStatThreads)
-    k_sums(const float* __restrict__ x, TrialArrays A, double* __restrict__ part,
-           int blocks_per_trial)
+    k_sums(const float* __restrict__ x, TrialArrays A, double* __restrict__ part)
 {
+    constexpr int Q = kInterpSpan / kStatThreads;
     const int trial = blockIdx.y;
-    const size_t N = A.length(trial);
+    const size_t N = A.length(trial), i0 = blockIdx.x * (size_t)kInterpSpan;
+    if (i0 >= N) return;
+    const int n = (int)min((size_t)kInterpSpan, N - i0);
     const float* xr = x + A.offset(trial);
-    const float shift = xr[0];
+    const double shift = (double)xr[0];
     double s1 = 0.0, s2 = 0.0;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < N;
-         i += (size_t)blocks_per_trial * blockDim.x) {
-        const double d = (double)xr[i] - (double)shift;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+        const int i = threadIdx.x + q * kStatThreads;
+        const double d = i < n ? (double)xr[i0 + i] - shift : 0.0;
         s1 += d;
         s2 += d * d;
     }
-    __shared__ double r1[kStatThreads], r2[kStatThreads];
-    r1[threadIdx.x] = s1;
-    r2[threadIdx.x] = s2;
-    __syncthreads();
-    for (int o = kStatThreads / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) {
-            r1[threadIdx.x] += r1[threadIdx.x + o];
-            r2[threadIdx.x] += r2[threadIdx.x + o];
-        }
-        __syncthreads();
-    }
+    const double2 s = block_sum2(s1, s2);
     if (threadIdx.x == 0) {
-        double* p = part + ((size_t)trial * blocks_per_trial + blockIdx.x) * 3;
-        p[0] = r1[0];
-        p[1] = r2[0];
-        p[2] = (double)shift;
+        double* p = part + ((size_t)trial * gridDim.x + blockIdx.x) * 3;
+        p[0] = s.x;
+        p[1] = s.y;
+        p[2] = shift;
     }
 }
 
-// mean and standard deviation per trial (population variance, ddof = 0).
-__global__ void k_stats(const double* __restrict__ part, TrialArrays A, int blocks_per_trial, int ntrials, double* __restrict__ mean,
-                        double* __restrict__ norm)
+// mean and standard deviation per trial (population variance, ddof = 0), a warp per trial:
+// `blocks` partial sums of it at most, in a fixed order.
+__global__ void k_stats(const double* __restrict__ part, TrialArrays A, int blocks, int ntrials,
+                        double* __restrict__ mean, double* __restrict__ norm)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31;
+    const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (t >= ntrials) return;
-    double s1 = 0.0, s2 = 0.0, shift = 0.0;
-    for (int b = 0; b < blocks_per_trial; ++b) {
-        const double* p = part + ((size_t)t * blocks_per_trial + b) * 3;
-        s1 += p[0];
-        s2 += p[1];
-        shift = p[2];
+    const double* p = part + (size_t)t * blocks * 3;
+    const int nb = (int)interp_blocks(A.length(t));
+    double s1 = 0.0, s2 = 0.0;
+    for (int b = lane; b < nb; b += 32) {
+        s1 += p[3 * b];
+        s2 += p[3 * b + 1];
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+        s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+    }
+    if (lane != 0) return;
     const double N = (double)A.length(t);
     const double d = s1 / N;
     const double var = s2 / N - d * d;
-    mean[t] = shift + d;
+    mean[t] = p[2] + d;
     norm[t] = sqrt(var);
 }
 
 // fast_running_median output (running_medians.py:82-85): float64 interpolation of the
-// scrunched running median back to every sample.
-__global__ void k_interp_rmed(TrialArrays A, int k, const float* __restrict__ rmed,
-                              double* __restrict__ out)
+// scrunched running median back to every sample, two samples a thread at a time, stored as one
+// 16-byte unit. Bound by the 8 bytes a sample that it writes.
+__global__ void __launch_bounds__(kStatThreads)
+    k_interp_rmed(TrialArrays A, int k, DivMagic g2k, const float* __restrict__ rmed,
+                  double* __restrict__ out)
 {
+    __shared__ double2 coef[kInterpCoefs];
     const int trial = blockIdx.y;
     const size_t N = A.length(trial);
     const float* fp = rmed + A.lo_offset(trial);
-    const size_t nl = A.lo_length(trial);
-    double* o = out + A.offset(trial);
-    const double half = 0.5 * (double)(k - 1);
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < N;
-         i += (size_t)gridDim.x * blockDim.x) {
-        const double xi = (double)i;
-        const double xl = (double)(nl - 1) * k + half;
-        double r;
-        if (xi < half) {
-            r = (double)fp[0];
-        } else if (xi >= xl) {
-            r = (double)fp[nl - 1];
-        } else {
-            const long long j = (2LL * (long long)i - (k - 1)) / (2LL * k);
-            const double xj = (double)j * k + half;
-            if (xj == xi) {
-                r = (double)fp[j];
-            } else {
-                const double slope =
-                    __ddiv_rn(__dsub_rn((double)fp[j + 1], (double)fp[j]), (double)k);
-                r = __dadd_rn(__dmul_rn(slope, __dsub_rn(xi, xj)), (double)fp[j]);
-            }
+    const size_t i0 = blockIdx.x * (size_t)kInterpSpan;
+    if (i0 >= N) return;
+    double* o = out + A.offset(trial) + i0;
+    const int n = (int)min((size_t)kInterpSpan, N - i0);
+    if (k == 1) {  // every sample is a point of the running median
+        for (int i = threadIdx.x; i < n; i += blockDim.x) o[i] = (double)fp[i0 + i];
+        return;
+    }
+    InterpSpan S;
+    S.load(fp, A.lo_length(trial), k, i0, n, coef);
+    __syncthreads();
+    if ((reinterpret_cast<uintptr_t>(o) & 15) == 0) {
+        for (int i = 2 * threadIdx.x; i < n; i += 2 * blockDim.x) {
+            const double a = S.value(i, k, g2k, coef);
+            if (i + 1 < n)
+                *reinterpret_cast<double2*>(o + i) = make_double2(a, S.value(i + 1, k, g2k, coef));
+            else
+                o[i] = a;
         }
-        o[i] = r;
+    } else {
+        for (int i = threadIdx.x; i < n; i += blockDim.x) o[i] = S.value(i, k, g2k, coef);
     }
 }
 
@@ -1211,7 +1198,6 @@ struct SearchPlan {
     float* d_y = nullptr;               // dereddened series
     float* d_norm = nullptr;            // normalised copy (when a cycle has f == 1)
     float* d_lores = nullptr;
-    double2* d_coef = nullptr;          // interpolation coefficients of the running median
     float* d_rmed = nullptr;
     double* d_part = nullptr;
     double* d_mean = nullptr;
@@ -1223,7 +1209,6 @@ struct SearchPlan {
     double* d_f = nullptr;
     int* d_useseg = nullptr;
     size_t* d_dsoff = nullptr;
-    int stat_blocks = 64;
     // optional per-stage CUDA-event timing: deredden+normalise, downsample, FFA + S/N
     bool timing = false;
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -1459,7 +1444,7 @@ static void plan_free_device(SearchPlan& P)
 {
     dfree(P.d_widths); dfree(P.d_xforms); dfree(P.d_items); dfree(P.d_plans);
     dfree(P.d_scratch); dfree(P.d_counters); dfree(P.d_ticket); dfree(P.d_ds); dfree(P.d_y);
-    dfree(P.d_norm); dfree(P.d_lores); dfree(P.d_coef); dfree(P.d_rmed); dfree(P.d_part);
+    dfree(P.d_norm); dfree(P.d_lores); dfree(P.d_rmed); dfree(P.d_part);
     dfree(P.d_mean); dfree(P.d_normv); dfree(P.d_len); dfree(P.d_off); dfree(P.d_lo_len);
     dfree(P.d_lo_off); dfree(P.d_f); dfree(P.d_useseg); dfree(P.d_dsoff);
     P.dev_ready = false;
@@ -1525,13 +1510,10 @@ static int plan_alloc_device(SearchPlan& P)
     if (P.cfg.deredden) {
         RT_TRY(dalloc(P, &P.d_y, P.total_len));
         RT_TRY(dalloc(P, &P.d_rmed, P.scrunch > 1 ? P.lo_total : P.total_len));
-        if (P.scrunch > 1) {
-            RT_TRY(dalloc(P, &P.d_lores, P.lo_total));
-            RT_TRY(dalloc(P, &P.d_coef, P.lo_total));
-        }
+        if (P.scrunch > 1) RT_TRY(dalloc(P, &P.d_lores, P.lo_total));
     }
     if (P.has_unit_factor) RT_TRY(dalloc(P, &P.d_norm, P.total_len));
-    RT_TRY(dalloc(P, &P.d_part, (size_t)T * P.stat_blocks * 3));
+    RT_TRY(dalloc(P, &P.d_part, (size_t)T * interp_blocks(P.max_len) * 3));
     RT_TRY(dalloc(P, &P.d_mean, T));
     RT_TRY(dalloc(P, &P.d_normv, T));
     RT_TRY(upload(P, &P.d_len, P.lengths));
@@ -1573,6 +1555,7 @@ static int plan_run(SearchPlan& P, const float* data, float* normalised_out, dou
     TrialArrays TA{P.d_len, P.d_off, P.d_lo_len, P.d_lo_off, 0, 0};
     const float* series = data;  // series before normalisation
     int launches = 0;
+    const dim3 stat_grid((unsigned)interp_blocks(P.max_len), (unsigned)T);
     if (P.timing) RT_TRY_CUDA(cudaEventRecord(P.ev[0], st));
     if (P.cfg.deredden) {
         const int k = P.scrunch;
@@ -1580,31 +1563,25 @@ static int plan_run(SearchPlan& P, const float* data, float* normalised_out, dou
             RT_TRY(launch_scrunch(data, TA, k, T, P.max_lo, P.d_lores, st));
             RT_TRY(launch_running_median(P.d_lores, P.d_lo_len, P.d_lo_off, T, P.max_lo,
                                          (int)P.cfg.rmed_minpts, P.d_rmed, st));
-            dim3 gc((unsigned)std::min<size_t>((P.max_lo + 255) / 256, 1024), (unsigned)T);
-            k_interp_coef<<<gc, 256, 0, st>>>(TA, k, P.d_rmed, P.d_coef);
-            RT_TRY_CUDA(cudaGetLastError());
-            launches += 3;
+            launches += 2;
         } else {
             RT_TRY(launch_running_median(data, P.d_len, P.d_off, T, P.max_len, P.rmed_width,
                                          P.d_rmed, st));
             launches += 1;
         }
-        dim3 g((unsigned)P.stat_blocks, (unsigned)T);
-        k_dered<<<g, kStatThreads, 0, st>>>(data, TA, k, div_magic(2u * (unsigned)k), P.d_rmed,
-                                            P.d_coef, P.d_y, P.d_part, P.stat_blocks);
+        k_dered<<<stat_grid, kStatThreads, 0, st>>>(data, TA, k, div_magic(2u * (unsigned)k),
+                                                    P.d_rmed, P.d_y, P.d_part);
         RT_TRY_CUDA(cudaGetLastError());
         launches += 1;
         series = P.d_y;
     } else if (!P.cfg.already_normalised) {
-        dim3 g((unsigned)P.stat_blocks, (unsigned)T);
-        k_sums<<<g, kStatThreads, 0, st>>>(data, TA, P.d_part, P.stat_blocks);
+        k_sums<<<stat_grid, kStatThreads, 0, st>>>(data, TA, P.d_part);
         RT_TRY_CUDA(cudaGetLastError());
         launches += 1;
     }
     const bool affine = !P.cfg.already_normalised;
     if (affine) {
-        k_stats<<<(T + 127) / 128, 128, 0, st>>>(P.d_part, TA, P.stat_blocks, T, P.d_mean,
-                                                 P.d_normv);
+        k_stats<<<(T + 3) / 4, 128, 0, st>>>(P.d_part, TA, (int)stat_grid.x, T, P.d_mean, P.d_normv);
         RT_TRY_CUDA(cudaGetLastError());
         launches += 1;
     }
@@ -2429,8 +2406,8 @@ extern "C" int rt_fast_running_median(const float* d_x, size_t size, size_t widt
         s = launch_scrunch(d_x, A, k, 1, nl, lores, st);
         if (s == RT_OK) s = launch_running_median(lores, nullptr, nullptr, 1, nl, w, rmed, st);
         if (s == RT_OK) {
-            k_interp_rmed<<<dim3(std::max(1, (int)std::min<size_t>((size + 255) / 256, 4096)), 1), 256, 0, st>>>(
-                A, k, rmed, d_out);
+            k_interp_rmed<<<(unsigned)((size + kInterpSpan - 1) / kInterpSpan), 256, 0, st>>>(
+                A, k, div_magic(2u * (unsigned)k), rmed, d_out);
             s = check_cuda(cudaGetLastError(), "fast_running_median");
         }
     } else {
@@ -2438,8 +2415,8 @@ extern "C" int rt_fast_running_median(const float* d_x, size_t size, size_t widt
         RT_TRY_CUDA(scratch_malloc((void**)&rmed, size * sizeof(float), st));
         s = launch_running_median(d_x, nullptr, nullptr, 1, size, w, rmed, st);
         if (s == RT_OK) {
-            k_interp_rmed<<<dim3(std::max(1, (int)std::min<size_t>((size + 255) / 256, 4096)), 1), 256, 0, st>>>(
-                one_series(size, size), 1, rmed, d_out);
+            k_interp_rmed<<<(unsigned)((size + kInterpSpan - 1) / kInterpSpan), 256, 0, st>>>(
+                one_series(size, size), 1, div_magic(2), rmed, d_out);
             s = check_cuda(cudaGetLastError(), "fast_running_median");
         }
     }
@@ -2459,32 +2436,24 @@ extern "C" int rt_deredden(const float* d_x, size_t size, double tsamp, double w
     RT_TRY(rmed_geometry(size, (size_t)ws, min_points, &k, &w, &nl));
     const TrialArrays A = one_series(size, nl);
     float *lores = nullptr, *rmed = nullptr;
-    double2* coef = nullptr;
     double* part = nullptr;
     int s = RT_OK;
-    const int blocks = 64;
+    const size_t blocks = interp_blocks(size);
     RT_TRY_CUDA(scratch_malloc((void**)&part, blocks * 3 * sizeof(double), st));
     if (k > 1) {
         RT_TRY_CUDA(scratch_malloc((void**)&lores, nl * sizeof(float), st));
         RT_TRY_CUDA(scratch_malloc((void**)&rmed, nl * sizeof(float), st));
-        RT_TRY_CUDA(scratch_malloc((void**)&coef, nl * sizeof(double2), st));
         s = launch_scrunch(d_x, A, k, 1, nl, lores, st);
         if (s == RT_OK) s = launch_running_median(lores, nullptr, nullptr, 1, nl, w, rmed, st);
-        if (s == RT_OK) {
-            k_interp_coef<<<dim3((unsigned)std::min<size_t>((nl + 255) / 256, 1024), 1), 256, 0, st>>>(
-                A, k, rmed, coef);
-            s = check_cuda(cudaGetLastError(), "deredden");
-        }
     } else {
         RT_TRY_CUDA(scratch_malloc((void**)&rmed, size * sizeof(float), st));
         s = launch_running_median(d_x, nullptr, nullptr, 1, size, w, rmed, st);
     }
     if (s == RT_OK) {
-        k_dered<<<dim3(blocks, 1), kStatThreads, 0, st>>>(d_x, A, k, div_magic(2u * (unsigned)k),
-                                                          rmed, coef, d_out, part, blocks);
+        k_dered<<<(unsigned)blocks, kStatThreads, 0, st>>>(d_x, A, k, div_magic(2u * (unsigned)k),
+                                                          rmed, d_out, part);
         s = check_cuda(cudaGetLastError(), "deredden");
     }
-    if (coef) cudaFreeAsync(coef, st);
     if (lores) cudaFreeAsync(lores, st);
     if (rmed) cudaFreeAsync(rmed, st);
     cudaFreeAsync(part, st);
@@ -2497,12 +2466,12 @@ extern "C" int rt_normalise(const float* d_x, size_t size, float* d_out, void* s
     if (size == 0) return RT_OK;
     const TrialArrays A = one_series(size, 0);
     double* part = nullptr;
-    const int blocks = 64;
+    const size_t blocks = interp_blocks(size);
     RT_TRY_CUDA(scratch_malloc((void**)&part, (blocks * 3 + 2) * sizeof(double), st));
     double* mean = part + blocks * 3;
     double* norm = mean + 1;
-    k_sums<<<dim3(blocks, 1), kStatThreads, 0, st>>>(d_x, A, part, blocks);
-    k_stats<<<1, 32, 0, st>>>(part, A, blocks, 1, mean, norm);
+    k_sums<<<(unsigned)blocks, kStatThreads, 0, st>>>(d_x, A, part);
+    k_stats<<<1, 32, 0, st>>>(part, A, (int)blocks, 1, mean, norm);
     k_normalise<<<dim3(std::max(1, (int)std::min<size_t>((size + 255) / 256, 4096)), 1), 256, 0, st>>>(
         d_x, A, mean, norm, d_out);
     int s = check_cuda(cudaGetLastError(), "normalise");
