@@ -352,6 +352,16 @@ int rt_search_backward_rows(rt_search_plan* plan, const float* d_z, const float*
  * d_gy = (g - mean(g) - z * mean(g z)) / std, with d_z the normalised series. */
 int rt_normalise_adjoint(const float* d_g, const float* d_z, size_t size, double std_,
                          float* d_gy, void* stream);
+/* The adjoints of normalise and then deredden over ntrials packed series at once: from d_gz,
+ * the gradient with respect to the searched series, to d_gx, the one with respect to the input
+ * d_x (both packed like the input). h_std: the standard deviation each series was normalised
+ * by (null: it was not; else d_z holds the normalised series). width_samples and min_points as
+ * for fast_running_median (min_points 0: no deredden); running medians of up to 257 points,
+ * RT_EINVAL beyond. d_gx may not alias d_x or d_z. */
+int rt_front_adjoint(const float* d_x, const float* d_z, const float* d_gz,
+                     const uint64_t* h_lengths, size_t ntrials, const double* h_std,
+                     size_t width_samples, size_t min_points, float* d_gx, void* stream);
+
 
 /* ---------------------------------------------------------------------------------------
  * Time series files into device memory: the data side of TimeSeries.from_presto_inf /

@@ -67,6 +67,7 @@ SIGNATURES = {
     "rt_ffa2_transpose": (ctypes.c_int, [_vp, _sz, _sz, _vp, _vp]),
     "rt_downsample_adjoint": (ctypes.c_int, [_vp, _sz, _d, _vp, _vp]),
     "rt_normalise_adjoint": (ctypes.c_int, [_vp, _vp, _sz, _d, _vp, _vp]),
+    "rt_front_adjoint": (ctypes.c_int, [_vp, _vp, _vp, _u64p, _sz, ctypes.POINTER(_d), _sz, _sz, _vp, _vp]),
     "rt_search_set_graph": (ctypes.c_int, [_vp, ctypes.c_int]),
     "rt_fold_shape": (ctypes.c_int, [_sz, _d, _d, _sz, ctypes.c_longlong, ctypes.POINTER(_sz), ctypes.POINTER(ctypes.c_int)]),
     "rt_fold": (ctypes.c_int, [_vp, _sz, _d, _d, _sz, ctypes.c_longlong, _vp, _vp]),

@@ -3,6 +3,8 @@
 // differentiable; these follow its forward arithmetic (snr.hpp:37-65, transforms.hpp:13-61,
 // downsample.hpp:44-82, time_series.py:67-93) so that the gradient is the one of the function
 // the forward computes.
+#include <string.h>
+
 #include <algorithm>
 #include <vector>
 
@@ -231,14 +233,25 @@ __global__ void k_downsample_adjoint(const float* __restrict__ gout, size_t N, d
 // ------------------------------------------------------------------------------------
 constexpr int kNormBwdThreads = 256;
 
-__global__ void k_norm_adj_sums(const float* __restrict__ g, const float* __restrict__ z,
-                                size_t N, double* __restrict__ part)
+// Packed series of a batch (all arrays on the device).
+struct AdjBatch {
+    const size_t *len, *off;        // [ntrials] lengths, offsets into the packed series
+    const size_t *lo_len, *lo_off;  // [ntrials] the same of the scrunched series
+    const double* inv_std;          // [ntrials]
+};
+
+__global__ void __launch_bounds__(kNormBwdThreads)
+    k_norm_adj_sums(const float* __restrict__ g, const float* __restrict__ z, AdjBatch B,
+                    double2* __restrict__ part)
 {
+    const int trial = blockIdx.y;
+    const size_t N = B.len[trial], off = B.off[trial];
     double s1 = 0.0, s2 = 0.0;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < N;
          i += (size_t)gridDim.x * blockDim.x) {
-        s1 += (double)g[i];
-        s2 += (double)g[i] * (double)z[i];
+        const double gv = (double)g[off + i];
+        s1 += gv;
+        s2 += gv * (double)z[off + i];
     }
     __shared__ double r1[kNormBwdThreads], r2[kNormBwdThreads];
     r1[threadIdx.x] = s1;
@@ -251,31 +264,176 @@ __global__ void k_norm_adj_sums(const float* __restrict__ g, const float* __rest
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        part[2 * blockIdx.x] = r1[0];
-        part[2 * blockIdx.x + 1] = r2[0];
+    if (threadIdx.x == 0) part[(size_t)trial * gridDim.x + blockIdx.x] = make_double2(r1[0], r2[0]);
+}
+
+// (Every CTA adds up its series' partial sums first, a warp at a time: by one thread that took
+// 20 of 26 us.)
+__global__ void __launch_bounds__(kNormBwdThreads)
+    k_norm_adj_apply(const float* __restrict__ g, const float* __restrict__ z, AdjBatch B,
+                     const double2* __restrict__ part, float* __restrict__ gy)
+{
+    __shared__ double s_m1, s_m2;
+    const int trial = blockIdx.y;
+    const size_t N = B.len[trial], off = B.off[trial];
+    if (threadIdx.x < 32) {
+        const double2* p = part + (size_t)trial * gridDim.x;
+        double a = 0.0, c = 0.0;
+        for (unsigned k = threadIdx.x; k < gridDim.x; k += 32) {
+            a += p[k].x;
+            c += p[k].y;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            a += __shfl_xor_sync(0xffffffffu, a, o);
+            c += __shfl_xor_sync(0xffffffffu, c, o);
+        }
+        if (threadIdx.x == 0) {
+            s_m1 = a / (double)N;
+            s_m2 = c / (double)N;
+        }
+    }
+    __syncthreads();
+    const double m1 = s_m1, m2 = s_m2, inv_std = B.inv_std[trial];
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < N;
+         i += (size_t)gridDim.x * blockDim.x)
+        gy[off + i] = (float)(((double)g[off + i] - m1 - (double)z[off + i] * m2) * inv_std);
+}
+
+// ------------------------------------------------------------------------------------
+// Deredden adjoint: y = x - r(x) with r = np.interp of the running median of the mean-scrunched
+// series (running_medians.py:49-85), so gx = gy - r^T gy: through the interpolation (each point
+// gathers from the samples around it), the median (to the element it selects) and the mean.
+// All in float64; every sum is a gather, so the result does not depend on scheduling.
+// ------------------------------------------------------------------------------------
+// Scrunched means, and the interpolation's transpose of g at every point j: with a = the
+// sample's position past point j over k, sum g (1 - a) over the samples from point j to j + 1
+// and g a over those from j - 1 to j; samples outside the points go to the end points. A warp
+// per point. k == 1: the samples themselves.
+__global__ void __launch_bounds__(256)
+    k_dered_adj_points(const float* __restrict__ x, const float* __restrict__ g, AdjBatch B, int k,
+                       double* __restrict__ lores, double* __restrict__ glo)
+{
+    const int trial = blockIdx.y, lane = threadIdx.x & 31;
+    const size_t N = B.len[trial], nl = B.lo_len[trial];
+    const float *xr = x + B.off[trial], *gr = g + B.off[trial];
+    double *lo = lores + B.lo_off[trial], *go = glo + B.lo_off[trial];
+    const double rk = 1.0 / (double)k;
+    for (size_t j = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5; j < nl;
+         j += ((size_t)gridDim.x * blockDim.x) >> 5) {
+        if (k == 1) {
+            if (lane == 0) {
+                lo[j] = (double)xr[j];
+                go[j] = (double)gr[j];
+            }
+            continue;
+        }
+        double s = 0.0, c = 0.0;
+        for (int i = lane; i < k; i += 32) s += (double)xr[j * k + i];
+        const size_t at = j * k + k / 2;  // first sample at or past point j
+        const size_t lo_i = j == 0 ? 0 : at - k;
+        const size_t hi_i = j + 1 == nl ? N : at + k;
+        for (size_t i = lo_i + lane; i < hi_i; i += 32) {
+            // 2 (i - point j), an exact integer
+            const double d = (double)(2LL * ((long long)i - (long long)(j * k)) - (k - 1)) * 0.5;
+            double w = 1.0;
+            if (i < at) w = j == 0 ? 1.0 : 1.0 + d * rk;
+            else if (j + 1 < nl) w = 1.0 - d * rk;
+            c += w * (double)gr[i];
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            s += __shfl_xor_sync(0xffffffffu, s, o);
+            c += __shfl_xor_sync(0xffffffffu, c, o);
+        }
+        if (lane == 0) {
+            lo[j] = s * rk;
+            go[j] = c;
+        }
     }
 }
 
-__global__ void k_norm_adj_apply(const float* __restrict__ g, const float* __restrict__ z,
-                                 size_t N, const double* __restrict__ part, int nblocks,
-                                 double inv_std, float* __restrict__ gy)
+// Index of the element that the running median selects at every point: the tile's values ranked
+// by (value, position) as in k_running_median_sorted.
+constexpr int kAdjTile = 128;
+constexpr int kAdjMaxWidth = 257;
+constexpr int kAdjSpan = kAdjTile + kAdjMaxWidth - 1;
+
+__global__ void __launch_bounds__(kAdjTile)
+    k_dered_adj_select(const double* __restrict__ lores, AdjBatch B, int width,
+                       unsigned* __restrict__ sel)
 {
-    __shared__ double s_m1, s_m2;
-    if (threadIdx.x == 0) {
-        double a = 0.0, c = 0.0;
-        for (int k = 0; k < nblocks; ++k) {
-            a += part[2 * k];
-            c += part[2 * k + 1];
-        }
-        s_m1 = a / (double)N;
-        s_m2 = c / (double)N;
+    __shared__ double sx[kAdjSpan];
+    __shared__ unsigned short sp[kAdjSpan];
+    const int trial = blockIdx.y;
+    const size_t nl = B.lo_len[trial], t0 = (size_t)blockIdx.x * kAdjTile;
+    if (t0 >= nl) return;
+    const double* lo = lores + B.lo_off[trial];
+    const int half = width / 2, span = kAdjTile + width - 1;
+    auto clamped = [&](long long i) { return i < 0 ? 0LL : i >= (long long)nl ? (long long)nl - 1 : i; };
+    for (int i = threadIdx.x; i < span; i += kAdjTile) {
+        sx[i] = lo[clamped((long long)t0 + i - half)];
+        sp[i] = 0xffff;
     }
     __syncthreads();
-    const double m1 = s_m1, m2 = s_m2;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < N;
+    for (int i = threadIdx.x; i < span; i += kAdjTile) {
+        const double v = sx[i];
+        int c = 0;
+        for (int j = 0; j < span; ++j) c += (sx[j] < v || (sx[j] == v && j < i)) ? 1 : 0;
+        sp[c] = (unsigned short)i;
+    }
+    __syncthreads();
+    const int t = threadIdx.x;
+    if (t0 + t >= nl) return;
+    int left = half, at = t + half;
+    for (int q = 0; q < span; ++q) {
+        const unsigned p = sp[q];
+        if (p - (unsigned)t < (unsigned)width && left-- == 0) {
+            at = (int)p;
+            break;
+        }
+    }
+    sel[B.lo_off[trial] + t0 + t] = (unsigned)clamped((long long)t0 + at - half);
+}
+
+// gradient of the scrunched series: element e gathers the points whose window selected it
+__global__ void k_dered_adj_gather(const double* __restrict__ glo, const unsigned* __restrict__ sel,
+                                   AdjBatch B, int width, int k, float* __restrict__ gsel)
+{
+    const int trial = blockIdx.y;
+    const size_t nl = B.lo_len[trial], lo = B.lo_off[trial];
+    const int half = width / 2;
+    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < nl;
+         e += (size_t)gridDim.x * blockDim.x) {
+        const size_t a = e >= (size_t)half ? e - half : 0, z = min(nl, e + half + 1);
+        double s = 0.0;
+        for (size_t t = a; t < z; ++t)
+            if (sel[lo + t] == (unsigned)e) s += glo[lo + t];
+        gsel[lo + e] = (float)(s / (double)k);
+    }
+}
+
+__global__ void k_dered_adj_apply(const float* __restrict__ gsel, AdjBatch B, int k,
+                                  float* __restrict__ gx)
+{
+    const int trial = blockIdx.y;
+    const size_t nl = B.lo_len[trial];
+    const float* s = gsel + B.lo_off[trial];
+    float* g = gx + B.off[trial];
+    // a CTA takes whole points, so that no thread divides
+    for (size_t j = blockIdx.x; j < nl; j += gridDim.x) {
+        const float v = s[j];
+        for (int i = threadIdx.x; i < k; i += blockDim.x) g[j * k + i] = __fsub_rn(g[j * k + i], v);
+    }
+}
+
+__global__ void k_dered_adj_apply1(const float* __restrict__ gsel, AdjBatch B, float* __restrict__ gx)
+{
+    const int trial = blockIdx.y;
+    const size_t nl = B.lo_len[trial], off = B.off[trial], lo = B.lo_off[trial];
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nl;
          i += (size_t)gridDim.x * blockDim.x)
-        gy[i] = (float)(((double)g[i] - m1 - (double)z[i] * m2) * inv_std);
+        gx[off + i] = __fsub_rn(gx[off + i], gsel[lo + i]);
 }
 
 }  // namespace rt
@@ -372,6 +530,62 @@ extern "C" int rt_downsample_adjoint(const float* d_gout, size_t size, double f,
     return check_cuda(cudaGetLastError(), "downsample_adjoint");
 }
 
+// Lengths and offsets of a batch on the device, with 1 / std of each series.
+static int adj_batch(const uint64_t* h_lengths, size_t ntrials, const double* h_std, size_t k,
+                     AdjBatch* B, void** blob, size_t* total, size_t* lo_total, size_t* max_len,
+                     cudaStream_t st)
+{
+    std::vector<size_t> h(5 * ntrials);
+    size_t off = 0, lo = 0, most = 0;
+    for (size_t t = 0; t < ntrials; ++t) {
+        h[t] = h_lengths[t];
+        h[ntrials + t] = off;
+        h[2 * ntrials + t] = h_lengths[t] / k;
+        h[3 * ntrials + t] = lo;
+        const double inv = h_std ? 1.0 / h_std[t] : 1.0;
+        memcpy(&h[4 * ntrials + t], &inv, sizeof(double));
+        off += h_lengths[t];
+        lo += h_lengths[t] / k;
+        most = std::max(most, (size_t)h_lengths[t]);
+    }
+    static_assert(sizeof(size_t) == sizeof(double), "one array for both");
+    RT_TRY_CUDA(scratch_malloc(blob, h.size() * sizeof(size_t), st));
+    // (pageable memory: the copy has read it when the call returns)
+    const cudaError_t e = cudaMemcpyAsync(*blob, h.data(), h.size() * sizeof(size_t),
+                                          cudaMemcpyHostToDevice, st);
+    if (e != cudaSuccess) {
+        cudaFreeAsync(*blob, st);
+        return check_cuda(e, "adjoint");
+    }
+    const size_t* d = static_cast<const size_t*>(*blob);
+    *B = AdjBatch{d, d + ntrials, d + 2 * ntrials, d + 3 * ntrials,
+                  reinterpret_cast<const double*>(d + 4 * ntrials)};
+    *total = off;
+    *lo_total = lo;
+    *max_len = most;
+    return RT_OK;
+}
+
+// gy = (g - mean g - z mean(g z)) / std of every series of the batch.
+static int normalise_adjoint(const float* d_g, const float* d_z, const AdjBatch& B, size_t ntrials,
+                             size_t max_len, float* d_gy, cudaStream_t st)
+{
+    const size_t most = std::max<size_t>(8, 148 * 16 / ntrials);
+    const unsigned blocks =
+        (unsigned)std::max<size_t>(1, std::min((max_len + kNormBwdThreads - 1) / kNormBwdThreads, most));
+    double2* part = nullptr;
+    RT_TRY_CUDA(scratch_malloc((void**)&part, blocks * ntrials * sizeof(double2), st));
+    const dim3 grid(blocks, (unsigned)ntrials);
+    k_norm_adj_sums<<<grid, kNormBwdThreads, 0, st>>>(d_g, d_z, B, part);
+    int s = check_cuda(cudaGetLastError(), "normalise_adjoint");
+    if (s == RT_OK) {
+        k_norm_adj_apply<<<grid, kNormBwdThreads, 0, st>>>(d_g, d_z, B, part, d_gy);
+        s = check_cuda(cudaGetLastError(), "normalise_adjoint");
+    }
+    cudaFreeAsync(part, st);
+    return s;
+}
+
 extern "C" int rt_normalise_adjoint(const float* d_g, const float* d_z, size_t size,
                                     double std_, float* d_gy, void* stream)
 {
@@ -379,16 +593,78 @@ extern "C" int rt_normalise_adjoint(const float* d_g, const float* d_z, size_t s
     if (size == 0) return RT_OK;
     if (!d_g || !d_z || !d_gy) return set_error(RT_EINVAL, "null argument");
     if (!(std_ > 0.0)) return set_error(RT_EINVAL, "std must be > 0");
-    const int blocks = (int)std::min<size_t>((size + kNormBwdThreads - 1) / kNormBwdThreads, 512);
-    double* part = nullptr;
-    RT_TRY_CUDA(scratch_malloc((void**)&part, (size_t)blocks * 2 * sizeof(double), st));
-    k_norm_adj_sums<<<blocks, kNormBwdThreads, 0, st>>>(d_g, d_z, size, part);
-    int s = check_cuda(cudaGetLastError(), "normalise_adjoint");
-    if (s == RT_OK) {
-        k_norm_adj_apply<<<blocks, kNormBwdThreads, 0, st>>>(d_g, d_z, size, part, blocks,
-                                                             1.0 / std_, d_gy);
-        s = check_cuda(cudaGetLastError(), "normalise_adjoint");
+    AdjBatch B;
+    void* blob = nullptr;
+    size_t total, lo, most;
+    const uint64_t len = size;
+    RT_TRY(adj_batch(&len, 1, &std_, 1, &B, &blob, &total, &lo, &most, st));
+    const int s = normalise_adjoint(d_g, d_z, B, 1, size, d_gy, st);
+    cudaFreeAsync(blob, st);
+    return s;
+}
+
+extern "C" int rt_front_adjoint(const float* d_x, const float* d_z, const float* d_gz,
+                                const uint64_t* h_lengths, size_t ntrials, const double* h_std,
+                                size_t width_samples, size_t min_points, float* d_gx, void* stream)
+{
+    cudaStream_t st = (cudaStream_t)stream;
+    if (!d_x || !d_gz || !d_gx || !h_lengths || (h_std && !d_z))
+        return set_error(RT_EINVAL, "null argument");
+    if (ntrials == 0) return RT_OK;
+    if (ntrials > 65535) return set_error(RT_EINVAL, "at most 65535 series per call");
+    size_t k = 1, width = 0;
+    if (min_points) {
+        // running_medians.py:72-80
+        if (!(min_points % 2)) return set_error(RT_EINVAL, "min_points must be an odd number");
+        k = (size_t)std::max(1.0, (double)width_samples / (double)min_points);
+        width = k == 1 ? width_samples : min_points;
+        if (!(width % 2)) return set_error(RT_EINVAL, "width must be an odd number");
+        if (width > (size_t)kAdjMaxWidth || k > (1u << 30))
+            return set_error(RT_EINVAL, "a running median of %zu points is too wide", width);
     }
-    cudaFreeAsync(part, st);
+    for (size_t t = 0; t < ntrials; ++t) {
+        if (h_lengths[t] == 0) return set_error(RT_EINVAL, "series %zu is empty", t);
+        if (min_points && !(width < h_lengths[t] / k))
+            return set_error(RT_EINVAL, "width must be < size");
+        if (min_points && h_lengths[t] / k >= (1ull << 32))
+            return set_error(RT_EINVAL, "series %zu is too long", t);
+        if (h_std && !(h_std[t] > 0.0)) return set_error(RT_EINVAL, "std must be > 0");
+    }
+    AdjBatch B;
+    void* blob = nullptr;
+    size_t total, lo_total, max_len;
+    RT_TRY(adj_batch(h_lengths, ntrials, h_std, k, &B, &blob, &total, &lo_total, &max_len, st));
+    int s = RT_OK;
+    if (h_std)
+        s = normalise_adjoint(d_gz, d_z, B, ntrials, max_len, d_gx, st);
+    else if (d_gx != d_gz)
+        s = check_cuda(cudaMemcpyAsync(d_gx, d_gz, total * sizeof(float), cudaMemcpyDeviceToDevice, st),
+                       "front_adjoint");
+    unsigned char* buf = nullptr;
+    if (s == RT_OK && min_points)
+        s = check_cuda(scratch_malloc((void**)&buf, lo_total * (2 * sizeof(double) + 8), st), "front_adjoint");
+    if (s == RT_OK && min_points) {
+        double* lores = reinterpret_cast<double*>(buf);
+        double* glo = lores + lo_total;
+        unsigned* sel = reinterpret_cast<unsigned*>(glo + lo_total);
+        float* gsel = reinterpret_cast<float*>(sel + lo_total);
+        const size_t max_lo = max_len / k;
+        const unsigned T = (unsigned)ntrials;
+        auto blocks = [](size_t n, size_t per) {
+            return (unsigned)std::max<size_t>(1, std::min<size_t>((n + per - 1) / per, 1 << 20));
+        };
+        k_dered_adj_points<<<dim3(blocks(max_lo, 8), T), 256, 0, st>>>(d_x, d_gx, B, (int)k, lores, glo);
+        k_dered_adj_select<<<dim3((unsigned)((max_lo + kAdjTile - 1) / kAdjTile), T), kAdjTile, 0, st>>>(
+            lores, B, (int)width, sel);
+        k_dered_adj_gather<<<dim3(blocks(max_lo, 128), T), 128, 0, st>>>(glo, sel, B, (int)width,
+                                                                        (int)k, gsel);
+        if (k == 1)
+            k_dered_adj_apply1<<<dim3(blocks(max_lo, 1024), T), 256, 0, st>>>(gsel, B, d_gx);
+        else
+            k_dered_adj_apply<<<dim3(blocks(max_lo, 1), T), 256, 0, st>>>(gsel, B, (int)k, d_gx);
+        s = check_cuda(cudaGetLastError(), "front_adjoint");
+    }
+    if (buf) cudaFreeAsync(buf, st);
+    cudaFreeAsync(blob, st);
     return s;
 }

@@ -239,18 +239,33 @@ class DifferentiableSearch(object):
                                 dtype=np.int64).reshape(-1, 6)
         return self._tr
 
+    # widest running median (points) of the native adjoint; torch's median takes wider ones
+    _max_native_width = 257
+
     def _through_front(self, x, gz_all, z_all, stds):
         """From the gradient with respect to the searched series to the one with respect to x:
         normalisation, then deredden."""
         torch = libcpp._t()
+        if not (self.normalise or self.deredden):
+            return gz_all
+        k = int(max(1, self.rmed_width_samples / float(self.rmed_minpts)))
+        width = self.rmed_width_samples if k == 1 else self.rmed_minpts
+        if not self.deredden or width <= self._max_native_width:
+            gx = torch.empty_like(gz_all)
+            xc = x.detach().contiguous()
+            std = (ctypes.c_double * self.bs.num_trials)(*[float(s) for s in stds])
+            _lib.check(_lib.load().rt_front_adjoint(
+                libcpp._ptr(xc), libcpp._ptr(z_all), libcpp._ptr(gz_all),
+                self.bs.lengths.ctypes.data_as(_lib._u64p), self.bs.num_trials,
+                std if self.normalise else None, self.rmed_width_samples,
+                self.rmed_minpts if self.deredden else 0, libcpp._ptr(gx), libcpp._stream()))
+            return gx
         gx = torch.empty_like(x) if self.normalise else gz_all
         if self.normalise:
             for t in range(self.bs.num_trials):
                 a, e = int(self.offsets[t]), int(self.offsets[t + 1])
                 gx[a:e] = normalise_adjoint(gz_all[a:e], z_all[a:e], float(stds[t]))
-        if self.deredden:
-            gx = gx - self._rmed_adjoint_batch(x.detach(), gx)
-        return gx
+        return gx - self._rmed_adjoint_batch(x.detach(), gx)
 
     def _rmed_adjoint_batch(self, x, g):
         """_rmed_adjoint over every trial: one batched call when all trials have the same
