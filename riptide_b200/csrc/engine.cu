@@ -1192,8 +1192,7 @@ struct SearchPlan {
     WorkItem* d_items = nullptr;
     StagePlan* d_plans = nullptr;
     float* d_scratch = nullptr;
-    int* d_counters = nullptr;          // done + slot_release + error
-    unsigned long long* d_ticket = nullptr;
+    int* d_counters = nullptr;          // ticket (8 bytes) + done + slot_release + error
     float* d_ds = nullptr;
     float* d_y = nullptr;               // dereddened series
     float* d_norm = nullptr;            // normalised copy (when a cycle has f == 1)
@@ -1443,7 +1442,7 @@ static void dfree(T*& p)
 static void plan_free_device(SearchPlan& P)
 {
     dfree(P.d_widths); dfree(P.d_xforms); dfree(P.d_items); dfree(P.d_plans);
-    dfree(P.d_scratch); dfree(P.d_counters); dfree(P.d_ticket); dfree(P.d_ds); dfree(P.d_y);
+    dfree(P.d_scratch); dfree(P.d_counters); dfree(P.d_ds); dfree(P.d_y);
     dfree(P.d_norm); dfree(P.d_lores); dfree(P.d_rmed); dfree(P.d_part);
     dfree(P.d_mean); dfree(P.d_normv); dfree(P.d_len); dfree(P.d_off); dfree(P.d_lo_len);
     dfree(P.d_lo_off); dfree(P.d_f); dfree(P.d_useseg); dfree(P.d_dsoff);
@@ -1480,6 +1479,9 @@ static int upload(SearchPlan& P, T** p, const std::vector<T>& v)
 
 static int plan_alloc_device(SearchPlan& P);
 
+// Counters of a run, in one array: the ticket, the stage counts, the slot releases, the error.
+static size_t plan_counters(const SearchPlan& P) { return 2 + (size_t)P.nseq * kMaxStages + kSlots + 1; }
+
 // Allocates and fills the plan's device buffers once. On failure every buffer allocated so
 // far is released again, so a failed call leaks nothing and can be retried.
 static int plan_prepare_device(SearchPlan& P)
@@ -1503,8 +1505,7 @@ static int plan_alloc_device(SearchPlan& P)
     RT_TRY(upload(P, &P.d_plans, P.plans));
     RT_TRY(upload(P, &P.d_xforms, P.xforms));
     RT_TRY(dalloc(P, &P.d_scratch, (size_t)kSlots * 2 * std::max<size_t>(P.slot_floats, 1)));
-    RT_TRY(dalloc(P, &P.d_counters, (size_t)P.nseq * kMaxStages + kSlots + 1));
-    RT_TRY(dalloc(P, &P.d_ticket, 1));
+    RT_TRY(dalloc(P, &P.d_counters, plan_counters(P)));
     // + 16 floats: bulk copies read whole 16-byte units around a block of rows
     RT_TRY(dalloc(P, &P.d_ds, P.ds_total + 16));
     if (P.cfg.deredden) {
@@ -1619,9 +1620,7 @@ static int plan_run(SearchPlan& P, const float* data, float* normalised_out, dou
     }
     if (P.timing) RT_TRY_CUDA(cudaEventRecord(P.ev[2], st));
     // counters
-    const size_t ncounters = (size_t)P.nseq * kMaxStages + kSlots + 1;
-    RT_TRY_CUDA(cudaMemsetAsync(P.d_counters, 0, ncounters * sizeof(int), st));
-    RT_TRY_CUDA(cudaMemsetAsync(P.d_ticket, 0, sizeof(unsigned long long), st));
+    RT_TRY_CUDA(cudaMemsetAsync(P.d_counters, 0, plan_counters(P) * sizeof(int), st));
     EngineArgs A;
     A.ds = P.d_ds;
     A.norm = zsrc;
@@ -1635,10 +1634,10 @@ static int plan_run(SearchPlan& P, const float* data, float* normalised_out, dou
     A.nfast = P.nfast;
     A.scratch = P.d_scratch;
     A.slot_floats = P.slot_floats;
-    A.done = P.d_counters;
-    A.slot_release = P.d_counters + (size_t)P.nseq * kMaxStages;
+    A.done = P.d_counters + 2;
+    A.slot_release = A.done + (size_t)P.nseq * kMaxStages;
     A.error = A.slot_release + kSlots;
-    A.ticket = P.d_ticket;
+    A.ticket = reinterpret_cast<unsigned long long*>(P.d_counters);
     A.phase_cycles = P.d_phase;
     A.spin_limit = P.spin_limit;
     A.dep_bias = P.dep_bias;
@@ -1664,8 +1663,7 @@ static int plan_run(SearchPlan& P, const float* data, float* normalised_out, dou
 static int plan_check_error(SearchPlan& P, cudaStream_t st)
 {
     int err = 0;
-    RT_TRY_CUDA(cudaMemcpyAsync(&err, P.d_counters + (size_t)P.nseq * kMaxStages + kSlots,
-                                sizeof(int), cudaMemcpyDeviceToHost, st));
+    RT_TRY_CUDA(cudaMemcpyAsync(&err, P.d_counters + plan_counters(P) - 1, sizeof(int), cudaMemcpyDeviceToHost, st));
     RT_TRY_CUDA(cudaStreamSynchronize(st));
     if (err == RT_ETIMEOUT)
         return set_error(RT_ETIMEOUT, "a bounded wait in the search kernel ran out");

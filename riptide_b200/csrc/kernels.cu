@@ -204,6 +204,16 @@ static FfaLayout stage_layout(int m, int b)
     return ffa_layout(kFfaSmemBytes - kStageTreeBytes, b, (size_t)m);
 }
 
+// Copies one float to shared memory in the background (no register, so any number is in flight).
+__device__ __forceinline__ void copy_async4(float* dst, const float* src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_async_wait()
+{
+    asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
 // Copies the source rows of a later-stage job (rows of b floats in global memory, laid out by
 // build_job_tree_warp) into `sbuf`, each with its halo.
 __device__ void stage_rows_halo(const JobTree& T, const float* __restrict__ src, int b, float* sbuf,
@@ -222,8 +232,7 @@ __device__ void stage_rows_halo(const JobTree& T, const float* __restrict__ src,
         const int k = r - T.src_off[lo];
         const float* from = src + (size_t)(k < rg.y ? rg.x + k : rg.z + k - rg.y) * b;
         float* to = sbuf + (size_t)r * stride;
-#pragma unroll 4
-        for (int c = lane; c < b + kHalo; c += 32) to[c] = __ldg(from + (c < b ? c : c % b));
+        for (int c = lane; c < b + kHalo; c += 32) copy_async4(to + c, from + (c < b ? c : c % b));
     }
 }
 
@@ -246,14 +255,14 @@ __global__ void __launch_bounds__(kThreads, 1)
         // raw input rows, as one block (it fits: no more rows than a level holds)
         const float* from = src + (size_t)J.root_row0 * b;
         const int n = J.root_rows * b;
-#pragma unroll 4
-        for (int i = threadIdx.x; i < n; i += kThreads) buf1[i] = __ldg(from + i);
+        for (int i = threadIdx.x; i < n; i += kThreads) copy_async4(buf1 + i, from + i);
         io.staged = buf1 - (ptrdiff_t)J.root_row0 * b;
     }
     if (threadIdx.x < 32) build_job_tree_warp(T, J, b, ffa_cap_rows(L, b), L.ops_units, stage == 0);
     cta_sync();
     if (T.error) {
         if (threadIdx.x == 0 && err) atomicExch(err, RT_EINTERNAL);
+        copy_async_wait();
         return;
     }
     if (stage > 0 && T.pstaged) {
@@ -262,6 +271,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         io.staged_rows = true;
     }
     build_ops(T, b, ops);
+    copy_async_wait();
     cta_sync();
     bool ok = true;
     const float* root = run_job_levels(T, b, buf1, buf0, stride, ops, io, &ok);
@@ -289,24 +299,30 @@ bool plan_stages(int m, int b, int rows_out, int cap_rows, int snr_rows, StagePl
         ++D;
         if (D > 20) return false;
     }
-    int ns = 0;
     P->D[0] = D;
     P->R[0] = (m + (1 << D) - 1) >> D;
     P->jobs[0] = 1 << D;
     P->jobs_per_node[0] = 1;
-    ns = 1;
+    int ns = 1;
+    // rows of a job of e levels: cap - 3 2^(e-1), two less for 1 to 3 levels (their staged
+    // source rows can be two more than the bound of the levels)
+    auto rows_of = [&](int e) {
+        const int R = cap_rows - 3 * (1 << (e - 1));
+        return e <= 3 && R > 4 ? R - 2 : R;
+    };
+    // most levels of a stage: the jobs keep half the capacity as rows
+    int emax = std::min({std::max(D, 1), max_depth + 1, kMaxTreeDepth + 1});
+    while (emax > 1 && cap_rows - 3 * (1 << (emax - 1)) < cap_rows / 2) --emax;
+    int left = (D + emax - 1) / emax;  // stages to come
+    if (left >= kMaxStages) return false;
     while (D > 0) {
-        if (ns >= kMaxStages) return false;
-        // largest step e such that R = cap - 3 * 2^(e-1) stays >= cap / 2 (at least 1 level)
-        int e = std::min({D, max_depth + 1, kMaxTreeDepth + 1});
-        int R = 0;
-        for (; e >= 1; --e) {
-            R = cap_rows - 3 * (1 << (e - 1));
-            if (R >= cap_rows / 2 || e == 1) break;
-        }
+        // The fewest stages. In the search the first ones take the most levels (sharing them out
+        // leaves more rows a job, but slowed two trials of 2^23 samples at bins 480-520 from
+        // 11.17 to 11.30 ms: the last stage, which also has the S/N to do, got more levels).
+        // A transform of its own shares them out (16384 x 488: 184 to 178 us).
+        const int e = snr_rows > 0 ? std::min(emax, D) : (D + left - 1) / left;
+        int R = rows_of(e);
         if (R < 1) return false;
-        // (the staged source rows of 1 to 3 levels can be two more than the bound of the levels)
-        if (e <= 3 && R > 4) R -= 2;
         const int Dn = D - e;
         const int node_rows = (m + (1 << Dn) - 1) >> Dn;
         const int need = (Dn == 0) ? rows_out : node_rows;
@@ -318,6 +334,7 @@ bool plan_stages(int m, int b, int rows_out, int cap_rows, int snr_rows, StagePl
         P->jobs_per_node[ns] = per_node;
         P->jobs[ns] = P->jobs_per_node[ns] << Dn;
         ++ns;
+        --left;
         D = Dn;
     }
     P->nstages = ns;
@@ -328,10 +345,18 @@ int ffa_transform(const float* in, int m, int b, int rows_out, float* out, float
                   int* d_err, cudaStream_t st)
 {
     const FfaLayout L = stage_layout(m, b);
-    const int cap = ffa_cap_rows(L, b);
+    int cap = ffa_cap_rows(L, b);
     StagePlan P;
     if (cap < 4 || !plan_stages(m, b, rows_out, cap, 0, &P))
         return set_error(RT_EINVAL, "FFA transform of %d x %d does not fit the device plan", m, b);
+    // A small transform has fewer jobs than the GPU has SMs: jobs of half the rows as long as
+    // that takes no further stage (300 x 251: 4 jobs a stage, 17 + 14 us, against 8 and 9 jobs).
+    for (int c = cap / 2; c >= 16 && P.nstages > 1 && P.jobs[P.nstages - 1] < 148; c /= 2) {
+        StagePlan Q;
+        if (!plan_stages(m, b, rows_out, c, 0, &Q) || Q.nstages != P.nstages) break;
+        P = Q;
+        cap = c;
+    }
     // what the device checks of every job (level rows and node lists that fit), for all of them:
     // a level d of a later-stage job of R rows holds at most R + 3 2^d rows
     for (int s = 0; s < P.nstages; ++s) {
@@ -409,8 +434,13 @@ int snr2(const float* x, size_t rows, size_t cols, const int* h_widths, int nw, 
     int wmax = 0;
     for (int k = 0; k < nw; ++k) wmax = std::max(wmax, h_widths[k]);
     const int nfast = detect_fast_widths(h_widths, nw);
-    const int tile = std::min<int>(snr_tile_rows((int)cols, wmax), 1024);
+    int tile = std::min<int>(snr_tile_rows((int)cols, wmax), 1024);
     if (tile < 1) return set_error(RT_EINVAL, "profiles of %zu bins are too long", cols);
+    // one CTA per SM (it holds the whole shared memory): whole warps of profiles per CTA, as few
+    // as give every SM some (4,099 profiles as 24 CTAs of 173 took 31 us)
+    const size_t per_warp = 32 / snr_tpr((int)cols);
+    const size_t share = ((rows + 147) / 148 + per_warp - 1) / per_warp * per_warp;
+    tile = (int)std::min<size_t>(tile, share);
     const int grid = (int)std::min<size_t>((rows + tile - 1) / tile, 148 * 4);
     if (nw > kMaxWidths) return set_error(RT_EINVAL, "at most %d trial widths are supported", kMaxWidths);
     WidthList W{};
@@ -445,7 +475,7 @@ int snr2(const float* x, size_t rows, size_t cols, const int* h_widths, int nw, 
 // Factors with f + 2 > kDsHalo use k_downsample_wide instead.
 //
 // Layout of the work: a lane owns 4 consecutive staged samples of each 128-sample chunk of
-// its warp's 512, read as 16-byte vectors (realigned in registers when the segment does not
+// its warp's share (512, 128 in the small shape), read as 16-byte vectors (realigned in registers when the segment does not
 // start on a 16-byte boundary, so the staged values and the order of the prefix sums do not
 // depend on where the series lies in memory). The prefix is a 4-sample scan in the lane and a
 // shuffle scan of the lanes' totals. Outputs of all cycles form one index range; a table gives
@@ -460,13 +490,13 @@ __device__ __forceinline__ size_t first_k_at_or_after(size_t i0, double f)
     return k;
 }
 
-constexpr int kDsThreads = 512;
-constexpr int kDsWarps = kDsThreads / 32;
-constexpr int kDsPerWarp = kDsStage / kDsWarps;  // staged samples per warp
-constexpr int kDsQuads = kDsPerWarp / 128;       // 128-sample chunks per warp, 4 samples a lane
 constexpr int kDsTab = 1024;                     // 32-output chunks with a tabulated cycle
-static_assert(kDsPerWarp % 128 == 0, "whole chunks");
-static_assert(kDsMaxCycles <= 256, "cycle numbers are stored in bytes");
+static_assert(kDsMaxCycles <= 256, "cycle numbers are stored in bytes, found by a thread each");
+// Threads and staged samples of the kernel's two shapes: the small one for a few short series
+// (up to 128 CTAs of the large one), where the factors allow its halo. 2^15 samples, 24 factors:
+// 36 us as 5 large CTAs.
+constexpr int kDsThreads = 512, kDsSmallThreads = 256;
+constexpr int kDsSmallStage = 1024, kDsSmallHalo = 256;
 
 // The 16-byte-aligned group A[j .. j+3] (j a multiple of 4), zero outside [lo, hi).
 __device__ __forceinline__ float4 ds_group(const float* A, int j, int lo, int hi)
@@ -485,9 +515,14 @@ __device__ __forceinline__ float ds_normalised(float x, double mean, double inv)
     return __double2float_rn(__ddiv_rn(__dsub_rn((double)x, mean), inv));
 }
 
-__global__ void __launch_bounds__(kDsThreads, 2)
+template <int kDsThreads, int kDsStage>
+__global__ void __launch_bounds__(kDsThreads, 1024 / kDsThreads)
     k_downsample_segments(DsJob job)
 {
+    constexpr int kDsWarps = kDsThreads / 32;
+    constexpr int kDsPerWarp = kDsStage / kDsWarps;  // staged samples per warp
+    constexpr int kDsQuads = kDsPerWarp / 128;       // 128-sample chunks per warp, 4 samples a lane
+    static_assert(kDsPerWarp % 128 == 0, "whole chunks");
     extern __shared__ __align__(16) unsigned char smem[];
     double* P = reinterpret_cast<double*>(smem);                    // kDsStage + 1 (+1 pad)
     float* zs = reinterpret_cast<float*>(P + kDsStage + 2);          // kDsStage
@@ -724,13 +759,17 @@ int launch_downsample(const DsJob& job_in, int ntrials, size_t max_len, cudaStre
     }
     // halo >= f + 1 for every segment factor (ds_use_segments: f + 2 <= kDsHalo), in whole warps
     const int halo = std::min(kDsHalo, ((int)ceil(fmax) + 2 + 31) & ~31);
-    job.seg = kDsStage - halo;
     if (any_seg) {
-        const size_t smem = (kDsStage + 2) * sizeof(double) + kDsStage * sizeof(float);
-        RT_TRY_CUDA(cudaFuncSetAttribute(k_downsample_segments,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        const size_t large = (max_len + (kDsStage - halo) - 1) / (kDsStage - halo) * ntrials;
+        const bool small = halo <= kDsSmallHalo && large <= 128;
+        const int stage = small ? kDsSmallStage : kDsStage;
+        job.seg = stage - halo;
+        const size_t smem = (stage + 2) * sizeof(double) + stage * sizeof(float);
+        void (*kernel)(DsJob) = small ? k_downsample_segments<kDsSmallThreads, kDsSmallStage>
+                                      : k_downsample_segments<kDsThreads, kDsStage>;
+        RT_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         dim3 grid((unsigned)((max_len + job.seg - 1) / job.seg), (unsigned)ntrials);
-        k_downsample_segments<<<grid, kDsThreads, smem, st>>>(job);
+        kernel<<<grid, small ? kDsSmallThreads : kDsThreads, smem, st>>>(job);
         RT_TRY_CUDA(cudaGetLastError());
     }
     for (int c = 0; c < job.ncycles; ++c) {
