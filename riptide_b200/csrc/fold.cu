@@ -382,7 +382,14 @@ extern "C" int rt_fold_batched(const float* d_in, size_t size, double tsamp,
     }
     const size_t job_bytes = (count * sizeof(FoldJob) + 255) & ~size_t(255);
     char* scratch = nullptr;
-    RT_TRY_CUDA(scratch_malloc((void**)&scratch, job_bytes + block * sizeof(float), stream));
+    bool no_block = false;
+    cudaError_t room = scratch_malloc((void**)&scratch, job_bytes + block * sizeof(float), stream);
+    if (room == cudaErrorMemoryAllocation && block > 0) {  // no room for blocks: none is written
+        cudaGetLastError();
+        no_block = true;
+        room = scratch_malloc((void**)&scratch, job_bytes, stream);
+    }
+    if (room != cudaSuccess) return check_cuda(room, "fold scratch memory");
     FoldJob* d_jobs = reinterpret_cast<FoldJob*>(scratch);
     float* d_blocks = reinterpret_cast<float*>(scratch + job_bytes);
     cudaError_t e = cudaMemcpyAsync(d_jobs, jobs.data(), count * sizeof(FoldJob),
@@ -390,7 +397,7 @@ extern "C" int rt_fold_batched(const float* d_in, size_t size, double tsamp,
     for (const Batch& B : batches) {
         if (e != cudaSuccess) break;
         const unsigned n = (unsigned)(B.end - B.first);
-        if (B.direct) {
+        if (B.direct || (no_block && B.block > 0)) {
             const size_t bx = std::min<size_t>((B.most + 127) / 128, 4096);
             k_fold<<<dim3((unsigned)bx, n), 128, 0, stream>>>(d_in, size, d_jobs + B.first, d_out);
             e = cudaGetLastError();
