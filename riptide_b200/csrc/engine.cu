@@ -318,8 +318,7 @@ __device__ void scheduler_warp(const EngineArgs& A, Handover& H, JobTree* trees,
         }
         signal_item_done(A, L);
     };
-    auto claim = [&]() {  // a pool entry with the next item, -1: no more
-        const long long t = (long long)atomicAdd(A.ticket, 1ull);
+    auto claimed = [&](long long t) {  // a pool entry with item t, -1: no more
         if (t >= A.nitems) {
             exhausted = true;
             return -1;
@@ -330,6 +329,7 @@ __device__ void scheduler_warp(const EngineArgs& A, Handover& H, JobTree* trees,
         if (A.phase_cycles) atomicAdd(A.phase_cycles + 10, 1ull);
         return i;
     };
+    auto claim = [&]() { return claimed((long long)atomicAdd(A.ticket, 1ull)); };
     int k = 0;
     for (;; ++k) {
         const int s = k & 1;
@@ -425,20 +425,23 @@ __device__ void scheduler_warp(const EngineArgs& A, Handover& H, JobTree* trees,
             build_job_tree_warp(trees[s], L.J, L.X.b, L.cap_rows, A.layout.ops_units, L.stage == 0);
             const bool fill = L.last && snr[s].b != L.X.b;
             __syncwarp();
-            if (fill) snr_params_fill_warp(snr[s], A.widths, A.nw, A.nfast, L.X.b);
+            if (fill) snr_coefs_warp(snr[s], L.X.b);
             if (k == 0) stage_item(A, L, trees[0], level_buffer(smem, A, staging_buffer(-1)), bar);
         }
         __syncwarp();
         if (lane == 0) {
             mbar_arrive(reinterpret_cast<uint64_t*>(H.full + s));
+            const bool more = !stop && ahead < 0 && !exhausted &&
+                              L.ticket + 8 * (long long)gridDim.x < A.nitems;
+            long long t = 0;
+            if (more) t = (long long)atomicAdd(A.ticket, 1ull);
             if (owed >= 0) {
                 settle(owed, stored[s]);
                 free_mask |= 1u << owed;
             }
             pending[s] = true;
             stored[s] = false;
-            if (!stop && ahead < 0 && !exhausted && L.ticket + 8 * (long long)gridDim.x < A.nitems)
-                ahead = claim();
+            if (more) ahead = claimed(t);
         }
         if (stop) break;
     }
@@ -466,12 +469,14 @@ __global__ void __launch_bounds__(kEngineThreads, 1) k_search_persistent(EngineA
         mbar_init(staged, 1);
         mbar_init(full, 1);
         mbar_init(full + 1, 1);
-        snr[0].b = snr[1].b = 0;
         H.pool[kPool].ok = 0;
         H.pool[kPool].ticket = A.nitems;
     }
     __syncthreads();
     if (threadIdx.x >= kThreads) {
+        // (read from memory for every profile length, they took longer than the node lists)
+        snr_widths_warp(snr[0], A.widths, A.nw, A.nfast);
+        snr_widths_warp(snr[1], A.widths, A.nw, A.nfast);
         scheduler_warp(A, H, trees, snr, smem);
         return;
     }

@@ -75,7 +75,7 @@ struct Node {
     int hbias, tbias;  // row r of the head / tail child is row hbias + r / tbias + r of the
                        // level below's buffer, of the staged rows, or of the transform
     int thr;    // last even row s with h(s) = s / 2 (odd rows: see head_row)
-    float kh;   // head slope of the node (merge_coef)
+    float kh;   // head slope of the node (merge_coef), where rows follow no pattern
 };
 
 // One pass over a job's shared-memory levels: level d from level d + 1 by row groups, or
@@ -132,43 +132,67 @@ RT_HD int max_full_depth(int b) { return b >= kWideMinBins ? kMaxJobDepth : kMax
 // share their tail row (t(s) = t(s + 1), and mostly their head row): for a node of n rows the
 // group of row s is (s + n % 2) / 2. For every n up to kRegularRows that number is t(s) itself,
 // and h(s) is t(s) (n even), t(s) - 1 (n odd, s odd), or one of the two (n odd, s even: t(s) up
-// to the middle row n / 2 or the even row before it, t(s) - 1 beyond it): the CPU tests check
-// every n and s. From n = 8195 on the float32 slope moves that middle row, and only the row
-// groups (which read each row's own numbers) are used.
+// to the middle row n / 2 or, where that is odd, the row before it, t(s) - 1 beyond it): the CPU
+// tests check every n and s. From n = 8195 on the float32 slope moves that middle row, and only
+// the row groups (which read each row's own numbers) are used.
 constexpr int kRegularRows = 8192;
 RT_HD int group_of(int n, int s) { return (s + (n & 1)) >> 1; }
 
 // h(s) of a node of at most kRegularRows rows, thr as in Node.
-__device__ __forceinline__ int head_row(const Node& nd, int s)
+__device__ __forceinline__ int head_threshold(int rows)
 {
-    return (s >> 1) - (int)((s > nd.thr) & ((s & 1) ^ 1));
+    return (rows & 1) ? (rows >> 1) & ~1 : 0x7fffffff;
 }
+__device__ __forceinline__ int head_row(int thr, int s)
+{
+    return (s >> 1) - (int)((s > thr) & ((s & 1) ^ 1));
+}
+__device__ __forceinline__ int head_row(const Node& nd, int s) { return head_row(nd.thr, s); }
 
 // Node q of a job's node list in heap order (1: the root, 2 q and 2 q + 1: the head and tail
 // children of q): its row range follows from the root's by the head/tail row maps along the
-// path to it. Every lane of a warp walks to a node of its own.
-__device__ __forceinline__ Node walk_to_node(const JobSpec& J, int q, int maxdepth)
+// path to it. Every lane of a warp walks to a node of its own. `regular`: at most kRegularRows
+// rows, whole-number maps (with the slopes, a division per level, the walk was most of the node
+// lists' time).
+__device__ __forceinline__ Node walk_to_node(const JobSpec& J, int q, int maxdepth, bool regular)
 {
     Node nd;
     nd.row0 = J.root_row0;
     nd.rows = J.root_rows;
     nd.lo = J.lo;
     nd.hi = J.hi;
+    nd.kh = 0.0f;
     const int d = 31 - __clz(q);
-    for (int k = 0; k < maxdepth; ++k) {
-        if (k >= d) break;
-        const int tail = (q >> (d - 1 - k)) & 1;
-        const int mh = nd.rows >> 1;
-        const int n = tail ? nd.rows - mh : mh;
-        const float slope = __fdiv_rn((float)n - 1.0f, (float)nd.rows - 1.0f);  // merge_coef
-        nd.row0 += tail ? mh : 0;
-        nd.rows = n;
-        nd.lo = merge_row(slope, nd.lo);
-        nd.hi = merge_row(slope, nd.hi - 1) + 1;
+    if (regular) {
+        for (int k = 0; k < maxdepth; ++k) {
+            if (k >= d) break;
+            const int mh = nd.rows >> 1, thr = head_threshold(nd.rows);
+            if ((q >> (d - 1 - k)) & 1) {
+                nd.lo = group_of(nd.rows, nd.lo);
+                nd.hi = group_of(nd.rows, nd.hi - 1) + 1;
+                nd.row0 += mh;
+                nd.rows -= mh;
+            } else {
+                nd.lo = head_row(thr, nd.lo);
+                nd.hi = head_row(thr, nd.hi - 1) + 1;
+                nd.rows = mh;
+            }
+        }
+    } else {
+        for (int k = 0; k < maxdepth; ++k) {
+            if (k >= d) break;
+            const int tail = (q >> (d - 1 - k)) & 1;
+            const int mh = nd.rows >> 1;
+            const int n = tail ? nd.rows - mh : mh;
+            const float slope = __fdiv_rn((float)n - 1.0f, (float)nd.rows - 1.0f);  // merge_coef
+            nd.row0 += tail ? mh : 0;
+            nd.rows = n;
+            nd.lo = merge_row(slope, nd.lo);
+            nd.hi = merge_row(slope, nd.hi - 1) + 1;
+        }
+        nd.kh = merge_coef(nd.rows).kh;
     }
-    nd.kh = merge_coef(nd.rows).kh;
-    const int half = (nd.rows >> 1) & ~1;
-    nd.thr = !(nd.rows & 1) ? 0x7fffffff : merge_row(nd.kh, half) == half >> 1 ? half : half - 2;
+    nd.thr = head_threshold(nd.rows);
     nd.hbias = nd.row0;
     nd.tbias = nd.row0 + (nd.rows >> 1);
     nd.off = nd.goff = nd.qoff = 0;
@@ -203,11 +227,12 @@ __device__ inline void build_job_tree_warp(JobTree& T, const JobSpec& J, int b, 
     }
     __syncwarp();
     int first_op = b < kWideMinBins ? -1 : depth - 1;
-    for (int half = 0; half < (depth == kMaxTreeDepth ? 2 : 1); ++half) {
+    const int halves = depth == kMaxTreeDepth ? 2 : 1;
+    for (int half = 0; half < halves; ++half) {
         const int q = half ? 32 + lane : lane + 1;
         const int d = 31 - __clz(q), i = q - (1 << d);  // level, node of the level
         const bool live = d <= depth && d < (half ? 6 : 5);
-        Node nd = walk_to_node(J, live ? q : 1, depth);
+        Node nd = walk_to_node(J, live ? q : 1, depth, regular);
         // rows stored, row groups, and row groups of tail children (the quads of the level
         // above) of the node, scanned together: 11, 10 and 10 bits. The fused level stores
         // whole nodes.
@@ -217,13 +242,55 @@ __device__ inline void build_job_tree_warp(JobTree& T, const JobSpec& J, int b, 
             const int grp = group_of(nd.rows, nd.hi - 1) - group_of(nd.rows, nd.lo) + 1;
             v = rows | (grp << 11) | ((i & 1) ? (unsigned)grp << 21 : 0u);
         }
+        // rows each level-G node needs from its two children, as consecutive staged blocks
+        const bool source = !raw && half == halves - 1;
+        const bool mine = source && live && d == depth;
+        int v2 = 0;
+        bool two = true;
+        int4 rg = make_int4(0, 0, 0, 0);
+        if (mine) {
+            rg = make_int4(nd.row0, 0, nd.row0 + (nd.rows >> 1), 0);
+            two = nd.rows >= 2;
+            if (two) {
+                const float kt = regular ? 0.f : merge_coef(nd.rows).kt;
+                const int hlo = regular ? head_row(nd, nd.lo) : merge_row(nd.kh, nd.lo);
+                const int hhi = regular ? head_row(nd, nd.hi - 1) : merge_row(nd.kh, nd.hi - 1);
+                const int tlo = regular ? group_of(nd.rows, nd.lo) : merge_row(kt, nd.lo);
+                const int thi = regular ? group_of(nd.rows, nd.hi - 1) : merge_row(kt, nd.hi - 1);
+                rg = make_int4(rg.x + hlo, hhi + 1 - hlo, rg.z + tlo, thi + 1 - tlo);
+            }
+            v2 = rg.y + rg.w;
+        }
+        // both scans along the nodes of a level, at most 2^depth of them
         unsigned incl = v;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
+        int incl2 = v2;
+        for (int o = 1; o < (1 << depth); o <<= 1) {
             const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (i >= o) incl += y;
+            const int y2 = __shfl_up_sync(0xffffffffu, incl2, o);
+            if (i >= o) {
+                incl += y;
+                incl2 += y2;
+            }
         }
         const unsigned excl = incl - v;
+        bool staged = false;
+        if (source) {
+            const int total = __shfl_sync(0xffffffffu, incl2, half ? 31 : (2 << depth) - 2);
+            staged = __all_sync(0xffffffffu, two) && total <= cap_rows;
+            if (lane == 0) {
+                T.src_off[1 << depth] = total;
+                T.pstaged = staged ? 1 : 0;
+            }
+            if (mine) {
+                T.src_rng[i] = rg;
+                T.src_off[i] = incl2 - v2;
+            }
+            if (staged && mine) {
+                nd.hbias += incl2 - v2 - rg.x;
+                nd.tbias += incl2 - v2 + rg.y - rg.z;
+            }
+            if (staged && b >= kWideMinBins) first_op = depth;
+        }
         if (live) {
             nd.off = excl & 0x7ff;
             nd.goff = (excl >> 11) & 0x3ff;
@@ -245,60 +312,26 @@ __device__ inline void build_job_tree_warp(JobTree& T, const JobSpec& J, int b, 
                 parent.hbias = nd.off - nd.lo;
             }
         }
-        if (!raw && half == (depth == kMaxTreeDepth ? 1 : 0)) {
-            // rows each level-G node needs from its two children, as consecutive staged blocks
-            const bool mine = live && d == depth;
-            int v2 = 0;
-            bool two = true;
-            int4 rg = make_int4(0, 0, 0, 0);
-            if (mine) {
-                rg = make_int4(nd.row0, 0, nd.row0 + (nd.rows >> 1), 0);
-                two = nd.rows >= 2;
-                if (two) {
-                    const float kt = regular ? 0.f : merge_coef(nd.rows).kt;
-                    const int hlo = merge_row(nd.kh, nd.lo), hhi = merge_row(nd.kh, nd.hi - 1);
-                    const int tlo = regular ? group_of(nd.rows, nd.lo) : merge_row(kt, nd.lo);
-                    const int thi = regular ? group_of(nd.rows, nd.hi - 1) : merge_row(kt, nd.hi - 1);
-                    rg = make_int4(rg.x + hlo, hhi + 1 - hlo, rg.z + tlo, thi + 1 - tlo);
-                }
-                v2 = rg.y + rg.w;
-                T.src_rng[i] = rg;
-            }
-            int incl2 = v2;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, incl2, o);
-                if (i >= o) incl2 += y;
-            }
-            if (mine) T.src_off[i] = incl2 - v2;
-            const int total = __shfl_sync(0xffffffffu, incl2, half ? 31 : (2 << depth) - 2);
-            const bool staged = __all_sync(0xffffffffu, two) && total <= cap_rows;
-            if (lane == 0) {
-                T.src_off[1 << depth] = total;
-                T.pstaged = staged ? 1 : 0;
-            }
-            if (staged && mine) {
-                T.nodes[q - 1].hbias += incl2 - v2 - rg.x;
-                T.nodes[q - 1].tbias += incl2 - v2 + rg.y - rg.z;
-            }
-            if (staged && b >= kWideMinBins) first_op = depth;
-        }
-        __syncwarp();
     }
     // the passes over levels first_op .. 0: two levels at a time from the deepest up, a single
-    // one last when their number is odd
-    if (lane == 0) {
-        int ns = 0, unit = 0;
-        for (int d = first_op; d >= 0; --d) {
-            const bool two = d >= 1 && regular;
-            const int count = two ? T.level_tails[d] : T.level_groups[d];
-            if (two) --d;
-            T.steps[ns++] = Step{d, two ? 1 : 0, unit, count};
-            unit += two ? 2 * count : count;
+    // one last when their number is odd; lane j has pass j
+    {
+        const int width = regular ? 2 : 1, ns = (first_op + width) / width;
+        int d = first_op - lane * width;
+        const bool live = lane < ns, two = live && regular && d >= 1;
+        const int count = !live ? 0 : two ? T.level_tails[d] : T.level_groups[d];
+        const int units = two ? 2 * count : count;
+        int end = units;
+        for (int o = 1; o < 8; o <<= 1) {  // at most kMaxTreeDepth + 1 passes
+            const int y = __shfl_up_sync(0xffffffffu, end, o);
+            if (lane >= o) end += y;
         }
-        T.first_op = first_op;
-        T.nsteps = ns;
-        if (unit > ops_units) T.error = 3;
+        if (live) T.steps[lane] = Step{two ? d - 1 : d, two ? 1 : 0, end - units, count};
+        if (lane == 7) {
+            T.first_op = first_op;
+            T.nsteps = ns;
+            if (end > ops_units) T.error = 3;
+        }
     }
     __syncwarp();
 }

@@ -76,23 +76,31 @@ __device__ inline void snr_params_fill(SnrParams& S, const int* widths, int nw, 
     cta_sync();
 }
 
-// The same parameters filled by one warp (no CTA barrier).
-__device__ inline void snr_params_fill_warp(SnrParams& S, const int* widths, int nw, int nfast,
-                                            int b)
+// The widths alone, by one warp; the coefficients follow for each profile length.
+__device__ inline void snr_widths_warp(SnrParams& S, const int* widths, int nw, int nfast)
 {
     const int lane = threadIdx.x & 31;
+    int wm = 0;
+    for (int k = lane; k < nw; k += 32) {
+        S.w[k] = widths[k];
+        wm = max(wm, S.w[k]);
+    }
+    wm = __reduce_max_sync(0xffffffffu, wm);
     if (lane == 0) {
         S.nw = nw;
         S.nfast = nfast;
-        int wm = 0;
-        for (int k = 0; k < nw; ++k) wm = widths[k] > wm ? widths[k] : wm;
         S.wmax = wm;
-        S.b = b;
+        S.b = 0;
     }
-    for (int k = lane; k < nw; k += 32) {
-        S.w[k] = widths[k];
-        boxcar_coefs(b, widths[k], &S.hb[k], &S.beta[k]);
-    }
+    __syncwarp();
+}
+
+// The coefficients for profiles of b bins, by one warp (no CTA barrier).
+__device__ inline void snr_coefs_warp(SnrParams& S, int b)
+{
+    const int lane = threadIdx.x & 31;
+    for (int k = lane; k < S.nw; k += 32) boxcar_coefs(b, S.w[k], &S.hb[k], &S.beta[k]);
+    if (lane == 0) S.b = b;
     __syncwarp();
 }
 

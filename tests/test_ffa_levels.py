@@ -72,3 +72,11 @@ def test_search_level_edges(bmin, bmax, n, tsamp):
     rp, rfb, rs = O.C().periodogram(*args)
     assert np.array_equal(p, rp) and np.array_equal(fb, rfb)
     assert np.allclose(s, rs, rtol=1e-5, atol=2e-5)
+
+
+def test_head_row_threshold():
+    # an odd node's even rows s > (n / 2 rounded down to even) have h(s) = s / 2 - 1, no others
+    for n in range(3, 8193, 2):
+        h, _ = _rows(n)
+        s = np.arange(0, n, 2)
+        assert np.array_equal(h[s], (s >> 1) - (s > ((n >> 1) & ~1))), n
