@@ -52,6 +52,17 @@ extern "C" int rt_ffa2(const float* d_in, size_t rows, size_t cols, float* d_out
         return set_error(RT_EINVAL, "ffa2 input of %zu x %zu is larger than supported", rows, cols);
     const int m = (int)rows, b = (int)cols;
     float* scratch = nullptr;
+    if (const size_t bytes = ffa_persistent_bytes(m, b, m)) {
+        void* room = nullptr;
+        const cudaError_t e = scratch_malloc(&room, bytes, st);
+        if (e == cudaSuccess) {
+            const int s = ffa_transform_persistent(d_in, m, b, m, d_out, room, nullptr, st);
+            cudaFreeAsync(room, st);
+            return s;
+        }
+        if (e != cudaErrorMemoryAllocation) return check_cuda(e, "ffa2 scratch");
+        cudaGetLastError();  // a launch per stage needs a little less
+    }
     const size_t sf = ffa_scratch_floats(m, b);
     if (sf) {
         const cudaError_t e = scratch_malloc((void**)&scratch, sf * sizeof(float), st);
@@ -71,21 +82,27 @@ extern "C" int rt_benchmark_ffa2(size_t rows, size_t cols, size_t loops, double*
         return RT_OK;
     }
     const int m = (int)rows, b = (int)cols;
-    float *in = nullptr, *out = nullptr, *scratch = nullptr;
+    float *in = nullptr, *out = nullptr;
+    void* scratch = nullptr;
     int* d_err = nullptr;
-    const size_t n = rows * cols, sf = ffa_scratch_floats(m, b);
+    const size_t n = rows * cols, persistent = ffa_persistent_bytes(m, b, m);  // as rt_ffa2
+    const size_t bytes = persistent ? persistent : ffa_scratch_floats(m, b) * sizeof(float);
     RT_TRY_CUDA(cudaMalloc((void**)&in, n * sizeof(float)));
     RT_TRY_CUDA(cudaMalloc((void**)&out, n * sizeof(float)));
     RT_TRY_CUDA(cudaMalloc((void**)&d_err, sizeof(int)));
-    if (sf) RT_TRY_CUDA(cudaMalloc((void**)&scratch, sf * sizeof(float)));
+    if (bytes) RT_TRY_CUDA(cudaMalloc(&scratch, bytes));
     RT_TRY_CUDA(cudaMemset(in, 0, n * sizeof(float)));
     RT_TRY_CUDA(cudaMemset(d_err, 0, sizeof(int)));
+    auto transform = [&]() {
+        return persistent ? ffa_transform_persistent(in, m, b, m, out, scratch, d_err, 0)
+                          : ffa_transform(in, m, b, m, out, static_cast<float*>(scratch), d_err, 0);
+    };
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
-    int s = ffa_transform(in, m, b, m, out, scratch, d_err, 0);  // warm-up
+    int s = transform();  // warm-up
     cudaEventRecord(e0, 0);
-    for (size_t i = 0; i < loops && s == RT_OK; ++i) s = ffa_transform(in, m, b, m, out, scratch, d_err, 0);
+    for (size_t i = 0; i < loops && s == RT_OK; ++i) s = transform();
     cudaEventRecord(e1, 0);
     cudaEventSynchronize(e1);
     float ms = 0.f;

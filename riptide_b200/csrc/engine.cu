@@ -58,6 +58,7 @@ struct EngineArgs {
     const float* ds;         // downsampled series arena
     const float* norm;       // normalised series arena (cycles with f == 1)
     float* snrs;
+    float* rows_out;         // kRowsOnly
     const XformRec* xforms;
     const WorkItem* items;
     long long nitems;
@@ -453,8 +454,29 @@ __device__ void scheduler_warp(const EngineArgs& A, Handover& H, JobTree* trees,
     }
 }
 
-// KINDS: the kinds of S/N code (snr_kind) the instance holds. The host picks the instance
-// (search_kernel_for).
+constexpr int kRowsOnly = 0;
+
+// The root rows of a job of a transform of its own, without halo, to A.rows_out: 16 bytes a
+// thread where the rows allow.
+__device__ __forceinline__ void store_rows_out(const EngineArgs& A, const ItemSlot& L,
+                                               const float* rows, int stride)
+{
+    const int b = L.X.b, n = L.J.hi - L.J.lo, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float* to = A.rows_out + (size_t)(L.J.root_row0 + L.J.lo) * b;
+    if ((b & 3) == 0 && (reinterpret_cast<uintptr_t>(A.rows_out) & 15) == 0) {
+        for (int r = warp; r < n; r += kWarps) {
+            const float4* from = reinterpret_cast<const float4*>(rows + (size_t)r * stride);
+            float4* row = reinterpret_cast<float4*>(to + (size_t)r * b);
+            for (int c = lane; c < b >> 2; c += 32) row[c] = from[c];
+        }
+    } else {
+        for (int r = warp; r < n; r += kWarps)
+            for (int c = lane; c < b; c += 32) to[(size_t)r * b + c] = rows[(size_t)r * stride + c];
+    }
+}
+
+// KINDS: the kinds of S/N code (snr_kind) the instance holds; kRowsOnly: none, the root rows of
+// the last stage are the result. The host picks the instance (search_kernel_for).
 template <int KINDS>
 __global__ void __launch_bounds__(kEngineThreads, 1) k_search_persistent(EngineArgs A)
 {
@@ -559,7 +581,10 @@ __global__ void __launch_bounds__(kEngineThreads, 1) k_search_persistent(EngineA
                 float* rows = run_job_levels(T, b, sbuf, other, fstride, ops, io, &ok);
                 if (!ok && threadIdx.x == 0) atomicExch(A.error, RT_ETIMEOUT);
                 mark(kPhLevels);
-                if (L.last) {
+                if (KINDS == kRowsOnly && L.last) {
+                    store_rows_out(A, L, rows, fstride);
+                    mark(kPhSnr);
+                } else if (L.last) {
                     float* work = rows == sbuf ? other : sbuf;
                     constexpr bool one = (KINDS & (KINDS - 1)) == 0;
                     const int kind = one ? KINDS : snr_kind(b, X.tune >> 16);
@@ -1551,6 +1576,130 @@ static int engine_grid(void (*kernel)(EngineArgs))
     return std::max(1, sms * std::max(per, 1));
 }
 
+// ------------------------------------------------------------------------------------
+// One transform by the persistent kernel (ffa2 of a large block): its jobs are the work items,
+// stage by stage, and its rows the result. Against a launch per stage, a job's node lists,
+// staging and stores run beside the levels of the one before: 16,384 x 488 values 176 to 155 us a
+// call, 8,000 x 1,000 198 to 162, 33,000 x 250 175 to 147. From kPersistentItems jobs: with fewer
+// the waits between the stages cost more (8,000 x 488: 88 against 80 us). Nodes counted one by one,
+// so that one may start before its whole stage is done, took as long and slowed the searches.
+// ------------------------------------------------------------------------------------
+struct TransformState {
+    unsigned long long ticket;
+    int error;
+    int done[kMaxStages];
+    int slot_release[kSlots];
+    XformRec xform;
+    StagePlan plan;
+};
+
+// Work items of the transform, its record and cleared counters.
+__global__ void k_transform_items(TransformState* S, WorkItem* items, XformRec X, StagePlan P)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, n = gridDim.x * blockDim.x;
+    if (t == 0) {
+        S->ticket = 0;
+        S->error = RT_OK;
+        S->xform = X;
+        S->plan = P;
+    }
+    if (t < kMaxStages) S->done[t] = 0;
+    if (t < kSlots) S->slot_release[t] = 0;
+    int first = 0;
+    for (int s = 0; s < P.nstages; ++s) {
+        for (int j = t; j < P.jobs[s]; j += n) items[first + j] = WorkItem{0, s << 24 | j};
+        first += P.jobs[s];
+    }
+}
+
+// A bounded wait that ran out leaves NaN, and the error where it is asked for.
+__global__ void k_transform_check(const TransformState* S, float* out, size_t n, int* d_err)
+{
+    if (S->error == RT_OK) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0 && d_err) *d_err = S->error;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
+         i += (size_t)gridDim.x * blockDim.x)
+        out[i] = __int_as_float(0x7fffffff);
+}
+
+struct TransformPlan {
+    FfaLayout layout;
+    StagePlan plan;
+    int cap, items;
+    size_t slot_floats, state_bytes, item_bytes;
+};
+
+static bool transform_plan(int m, int b, int rows_out, TransformPlan& T)
+{
+    T.layout = ffa_layout(kEngineDynBytes, b, (size_t)m);
+    T.cap = ffa_cap_rows(T.layout, b);
+    if (T.cap < 4 || T.cap > 0xffff || !plan_stages(m, b, rows_out, T.cap, 0, &T.plan)) return false;
+    if (T.plan.nstages < 2) return false;
+    T.items = 0;
+    for (int s = 0; s < T.plan.nstages; ++s) {
+        if (T.plan.jobs[s] >= 1 << 24) return false;
+        T.items += T.plan.jobs[s];
+    }
+    T.slot_floats = ((size_t)m * ffa_stride(b) + 3) & ~size_t(3);
+    T.state_bytes = (sizeof(TransformState) + 255) & ~size_t(255);
+    T.item_bytes = ((size_t)T.items * sizeof(WorkItem) + 255) & ~size_t(255);
+    return true;
+}
+
+size_t ffa_persistent_bytes(int m, int b, int rows_out)
+{
+    TransformPlan T;
+    if (!transform_plan(m, b, rows_out, T) || T.items < kPersistentItems) return 0;
+    return T.state_bytes + T.item_bytes + 2 * T.slot_floats * sizeof(float);
+}
+
+int ffa_transform_persistent(const float* in, int m, int b, int rows_out, float* out, void* scratch,
+                             int* d_err, cudaStream_t st)
+{
+    TransformPlan T;
+    if (!transform_plan(m, b, rows_out, T))
+        return set_error(RT_EINTERNAL, "no plan for an FFA transform of %d x %d", m, b);
+    unsigned char* base = static_cast<unsigned char*>(scratch);
+    TransformState* S = reinterpret_cast<TransformState*>(base);
+    WorkItem* items = reinterpret_cast<WorkItem*>(base + T.state_bytes);
+    XformRec X;
+    memset(&X, 0, sizeof(X));
+    X.tau = 1.0;
+    X.b = b;
+    X.m = m;
+    X.rows_eval = rows_out;
+    X.stdnoise = 1.0f;
+    // bulk copies of whole 16-byte units stay inside the block if it starts and ends with one
+    X.src_norm = (reinterpret_cast<uintptr_t>(in) & 15) != 0 || ((size_t)m * b) % 4 != 0;
+    X.tune = T.cap;
+    k_transform_items<<<std::min(148, (T.items + 255) / 256 + 1), 256, 0, st>>>(S, items, X, T.plan);
+    RT_TRY_CUDA(cudaGetLastError());
+    EngineArgs A;
+    memset(&A, 0, sizeof(A));
+    A.ds = A.norm = in;
+    A.rows_out = out;
+    A.xforms = &S->xform;
+    A.items = items;
+    A.nitems = T.items;
+    A.plans = &S->plan;
+    A.scratch = reinterpret_cast<float*>(base + T.state_bytes + T.item_bytes);
+    A.slot_floats = T.slot_floats;
+    A.done = S->done;
+    A.slot_release = S->slot_release;
+    A.error = &S->error;
+    A.ticket = &S->ticket;
+    A.spin_limit = kSpinLimit;
+    A.layout = T.layout;
+    void (*kernel)(EngineArgs) = k_search_persistent<kRowsOnly>;
+    RT_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)kEngineDynBytes));
+    kernel<<<std::min(engine_grid(kernel), T.items), kEngineThreads, kEngineDynBytes, st>>>(A);
+    RT_TRY_CUDA(cudaGetLastError());
+    k_transform_check<<<148, 256, 0, st>>>(S, out, (size_t)rows_out * b, d_err);
+    RT_TRY_CUDA(cudaGetLastError());
+    return RT_OK;
+}
+
 // Launches the whole search of the plan on `st`. data: packed input series (device).
 static int plan_run(SearchPlan& P, const float* data, float* normalised_out, double* periods,
                     uint32_t* foldbins, float* snrs, cudaStream_t st)
@@ -1627,6 +1776,7 @@ static int plan_run(SearchPlan& P, const float* data, float* normalised_out, dou
     // counters
     RT_TRY_CUDA(cudaMemsetAsync(P.d_counters, 0, plan_counters(P) * sizeof(int), st));
     EngineArgs A;
+    memset(&A, 0, sizeof(A));
     A.ds = P.d_ds;
     A.norm = zsrc;
     A.snrs = snrs;

@@ -27,6 +27,14 @@ void release_scratch();
 int ffa_transform(const float* in, int m, int b, int rows_out, float* out, float* scratch,
                   int* d_err, cudaStream_t st);
 
+// The same by the persistent search kernel, with ffa_persistent_bytes(m, b, rows_out) bytes of
+// 256-byte aligned scratch (0: not for this size). Its waits are bounded: one that runs out
+// leaves NaN in `out`.
+constexpr int kPersistentItems = 1000;
+size_t ffa_persistent_bytes(int m, int b, int rows_out);
+int ffa_transform_persistent(const float* in, int m, int b, int rows_out, float* out, void* scratch,
+                             int* d_err, cudaStream_t st);
+
 int snr2(const float* x, size_t rows, size_t cols, const int* h_widths, int nw, float stdnoise,
          float* out, cudaStream_t st);
 int rollback(const float* x, size_t size, size_t shift, float* out, cudaStream_t st);
