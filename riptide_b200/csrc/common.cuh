@@ -125,4 +125,22 @@ __device__ __forceinline__ float ordered_to_float(unsigned u)
     return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
 }
 
+// A whole number below 2^52 as a double and the floor of a double in [0, 2^51) as both, by the
+// place of a number's units in the mantissa of 2^52 + number: on the FP64 units, for kernels
+// that the rate of the conversion instructions bounds.
+__device__ __forceinline__ double whole_double(size_t k)
+{
+    return __longlong_as_double((long long)(k | 0x4330000000000000ull)) - 4503599627370496.0;
+}
+__device__ __forceinline__ double floor_index(double v, size_t& i)
+{
+    const double u = __dadd_rd(v, 4503599627370496.0);
+    i = (size_t)__double_as_longlong(u) & 0xfffffffffffffull;
+    return u - 4503599627370496.0;
+}
+__device__ __forceinline__ double floor_double(double v)
+{
+    return __dadd_rd(v, 4503599627370496.0) - 4503599627370496.0;
+}
+
 }  // namespace rt

