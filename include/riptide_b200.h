@@ -164,7 +164,9 @@ int rt_search_plan_create(const uint64_t* h_lengths, size_t ntrials,
 /* Engine tile choices (0 = default), as picked by an autotuner:
  *   rows_fraction       rows per job as a fraction (0, 1] of what the shared memory holds,
  *                       for transforms of up to 8 jobs' worth of rows;
- *   snr_threads         threads per profile in the S/N: 8 (bins <= 264 only) or 16;
+ *   snr_threads         threads per profile in the S/N: 16 where 16 segments of 33 phases hold a
+ *                       profile (bins <= 528); 8 or 0: the default, 4 threads up to 132 bins,
+ *                       8 up to 264, 16 up to 528, 32 beyond;
  *   lag_items           work items between two stages of a multi-stage transform (640);
  *   rows_fraction_deep  the same fraction for transforms of more rows than that (0: the
  *                       value of rows_fraction).
@@ -183,7 +185,7 @@ int rt_search_plan_create_tuned(const uint64_t* h_lengths, size_t ntrials,
  * (riptide_b200.tuning): the first rule whose ranges hold a transform's (rows, bins) sets
  * its choices; a field left 0 keeps the plan-wide value of `tuning`.
  *   rows_fraction  rows per job, as a fraction of what shared memory holds at these bins;
- *   snr_threads    threads per profile in the S/N: 8 (bins <= 264 only) or 16;
+ *   snr_threads    threads per profile in the S/N, as above;
  *   max_levels     levels a job computes in shared memory (1..8, default 8): fewer levels cut
  *                  a deep transform into more stages, whose outputs pass through L2.
  * Results do not depend on these; only the speed does. No counterpart in the reference. */
@@ -407,7 +409,7 @@ int rt_fold_shape(size_t size, double tsamp, double period, size_t bins, long lo
 /* fold of d_in (size float32 samples) into d_out (rows x bins, rt_fold_shape). */
 int rt_fold(const float* d_in, size_t size, double tsamp, double period, size_t bins,
             long long subints, float* d_out, void* stream);
-/* `count` folds of the same series in one launch (candidate folding): fold c at h_periods[c]
+/* `count` folds of the same series in one call (candidate folding): fold c at h_periods[c]
  * with h_bins[c] bins and h_subints[c], written at d_out + h_out_offsets[c]. */
 int rt_fold_batched(const float* d_in, size_t size, double tsamp, const double* h_periods,
                     const size_t* h_bins, const long long* h_subints, size_t count,

@@ -72,9 +72,8 @@ __device__ __forceinline__ float folded(const float* x, size_t N, const FoldJob&
 // neighbouring lanes sum a window (about six samples a lane, so that the loads of a warp cover
 // few lines and the per-window arithmetic stays small), and the next window is the next lanes'.
 // Bound: instructions (81% of the issue slots), most of them a window's own, and conversions to
-// float64 (57% of their rate). 48 folds of 2^22 samples
-// into 256 bins, 32 sub-integrations: 385 us with a thread per output value; 180 us for both
-// kernels.
+// float64 (57% of their rate). 48 folds of 2^22 samples into 256 bins, 32 sub-integrations: 385 us
+// with a thread per output value; 180 us for both kernels.
 // ------------------------------------------------------------------------------------
 constexpr int kFoldThreads = 256;
 

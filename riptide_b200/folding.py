@@ -39,7 +39,7 @@ def fold_shape(nsamp, tsamp, period, bins, subints=None):
 
 
 def fold_batched(ts, periods, bins, subints=None):
-    """Fold one TimeSeries at many periods in one launch (candidate folding). `bins` and
+    """Fold one TimeSeries at many periods in one call (candidate folding). `bins` and
     `subints` are scalars or one per period. Returns a list of numpy float32 arrays shaped as
     fold() returns them."""
     torch = libcpp._t()
@@ -82,7 +82,7 @@ def candidate_subints(period, subints, length):
 
 
 def fold_candidates(ts, periods, bins, subints=1):
-    """Fold one TimeSeries at every candidate period in one launch, with the candidate stage's
+    """Fold one TimeSeries at every candidate period in one call, with the candidate stage's
     rule for sub-integrations (candidate_subints). Returns the list of folded arrays."""
     subs = [candidate_subints(float(p), subints, ts.length) for p in np.asarray(periods).ravel()]
     return fold_batched(ts, periods, bins, subs)

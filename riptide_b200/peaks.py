@@ -8,7 +8,7 @@ fitted to the control points (a constant `smin` below `minseg` segments), and th
 above both the threshold and `smin` are clustered in frequency (radius clrad / T_obs), one
 peak per cluster at its highest S/N.
 
-Here the segment statistics (sorts of every segment's S/N and frequencies) and the
+Here the segment statistics (order statistics of every segment's S/N and frequencies) and the
 thresholding of every periodogram point run on the GPU (rt_peak_segments, rt_peak_select);
 the polynomial fits (np.polyfit, a few hundred points each) and the clustering of the
 selected points run on the host with the reference's numpy calls, so that the peaks are the

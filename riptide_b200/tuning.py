@@ -7,8 +7,9 @@ The persistent search kernel has choices that change its speed but not its resul
                       more per-job overhead);
   rows_fraction_deep  the same for the transforms of more than 8 jobs' worth of rows, the ones
                       cut into several stages;
-  snr_threads         threads per profile in the S/N (8 or 16; 8 only for b <= 264): more
-                      threads per profile finish a job's last, partial round sooner;
+  snr_threads         threads per profile in the S/N: 16 (for b <= 528), or the default (8 or
+                      0), the fewest whose 33 phases each hold a profile: more threads per
+                      profile finish a job's last, partial round sooner;
   lag_items           work items between two stages of a multi-stage transform: a longer lag
                       leaves the previous stage more time to finish (fewer waits), a shorter
                       one keeps its output in L2.
