@@ -143,4 +143,34 @@ __device__ __forceinline__ double floor_double(double v)
     return __dadd_rd(v, 4503599627370496.0) - 4503599627370496.0;
 }
 
+// Kernels that follow one another in an entry point or a search run begin while the one before
+// drains: each lets its successor be scheduled as soon as all its own CTAs have started, and waits
+// for its predecessor (and for its writes) before it touches memory. Every kernel launched by
+// launch_dependent has to begin with after_previous_kernel(), in every thread.
+// The seven kernels of a search of 2^15 samples: 101 to 88 us; the two of a 300 x 251 transform:
+// 24 to 20. (The running median of one long series keeps plain launches: 2^22 samples took 45
+// against 32 us.)
+__device__ __forceinline__ void after_previous_kernel()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <typename... P, typename... A>
+cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+                             cudaStream_t st, A&&... args)
+{
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 }  // namespace rt

@@ -113,6 +113,7 @@ __global__ void __launch_bounds__(256) k_search_periods(const XformRec* __restri
                                                         double* __restrict__ periods,
                                                         uint32_t* __restrict__ foldbins)
 {
+    after_previous_kernel();
     const int lane = threadIdx.x & 31;
     for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n;
          i += (gridDim.x * blockDim.x) >> 5) {
@@ -485,6 +486,7 @@ __global__ void __launch_bounds__(kEngineThreads, 1) k_search_persistent(EngineA
     __shared__ JobTree trees[2];
     __shared__ SnrParams snr[2];
 
+    after_previous_kernel();
     uint64_t* full = reinterpret_cast<uint64_t*>(H.full);
     uint64_t* staged = reinterpret_cast<uint64_t*>(&H.staged);
     if (threadIdx.x == 0) {
@@ -762,6 +764,7 @@ __global__ void __launch_bounds__(256)
     k_scrunch_batched(const float* __restrict__ x, TrialArrays A, int k, ScrunchTab T, int pts,
                       float* __restrict__ lores)
 {
+    after_previous_kernel();
     extern __shared__ float sm_scb[];
     __shared__ ScrunchTab S;
     const int nleaves = T.nleaves;
@@ -1034,6 +1037,7 @@ __global__ void __launch_bounds__(kStatThreads)
     k_dered(const float* __restrict__ x, TrialArrays A, int k, DivMagic g2k,
             const float* __restrict__ rmed, float* __restrict__ y, double* __restrict__ part)
 {
+    after_previous_kernel();
     constexpr int Q = kInterpSpan / kStatThreads;
     __shared__ double2 coef[kInterpCoefs];
     const int trial = blockIdx.y;
@@ -1110,6 +1114,7 @@ __global__ void __launch_bounds__(kStatThreads)
 __global__ void k_stats(const double* __restrict__ part, TrialArrays A, int blocks, int ntrials,
                         double* __restrict__ mean, double* __restrict__ norm)
 {
+    after_previous_kernel();
     const int lane = threadIdx.x & 31;
     const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (t >= ntrials) return;
@@ -1711,22 +1716,23 @@ static int plan_run(SearchPlan& P, const float* data, float* normalised_out, dou
     const float* series = data;  // series before normalisation
     int launches = 0;
     const dim3 stat_grid((unsigned)interp_blocks(P.max_len), (unsigned)T);
+    // (here, so that the kernels follow one another)
+    RT_TRY_CUDA(cudaMemsetAsync(P.d_counters, 0, plan_counters(P) * sizeof(int), st));
     if (P.timing) RT_TRY_CUDA(cudaEventRecord(P.ev[0], st));
     if (P.cfg.deredden) {
         const int k = P.scrunch;
         if (k > 1) {
             RT_TRY(launch_scrunch(data, TA, k, T, P.max_lo, P.d_lores, st));
             RT_TRY(launch_running_median(P.d_lores, P.d_lo_len, P.d_lo_off, T, P.max_lo,
-                                         (int)P.cfg.rmed_minpts, P.d_rmed, st));
+                                         (int)P.cfg.rmed_minpts, P.d_rmed, st, true));
             launches += 2;
         } else {
             RT_TRY(launch_running_median(data, P.d_len, P.d_off, T, P.max_len, P.rmed_width,
-                                         P.d_rmed, st));
+                                         P.d_rmed, st, true));
             launches += 1;
         }
-        k_dered<<<stat_grid, kStatThreads, 0, st>>>(data, TA, k, div_magic(2u * (unsigned)k),
-                                                    P.d_rmed, P.d_y, P.d_part);
-        RT_TRY_CUDA(cudaGetLastError());
+        RT_TRY_CUDA(launch_dependent(k_dered, stat_grid, dim3(kStatThreads), 0, st, data, TA, k,
+                                     div_magic(2u * (unsigned)k), P.d_rmed, P.d_y, P.d_part));
         launches += 1;
         series = P.d_y;
     } else if (!P.cfg.already_normalised) {
@@ -1736,8 +1742,8 @@ static int plan_run(SearchPlan& P, const float* data, float* normalised_out, dou
     }
     const bool affine = !P.cfg.already_normalised;
     if (affine) {
-        k_stats<<<(T + 3) / 4, 128, 0, st>>>(P.d_part, TA, (int)stat_grid.x, T, P.d_mean, P.d_normv);
-        RT_TRY_CUDA(cudaGetLastError());
+        RT_TRY_CUDA(launch_dependent(k_stats, dim3((T + 3) / 4), dim3(128), 0, st, P.d_part, TA,
+                                     (int)stat_grid.x, T, P.d_mean, P.d_normv));
         launches += 1;
     }
     if (P.timing) RT_TRY_CUDA(cudaEventRecord(P.ev[1], st));
@@ -1773,8 +1779,6 @@ static int plan_run(SearchPlan& P, const float* data, float* normalised_out, dou
         launches += seg ? 1 : 0;
     }
     if (P.timing) RT_TRY_CUDA(cudaEventRecord(P.ev[2], st));
-    // counters
-    RT_TRY_CUDA(cudaMemsetAsync(P.d_counters, 0, plan_counters(P) * sizeof(int), st));
     EngineArgs A;
     memset(&A, 0, sizeof(A));
     A.ds = P.d_ds;
@@ -1802,12 +1806,11 @@ static int plan_run(SearchPlan& P, const float* data, float* normalised_out, dou
                                      (int)kEngineDynBytes));
     if (A.nitems > 0) {
         const int nx = (int)P.xforms.size();
-        k_search_periods<<<std::min((nx + 7) / 8, 148 * 8), 256, 0, st>>>(P.d_xforms, nx, periods,
-                                                                         foldbins);
-        RT_TRY_CUDA(cudaGetLastError());
+        RT_TRY_CUDA(launch_dependent(k_search_periods, dim3(std::min((nx + 7) / 8, 148 * 8)),
+                                     dim3(256), 0, st, P.d_xforms, nx, periods, foldbins));
         launches += 1;
-        kernel<<<engine_grid(kernel), kEngineThreads, kEngineDynBytes, st>>>(A);
-        RT_TRY_CUDA(cudaGetLastError());
+        RT_TRY_CUDA(launch_dependent(kernel, dim3(engine_grid(kernel)), dim3(kEngineThreads),
+                                     kEngineDynBytes, st, A));
         launches += 1;
     }
     if (P.timing) RT_TRY_CUDA(cudaEventRecord(P.ev[3], st));

@@ -240,6 +240,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     k_ffa_stage(const float* __restrict__ src, float* __restrict__ dst, int m, int b,
                 int rows_out, StagePlan P, int stage, FfaLayout L, int* err)
 {
+    after_previous_kernel();
     extern __shared__ __align__(16) unsigned char smem[];
     JobTree& T = *reinterpret_cast<JobTree*>(smem);
     uint4* ops = reinterpret_cast<uint4*>(smem + kStageTreeBytes);
@@ -372,9 +373,8 @@ int ffa_transform(const float* in, int m, int b, int rows_out, float* out, float
     const float* src = in;
     for (int s = 0; s < P.nstages; ++s) {
         float* dst = (s == P.nstages - 1) ? out : scratch + (size_t)(s & 1) * m * b;
-        k_ffa_stage<<<P.jobs[s], kThreads, kFfaSmemBytes, st>>>(src, dst, m, b, rows_out, P, s,
-                                                               L, d_err);
-        RT_TRY_CUDA(cudaGetLastError());
+        RT_TRY_CUDA(launch_dependent(k_ffa_stage, dim3(P.jobs[s]), dim3(kThreads), kFfaSmemBytes, st,
+                                     src, dst, m, b, rows_out, P, s, L, d_err));
         src = dst;
     }
     return RT_OK;
@@ -519,6 +519,7 @@ template <int kDsThreads, int kDsStage>
 __global__ void __launch_bounds__(kDsThreads, 1024 / kDsThreads)
     k_downsample_segments(DsJob job)
 {
+    after_previous_kernel();
     constexpr int kDsWarps = kDsThreads / 32;
     constexpr int kDsPerWarp = kDsStage / kDsWarps;  // staged samples per warp
     constexpr int kDsQuads = kDsPerWarp / 128;       // 128-sample chunks per warp, 4 samples a lane
@@ -769,8 +770,8 @@ int launch_downsample(const DsJob& job_in, int ntrials, size_t max_len, cudaStre
                                       : k_downsample_segments<kDsThreads, kDsStage>;
         RT_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         dim3 grid((unsigned)((max_len + job.seg - 1) / job.seg), (unsigned)ntrials);
-        kernel<<<grid, small ? kDsSmallThreads : kDsThreads, smem, st>>>(job);
-        RT_TRY_CUDA(cudaGetLastError());
+        RT_TRY_CUDA(launch_dependent(kernel, grid, dim3(small ? kDsSmallThreads : kDsThreads), smem,
+                                     st, job));
     }
     for (int c = 0; c < job.ncycles; ++c) {
         if (job.use_seg_host[c] || job.skip_host[c]) continue;
@@ -843,6 +844,7 @@ __global__ void __launch_bounds__(kRmedThreads)
                             const size_t* __restrict__ offsets, size_t one_len, int width, int tile,
                             float* __restrict__ out)
 {
+    after_previous_kernel();
     __shared__ __align__(16) float sx[kRmedSortSpan];            // values in position order
     __shared__ float sv[kRmedSortSpan];                          // ... in sorted order
     __shared__ __align__(16) unsigned short sp[kRmedSortSpan];   // their positions
@@ -919,13 +921,18 @@ __global__ void __launch_bounds__(kRmedThreads)
 }
 
 int launch_running_median(const float* x, const size_t* d_lengths, const size_t* d_offsets,
-                          int ntrials, size_t max_len, int width, float* out, cudaStream_t st)
+                          int ntrials, size_t max_len, int width, float* out, cudaStream_t st,
+                          bool dependent)
 {
     if (width >= 1 && width <= kRmedMaxWidth) {
         // about as many outputs as the window has values: smaller tiles sort more overhang,
         // larger ones compare each value with more others
         const int tile = width <= 129 ? 128 : 256;
         dim3 grid((unsigned)((max_len + tile - 1) / tile), (unsigned)ntrials);
+        if (dependent)
+            return check_cuda(launch_dependent(k_running_median_sorted, grid, dim3(kRmedThreads), 0, st,
+                                               x, d_lengths, d_offsets, max_len, width, tile, out),
+                              "running_median");
         k_running_median_sorted<<<grid, kRmedThreads, 0, st>>>(x, d_lengths, d_offsets, max_len,
                                                                width, tile, out);
         return check_cuda(cudaGetLastError(), "running_median");

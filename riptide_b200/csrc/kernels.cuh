@@ -43,9 +43,10 @@ int fused_rollback_add(const float* x, const float* y, size_t size, size_t shift
 int circular_prefix_sum(const float* x, size_t size, size_t nsum, float* out, cudaStream_t st);
 int launch_periods(double* periods, uint32_t* foldbins, size_t rows_eval, double tau, int bins,
                    size_t rows, cudaStream_t st);
-// (d_lengths null: one series of max_len samples)
+// (d_lengths null: one series of max_len samples; dependent: by launch_dependent)
 int launch_running_median(const float* x, const size_t* d_lengths, const size_t* d_offsets,
-                          int ntrials, size_t max_len, int width, float* out, cudaStream_t st);
+                          int ntrials, size_t max_len, int width, float* out, cudaStream_t st,
+                          bool dependent = false);
 
 // Downsampling of many series by many factors in one pass (device arrays).
 constexpr int kDsStage = 8192;        // input samples staged per CTA (segment + halo)
