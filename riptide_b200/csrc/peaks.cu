@@ -40,7 +40,7 @@ struct SegTrial {
 // of the ranks by a scan, and gathers the few values in them, which are ranked against one
 // another. A span with more than kSelList values is divided again, until it holds one key.
 // The CTA holds its columns in shared memory, one read of the periodogram. Bound: the warps'
-// instructions, six to ten a value and pass. 1,068 segments of 1,174 points by 10 widths: 760 us
+// instructions, six to ten a value and pass. 1,048 segments of 1,174 points by 10 widths: 750 us
 // by bitonic sorts of columns padded to 2,048; by selection 80 us.
 // ------------------------------------------------------------------------------------
 constexpr int kSelSpans = 1024;  // 32 per lane
