@@ -215,6 +215,15 @@ typedef struct rt_search_transform {
     float stdnoise;
 } rt_search_transform;
 int rt_search_plan_transforms(const rt_search_plan* plan, rt_search_transform* h_out);
+/* Memory of a plan, for checks of its bounds (host only). The outputs of the stages of a
+ * transform lie in a ring of ring_slots x ring_slot_bytes of device memory. The search kernel
+ * has shared_bytes of dynamic shared memory per CTA: ops_bytes of row operations, two buffers of
+ * buffer_bytes for the rows of a level, and the rest for reads past the last row. */
+typedef struct rt_search_memory_t {
+    uint64_t ring_slots, ring_slot_bytes;
+    uint64_t shared_bytes, ops_bytes, buffer_bytes;
+} rt_search_memory_t;
+int rt_search_plan_memory(const rt_search_plan* plan, rt_search_memory_t* h_out);
 /* Per-trial mean and (population) standard deviation of the series the last run normalised
  * (after deredden); 0 and 1 when the plan does not normalise. Synchronises `stream`. */
 int rt_search_normalisation(rt_search_plan* plan, double* h_mean, double* h_std, void* stream);

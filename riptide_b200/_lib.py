@@ -59,6 +59,7 @@ SIGNATURES = {
     "rt_search_inject_fault": (ctypes.c_int, [_vp, ctypes.c_int, ctypes.c_int]),
     "rt_search_plan_prepare": (ctypes.c_int, [_vp]),
     "rt_search_plan_transforms": (ctypes.c_int, [_vp, _vp]),
+    "rt_search_plan_memory": (ctypes.c_int, [_vp, _vp]),
     "rt_search_normalisation": (ctypes.c_int, [_vp, ctypes.POINTER(_d), ctypes.POINTER(_d), _vp]),
     "rt_search_backward_rows": (ctypes.c_int, [_vp, _vp, _vp, _vp, _sz, _vp]),
     "rt_peak_segments": (ctypes.c_int, [_vp, _vp, _sz, _u64p, _sz, ctypes.POINTER(_d), _d, _d, _u64p, _vp, _vp, _vp]),
@@ -105,6 +106,11 @@ class PlanStats(ctypes.Structure):
         "num_trials", "num_cycles", "num_transforms", "num_work_items", "num_multistage",
         "total_rows", "total_samples", "downsampled_samples", "folded_samples",
         "scrunch_factor")]
+
+
+class SearchMemory(ctypes.Structure):
+    _fields_ = [(n, ctypes.c_uint64) for n in (
+        "ring_slots", "ring_slot_bytes", "shared_bytes", "ops_bytes", "buffer_bytes")]
 
 
 class TileRule(ctypes.Structure):

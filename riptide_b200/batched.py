@@ -84,6 +84,12 @@ class BatchedSearch(object):
     def total_rows(self):
         return int(self.row_offsets[-1])
 
+    def memory(self):
+        """Sizes of the plan's stage ring and of the search kernel's shared memory, in bytes."""
+        m = _lib.SearchMemory()
+        _lib.check(_lib.load().rt_search_plan_memory(self._plan, ctypes.byref(m)))
+        return {k: int(getattr(m, k)) for k, _ in _lib.SearchMemory._fields_}
+
     def allocate_outputs(self, device="cuda"):
         """Device tensors (periods f64[L], foldbins i32[L], snrs f32[L, nw]) of the batch."""
         torch = libcpp._t()

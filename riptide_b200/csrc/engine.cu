@@ -1342,7 +1342,17 @@ static int plan_build(SearchPlan& P)
 
     // (the first cycle has the smallest factor, and so the most rows)
     const size_t most_rows = C > 0 ? downsampled_size(P.max_len, P.f[0]) / c.bins_min : 0;
-    P.layout = ffa_layout(kEngineDynBytes, (int)c.bins_min, most_rows);
+    // Room behind the second level buffer for the reads of the S/N past its last row, by every
+    // number of threads that a transform of the plan may be given. (A one-stage transform can fill
+    // the buffer to its last row; the last stage of others has at most kThreads / tpr rows.)
+    int pad = kPadFloats;
+    for (int b = (int)c.bins_min; b <= (int)c.bins_max; ++b) {
+        bool tuned = P.tuning.snr_threads == 16;
+        for (const rt_tile_rule& R : P.rules)
+            tuned |= R.snr_threads == 16 && (unsigned)b >= R.bins_min && (unsigned)b <= R.bins_max;
+        pad = std::max({pad, snr_overread(b, snr_tpr(b)), tuned ? snr_overread(b, 16) : 0});
+    }
+    P.layout = ffa_layout(kEngineDynBytes, (int)c.bins_min, most_rows, pad);
     size_t ds_total = 0;
     for (int t = 0; t < T; ++t) {
         const size_t N = P.lengths[t];
@@ -2314,6 +2324,18 @@ extern "C" int rt_search_plan_stats(const rt_search_plan* plan, rt_search_plan_s
     for (const XformRec& X : P.xforms) fold += (uint64_t)X.m * X.b;
     st->folded_samples = fold;
     st->scrunch_factor = (uint64_t)P.scrunch;
+    return RT_OK;
+}
+
+extern "C" int rt_search_plan_memory(const rt_search_plan* plan, rt_search_memory_t* h_out)
+{
+    if (!plan || !h_out) return set_error(RT_EINVAL, "null argument");
+    const SearchPlan& P = plan->p;
+    h_out->ring_slots = kSlots;
+    h_out->ring_slot_bytes = 2 * P.slot_floats * sizeof(float);
+    h_out->shared_bytes = kEngineDynBytes;
+    h_out->ops_bytes = (uint64_t)P.layout.ops_units * 16;
+    h_out->buffer_bytes = (uint64_t)P.layout.buf_floats * sizeof(float);
     return RT_OK;
 }
 

@@ -907,14 +907,14 @@ struct FfaLayout {
 };
 
 // Layout of `bytes` of shared memory for transforms of at least bmin bins and at most max_rows
-// rows: fixed by the smallest b, which has the most rows per level.
-RT_HD FfaLayout ffa_layout(size_t bytes, int bmin, size_t max_rows)
+// rows: fixed by the smallest b, which has the most rows per level. `pad` floats stay free behind
+// the second buffer, for what the boxcar S/N reads past the end of its last row (snr_overread).
+RT_HD FfaLayout ffa_layout(size_t bytes, int bmin, size_t max_rows, int pad = kPadFloats)
 {
     FfaLayout L;
     const int most = (int)(bytes / (2 * sizeof(float) * ffa_stride(bmin)));
     L.ops_units = (ffa_ops_units(most, max_rows <= (size_t)kRegularRows) + 3) & ~3;
-    // (kPadFloats behind the second buffer: the boxcar S/N reads past the end of its rows)
-    L.buf_floats = (int)((bytes - (size_t)L.ops_units * 16 - kPadFloats * sizeof(float)) /
+    L.buf_floats = (int)((bytes - (size_t)L.ops_units * 16 - pad * sizeof(float)) /
                          (2 * sizeof(float))) & ~15;
     return L;
 }

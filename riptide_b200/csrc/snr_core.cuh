@@ -179,9 +179,9 @@ RT_HD int snr_phases(int b, int tpr)
 // warp-level synchronisation: a profile's TPR threads are lanes of one warp. Writes
 // out[r * out_stride + k]. `groups` profiles are processed at a time (C holds `groups` rows).
 // kUnrolled: kSnrPhases phases per thread. kGuard: X must not be read past a row's end; without
-// it all TPR * kSnrPhases values from the row's start are read: anything may be past bin b - 1,
-// it only reaches prefix values past b - 1, which the wrap-around part replaces as far as they
-// are read.
+// it all TPR * kSnrPhases values from the row's start are read (snr_overread floats past the last
+// row, for which the caller has room): anything may be past bin b - 1, it only reaches prefix
+// values past b - 1, which the wrap-around part replaces as far as they are read.
 template <int TPR, int SB, bool kUnrolled, bool kGuard>
 __device__ __forceinline__ void snr_rows_impl(const float* X, int xs, int nrows, int b,
                                               const SnrParams& S, float stdnoise,
@@ -344,6 +344,14 @@ RT_HD int prefix_stride(int b, int wmax, int tpr)
 RT_HD int snr_tpr(int b)
 {
     return b <= 4 * kSnrPhases ? 4 : b <= 8 * kSnrPhases ? 8 : b <= 16 * kSnrPhases ? 16 : 32;
+}
+
+// Floats past the end of a row of ffa_stride(b) floats that the S/N reads without its guard: up to
+// 516 (529 bins, 32 threads) by the threads of snr_tpr, 508 by 16 threads for any b they hold.
+RT_HD int snr_overread(int b, int tpr)
+{
+    const int past = tpr * kSnrPhases - ffa_stride(b);
+    return b <= tpr * kSnrPhases && past > 0 ? past : 0;
 }
 
 // Kinds of S/N code a kernel instance may hold, one bit each: 4, 8, 16 or 32 threads a profile
