@@ -125,6 +125,18 @@ __device__ __forceinline__ float ordered_to_float(unsigned u)
     return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
 }
 
+// Integers in the order of the values, distinct for distinct bits; a NaN is the largest.
+__device__ __forceinline__ unsigned order_key(float v)
+{
+    const unsigned u = __float_as_uint(v);
+    return v != v ? 0xffffffffu : u ^ ((u >> 31) ? 0xffffffffu : 0x80000000u);
+}
+__device__ __forceinline__ unsigned long long order_key(double v)
+{
+    const unsigned long long u = (unsigned long long)__double_as_longlong(v);
+    return v != v ? ~0ull : u ^ ((u >> 63) ? ~0ull : 1ull << 63);
+}
+
 // A whole number below 2^52 as a double and the floor of a double in [0, 2^51) as both, by the
 // place of a number's units in the mantissa of 2^52 + number: on the FP64 units, for kernels
 // that the rate of the conversion instructions bounds.

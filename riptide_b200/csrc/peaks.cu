@@ -58,20 +58,10 @@ struct SelWarp {
     unsigned long long found[2];
 };
 
-// Integers in the order of the values; a NaN is the largest.
-__device__ __forceinline__ unsigned order_key(float v)
-{
-    const unsigned u = __float_as_uint(v);
-    return v != v ? 0xffffffffu : u ^ ((u >> 31) ? 0xffffffffu : 0x80000000u);
-}
+// Values of the keys (order_key).
 __device__ __forceinline__ float key_value(unsigned k)
 {
     return __uint_as_float(k ^ ((k >> 31) ? 0x80000000u : 0xffffffffu));
-}
-__device__ __forceinline__ unsigned long long order_key(double v)
-{
-    const unsigned long long u = (unsigned long long)__double_as_longlong(v);
-    return v != v ? ~0ull : u ^ ((u >> 63) ? ~0ull : 1ull << 63);
 }
 __device__ __forceinline__ double key_value(unsigned long long k)
 {
