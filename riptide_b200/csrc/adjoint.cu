@@ -354,7 +354,7 @@ __global__ void __launch_bounds__(256)
 }
 
 // Index of the element that the running median selects at every point: the tile's values ranked
-// by (value, position) as in k_running_median_sorted.
+// by (value, position) as in k_running_median_sorted, compared by their order_key.
 constexpr int kAdjTile = 128;
 constexpr int kAdjMaxWidth = 257;
 constexpr int kAdjSpan = kAdjTile + kAdjMaxWidth - 1;
@@ -363,7 +363,7 @@ __global__ void __launch_bounds__(kAdjTile)
     k_dered_adj_select(const double* __restrict__ lores, AdjBatch B, int width,
                        unsigned* __restrict__ sel)
 {
-    __shared__ double sx[kAdjSpan];
+    __shared__ unsigned long long sk[kAdjSpan];
     __shared__ unsigned short sp[kAdjSpan];
     const int trial = blockIdx.y;
     const size_t nl = B.lo_len[trial], t0 = (size_t)blockIdx.x * kAdjTile;
@@ -372,14 +372,14 @@ __global__ void __launch_bounds__(kAdjTile)
     const int half = width / 2, span = kAdjTile + width - 1;
     auto clamped = [&](long long i) { return i < 0 ? 0LL : i >= (long long)nl ? (long long)nl - 1 : i; };
     for (int i = threadIdx.x; i < span; i += kAdjTile) {
-        sx[i] = lo[clamped((long long)t0 + i - half)];
-        sp[i] = 0xffff;
+        // (+ 0.0: a zero's sign is left out)
+        sk[i] = order_key(__dadd_rn(lo[clamped((long long)t0 + i - half)], 0.0));
     }
     __syncthreads();
     for (int i = threadIdx.x; i < span; i += kAdjTile) {
-        const double v = sx[i];
+        const unsigned long long v = sk[i];
         int c = 0;
-        for (int j = 0; j < span; ++j) c += (sx[j] < v || (sx[j] == v && j < i)) ? 1 : 0;
+        for (int j = 0; j < span; ++j) c += (sk[j] < v || (sk[j] == v && j < i)) ? 1 : 0;
         sp[c] = (unsigned short)i;
     }
     __syncthreads();
