@@ -58,8 +58,16 @@ int rt_circular_prefix_sum(const float* d_x, size_t size, size_t nsum, float* d_
 
 /* ffa2: FFA transform of a rows x cols C-order block, bit-identical to the reference.
  * Replaces python_bindings.cpp:84-96 (transforms.hpp:53-61). Allocates its own scratch for
- * blocks larger than one CTA's shared memory. */
+ * blocks larger than one CTA's shared memory. Returns once enqueued. Large blocks are computed by
+ * one kernel whose CTAs wait for one another; its waits are bounded, and one that runs out leaves
+ * NaN in all of d_out. */
 int rt_ffa2(const float* d_in, size_t rows, size_t cols, float* d_out, void* stream);
+/* The same, with a status for callers that do not look for NaN: *d_status (device memory) is
+ * RT_OK or, after a wait that ran out, RT_ETIMEOUT once the call's work is done. wait_polls: bound
+ * of the waits in polls, as for rt_search_set_wait_limit (0: its default). fault: RT_FAULT_NONE,
+ * or RT_FAULT_STAGE_WAIT to make a wait run out in a test (see rt_search_inject_fault). */
+int rt_ffa2_status(const float* d_in, size_t rows, size_t cols, float* d_out, int32_t* d_status,
+                   long long wait_polls, int fault, void* stream);
 
 /* ffa2 without any device allocation, for callers that cannot allocate: pipelines whose
  * device memory is reserved up front by another framework's pool, and real-time loops that

@@ -31,6 +31,7 @@ SIGNATURES = {
     "rt_fused_rollback_add": (ctypes.c_int, [_vp, _vp, _sz, _sz, _vp, _vp]),
     "rt_circular_prefix_sum": (ctypes.c_int, [_vp, _sz, _sz, _vp, _vp]),
     "rt_ffa2": (ctypes.c_int, [_vp, _sz, _sz, _vp, _vp]),
+    "rt_ffa2_status": (ctypes.c_int, [_vp, _sz, _sz, _vp, _vp, ctypes.c_longlong, ctypes.c_int, _vp]),
     "rt_ffa2_noalloc": (ctypes.c_int, [_vp, _sz, _sz, _vp, _vp]),
     "rt_benchmark_ffa2": (ctypes.c_int, [_sz, _sz, _sz, ctypes.POINTER(_d)]),
     "rt_snr2": (ctypes.c_int, [_vp, _sz, _sz, _u64p, _sz, ctypes.c_float, _vp, _vp]),
@@ -173,6 +174,14 @@ def check(status):
     if status == RT_EIO:
         raise OSError(msg)
     raise RiptideError(f"[status {status}] {msg}")
+
+
+def check_device(status, what):
+    """Raise the exception of a status that a kernel left behind."""
+    if status == RT_ETIMEOUT:
+        raise RiptideError(f"[status {status}] a bounded wait in {what} ran out")
+    if status != RT_OK:
+        raise RiptideError(f"[status {status}] {what} reported an error")
 
 
 def u64_array(values):

@@ -44,9 +44,12 @@ extern "C" int rt_circular_prefix_sum(const float* d_x, size_t size, size_t nsum
 // ------------------------------------------------------------------------------------
 // ffa2
 // ------------------------------------------------------------------------------------
-extern "C" int rt_ffa2(const float* d_in, size_t rows, size_t cols, float* d_out, void* stream)
+// d_status (or null) receives the status of the transform, in stream order. wait_polls, dep_bias:
+// see ffa_transform_persistent.
+static int ffa2(const float* d_in, size_t rows, size_t cols, float* d_out, int* d_status,
+                long long wait_polls, int dep_bias, cudaStream_t st)
 {
-    cudaStream_t st = (cudaStream_t)stream;
+    if (d_status) RT_TRY_CUDA(cudaMemsetAsync(d_status, 0, sizeof(int), st));  // RT_OK
     if (rows == 0 || cols == 0) return RT_OK;
     if (rows >= (1u << 24) || cols > 4096)
         return set_error(RT_EINVAL, "ffa2 input of %zu x %zu is larger than supported", rows, cols);
@@ -56,7 +59,8 @@ extern "C" int rt_ffa2(const float* d_in, size_t rows, size_t cols, float* d_out
         void* room = nullptr;
         const cudaError_t e = scratch_malloc(&room, bytes, st);
         if (e == cudaSuccess) {
-            const int s = ffa_transform_persistent(d_in, m, b, m, d_out, room, nullptr, st);
+            const int s = ffa_transform_persistent(d_in, m, b, m, d_out, room, d_status, st,
+                                                   wait_polls, dep_bias);
             cudaFreeAsync(room, st);
             return s;
         }
@@ -68,10 +72,26 @@ extern "C" int rt_ffa2(const float* d_in, size_t rows, size_t cols, float* d_out
         const cudaError_t e = scratch_malloc((void**)&scratch, sf * sizeof(float), st);
         if (e != cudaSuccess) return check_cuda(e, "ffa2 scratch");
     }
-    // (the plan is checked on the host before any launch: nothing to read back)
-    const int s = ffa_transform(d_in, m, b, m, d_out, scratch, nullptr, st);
+    // (the plan is checked on the host before any launch: no kernel waits for another here)
+    const int s = ffa_transform(d_in, m, b, m, d_out, scratch, d_status, st);
     if (scratch) cudaFreeAsync(scratch, st);
     return s;
+}
+
+extern "C" int rt_ffa2(const float* d_in, size_t rows, size_t cols, float* d_out, void* stream)
+{
+    return ffa2(d_in, rows, cols, d_out, nullptr, 0, 0, (cudaStream_t)stream);
+}
+
+extern "C" int rt_ffa2_status(const float* d_in, size_t rows, size_t cols, float* d_out,
+                              int32_t* d_status, long long wait_polls, int fault, void* stream)
+{
+    if (!d_status) return set_error(RT_EINVAL, "null argument");
+    if (wait_polls < 0) return set_error(RT_EINVAL, "the wait limit must not be negative");
+    if (fault != RT_FAULT_NONE && fault != RT_FAULT_STAGE_WAIT)
+        return set_error(RT_EINVAL, "unknown fault kind %d", fault);
+    return ffa2(d_in, rows, cols, d_out, d_status, wait_polls, fault == RT_FAULT_STAGE_WAIT ? 1 : 0,
+                (cudaStream_t)stream);
 }
 
 extern "C" int rt_benchmark_ffa2(size_t rows, size_t cols, size_t loops, double* h_seconds)

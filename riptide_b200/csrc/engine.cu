@@ -1669,7 +1669,7 @@ size_t ffa_persistent_bytes(int m, int b, int rows_out)
 }
 
 int ffa_transform_persistent(const float* in, int m, int b, int rows_out, float* out, void* scratch,
-                             int* d_err, cudaStream_t st)
+                             int* d_err, cudaStream_t st, long long wait_polls, int dep_bias)
 {
     TransformPlan T;
     if (!transform_plan(m, b, rows_out, T))
@@ -1703,7 +1703,8 @@ int ffa_transform_persistent(const float* in, int m, int b, int rows_out, float*
     A.slot_release = S->slot_release;
     A.error = &S->error;
     A.ticket = &S->ticket;
-    A.spin_limit = kSpinLimit;
+    A.spin_limit = wait_polls > 0 ? wait_polls : kSpinLimit;
+    A.dep_bias = dep_bias;
     A.layout = T.layout;
     void (*kernel)(EngineArgs) = k_search_persistent<kRowsOnly>;
     RT_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,

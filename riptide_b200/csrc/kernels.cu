@@ -263,6 +263,9 @@ __global__ void __launch_bounds__(kThreads, 1)
     cta_sync();
     if (T.error) {
         if (threadIdx.x == 0 && err) atomicExch(err, RT_EINTERNAL);
+        float* to = dst + (size_t)(J.root_row0 + J.lo) * b;
+        for (size_t i = threadIdx.x; i < (size_t)(J.hi - J.lo) * b; i += kThreads)
+            to[i] = __int_as_float(0x7fffffff);  // and so in every row computed from these
         copy_async_wait();
         return;
     }

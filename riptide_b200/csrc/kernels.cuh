@@ -23,17 +23,19 @@ void release_scratch();
 
 // FFA transform of an m x b block (device pointers). rows_out <= m root rows are produced
 // (the reference's ffa2 uses rows_out = m). `scratch` holds ffa_scratch_floats(m, b)
-// floats. Errors of the device plan are reported through d_err.
+// floats. Errors of the device plan are reported through d_err and leave NaN in the rows concerned.
 int ffa_transform(const float* in, int m, int b, int rows_out, float* out, float* scratch,
                   int* d_err, cudaStream_t st);
 
 // The same by the persistent search kernel, with ffa_persistent_bytes(m, b, rows_out) bytes of
-// 256-byte aligned scratch (0: not for this size). Its waits are bounded: one that runs out
-// leaves NaN in `out`.
+// 256-byte aligned scratch (0: not for this size). Its waits are bounded, by `wait_polls` polls
+// (0: kSpinLimit): one that runs out leaves NaN in all of `out` and RT_ETIMEOUT in *d_err.
+// `dep_bias` is added to what a later stage waits for (fault injection).
 constexpr int kPersistentItems = 1000;
 size_t ffa_persistent_bytes(int m, int b, int rows_out);
 int ffa_transform_persistent(const float* in, int m, int b, int rows_out, float* out, void* scratch,
-                             int* d_err, cudaStream_t st);
+                             int* d_err, cudaStream_t st, long long wait_polls = 0,
+                             int dep_bias = 0);
 
 int snr2(const float* x, size_t rows, size_t cols, const int* h_widths, int nw, float stdnoise,
          float* out, cudaStream_t st);

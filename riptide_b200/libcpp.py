@@ -124,12 +124,22 @@ def circular_prefix_sum(x, nsum):
 
 def ffa2(arr):
     """FFA transform of a 2D (rows, cols) array, bit-identical to the reference
-    (python_bindings.cpp:84-96)."""
+    (python_bindings.cpp:84-96). The result of a CUDA tensor is computed in stream order; if a
+    bounded wait of the kernel runs out, it is NaN throughout. For a numpy array that raises
+    RiptideError."""
     t, dev = _as_f32(arr, 2)
-    out = _empty(t.shape, t.dtype, t)
     rows, cols = t.shape
-    _lib.check(_lib.load().rt_ffa2(_ptr(t), rows, cols, _ptr(out), _stream()))
-    return _out(out, dev)
+    if dev:
+        out = _empty(t.shape, t.dtype, t)
+        _lib.check(_lib.load().rt_ffa2(_ptr(t), rows, cols, _ptr(out), _stream()))
+        return out
+    # the transform, and behind it its status: one copy back for both
+    out = _empty((rows * cols + 1,), t.dtype, t)
+    _lib.check(_lib.load().rt_ffa2_status(_ptr(t), rows, cols, _ptr(out), _ptr(out[rows * cols:]), 0,
+                                          _lib.RT_FAULT_NONE, _stream()))
+    host = _out(out, dev)
+    _lib.check_device(int(host[rows * cols:].view(np.int32)[0]), "ffa2")
+    return host[:rows * cols].reshape(rows, cols)
 
 
 def benchmark_ffa2(rows, cols, loops):
