@@ -224,7 +224,9 @@ typedef struct rt_search_transform {
 } rt_search_transform;
 int rt_search_plan_transforms(const rt_search_plan* plan, rt_search_transform* h_out);
 /* Memory of a plan, for checks of its bounds (host only). The outputs of the stages of a
- * transform lie in a ring of ring_slots x ring_slot_bytes of device memory. The search kernel
+ * transform lie in a ring of ring_slots x ring_slot_bytes of device memory: a slot for
+ * each transform of several stages in a power of two up to 256, halved where the device has no room
+ * for them (by the first run, or rt_search_plan_prepare). The search kernel
  * has shared_bytes of dynamic shared memory per CTA: ops_bytes of row operations, two buffers of
  * buffer_bytes for the rows of a level, and the rest for reads past the last row. */
 typedef struct rt_search_memory_t {
@@ -278,10 +280,12 @@ int rt_search_set_wait_limit(rt_search_plan* plan, long long polls);
  * stage has, a count that is never reached, so the run ends with RT_ETIMEOUT after the wait
  * limit; RT_FAULT_ALLOC: the plan's device buffers are released and allocation number `arg`
  * (from 1) of the next run fails with RT_ENOMEM (everything allocated before it is released
- * again); RT_FAULT_NONE clears both. No counterpart in the reference. */
+ * again); RT_FAULT_RING: they are released, and there is no room for a stage ring of more than
+ * `arg` slots; RT_FAULT_NONE clears all three. No counterpart in the reference. */
 #define RT_FAULT_NONE 0
 #define RT_FAULT_STAGE_WAIT 1
 #define RT_FAULT_ALLOC 2
+#define RT_FAULT_RING 3
 int rt_search_inject_fault(rt_search_plan* plan, int kind, int arg);
 void rt_search_plan_destroy(rt_search_plan* plan);
 

@@ -15,7 +15,7 @@ LIB_PATH = os.path.join(HERE, "_riptide_b200.so")
 
 RT_OK, RT_EINVAL, RT_ECUDA, RT_ENOMEM, RT_ETIMEOUT, RT_EINTERNAL, RT_EIO = 0, 1, 2, 3, 4, 5, 6
 RT_SAMPLES_F32, RT_SAMPLES_U8, RT_SAMPLES_I8 = 0, 1, 2
-RT_FAULT_NONE, RT_FAULT_STAGE_WAIT, RT_FAULT_ALLOC = 0, 1, 2
+RT_FAULT_NONE, RT_FAULT_STAGE_WAIT, RT_FAULT_ALLOC, RT_FAULT_RING = 0, 1, 2, 3
 
 _sz = ctypes.c_size_t
 _vp = ctypes.c_void_p

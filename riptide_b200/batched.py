@@ -195,10 +195,11 @@ class BatchedSearch(object):
         """Host-side fault injection for tests of the error paths (no GPU fault is raised):
         "stage_wait" makes later-stage work items wait on a count that is never reached (the
         run ends with RT_ETIMEOUT after the wait limit); "alloc" releases the plan's device
-        buffers and makes allocation number `arg` of the next run fail (RT_ENOMEM); None
-        clears both."""
+        buffers and makes allocation number `arg` of the next run fail (RT_ENOMEM); "ring"
+        releases them and leaves no room for a stage ring of more than `arg` slots; None clears
+        all three."""
         kinds = {None: _lib.RT_FAULT_NONE, "stage_wait": _lib.RT_FAULT_STAGE_WAIT,
-                 "alloc": _lib.RT_FAULT_ALLOC}
+                 "alloc": _lib.RT_FAULT_ALLOC, "ring": _lib.RT_FAULT_RING}
         _lib.check(_lib.load().rt_search_inject_fault(self._plan, kinds[kind], int(arg)))
 
     def close(self):

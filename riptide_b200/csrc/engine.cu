@@ -50,7 +50,7 @@ constexpr size_t kEngineTreeBytes = (sizeof(JobTree) + 255) & ~size_t(255);
 constexpr size_t kEngineSnrBytes = (sizeof(SnrParams) + 255) & ~size_t(255);
 constexpr size_t kEngineDynBytes = kFfaSmemBytes - 2 * (kEngineTreeBytes + kEngineSnrBytes);
 
-constexpr int kSlots = 256;          // scratch slots for multi-stage transforms
+constexpr int kSlots = 256;          // most scratch slots for multi-stage transforms
 constexpr size_t kLagItems = 640;    // work items emitted between two stages of a transform
 constexpr long long kSpinLimit = 20000000LL;  // default bound of the waits (about 2-20 s with backoff)
 
@@ -65,10 +65,11 @@ struct EngineArgs {
     const StagePlan* plans;
     const int* widths;
     int nw, nfast;
-    float* scratch;          // kSlots * 2 * slot_floats
+    float* scratch;          // slots * 2 * slot_floats
     size_t slot_floats;
     int* done;               // [nseq * kMaxStages]
-    int* slot_release;       // [kSlots]
+    int* slot_release;       // [slots]: transform `seq` has slot seq & slot_mask, after
+    int slot_mask, slot_shift;  // seq >> slot_shift others
     unsigned long long* ticket;
     int* error;              // RT_OK or an error code
     unsigned long long* phase_cycles;  // optional [kPhases] SM-cycle totals (thread 0 of each CTA)
@@ -191,7 +192,7 @@ __device__ __forceinline__ void signal_item_done(const EngineArgs& A, const Item
     const int prev = atomicAdd(d, 1);
     if (prev + 1 == P.jobs_of_stage) {
         __threadfence();
-        atomicAdd(A.slot_release + (P.X.seq % kSlots), 1);
+        atomicAdd(A.slot_release + (P.X.seq & A.slot_mask), 1);
     }
 }
 
@@ -220,8 +221,8 @@ __device__ __forceinline__ void sched_decode(const EngineArgs& A, long long t, I
     if (J.hi > J.lo && X.seq >= 0) {
         const int seq = X.seq;
         if (stage == 0) {
-            dep = A.slot_release + (seq % kSlots);
-            target = seq / kSlots;
+            dep = A.slot_release + (seq & A.slot_mask);
+            target = seq >> A.slot_shift;
         } else {
             dep = A.done + (size_t)seq * kMaxStages + stage - 1;
             target = P.jobs[stage - 1] + A.dep_bias;
@@ -243,7 +244,7 @@ __device__ __forceinline__ float* level_buffer(unsigned char* smem, const Engine
 
 __device__ __forceinline__ float* stage_output(const EngineArgs& A, const XformRec& X, int stage)
 {
-    return A.scratch + ((size_t)(X.seq % kSlots) * 2 + (stage & 1)) * A.slot_floats;
+    return A.scratch + ((size_t)(X.seq & A.slot_mask) * 2 + (stage & 1)) * A.slot_floats;
 }
 
 // Whether an item's source rows come by bulk copies (issued by the scheduling warp).
@@ -1219,6 +1220,8 @@ struct SearchPlan {
     std::vector<WorkItem> items;
     int nseq = 0;
     size_t slot_floats = 0;
+    int slots = 0;                       // scratch slots of the ring, a power of two
+    int item_slots = 0;                  // ... that the work items are made for
     FfaLayout layout{};                  // shared-memory layout of the persistent kernel
     // device buffers
     bool dev_ready = false;
@@ -1256,6 +1259,7 @@ struct SearchPlan {
     int dep_bias = 0;
     int alloc_fail_at = 0;   // 1-based device allocation that fails; 0: none
     int alloc_calls = 0;
+    int ring_fails_above = 0;  // slots of the largest ring that there is room for; 0: no limit
     cudaGraphExec_t gexec = nullptr;
     cudaStream_t cap_stream = nullptr;
     const void* gkey[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
@@ -1291,24 +1295,26 @@ static int plan_cycles(SearchPlan& P)
     return RT_OK;
 }
 
-// Emits the work items of all transforms. Order: (trial, cycle, bins). For a transform that
-// needs several stages, stage s + 1 is emitted at least kLagItems items after stage s, so that
-// by the time a CTA takes it the previous stage has usually completed; the transform that
-// reuses a scratch slot starts only after every stage of the previous occupant is emitted.
-static int plan_build(SearchPlan& P)
+// Slots of the ring of stage outputs, a power of two: one per multi-stage transform, up to kSlots.
+static int ring_slots(const SearchPlan& P)
 {
-    RT_TRY(plan_cycles(P));
-    const rt_search_config& c = P.cfg;
-    const int T = (int)P.lengths.size();
-    const int C = (int)P.f.size();
-    P.out_rows_off.assign(T + 1, 0);
-    P.ds_off.assign((size_t)T * C, 0);
-    std::map<std::pair<int, long long>, int> plan_index;
+    int n = 1;
+    while (n < kSlots && n < P.nseq) n *= 2;
+    return n;
+}
+
+// Emits the work items of all transforms, in order. For a transform that needs several stages,
+// stage s + 1 is emitted at least kLagItems items after stage s, so that by the time a CTA takes
+// it the previous stage has usually completed; the transform that reuses a scratch slot starts
+// only after every stage of the previous occupant is emitted.
+static void plan_items(SearchPlan& P)
+{
+    P.items.clear();
+    P.item_slots = P.slots;
     const size_t lag_items = P.tuning.lag_items > 0 ? (size_t)P.tuning.lag_items : kLagItems;
     std::set<std::tuple<size_t, int, int>> deferred;  // (due item count, xform, stage)
-    std::vector<int> seq_xform;                        // xform of each multi-stage sequence
-    std::vector<std::tuple<size_t, int, int>> seq_pending;  // its deferred entry, if any
-    std::vector<char> seq_has_pending;
+    std::vector<std::tuple<size_t, int, int>> seq_pending(P.nseq);  // its deferred entry, if any
+    std::vector<char> seq_has_pending(P.nseq, 0);
 
     auto emit_stage = [&](int xi, int stage) {
         const StagePlan& sp = P.plans[P.xforms[xi].plan];
@@ -1339,6 +1345,28 @@ static int plan_build(SearchPlan& P)
             emit_stage(std::get<1>(e), std::get<2>(e));
         }
     };
+    for (int xi = 0; xi < (int)P.xforms.size(); ++xi) {
+        if (P.xforms[xi].seq >= P.slots) finish_seq(P.xforms[xi].seq - P.slots);
+        emit_stage(xi, 0);
+        flush();
+    }
+    while (!deferred.empty()) {
+        const auto e = *deferred.begin();
+        deferred.erase(deferred.begin());
+        emit_stage(std::get<1>(e), std::get<2>(e));
+    }
+}
+
+// The transforms of a plan, in the order (trial, cycle, bins), and their work items.
+static int plan_build(SearchPlan& P)
+{
+    RT_TRY(plan_cycles(P));
+    const rt_search_config& c = P.cfg;
+    const int T = (int)P.lengths.size();
+    const int C = (int)P.f.size();
+    P.out_rows_off.assign(T + 1, 0);
+    P.ds_off.assign((size_t)T * C, 0);
+    std::map<std::pair<int, long long>, int> plan_index;
 
     // (the first cycle has the smallest factor, and so the most rows)
     const size_t most_rows = C > 0 ? downsampled_size(P.max_len, P.f[0]) / c.bins_min : 0;
@@ -1424,32 +1452,22 @@ static int plan_build(SearchPlan& P)
                 X.plan = pi;
                 X.seq = -1;
                 X.tune = capr | (tpr << 16);
-                const int xi = (int)P.xforms.size();
                 if (multi) {
                     X.seq = P.nseq++;
                     // stage outputs use the level stride (16-byte aligned rows)
                     P.slot_floats = std::max(P.slot_floats, rows * (size_t)ffa_stride((int)b));
-                    seq_xform.push_back(xi);
-                    seq_pending.emplace_back();
-                    seq_has_pending.push_back(0);
-                    if (X.seq >= kSlots) finish_seq(X.seq - kSlots);
                 }
                 P.xforms.push_back(X);
                 P.snr_kinds |= snr_kind((int)b, tpr);
                 P.xform_tc.push_back(make_int2(t, ci));
                 rows_total += re;
-                emit_stage(xi, 0);
-                flush();
             }
         }
         P.out_rows_off[t + 1] = P.out_rows_off[t] + rows_total;
     }
-    while (!deferred.empty()) {
-        const auto e = *deferred.begin();
-        deferred.erase(deferred.begin());
-        emit_stage(std::get<1>(e), std::get<2>(e));
-    }
     P.ds_total = ds_total;
+    P.slots = ring_slots(P);
+    plan_items(P);
 
     // deredden geometry (time_series.py:119, running_medians.py:72-80)
     P.lo_len.assign(T, 0);
@@ -1514,18 +1532,26 @@ static int dalloc(SearchPlan& P, T** p, size_t n)
 }
 
 template <class T>
+static int copy_up(T* p, const std::vector<T>& v)
+{
+    if (!v.empty()) RT_TRY_CUDA(cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
+    return RT_OK;
+}
+
+template <class T>
 static int upload(SearchPlan& P, T** p, const std::vector<T>& v)
 {
     RT_TRY(dalloc(P, p, v.size()));
-    if (!v.empty())
-        RT_TRY_CUDA(cudaMemcpy(*p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
-    return RT_OK;
+    return copy_up(*p, v);
 }
 
 static int plan_alloc_device(SearchPlan& P);
 
 // Counters of a run, in one array: the ticket, the stage counts, the slot releases, the error.
-static size_t plan_counters(const SearchPlan& P) { return 2 + (size_t)P.nseq * kMaxStages + kSlots + 1; }
+static size_t plan_counters(const SearchPlan& P)
+{
+    return 2 + (size_t)P.nseq * kMaxStages + P.slots + 1;
+}
 
 // Allocates and fills the plan's device buffers once. On failure every buffer allocated so
 // far is released again, so a failed call leaks nothing and can be retried.
@@ -1542,15 +1568,30 @@ static int plan_prepare_device(SearchPlan& P)
     return RT_OK;
 }
 
+// The ring of stage outputs, with half the slots as often as there is no room for it. The halo of
+// its rows adds 5% to the ring at 240 bins and 80% at 20 (a series of 2^26 samples: 247 GB). With
+// half the slots a transform takes its slot over from one 128 back; kLagItems are those of 213
+// transforms at most. The work items follow the slots.
+static int plan_alloc_ring(SearchPlan& P)
+{
+    int s = RT_ENOMEM;
+    for (P.slots = ring_slots(P);; P.slots /= 2) {
+        const bool no_room = P.ring_fails_above > 0 && P.slots > P.ring_fails_above;
+        if (!no_room) s = dalloc(P, &P.d_scratch, (size_t)P.slots * 2 * std::max<size_t>(P.slot_floats, 1));
+        if (s != RT_ENOMEM || P.slots == 1 || P.alloc_calls == P.alloc_fail_at) break;
+    }
+    if (s == RT_OK && P.slots != P.item_slots) plan_items(P);
+    return s;
+}
+
 static int plan_alloc_device(SearchPlan& P)
 {
     const int T = (int)P.lengths.size();
     RT_TRY(upload(P, &P.d_widths, P.widths));
-    RT_TRY(upload(P, &P.d_items, P.items));
+    RT_TRY(dalloc(P, &P.d_items, P.items.size()));
     RT_TRY(upload(P, &P.d_plans, P.plans));
-    RT_TRY(upload(P, &P.d_xforms, P.xforms));
-    RT_TRY(dalloc(P, &P.d_scratch, (size_t)kSlots * 2 * std::max<size_t>(P.slot_floats, 1)));
-    RT_TRY(dalloc(P, &P.d_counters, plan_counters(P)));
+    RT_TRY(dalloc(P, &P.d_xforms, P.xforms.size()));
+    RT_TRY(dalloc(P, &P.d_counters, 2 + (size_t)P.nseq * kMaxStages + kSlots + 1));
     // + 16 floats: bulk copies read whole 16-byte units around a block of rows
     RT_TRY(dalloc(P, &P.d_ds, P.ds_total + 16));
     if (P.cfg.deredden) {
@@ -1569,6 +1610,9 @@ static int plan_alloc_device(SearchPlan& P)
     RT_TRY(upload(P, &P.d_f, P.f));
     RT_TRY(upload(P, &P.d_useseg, P.use_seg));
     RT_TRY(upload(P, &P.d_dsoff, P.ds_off));
+    RT_TRY(plan_alloc_ring(P));  // (last: the other buffers' sizes are fixed)
+    RT_TRY(copy_up(P.d_items, P.items));
+    RT_TRY(copy_up(P.d_xforms, P.xforms));
     return RT_OK;
 }
 
@@ -1603,8 +1647,10 @@ struct TransformState {
     unsigned long long ticket;
     int error;
     int done[kMaxStages];
-    int slot_release[kSlots];
-    XformRec xform;
+    int slot_release;  // (one transform, one slot)
+    // (apart from the counters, which every CTA changes: on their cache line, 16,001 x 499 took
+    // 169.8 instead of 167.4 us)
+    alignas(256) XformRec xform;
     StagePlan plan;
 };
 
@@ -1615,11 +1661,11 @@ __global__ void k_transform_items(TransformState* S, WorkItem* items, XformRec X
     if (t == 0) {
         S->ticket = 0;
         S->error = RT_OK;
+        S->slot_release = 0;
         S->xform = X;
         S->plan = P;
     }
     if (t < kMaxStages) S->done[t] = 0;
-    if (t < kSlots) S->slot_release[t] = 0;
     int first = 0;
     for (int s = 0; s < P.nstages; ++s) {
         for (int j = t; j < P.jobs[s]; j += n) items[first + j] = WorkItem{0, s << 24 | j};
@@ -1700,7 +1746,7 @@ int ffa_transform_persistent(const float* in, int m, int b, int rows_out, float*
     A.scratch = reinterpret_cast<float*>(base + T.state_bytes + T.item_bytes);
     A.slot_floats = T.slot_floats;
     A.done = S->done;
-    A.slot_release = S->slot_release;
+    A.slot_release = &S->slot_release;
     A.error = &S->error;
     A.ticket = &S->ticket;
     A.spin_limit = wait_polls > 0 ? wait_polls : kSpinLimit;
@@ -1806,7 +1852,9 @@ static int plan_run(SearchPlan& P, const float* data, float* normalised_out, dou
     A.slot_floats = P.slot_floats;
     A.done = P.d_counters + 2;
     A.slot_release = A.done + (size_t)P.nseq * kMaxStages;
-    A.error = A.slot_release + kSlots;
+    A.slot_mask = P.slots - 1;
+    while ((P.slots >> A.slot_shift) > 1) ++A.slot_shift;
+    A.error = A.slot_release + P.slots;
     A.ticket = reinterpret_cast<unsigned long long*>(P.d_counters);
     A.phase_cycles = P.d_phase;
     A.spin_limit = P.spin_limit;
@@ -2332,7 +2380,7 @@ extern "C" int rt_search_plan_memory(const rt_search_plan* plan, rt_search_memor
 {
     if (!plan || !h_out) return set_error(RT_EINVAL, "null argument");
     const SearchPlan& P = plan->p;
-    h_out->ring_slots = kSlots;
+    h_out->ring_slots = (uint64_t)P.slots;
     h_out->ring_slot_bytes = 2 * P.slot_floats * sizeof(float);
     h_out->shared_bytes = kEngineDynBytes;
     h_out->ops_bytes = (uint64_t)P.layout.ops_units * 16;
@@ -2497,6 +2545,7 @@ extern "C" int rt_search_inject_fault(rt_search_plan* plan, int kind, int arg)
         case RT_FAULT_NONE:
             P.dep_bias = 0;
             P.alloc_fail_at = 0;
+            P.ring_fails_above = 0;
             break;
         case RT_FAULT_STAGE_WAIT:
             P.dep_bias = 1;
@@ -2505,6 +2554,11 @@ extern "C" int rt_search_inject_fault(rt_search_plan* plan, int kind, int arg)
             if (arg < 1) return set_error(RT_EINVAL, "the failing allocation is numbered from 1");
             P.alloc_fail_at = arg;
             plan_free_device(P);  // the next run allocates again
+            break;
+        case RT_FAULT_RING:
+            if (arg < 1) return set_error(RT_EINVAL, "a ring has one slot or more");
+            P.ring_fails_above = arg;
+            plan_free_device(P);
             break;
         default:
             return set_error(RT_EINVAL, "unknown fault kind %d", kind);

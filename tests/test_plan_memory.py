@@ -1,7 +1,7 @@
-"""Bounds of a plan's shared memory, by arithmetic on the host: the boxcar S/N of the search kernel
-reads whole segments of 33 phases, past the end of a row, for whatever number of threads the plan
-may give a profile; the last row of a full level buffer is the one that could leave the CTA's
-shared memory."""
+"""Bounds of a plan's memory, by arithmetic on the host. Shared memory: the boxcar S/N of the search
+kernel reads whole segments of 33 phases, past the end of a row, for whatever number of threads the
+plan may give a profile; the last row of a full level buffer is the one that could leave the CTA's
+shared memory. Device memory: the ring of stage outputs."""
 import numpy as np
 import pytest
 
@@ -50,6 +50,73 @@ def test_snr_reads_stay_in_shared_memory(rows, kw, tuned):
                 for tpr in _threads(b, tuned):
                     if b <= 33 * tpr:
                         assert _last_read(mem, b, tpr) <= mem["shared_bytes"], (bmin, bmax, b, tpr)
+
+
+def _transforms(bs):
+    import ctypes
+
+    from riptide_b200 import _lib
+
+    arr = (_lib.SearchTransform * bs.stats["num_transforms"])()
+    _lib.check(_lib.load().rt_search_plan_transforms(bs._plan, ctypes.cast(arr, ctypes.c_void_p)))
+    return arr
+
+
+# the outputs of the stages take a slot of two copies for each transform of several stages, in a power
+# of two up to 256
+@pytest.mark.parametrize("bmin,bmax,n,trials", [
+    (20, 22, 1 << 26, 1), (20, 23, 1 << 20, 40), (240, 260, 1 << 22, 4), (240, 260, 1 << 16, 1)])
+def test_stage_ring_slots(bmin, bmax, n, trials):
+    from riptide_b200 import BatchedSearch
+
+    bs = BatchedSearch([n] * trials, 1e-3, period_min=1e-3 * bmin, period_max=4e-3 * bmin,
+                       bins_min=bmin, bins_max=bmax, widths=[1], deredden=False)
+    try:
+        mem, multi = bs.memory(), bs.stats["num_multistage"]
+        most = max(4 * t.rows * _stride(t.bins) for t in _transforms(bs))
+        assert mem["ring_slots"] == min(256, 1 << max(0, multi - 1).bit_length())
+        assert mem["ring_slot_bytes"] <= 2 * most
+    finally:
+        bs.close()
+
+
+# no room for all of the ring (injected on the host): fewer slots, the same periodograms
+@pytest.mark.gpu
+@pytest.mark.parametrize("bmin,bmax,n", [(20, 23, 60000), (2, 4, 9000)])
+def test_less_room_for_the_ring(bmin, bmax, n):
+    import torch
+
+    import riptide_b200 as rb
+
+    rng = np.random.default_rng(n)
+    trials = 60
+    x = rng.standard_normal((trials, n)).astype(np.float32)
+    w = [1] if bmin < 4 else [1, 2, 3]
+    lim = (1e-3 * bmin, 8e-3 * bmin)
+    kw = dict(period_min=lim[0], period_max=lim[1], bins_min=bmin, bins_max=bmax, widths=w,
+              deredden=False, already_normalised=True)
+    bs = rb.BatchedSearch([n] * trials, 1e-3, **kw)
+    assert bs.stats["num_multistage"] > 256 == bs.memory()["ring_slots"]
+    d = torch.from_numpy(x.ravel()).cuda()
+    want = [t.clone() for t in bs.run(d)]
+    off = bs.row_offsets
+    for t in (0, 17, trials - 1):
+        p, fb, s = [v[off[t]:off[t + 1]].cpu().numpy() for v in want]
+        rp, rfb, rs = O.C().periodogram(x[t], 1e-3, np.array(w), *lim, bmin, bmax)
+        assert np.array_equal(p, rp) and np.array_equal(fb, rfb)
+        assert np.allclose(s, rs, rtol=1e-5, atol=2e-5), t
+    for room, slots in ((255, 128), (40, 32), (1, 1), (3, 2), (256, 256)):
+        bs.inject_fault("ring", room)
+        got = bs.run(d)
+        assert bs.memory()["ring_slots"] == slots
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+    bs.inject_fault("ring", 100)
+    bs.inject_fault("alloc", 5)
+    with pytest.raises(MemoryError):
+        bs.run(d)
+    bs.inject_fault(None)
+    assert all(torch.equal(a, b) for a, b in zip(bs.run(d), want))
+    bs.close()
 
 
 # bins and threads whose reads leave the smallest room behind the second buffer, with the rows of
