@@ -38,6 +38,9 @@ int rt_version(void);
 /* Gives back the device memory (at most 512 MiB) that the library keeps for the scratch of
  * later calls on the current device. */
 int rt_release_scratch(void);
+/* For tests of the paths without room: scratch allocation number `nth` (from 1) that the calling
+ * thread makes from now on fails as for lack of device memory, once; 0 clears it. */
+int rt_inject_scratch_fault(int nth);
 
 /* ---------------------------------------------------------------------------------
  * Drop-ins for the riptide.libcpp functions (device buffers).

@@ -27,6 +27,7 @@ SIGNATURES = {
     "rt_last_error": (ctypes.c_char_p, []),
     "rt_version": (ctypes.c_int, []),
     "rt_release_scratch": (ctypes.c_int, []),
+    "rt_inject_scratch_fault": (ctypes.c_int, [ctypes.c_int]),
     "rt_rollback": (ctypes.c_int, [_vp, _sz, _sz, _vp, _vp]),
     "rt_fused_rollback_add": (ctypes.c_int, [_vp, _vp, _sz, _sz, _vp, _vp]),
     "rt_circular_prefix_sum": (ctypes.c_int, [_vp, _sz, _sz, _vp, _vp]),

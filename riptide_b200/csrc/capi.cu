@@ -23,6 +23,13 @@ extern "C" int rt_release_scratch(void)
     return RT_OK;
 }
 
+extern "C" int rt_inject_scratch_fault(int nth)
+{
+    if (nth < 0) return set_error(RT_EINVAL, "scratch allocations are numbered from 1");
+    rt::inject_scratch_fault(nth);
+    return RT_OK;
+}
+
 extern "C" int rt_rollback(const float* d_x, size_t size, size_t shift, float* d_out,
                            void* stream)
 {

@@ -53,8 +53,13 @@ const char* last_error() { return g_err; }
 static std::mutex g_pool_mutex;
 static std::map<int, cudaMemPool_t> g_pools;  // by device
 
+static thread_local int g_scratch_fault = 0;  // scratch allocations until one fails; 0: none does
+
+void inject_scratch_fault(int nth) { g_scratch_fault = nth; }
+
 cudaError_t scratch_malloc(void** p, size_t bytes, cudaStream_t st)
 {
+    if (g_scratch_fault > 0 && --g_scratch_fault == 0) return cudaErrorMemoryAllocation;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;

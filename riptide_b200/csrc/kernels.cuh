@@ -18,8 +18,10 @@ const char* last_error();
 // 400 us a call. release_scratch gives the kept memory of the current device back; a plan that
 // runs out of device memory does so before it tries again.
 constexpr size_t kScratchKept = size_t(512) << 20;
+// inject_scratch_fault: the nth allocation of the calling thread from now on fails (0: none).
 cudaError_t scratch_malloc(void** p, size_t bytes, cudaStream_t st);
 void release_scratch();
+void inject_scratch_fault(int nth);
 
 // FFA transform of an m x b block (device pointers). rows_out <= m root rows are produced
 // (the reference's ffa2 uses rows_out = m). `scratch` holds ffa_scratch_floats(m, b)
