@@ -112,14 +112,32 @@ extern "C" int rt_benchmark_ffa2(size_t rows, size_t cols, size_t loops, double*
     float *in = nullptr, *out = nullptr;
     void* scratch = nullptr;
     int* d_err = nullptr;
-    const size_t n = rows * cols, persistent = ffa_persistent_bytes(m, b, m);  // as rt_ffa2
-    const size_t bytes = persistent ? persistent : ffa_scratch_floats(m, b) * sizeof(float);
-    RT_TRY_CUDA(cudaMalloc((void**)&in, n * sizeof(float)));
-    RT_TRY_CUDA(cudaMalloc((void**)&out, n * sizeof(float)));
-    RT_TRY_CUDA(cudaMalloc((void**)&d_err, sizeof(int)));
-    if (bytes) RT_TRY_CUDA(cudaMalloc(&scratch, bytes));
-    RT_TRY_CUDA(cudaMemset(in, 0, n * sizeof(float)));
-    RT_TRY_CUDA(cudaMemset(d_err, 0, sizeof(int)));
+    const size_t n = rows * cols, sf = ffa_scratch_floats(m, b);
+    size_t persistent = ffa_persistent_bytes(m, b, m);  // as rt_ffa2, also where that finds no room
+    cudaError_t e = cudaMalloc((void**)&in, n * sizeof(float));
+    if (e == cudaSuccess) e = cudaMalloc((void**)&out, n * sizeof(float));
+    if (e == cudaSuccess) e = cudaMalloc((void**)&d_err, sizeof(int));
+    if (e == cudaSuccess && persistent) {
+        e = scratch_malloc(&scratch, persistent, 0);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            persistent = 0;
+            e = cudaSuccess;
+        }
+    }
+    if (e == cudaSuccess && !persistent && sf) e = scratch_malloc(&scratch, sf * sizeof(float), 0);
+    if (e == cudaSuccess) e = cudaMemset(in, 0, n * sizeof(float));
+    if (e == cudaSuccess) e = cudaMemset(d_err, 0, sizeof(int));
+    auto release = [&]() {
+        cudaFree(in);
+        cudaFree(out);
+        cudaFree(d_err);
+        if (scratch) cudaFreeAsync(scratch, 0);
+    };
+    if (e != cudaSuccess) {
+        release();
+        return check_cuda(e, "benchmark_ffa2");
+    }
     auto transform = [&]() {
         return persistent ? ffa_transform_persistent(in, m, b, m, out, scratch, d_err, 0)
                           : ffa_transform(in, m, b, m, out, static_cast<float*>(scratch), d_err, 0);
@@ -136,10 +154,7 @@ extern "C" int rt_benchmark_ffa2(size_t rows, size_t cols, size_t loops, double*
     cudaEventElapsedTime(&ms, e0, e1);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    cudaFree(in);
-    cudaFree(out);
-    cudaFree(d_err);
-    if (scratch) cudaFree(scratch);
+    release();
     if (s != RT_OK) return s;
     *h_seconds = (double)ms * 1e-3 / (double)loops;
     return RT_OK;

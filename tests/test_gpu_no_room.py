@@ -1,4 +1,4 @@
-"""ffa2 without room for the scratch memory that it would like to have (a scratch allocation that
+"""ffa2 and benchmark_ffa2 without room for the scratch memory that it would like to have (a scratch allocation that
 fails, injected on the host): a launch per stage instead of the persistent kernel, an error where
 there is no other way, and the next call as before."""
 import numpy as np
@@ -44,3 +44,23 @@ def test_ffa2_without_room(no_room):
     with pytest.raises(MemoryError):
         libcpp.ffa2(x)
     assert np.array_equal(libcpp.ffa2(x), O.C().ffa2(x))
+
+
+def test_benchmark_ffa2(no_room):
+    # by stages where the persistent kernel's copies find no room; nothing is left allocated
+    import torch
+
+    from riptide_b200 import _lib, libcpp
+
+    assert libcpp.benchmark_ffa2(33000, 250, 2) > 0
+    torch.cuda.synchronize()
+    _lib.check(_lib.load().rt_release_scratch())
+    free = torch.cuda.mem_get_info()[0]
+    no_room(1)
+    assert libcpp.benchmark_ffa2(33000, 250, 2) > 0
+    no_room(1)
+    with pytest.raises(MemoryError):
+        libcpp.benchmark_ffa2(300, 251, 2)
+    torch.cuda.synchronize()
+    _lib.check(_lib.load().rt_release_scratch())
+    assert abs(torch.cuda.mem_get_info()[0] - free) <= 2 << 20
