@@ -51,7 +51,28 @@ const char* last_error() { return g_err; }
 // Device scratch
 // ------------------------------------------------------------------------------------
 static std::mutex g_pool_mutex;
-static std::map<int, cudaMemPool_t> g_pools;  // by device
+// by device and context: a pool ends with the context that it was made in (cudaDeviceReset)
+static std::map<std::pair<int, unsigned long long>, cudaMemPool_t> g_pools;
+
+static cudaError_t pool_key(std::pair<int, unsigned long long>* key)
+{
+    typedef CUresult (*ContextId)(CUcontext, unsigned long long*);
+    static const ContextId context_id = [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &found) != cudaSuccess)
+            p = nullptr;
+        return reinterpret_cast<ContextId>(p);
+    }();
+    cudaError_t e = cudaGetDevice(&key->first);
+    if (e != cudaSuccess) return e;
+    key->second = 0;
+    if (!context_id) return cudaErrorNotSupported;
+    if (context_id(nullptr, &key->second) == CUDA_SUCCESS) return cudaSuccess;
+    e = cudaFree(nullptr);  // no context yet, or none since a reset
+    if (e != cudaSuccess) return e;
+    return context_id(nullptr, &key->second) == CUDA_SUCCESS ? cudaSuccess : cudaErrorDeviceUninitialized;
+}
 
 static thread_local int g_scratch_fault = 0;  // scratch allocations until one fails; 0: none does
 
@@ -60,19 +81,19 @@ void inject_scratch_fault(int nth) { g_scratch_fault = nth; }
 cudaError_t scratch_malloc(void** p, size_t bytes, cudaStream_t st)
 {
     if (g_scratch_fault > 0 && --g_scratch_fault == 0) return cudaErrorMemoryAllocation;
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
+    std::pair<int, unsigned long long> key;
+    cudaError_t e = pool_key(&key);
     if (e != cudaSuccess) return e;
     cudaMemPool_t pool = nullptr;
     {
         std::lock_guard<std::mutex> lock(g_pool_mutex);
-        auto it = g_pools.find(dev);
+        auto it = g_pools.find(key);
         if (it == g_pools.end()) {
             cudaMemPoolProps props;
             memset(&props, 0, sizeof(props));
             props.allocType = cudaMemAllocationTypePinned;
             props.location.type = cudaMemLocationTypeDevice;
-            props.location.id = dev;
+            props.location.id = key.first;
             e = cudaMemPoolCreate(&pool, &props);
             if (e != cudaSuccess) return e;
             cuuint64_t kept = kScratchKept;
@@ -81,7 +102,7 @@ cudaError_t scratch_malloc(void** p, size_t bytes, cudaStream_t st)
                 cudaMemPoolDestroy(pool);
                 return e;
             }
-            g_pools[dev] = pool;
+            g_pools[key] = pool;
         } else {
             pool = it->second;
         }
@@ -91,10 +112,10 @@ cudaError_t scratch_malloc(void** p, size_t bytes, cudaStream_t st)
 
 void release_scratch()
 {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return;
+    std::pair<int, unsigned long long> key;
+    if (pool_key(&key) != cudaSuccess) return;
     std::lock_guard<std::mutex> lock(g_pool_mutex);
-    auto it = g_pools.find(dev);
+    auto it = g_pools.find(key);
     if (it != g_pools.end()) cudaMemPoolTrimTo(it->second, 0);
 }
 
