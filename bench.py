@@ -195,9 +195,14 @@ def barrier(world):
 
 # --------------------------------------------------------------------------------------
 def bench_reference(args):
-    """--impl reference: the reference's CPU implementation on the host cores."""
+    """--impl reference: the reference's CPU implementation on the host cores, its own compiled
+    module; without that there is nothing to time under its name."""
     world, rank, local = int(os.environ.get("WORLD_SIZE", "1")), int(os.environ.get("RANK", "0")), 0
     if rank != 0:
+        return 0
+    if cpu_kind() != "reference":
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's libcpp module is not "
+                          "built (oracle/_ref): its sources are not present"}), flush=True)
         return 0
     from riptide_b200 import synth
 
@@ -214,14 +219,13 @@ def bench_reference(args):
         pool.close()
     step = float(np.mean(times))
     value = nsample / step
-    kind = cpu_kind()
     line = {
         "impl": "reference", "metric": METRIC, "value": value, "unit": "trials/s", "n_gpus": world,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": step * 1e3,
         "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32",
         "data": "synthetic",
         "config": {"workload": cfg["name"], "trials_per_step": nsample},
-        "cpu_baseline": {"value": value, "unit": "trials/s", "cores": ncores, "kind": kind,
+        "cpu_baseline": {"value": value, "unit": "trials/s", "cores": ncores, "kind": "reference",
                          "sample": f"{nsample} trials of the workload per step, one per process"},
         "e2e": {"value": value, "unit": "trials/s", "h2d_bytes_per_step": 0,
                 "d2h_bytes_per_step": 0},
