@@ -698,7 +698,9 @@ __global__ void __launch_bounds__(kDsThreads, 1024 / kDsThreads)
     // the cycle boundaries inside the chunk. Sample positions are made relative to seg0:
     // start - seg0 and end - seg0 are exact (seg0 is an integer at most start), so floor,
     // weights and clamping give the same values as the absolute FP64 bounds of
-    // downsample.hpp:58-72.
+    // downsample.hpp:58-72. The product is rounded by itself: fused with the subtraction, it lies
+    // below seg0 where k f rounds up to it (f = 1.2: at every segment), and the first sample
+    // would be the one before the staged ones.
     const double seg0d = (double)seg0;
     const double lastd = (double)(N - 1 - seg0);
     const double rinv = 1.0 / inv;
@@ -719,9 +721,9 @@ __global__ void __launch_bounds__(kDsThreads, 1024 / kDsThreads)
         while (s_cnt[c + 1] <= q) ++c;
         const double f = s_f[c];
         const size_t k = (size_t)(s_kb[c] + q);
-        const double start = (double)k * f;
-        const double end = start + f;
-        const double sr = start - seg0d, er = end - seg0d;
+        const double start = __dmul_rn((double)k, f);
+        const double end = __dadd_rn(start, f);
+        const double sr = __dsub_rn(start, seg0d), er = __dsub_rn(end, seg0d);
         // floors of values in [0, 2^13) as doubles; their integer values via the 2^52 + 2^51
         // rounding constant (exact for integral doubles below 2^51)
         const double fl = floor(sr);
