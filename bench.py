@@ -754,7 +754,7 @@ def bench_fold(args, cfg, data, lengths):
     cpu = (time.perf_counter() - t0) / len(sample)
     return {"candidates": int(args.fold), "s_all": best, "ms_per_candidate": best * 1e3 / args.fold,
             "cpu_ms_per_candidate_1_core": cpu * 1e3, "cpu_kind": "port",
-            "api": "fold_candidates (rt_fold_batched, one launch), host series copied in"}
+            "api": "fold_candidates (rt_fold_batched, one call), host series copied in"}
 
 
 def main():

@@ -10,7 +10,8 @@
 //      (trial, cycle, bins) transforms and writes the periodogram rows (S/N fused).
 // Transforms too large for one CTA are split in stages; jobs of a stage wait for the previous
 // stage through per-transform counters, and stage-0 jobs wait until their scratch slot is
-// released. Every wait is bounded and reports RT_ETIMEOUT instead of hanging.
+// released. These waits, for other CTAs, are bounded and report RT_ETIMEOUT instead of hanging;
+// inside a CTA, the compute warps wait for the scheduling warp, which always hands an item over.
 #include <string.h>
 
 #include <algorithm>
@@ -520,7 +521,7 @@ __global__ void __launch_bounds__(kEngineThreads, 1) k_search_persistent(EngineA
     for (int k = 0;; ++k) {
         const int sl = k & 1;
         // the scheduling warp's own waits are bounded and it always hands a slot over: this
-        // limit is far beyond them
+        // limit, hours, is only there so that the loop has one
         if (!mbar_wait(full + sl, (k >> 1) & 1, 1ll << 40)) break;
         mark(kPhWait);
         ItemSlot& L = H.pool[H.item[sl]];
