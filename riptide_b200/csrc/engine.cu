@@ -1614,6 +1614,9 @@ static int plan_alloc_device(SearchPlan& P)
     RT_TRY(plan_alloc_ring(P));  // (last: the other buffers' sizes are fixed)
     RT_TRY(copy_up(P.d_items, P.items));
     RT_TRY(copy_up(P.d_xforms, P.xforms));
+    // a copy from pageable memory returns when the data is staged; the run may be on a stream that
+    // does not wait for the default stream, which the copies are on
+    RT_TRY_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
     return RT_OK;
 }
 
